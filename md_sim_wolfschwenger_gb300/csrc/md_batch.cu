@@ -195,7 +195,7 @@ int pack(md_batch* b) {
     }
     b->coat = b->coat || s.ctx->cfg.ENABLE_COATING_POT;
   }
-  b->np = scatter_particles(b->kcmax, false);
+  b->np = scatter_particles(b->kcmax);
   if (any_simt && !b->np) return set_err(nullptr, MD_ERR_UNSUPPORTED, "kc too large for the packed k-space scatter");
   // task tables, one per kernel shape: R + 1 offsets each on the host
   std::vector<int> toff;
@@ -456,7 +456,7 @@ int md_batch_add(md_batch* b, md_ctx* c, int64_t nsteps, double dt, int64_t* id)
   if (c->device != b->device) return set_err(c, MD_ERR_INVALID, "context and batch on different devices");
   for (const Slot& s : b->slots)
     if (s.ctx == c) return set_err(c, MD_ERR_INVALID, "context already in the batch");
-  if (!scatter_particles((int)c->kc, false)) return set_err(c, MD_ERR_UNSUPPORTED, "kc too large");
+  if (!scatter_particles((int)c->kc)) return set_err(c, MD_ERR_UNSUPPORTED, "kc too large");
   if ((st = prepare_dt(c, dt))) return st;
   if ((st = ensure_records(c, nsteps))) return st;
   CK(c, cudaStreamSynchronize(c->stream));

@@ -135,6 +135,8 @@ RealParams real_params(md_ctx* c, void* B, void* F, void* ov) {
   const md_config& g = c->cfg;
   const double L = c->L, a = c->alpha * L, rcb = c->rc / L;
   p.n = (int)c->n;
+  p.gtab = c->gtab;
+  p.etab = c->etab;
   p.grid = c->grid;
   p.alpha = a;
   p.rc = rcb;
@@ -269,6 +271,17 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.tc_yz = c->tcs.yz;
   p.tc_sfa = c->tcs.sfa;
   p.tc_sfb = c->tcs.sfb;
+  p.k64_T = c->k64_T;
+  p.k64_R = c->k64_R;
+  p.k64_nblk = c->k64s.nblk;
+  p.k64_threads = c->k64s.threads;
+  p.k64_chunk = c->k64s.chunk;
+  p.k64_nchunk = c->k64s.nchunk;
+  p.k64_task = c->k64_task;
+  p.k64_kidx = c->k64_kidx;
+  p.k64_row = c->k64_row;
+  p.k64_rowt = c->k64_rowt;
+  p.k64_ad = c->k64_ad;
   p.tc_wait = c->tc_wait;
   p.err = &c->sc->err;
   return p;
@@ -643,6 +656,74 @@ static int setup_tc(md_ctx* c) {
   return MD_OK;
 }
 
+// FP64 k space: tasks of four consecutive |nx| of one k row, rows by nz then
+// ny, and the buffers of the launches (md_kspace64.cu).
+static int setup_k64(md_ctx* c) {
+  const int kc = (int)c->kc, nk = c->klist.nk;
+  std::map<std::pair<int, int>, std::vector<std::pair<int, int>>> byrow;  // (nz, ny) -> (nx, k)
+  for (int k = 0; k < nk; k++)
+    if (c->klist.kreal[k]) byrow[{c->klist.kz[k], c->klist.ky[k]}].push_back({c->klist.kx[k], k});
+  std::vector<int4> task;
+  std::vector<int> kidx;
+  std::vector<double2> row;
+  std::vector<int2> rowt;
+  for (const auto& e : byrow) {
+    const int nz = e.first.first, ny = e.first.second;
+    int top = 0;
+    for (const auto& q : e.second) top = std::max(top, std::abs(q.first));
+    const int nt = top / 4 + 1, t0 = (int)task.size();
+    for (int t = 0; t < nt; t++) task.push_back(make_int4((int)row.size(), ny, nz, 4 * t));
+    kidx.resize(8 * task.size(), -1);
+    for (const auto& q : e.second) {
+      const int ax = std::abs(q.first);
+      kidx[8 * (size_t)(t0 + ax / 4) + 2 * (ax % 4) + (q.first < 0 ? 1 : 0)] = q.second;
+    }
+    row.push_back(make_double2((double)ny, (double)nz));
+    rowt.push_back(make_int2(t0, nt));
+  }
+  const int T = (int)task.size(), R = (int)row.size();
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+  const md::K64Shape sh = md::kspace64_shape(kc, (int)c->n, T, nsm);
+  void* old[] = {c->k64_task, c->k64_kidx, c->k64_row, c->k64_rowt, c->k64_ad};
+  for (void* q : old) dfree(c, q);
+  c->k64_task = nullptr;
+  c->k64_kidx = nullptr;
+  c->k64_row = nullptr;
+  c->k64_rowt = nullptr;
+  c->k64_ad = nullptr;
+  c->k64_T = 0;
+  int st;
+  if ((st = dalloc(c, &c->k64_task, sizeof(int4) * (size_t)T))) return st;
+  if ((st = dalloc(c, &c->k64_kidx, sizeof(int) * kidx.size()))) return st;
+  if ((st = dalloc(c, &c->k64_row, sizeof(double2) * (size_t)R))) return st;
+  if ((st = dalloc(c, &c->k64_rowt, sizeof(int2) * (size_t)R))) return st;
+  if ((st = dalloc(c, &c->k64_ad, 8 * sizeof(double2) * (size_t)T))) return st;
+  const size_t sp = 8 * (size_t)T * (size_t)sh.nchunk;
+  if (sp > c->spart_cap) {
+    dfree(c, c->Spart);
+    c->Spart = nullptr;
+    c->spart_cap = 0;
+    if ((st = dalloc(c, &c->Spart, sizeof(double2) * sp))) return st;
+    c->spart_cap = sp;
+  }
+  if (sh.nchunk > c->musum_cap) {
+    dfree(c, c->musum_part);
+    c->musum_part = nullptr;
+    c->musum_cap = 0;
+    if ((st = dalloc(c, &c->musum_part, 24 * (size_t)sh.nchunk))) return st;
+    c->musum_cap = sh.nchunk;
+  }
+  CK(c, cudaMemcpy(c->k64_task, task.data(), sizeof(int4) * (size_t)T, cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->k64_kidx, kidx.data(), sizeof(int) * kidx.size(), cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->k64_row, row.data(), sizeof(double2) * (size_t)R, cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->k64_rowt, rowt.data(), sizeof(int2) * (size_t)R, cudaMemcpyHostToDevice));
+  c->k64s = sh;
+  c->k64_T = T;
+  c->k64_R = R;
+  return MD_OK;
+}
+
 extern "C" {
 
 const char* md_strerror(int s) {
@@ -774,6 +855,14 @@ int md_ctx_create(const md_config* cfg, int64_t n, int precision, md_ctx** out) 
       return fail(set_err(nullptr, MD_ERR_CUDA, "initial memset failed"));
   }
   if ((st = dalloc(c, &c->sc, sizeof(DevScalars)))) return fail(st);
+  if (fp64(c)) {
+    const mdh::RealTables t = mdh::real_tables64(cfg->irPi);
+    if ((st = dalloc(c, &c->gtab, 8 * t.g.size())) || (st = dalloc(c, &c->etab, 8 * t.e.size()))) return fail(st);
+    if (cudaMemcpyAsync(c->gtab, t.g.data(), 8 * t.g.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaMemcpyAsync(c->etab, t.e.data(), 8 * t.e.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+      return fail(set_err(nullptr, MD_ERR_CUDA, "table upload failed"));
+  }
   static const int one = 1;
   if (cudaMemsetAsync(c->sc, 0, sizeof(DevScalars), c->stream) != cudaSuccess ||
       cudaMemcpyAsync(&c->sc->flags.soverflow, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
@@ -1006,7 +1095,7 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
   if (!c || !c->have_particles) return set_err(c, MD_ERR_INVALID, "particles not set");
   if (!(alpha > 0) || !(rc > 0) || rc > 0.5 * c->L * (1 + 1e-12) || kc < 1 || kc > 96)
     return set_err(c, MD_ERR_INVALID, "bad Ewald parameters (alpha>0, 0<rc<=L/2, 1<=kc<=96)");
-  if (kscatter_smem((int)kc, fp64(c)) == 0) return set_err(c, MD_ERR_UNSUPPORTED, "kc too large for shared memory");
+  if (!fp64(c) && kscatter_smem((int)kc) == 0) return set_err(c, MD_ERR_UNSUPPORTED, "kc too large for shared memory");
   invalidate_graph(c);
   CK(c, cudaStreamSynchronize(c->stream));
   c->alpha = alpha;
@@ -1017,19 +1106,21 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
   const double w = std::pow(c->cfg.my_pi / ab, 2.0);
   c->klist = mdh::build_klist((int)kc, w);
   c->grid = mdh::choose_grid(rc / c->L, c->n, 2);
-  // structure-factor grid (segment blocks x particle chunks): the fewest
-  // whole waves of resident blocks that keep every FP32 chunk sum within 512
-  // particles, with the chunk count chosen to fill those waves
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const int nsegb = (int)((c->klist.seg.size() + md::sk_threads() - 1) / md::sk_threads());
-  const int64_t slots = (int64_t)nsm * md::sk_resident_blocks((int)kc, fp64(c));
-  const int64_t nch_min = std::max<int64_t>(1, (c->n + 511) / 512);
-  const int64_t waves = std::max<int64_t>(1, (nsegb * nch_min + slots - 1) / slots);
-  int64_t nch = std::max<int64_t>(nch_min, waves * slots / nsegb);
-  nch = std::min<int64_t>(nch, (c->n + 31) / 32);
-  c->chunk = (int)(((c->n + nch - 1) / nch + 31) / 32 * 32);
-  c->nchunk = (int)((c->n + c->chunk - 1) / c->chunk);
+  if (!fp64(c)) {
+    // structure-factor grid (segment blocks x particle chunks): the fewest
+    // whole waves of resident blocks that keep every FP32 chunk sum within 512
+    // particles, with the chunk count chosen to fill those waves
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+    const int nsegb = (int)((c->klist.seg.size() + md::sk_threads() - 1) / md::sk_threads());
+    const int64_t slots = (int64_t)nsm * md::sk_resident_blocks((int)kc);
+    const int64_t nch_min = std::max<int64_t>(1, (c->n + 511) / 512);
+    const int64_t waves = std::max<int64_t>(1, (nsegb * nch_min + slots - 1) / slots);
+    int64_t nch = std::max<int64_t>(nch_min, waves * slots / nsegb);
+    nch = std::min<int64_t>(nch, (c->n + 31) / 32);
+    c->chunk = (int)(((c->n + nch - 1) / nch + 31) / 32 * 32);
+    c->nchunk = (int)((c->n + c->chunk - 1) / c->chunk);
+  }
   // (re)allocate Ewald-sized buffers
   const int ncell = c->grid.ncell;
   if (ncell + 1 > c->ncell_cap) {
@@ -1056,18 +1147,20 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
     for (void* p : old) dfree(c, p);
     const size_t cap = need;
     int st;
-    if ((st = dalloc(c, &c->kseg, sizeof(KSeg) * cap))) return st;
-    if ((st = dalloc(c, &c->koff, sizeof(int) * cap))) return st;
     if ((st = dalloc(c, &c->ek, sizeof(double) * cap))) return st;
-    if ((st = dalloc(c, &c->eS, 2 * tsz(c) * cap))) return st;
     if ((st = dalloc(c, &c->Sfull, sizeof(double2) * cap))) return st;
-    if ((st = dalloc(c, &c->rseg, sizeof(KSeg) * cap))) return st;
-    if ((st = dalloc(c, &c->rowpos, sizeof(int) * cap))) return st;
-    if ((st = dalloc(c, &c->chunks, sizeof(int2) * cap))) return st;
+    if (!fp64(c)) {  // row segments of the CUDA-core kernels
+      if ((st = dalloc(c, &c->kseg, sizeof(KSeg) * cap))) return st;
+      if ((st = dalloc(c, &c->koff, sizeof(int) * cap))) return st;
+      if ((st = dalloc(c, &c->eS, 8 * cap))) return st;
+      if ((st = dalloc(c, &c->rseg, sizeof(KSeg) * cap))) return st;
+      if ((st = dalloc(c, &c->rowpos, sizeof(int) * cap))) return st;
+      if ((st = dalloc(c, &c->chunks, sizeof(int2) * cap))) return st;
+    }
     c->ksize_cap = cap;
   }
   const size_t sp = nk * (size_t)c->nchunk;
-  if (sp > c->spart_cap) {
+  if (!fp64(c) && sp > c->spart_cap) {
     dfree(c, c->Spart);
     c->Spart = nullptr;
     int st;
@@ -1082,21 +1175,25 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
     if ((st = dalloc(c, &c->ptab, pt))) return st;
     c->ptab_cap = pt;
   }
-  if (c->nchunk > c->musum_cap) {
+  if (!fp64(c) && c->nchunk > c->musum_cap) {
     dfree(c, c->musum_part);
     c->musum_part = nullptr;
     int st;
     if ((st = dalloc(c, &c->musum_part, 24 * (size_t)c->nchunk))) return st;
     c->musum_cap = c->nchunk;
   }
-  CK(c, cudaMemcpy(c->kseg, c->klist.seg.data(), sizeof(KSeg) * nseg, cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->koff, c->klist.koff.data(), sizeof(int) * nseg, cudaMemcpyHostToDevice));
   CK(c, cudaMemcpy(c->ek, c->klist.ek.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->rseg, c->klist.rseg.data(), sizeof(KSeg) * nrseg, cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->rowpos, c->klist.rowpos.data(), sizeof(int) * nk, cudaMemcpyHostToDevice));
-  // the padding entries of the scatter layout are never written: zero
-  CK(c, cudaMemset(c->eS, 0, 2 * tsz(c) * nks));
-  CK(c, cudaMemcpy(c->chunks, c->klist.chunks.data(), sizeof(int) * c->klist.chunks.size(), cudaMemcpyHostToDevice));
+  if (!fp64(c)) {
+    CK(c, cudaMemcpy(c->kseg, c->klist.seg.data(), sizeof(KSeg) * nseg, cudaMemcpyHostToDevice));
+    CK(c, cudaMemcpy(c->koff, c->klist.koff.data(), sizeof(int) * nseg, cudaMemcpyHostToDevice));
+    CK(c, cudaMemcpy(c->rseg, c->klist.rseg.data(), sizeof(KSeg) * nrseg, cudaMemcpyHostToDevice));
+    CK(c, cudaMemcpy(c->rowpos, c->klist.rowpos.data(), sizeof(int) * nk, cudaMemcpyHostToDevice));
+    // the padding entries of the scatter layout are never written: zero
+    CK(c, cudaMemset(c->eS, 0, 8 * nks));
+    CK(c, cudaMemcpy(c->chunks, c->klist.chunks.data(), sizeof(int) * c->klist.chunks.size(), cudaMemcpyHostToDevice));
+  } else if (int st = setup_k64(c)) {
+    return st;
+  }
   if (int st = setup_tc(c)) return st;
   {
     // k-space self-interaction: B_i holds -cflux sum_k e(k) (n . mu_i) n of

@@ -88,6 +88,9 @@ struct md_ctx {
   int4* xi4 = nullptr;
   double4_32a* xd = nullptr;
   void* mu = nullptr;
+  // tables of the FP64 pair terms (FP64 path)
+  double* gtab = nullptr;
+  double2* etab = nullptr;
   // stage outputs (T)
   void *Br = nullptr, *Fr = nullptr, *ov = nullptr, *Bk = nullptr, *Fk = nullptr, *Br2 = nullptr, *Bk2 = nullptr;
   void *k1m = nullptr, *k1e = nullptr, *m2 = nullptr, *e2 = nullptr, *th = nullptr;
@@ -113,6 +116,14 @@ struct md_ctx {
   size_t ptab_cap = 0;
   size_t ksize_cap = 0, spart_cap = 0;
   int musum_cap = 0;
+  // FP64 k space (md_kspace64.cu)
+  int k64_T = 0, k64_R = 0;
+  K64Shape k64s{};
+  int4* k64_task = nullptr;
+  int* k64_kidx = nullptr;
+  double2* k64_row = nullptr;
+  int2* k64_rowt = nullptr;
+  double2* k64_ad = nullptr;
   // tensor-core k space (mixed path; md_ktc.cu): engine choice, k rows and
   // their buffers (tc_rows = 0 while the engine is off)
   int kengine = MD_KSPACE_AUTO;

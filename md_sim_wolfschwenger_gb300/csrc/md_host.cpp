@@ -587,6 +587,62 @@ KList build_klist(int kc, double w) {
   return L;
 }
 
+// ============================================== FP64 pair-term tables
+
+// Taylor coefficients of y = erfcx about c from y' = 2 s y - 2 / sqrt(pi):
+// (n + 1) a_{n+1} = 2 c a_n + 2 a_{n-1} - [n = 0] 2 / sqrt(pi), in long double
+// (the recurrence cancels by ~2 c^2 per order, up to 72).  Degree 6,
+// economised to 5: on |u| <= h, u^6 = h^6 (T6(u/h) + 48 (u/h)^4 - 18 (u/h)^2
+// + 1) / 32, and dropping the T6 part leaves < 2e-17.
+namespace {
+struct ErfcxTaylor {
+  std::vector<long double> a;  // [kGIntervals][6], the part that does not depend on the configuration
+  std::vector<double> e;
+};
+const ErfcxTaylor& erfcx_taylor() {
+  static const ErfcxTaylor t = [] {
+    ErfcxTaylor r;
+    const long double tsp = 1.128379167095512573896158903121545172L;  // 2 / sqrt(pi)
+    const long double h2 = 1.0L / 65536;                              // (1/256)^2
+    for (int k = 0; k < md::kGIntervals; k++) {
+      const long double c = (k + 0.5L) / 128;
+      long double a[7];
+      a[0] = expl(c * c) * erfcl(c);
+      a[1] = 2 * c * a[0] - tsp;
+      for (int n = 1; n < 6; n++) a[n + 1] = 2 * (c * a[n] + a[n - 1]) / (n + 1);
+      a[4] += a[6] * h2 * 1.5L;
+      a[2] -= a[6] * h2 * h2 * 0.5625L;
+      a[0] += a[6] * h2 * h2 * h2 / 32;
+      r.a.insert(r.a.end(), a, a + 6);
+    }
+    for (int k = 0; k < md::kEEntries; k++) {
+      r.e.push_back(k / 64.0);
+      r.e.push_back((double)expl(-k / 64.0L));
+    }
+    return r;
+  }();
+  return t;
+}
+}  // namespace
+
+RealTables real_tables64(double irPi) {
+  const ErfcxTaylor& t = erfcx_taylor();
+  RealTables r;
+  r.e = t.e;
+  r.g.resize(8 * (size_t)md::kGIntervals);
+  for (int k = 0; k < md::kGIntervals; k++) {
+    const long double c = (k + 0.5L) / 128;
+    for (int q = 0; q < 6; q++) {
+      long double v = t.a[6 * (size_t)k + 5 - q];
+      if (q == 5) v += 2 * (long double)irPi * c;
+      if (q == 4) v += 2 * (long double)irPi;
+      r.g[8 * (size_t)k + q] = (double)v;
+    }
+    r.g[8 * (size_t)k + 6] = (double)c;
+  }
+  return r;
+}
+
 // ============================================================ cell grid
 
 // Cells of edge >= rc / reach; a stencil of +-reach cells must not wrap onto

@@ -76,6 +76,15 @@ KList build_klist(int kc, double w);
 int init_system(const md_config& c, int64_t n, uint64_t seed, double* rMag, double* rHydr, double* pos, double* mm,
                 double* ea, double* lBox, std::string* err);
 
+// ----------------------------------------------- FP64 pair-term tables
+// g: per interval of width 1/128 in s = alpha r, six coefficients (highest
+// first) of G(s) = erfcx(s) + 2 irPi s about the interval's centre (irPi: the
+// configuration's 1 / sqrt(pi)), the centre, one pad; e: (k/64, exp(-k/64)).
+struct RealTables {
+  std::vector<double> g, e;
+};
+RealTables real_tables64(double irPi);
+
 // ----------------------------------------------------------- cell grid
 md::CellGrid choose_grid(double rc_box, int64_t n, int reach);
 

@@ -33,7 +33,7 @@ int sk_blocks(const KParams& p);
 // Threads (segments) per structure-factor block, and how many such blocks
 // one SM holds at once for kc.
 int sk_threads();
-int sk_resident_blocks(int kc, bool fp64);
+int sk_resident_blocks(int kc);
 int skred_blocks(const KParams& p);
 int scatter_blocks(const KParams& p, int np);
 int int_blocks(int n);
@@ -118,15 +118,23 @@ int launch_kspace_tc_packed(cudaStream_t st, const KParams* ps, const Packed& sf
 // One warp waits on an mbarrier that gets an arrival only when `arrive` is
 // set; a wait that gives up after `limit` cycles sets kErrTcWait in *err.
 int launch_tc_wait_probe(cudaStream_t st, int* err, int arrive, long long limit);
+// FP64 k space (md_kspace64.cu): launch shape for kc, n particles and the
+// given number of tasks.
+struct K64Shape {
+  int nblk, threads, chunk, nchunk;
+};
+K64Shape kspace64_shape(int kc, int n, int tasks, int nsm);
+int launch_phase64(cudaStream_t st, const KParams& p);
+int launch_kspace64(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev);
 // Per-particle phase tables (once per step; positions are frozen across the
 // two Heun stages).
 int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64);
 int launch_phase_tables_packed(cudaStream_t st, const KParams* ps, const Packed& phase);
 // FP32 FMA-chain calibration: returns FLOPs issued by one launch.
 double launch_fma_calibration(cudaStream_t st, float* out, int blocks, int threads);
-size_t kscatter_smem(int kc, bool fp64);
-size_t ksf_smem(int kc, bool fp64);
-int scatter_particles(int kc, bool fp64);
+size_t kscatter_smem(int kc);
+size_t ksf_smem(int kc);
+int scatter_particles(int kc);
 
 // Integrator.
 int launch_heun1(cudaStream_t st, const IntParams& p, bool fp64);

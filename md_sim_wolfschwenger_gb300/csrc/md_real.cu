@@ -37,7 +37,8 @@
 // erfc on the mixed path: the Chebyshev fit erfcc of Numerical Recipes
 // (Press et al., 2nd ed., section 6.2), relative error < 1.2e-7 for x >= 0,
 // written as t exp(-x^2) exp(P(t)) so that exp(-x^2) is shared with the
-// Gaussian term; exponentials with __expf.  The FP64 path calls erfc/exp.
+// Gaussian term; exponentials with __expf.  The FP64 path takes both from
+// tables of polynomials (ewald64).
 //
 // Overlap push: CompInteractVecs moves cores apart in place while it walks
 // the pairs, so later pairs see moved positions.  Here every overlap is
@@ -46,7 +47,8 @@
 // dCont for the Ewald terms, and the displacement is applied with the
 // translation step.  For configurations without overlaps the two agree.
 //
-// Roofline: FP32/SFU issue bound.  Algorithmic FLOPs per unordered in-range
+// Roofline: mixed path FP32/SFU issue bound, FP64 path bound by the FP64 pipe
+// (see the FP64 pair terms).  Algorithmic FLOPs per unordered in-range
 // pair (counted from the reference formula): 113 full, 58 field only.
 #include <algorithm>
 
@@ -82,62 +84,66 @@ __device__ __forceinline__ float erfc_nr(float z, float ez2) {
   return t * ez2 * __expf(q);
 }
 
-// Ewald pair terms for the pair vector (dx, dy, dz) from i to j (r2 < rc2).
-template <typename T, bool FULL, bool COAT>
-__device__ __forceinline__ void pair_terms(const RealParams& p, T dx, T dy, T dz, T r2, const typename V4<T>::t& mi,
-                                           const typename V4<T>::t& mj, int oi, int oj, Acc<T>& a) {
+// Coating potentials of a pair inside rCutSR (CompSterRep,
+// CompElectrostatRep, CompForceVdW): the scalar force along the unit vector,
+// in FP64.  rd: the pair distance (clamped to contact here, as the
+// reference's list length is); oi, oj: particle indices.
+__device__ __forceinline__ double coat_force(const RealParams& p, double rd, int oi, int oj) {
+  const double ri = p.rMag_u[oi], rj = p.rMag_u[oj];
+  const double dc = ri + rj + p.cont_eps;
+  if (rd < dc) rd = dc;
+  // steric repulsion is asymmetric: dDelta and the prefactor use the
+  // pair's lower particle index as "idx1" (interaction.cpp:768-775)
+  const double ra = oi < oj ? ri : rj, rb = oi < oj ? rj : ri;
+  const double dDelta = 2.0 * (ra + p.eff_len);
+  double s = rd <= dDelta ? (2.0 * rb / (ra + rb)) * p.ster * ra * ra * log(dDelta / rd) : 0.0;
+  s += (ri * rj / (ri + rj)) * p.elec * exp(-p.kappa * (rd - ri - rj));
+  const double g1 = (rd - ri - rj) * (rd + ri + rj), g2 = rd * rd - (ri - rj) * (ri - rj);
+  const double c4 = 4.0 * ri * rj;
+  s += -p.vdw * rd * (c4 * c4 * c4) / (6.0 * g1 * g1 * g2 * g2);
+  return s;
+}
+
+// Ewald pair terms for the pair vector (dx, dy, dz) from i to j (r2 < rc2),
+// mixed path: with coating potentials and in the direct cell scan.
+template <bool FULL, bool COAT>
+__device__ __forceinline__ void pair_terms(const RealParams& p, float dx, float dy, float dz, float r2, const float4& mi,
+                                           const float4& mj, int oi, int oj, Acc<float>& a) {
   a.np++;
-  T ir0, r0;
-  if constexpr (std::is_same<T, float>::value) {
-    ir0 = rsqrtf(r2);
-    r0 = r2 * ir0;
-  } else {
-    ir0 = rsqrt(r2);
-    r0 = r2 * ir0;
-  }
-  const T ux = dx * ir0, uy = dy * ir0, uz = dz * ir0;
-  T r = r0, ire = ir0;
-  const T dcont = mi.w + mj.w + (T)p.cont_eps;
+  const float ir0 = rsqrtf(r2), r0 = r2 * ir0;
+  const float ux = dx * ir0, uy = dy * ir0, uz = dz * ir0;
+  float r = r0, ire = ir0;
+  const float dcont = mi.w + mj.w + (float)p.cont_eps;
   if (r < dcont) {
     if constexpr (FULL) {
-      const T h = (T)0.5 * (dcont - r);
+      const float h = 0.5f * (dcont - r);
       a.o0 -= h * ux;
       a.o1 -= h * uy;
       a.o2 -= h * uz;
     }
     r = dcont;
-    if constexpr (std::is_same<T, float>::value)
-      ire = __fdividef(1.0f, r);
-    else
-      ire = 1.0 / r;
+    ire = __fdividef(1.0f, r);
   }
-  const T ire2 = ire * ire;
-  const T re2 = r * r;
-  T e, erfcv;
-  if constexpr (std::is_same<T, float>::value) {
-    e = __expf(-(float)p.al2 * re2);
-    erfcv = erfc_nr((float)p.alpha * r, e);
-  } else {
-    e = exp(-p.al2 * re2);
-    erfcv = erfc(p.alpha * r);
-  }
-  const T t = (T)p.c2a * e * ire2;
-  const T a1 = erfcv * ire2 * ire + t;
-  const T a2 = (T)3 * a1 * ire2 + (T)2 * (T)p.al2 * t;
-  const T d1 = mi.x * ux + mi.y * uy + mi.z * uz;
-  const T d2 = mj.x * ux + mj.y * uy + mj.z * uz;
-  const T c1 = a2 * d2 * re2;
+  const float ire2 = ire * ire;
+  const float re2 = r * r;
+  const float e = __expf(-(float)p.al2 * re2), erfcv = erfc_nr((float)p.alpha * r, e);
+  const float t = (float)p.c2a * e * ire2;
+  const float a1 = erfcv * ire2 * ire + t;
+  const float a2 = 3.0f * a1 * ire2 + 2.0f * (float)p.al2 * t;
+  const float d1 = mi.x * ux + mi.y * uy + mi.z * uz;
+  const float d2 = mj.x * ux + mj.y * uy + mj.z * uz;
+  const float c1 = a2 * d2 * re2;
   a.b0 += c1 * ux - a1 * mj.x;
   a.b1 += c1 * uy - a1 * mj.y;
   a.b2 += c1 * uz - a1 * mj.z;
   if constexpr (FULL) {
-    const T a3 = (T)5 * a2 * ire2 + (T)4 * (T)p.al4 * t;
-    const T m12 = mi.x * mj.x + mi.y * mj.y + mi.z * mj.z;
-    const T s1 = (a2 * m12 - a3 * d1 * d2 * re2) * r;
-    const T s2 = a2 * r;
-    const T vx = s1 * ux + s2 * (d2 * mi.x + d1 * mj.x);
-    const T vy = s1 * uy + s2 * (d2 * mi.y + d1 * mj.y);
-    const T vz = s1 * uz + s2 * (d2 * mi.z + d1 * mj.z);
+    const float a3 = 5.0f * a2 * ire2 + 4.0f * (float)p.al4 * t;
+    const float m12 = mi.x * mj.x + mi.y * mj.y + mi.z * mj.z;
+    const float s1 = (a2 * m12 - a3 * d1 * d2 * re2) * r;
+    const float s2 = a2 * r;
+    const float vx = s1 * ux + s2 * (d2 * mi.x + d1 * mj.x);
+    const float vy = s1 * uy + s2 * (d2 * mi.y + d1 * mj.y);
+    const float vz = s1 * uz + s2 * (d2 * mi.z + d1 * mj.z);
     a.f0 -= vx;
     a.f1 -= vy;
     a.f2 -= vz;
@@ -145,24 +151,10 @@ __device__ __forceinline__ void pair_terms(const RealParams& p, T dx, T dy, T dz
     a.p1 += r * ux * vz;
     a.p2 += r * uy * vz;
     if constexpr (COAT) {
-      // Coating potentials for pairs inside rCutSR (intRangeSR uses the
-      // unclamped distance, interaction.cpp:115), evaluated in FP64 with the
-      // clamped distance like the reference's list length.
+      // pairs inside rCutSR (intRangeSR uses the unclamped distance,
+      // interaction.cpp:115), in FP64
       if ((double)r2 < p.rcut_sr2) {
-        double rd = sqrt((double)dx * dx + (double)dy * dy + (double)dz * dz);
-        const double ri = p.rMag_u[oi], rj = p.rMag_u[oj];
-        const double dc = ri + rj + p.cont_eps;
-        if (rd < dc) rd = dc;
-        // steric repulsion is asymmetric: dDelta and the prefactor use the
-        // pair's lower particle index as "idx1" (interaction.cpp:768-775)
-        const double ra = oi < oj ? ri : rj, rb = oi < oj ? rj : ri;
-        const double dDelta = 2.0 * (ra + p.eff_len);
-        double s = rd <= dDelta ? (2.0 * rb / (ra + rb)) * p.ster * ra * ra * log(dDelta / rd) : 0.0;
-        s += (ri * rj / (ri + rj)) * p.elec * exp(-p.kappa * (rd - ri - rj));
-        const double g1 = (rd - ri - rj) * (rd + ri + rj), g2 = rd * rd - (ri - rj) * (ri - rj);
-        const double c4 = 4.0 * ri * rj;
-        s += -p.vdw * rd * (c4 * c4 * c4) / (6.0 * g1 * g1 * g2 * g2);
-        const T sv = (T)s;
+        const float sv = (float)coat_force(p, sqrt((double)dx * dx + (double)dy * dy + (double)dz * dz), oi, oj);
         a.f0 -= sv * ux;
         a.f1 -= sv * uy;
         a.f2 -= sv * uz;
@@ -172,6 +164,175 @@ __device__ __forceinline__ void pair_terms(const RealParams& p, T dx, T dy, T dz
       }
     }
   }
+}
+
+// ------------------------------------------------------- FP64 pair terms
+// GB300 issues an FP64 instruction of a warp in 64 cycles of an SM quarter
+// (2 FMA per SM and cycle, 1/64 of FP32), so the FP64 passes are bound by the
+// number of FP64 instructions per pair and by nothing else; table loads,
+// integer and FP32 work are free beside them.  Hence
+//  - the box fold is decided in FP32 on the float copies of the coordinates
+//    (FP64 only next to half a box, where they cannot decide);
+//  - 1/r comes from an FP32 seed and one third-order step (5 FP64
+//    instructions); conversions between the formats are integer operations;
+//  - erfc and exp come from tables (RealParams::gtab, etab): with s = alpha r,
+//    exp(-s^2) = E_k P(s^2 - k/64) and erfc(s) + (2 s / sqrt(pi)) exp(-s^2) =
+//    exp(-s^2) G(s), G = erfcx(s) + 2 s / sqrt(pi) (with the configuration's pi), each interval of width
+//    1/128 a polynomial of degree 5; both to ~1e-16 (Taylor coefficients from
+//    the differential equation of erfcx, economised with Chebyshev's T6).
+// 78 FP64 instructions per pair (field, force and pressure), 50 for the field
+// alone, against ~230 / ~170 with the library's erfc, exp and rsqrt.
+
+// FP64 <-> FP32 in integer operations: widening is exact for normal numbers,
+// narrowing truncates (both arguments are normal, positive here).
+__device__ __forceinline__ double widen(float v) {
+  const unsigned b = __float_as_uint(v);
+  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  return __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
+}
+
+// Minimum-image difference b - a of box coordinates, with the reference's
+// fold (d > 1/2 -> d - 1, d < -1/2 -> d + 1); af, bf: their float copies.
+__device__ __forceinline__ double fold64(double a, double b, float af, float bf) {
+  const float d = bf - af;
+  const float ad = fabsf(d);
+  double v = b - a;
+  if (fabsf(ad - 0.5f) < 1e-5f) {
+    if (v > 0.5)
+      v -= 1.0;
+    else if (v < -0.5)
+      v += 1.0;
+  } else if (ad > 0.5f) {
+    v -= __hiloint2double(d > 0.f ? 0x3ff00000 : (int)0xbff00000, 0);
+  }
+  return v;
+}
+
+// Ewald factors at distance r (ire = 1/r, s = alpha r, x = alpha^2 r^2 from
+// r^2 itself: the exponential magnifies its error): q = exp(-x) / r^2 and
+// g = G(s) / r; the pair coefficient a1 = q g, the Gaussian term t = c2a q.
+__device__ __forceinline__ void ewald64(const RealParams& p, double ire, double ire2, double s, double x, double& q,
+                                        double& g) {
+  const float sf = narrow(s), xf = sf * sf;
+  const int k = (int)(sf * 128.0f), kx = (int)fmaf(xf, 64.0f, 0.5f);
+  double e, G;
+  if ((unsigned)k < (unsigned)kGIntervals) {
+    const double2* c = (const double2*)(p.gtab + 8 * k);  // c5, c4, .. c0, centre
+    const double2 c01 = c[0], c23 = c[1], c45 = c[2];
+    const double u = s - c[3].x;
+    const double2 ek = p.etab[kx];  // (k/64, exp(-k/64))
+    const double v = ek.x - x;      // exp(v), |v| <= 1/128
+    G = fma(fma(fma(fma(fma(c01.x, u, c01.y), u, c23.x), u, c23.y), u, c45.x), u, c45.y);
+    constexpr double h2 = 1.0 / 16384.0;  // (1/128)^2: economised exp series of degree 5
+    double w = fma(1.0 / 120.0, v, 1.0 / 24.0 + h2 * (48.0 / 32.0 / 720.0));
+    w = fma(w, v, 1.0 / 6.0);
+    w = fma(w, v, 0.5 - h2 * h2 * (18.0 / 32.0 / 720.0));
+    w = fma(w, v, 1.0);
+    e = fma(w * ek.y, v, ek.y);
+  } else {  // alpha r beyond the tables (s >= 6)
+    e = exp(-x);
+    G = erfcx(s) + p.c2a / p.alpha * s;
+  }
+  q = e * ire2;
+  g = G * ire;
+}
+
+// Pair terms on the FP64 path for sorted particle j and self coordinates
+// di / fi, moment mi.
+template <bool FULL, bool COAT>
+__device__ __forceinline__ void pair64(const RealParams& p, const double4_32a& di, const float4& fi,
+                                       const double4_32a& mi, int oi, int j, Acc<double>& a) {
+  const double4_32a dj = p.s.xd[j];
+  const float4 fj = p.s.xf[j];
+  const double4_32a mj = ((const double4_32a*)p.s.mu)[j];
+  double dx = fold64(di.x, dj.x, fi.x, fj.x), dy = fold64(di.y, dj.y, fi.y, fj.y), dz = fold64(di.z, dj.z, fi.z, fj.z);
+  double r2 = dx * dx + dy * dy + dz * dz;
+  if (!(r2 < p.rc2)) return;
+  a.np++;
+  bool sr = false;
+  if constexpr (FULL && COAT) sr = r2 < p.rcut_sr2;
+  double ire;
+  if (r2 > 1e-30) {
+    const double y0 = widen(rsqrtf(narrow(r2)));
+    const double ee = fma(-r2 * y0, y0, 1.0);
+    ire = fma(y0 * ee, fma(0.375, ee, 0.5), y0);
+  } else {
+    ire = rsqrt(r2);  // (nearly) coincident particles
+  }
+  double r = r2 * ire;
+  const double r0 = r;
+  const float dcf = (fi.w + fj.w + p.pk.eps) * 1.00001f;
+  if (!(narrow(r) > dcf)) {  // near contact or overlapping
+    const double dcont = mi.w + mj.w + p.cont_eps;
+    if (r < dcont) {
+      if constexpr (FULL) {
+        const double h = 0.5 * (dcont - r) * ire;
+        a.o0 -= h * dx;
+        a.o1 -= h * dy;
+        a.o2 -= h * dz;
+      }
+      // the pair vector rescaled to the contact length
+      const double c = dcont * ire;
+      dx *= c;
+      dy *= c;
+      dz *= c;
+      r = dcont;
+      r2 = r * r;
+      ire = 1.0 / r;
+    }
+  }
+  const double ire2 = ire * ire;
+  double q, g;
+  ewald64(p, ire, ire2, p.alpha * r, p.al2 * r2, q, g);
+  const double a1 = q * g, t = p.c2a * q;
+  const double a2 = fma(3.0 * ire2, a1, 2.0 * p.al2 * t);
+  const double D2 = mj.x * dx + mj.y * dy + mj.z * dz;
+  const double e2 = a2 * D2;
+  a.b0 = fma(e2, dx, fma(-a1, mj.x, a.b0));
+  a.b1 = fma(e2, dy, fma(-a1, mj.y, a.b1));
+  a.b2 = fma(e2, dz, fma(-a1, mj.z, a.b2));
+  if constexpr (FULL) {
+    const double a3 = fma(5.0 * ire2, a2, 4.0 * p.al4 * t);
+    const double D1 = mi.x * dx + mi.y * dy + mi.z * dz;
+    const double m12 = mi.x * mj.x + mi.y * mj.y + mi.z * mj.z;
+    double t1 = fma(-a3 * D1, D2, a2 * m12);
+    const double e1 = a2 * D1;
+    if constexpr (COAT) {
+      if (sr) t1 += coat_force(p, r0, oi, p.s.perm[j]) * ire;  // along d / r
+    }
+    const double vx = fma(t1, dx, fma(e2, mi.x, e1 * mj.x));
+    const double vy = fma(t1, dy, fma(e2, mi.y, e1 * mj.y));
+    const double vz = fma(t1, dz, fma(e2, mi.z, e1 * mj.z));
+    a.f0 -= vx;
+    a.f1 -= vy;
+    a.f2 -= vz;
+    a.p0 = fma(dx, vy, a.p0);
+    a.p1 = fma(dx, vz, a.p1);
+    a.p2 = fma(dy, vz, a.p2);
+  }
+}
+
+// Sums of W values (a power of two) over the warp with W - 1 + log2(32 / W)
+// FP64 additions per lane instead of 5 W: each butterfly step halves the
+// values a lane carries.  Returns the sum of value (lane / (32 / W)).
+template <int W>
+__device__ __forceinline__ double warp_sums(double (&v)[W], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = W / 2; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < h; q++) {
+      const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(kFull, give, o);
+    }
+  }
+  double s = v[0];
+  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s;
 }
 
 // ------------------------------------------------- packed pair terms (FP32)
@@ -346,7 +507,7 @@ template <typename T>
 struct Self {
   int4 si;
   double4_32a di;
-  float x, y, z;
+  float x, y, z, w;
   int oi;
 };
 
@@ -361,6 +522,7 @@ __device__ __forceinline__ Self<T> load_self(const RealParams& p, int k) {
     s.x = (float)s.si.x * sc;
     s.y = (float)s.si.y * sc;
     s.z = (float)s.si.z * sc;
+    s.w = 0.f;
     s.oi = s.si.w;
   } else {
     s.di = p.s.xd[k];
@@ -368,6 +530,7 @@ __device__ __forceinline__ Self<T> load_self(const RealParams& p, int k) {
     s.x = f.x;
     s.y = f.y;
     s.z = f.z;
+    s.w = f.w;
     s.oi = COAT ? p.s.perm[k] : 0;
   }
   return s;
@@ -768,32 +931,16 @@ __device__ __forceinline__ void real_eval(const RealParams& p, int bx) {
       if (dxf * dxf + dyf * dyf + dzf * dzf < rc2_fix) {
         const float sc = 2.3283064365386963e-10f;  // 2^-32
         const float dx = dxf * sc, dy = dyf * sc, dz = dzf * sc;
-        pair_terms<T, FULL, COAT>(p, dx, dy, dz, dx * dx + dy * dy + dz * dz, mi, mj, me.oi, COAT ? sj.w : 0, a);
+        pair_terms<FULL, COAT>(p, dx, dy, dz, dx * dx + dy * dy + dz * dz, mi, mj, me.oi, COAT ? sj.w : 0, a);
       }
     }
   };
-  // pair vector from i to sorted particle j, and the in-range test
+  // pair terms of sorted particle j, with the in-range test
   auto eval = [&](int j) {
-    const T4 mj = ((const T4*)p.s.mu)[j];
     if constexpr (F32) {
-      const int4 sj = p.s.xi[j];
-      const float dxf = (float)(sj.x - me.si.x), dyf = (float)(sj.y - me.si.y), dzf = (float)(sj.z - me.si.z);
-      if (dxf * dxf + dyf * dyf + dzf * dzf < rc2_fix) {
-        const float sc = 2.3283064365386963e-10f;
-        const float dx = dxf * sc, dy = dyf * sc, dz = dzf * sc;
-        pair_terms<T, FULL, COAT>(p, dx, dy, dz, dx * dx + dy * dy + dz * dz, mi, mj, me.oi, COAT ? sj.w : 0, a);
-      }
+      eval_loaded(p.s.xi[j], ((const T4*)p.s.mu)[j]);
     } else {
-      const double4_32a dj = p.s.xd[j];
-      double dx = dj.x - me.di.x, dy = dj.y - me.di.y, dz = dj.z - me.di.z;
-      dx -= (double)(dx > 0.5);
-      dx += (double)(dx < -0.5);
-      dy -= (double)(dy > 0.5);
-      dy += (double)(dy < -0.5);
-      dz -= (double)(dz > 0.5);
-      dz += (double)(dz < -0.5);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < p.rc2) pair_terms<T, FULL, COAT>(p, dx, dy, dz, r2, mi, mj, me.oi, COAT ? p.s.perm[j] : 0, a);
+      pair64<FULL, COAT>(p, me.di, make_float4(me.x, me.y, me.z, me.w), mi, me.oi, j, a);
     }
   };
 
@@ -870,41 +1017,64 @@ __device__ __forceinline__ void real_eval(const RealParams& p, int bx) {
     a.b1 += a2.b1.x + a2.b1.y;
     a.b2 += a2.b2.x + a2.b2.y;
   }
-  a.b0 = warp_sum(a.b0);
-  a.b1 = warp_sum(a.b1);
-  a.b2 = warp_sum(a.b2);
-  if constexpr (FULL) {
-    a.f0 = warp_sum(a.f0);
-    a.f1 = warp_sum(a.f1);
-    a.f2 = warp_sum(a.f2);
-    a.o0 = warp_sum(a.o0);
-    a.o1 = warp_sum(a.o1);
-    a.o2 = warp_sum(a.o2);
-    a.p0 = warp_sum(a.p0);
-    a.p1 = warp_sum(a.p1);
-    a.p2 = warp_sum(a.p2);
-    a.np = warp_sum(a.np);
-  }
-  if (lane == 0) {
-    T* B = (T*)p.B;
-    const int n = p.n;
-    B[k] = a.b0;
-    B[n + k] = a.b1;
-    B[2 * n + k] = a.b2;
+  T* B = (T*)p.B;
+  T* F = (T*)p.F;
+  T* O = (T*)p.ov;
+  const int n = p.n;
+  if constexpr (F32) {
+    a.b0 = warp_sum(a.b0);
+    a.b1 = warp_sum(a.b1);
+    a.b2 = warp_sum(a.b2);
     if constexpr (FULL) {
-      T* F = (T*)p.F;
-      T* O = (T*)p.ov;
-      F[k] = a.f0;
-      F[n + k] = a.f1;
-      F[2 * n + k] = a.f2;
-      O[k] = a.o0;
-      O[n + k] = a.o1;
-      O[2 * n + k] = a.o2;
-      p.Ppart[3 * k] = (double)a.p0;
-      p.Ppart[3 * k + 1] = (double)a.p1;
-      p.Ppart[3 * k + 2] = (double)a.p2;
-      if (p.npairs) atomicAdd(p.npairs, (unsigned long long)a.np);
+      a.f0 = warp_sum(a.f0);
+      a.f1 = warp_sum(a.f1);
+      a.f2 = warp_sum(a.f2);
+      a.o0 = warp_sum(a.o0);
+      a.o1 = warp_sum(a.o1);
+      a.o2 = warp_sum(a.o2);
+      a.p0 = warp_sum(a.p0);
+      a.p1 = warp_sum(a.p1);
+      a.p2 = warp_sum(a.p2);
+      a.np = warp_sum(a.np);
     }
+    if (lane == 0) {
+      B[k] = a.b0;
+      B[n + k] = a.b1;
+      B[2 * n + k] = a.b2;
+      if constexpr (FULL) {
+        F[k] = a.f0;
+        F[n + k] = a.f1;
+        F[2 * n + k] = a.f2;
+        O[k] = a.o0;
+        O[n + k] = a.o1;
+        O[2 * n + k] = a.o2;
+        p.Ppart[3 * k] = (double)a.p0;
+        p.Ppart[3 * k + 1] = (double)a.p1;
+        p.Ppart[3 * k + 2] = (double)a.p2;
+      }
+    }
+  } else if constexpr (FULL) {
+    double v[16] = {a.b0, a.b1, a.b2, a.f0, a.f1, a.f2, a.p0, a.p1, a.p2, a.o0, a.o1, a.o2, 0, 0, 0, 0};
+    const double s = warp_sums<16>(v, lane);
+    const int q = lane >> 1;
+    if ((lane & 1) == 0 && q < 12) {
+      if (q < 3)
+        B[q * n + k] = s;
+      else if (q < 6)
+        F[(q - 3) * n + k] = s;
+      else if (q < 9)
+        p.Ppart[3 * k + q - 6] = s;
+      else
+        O[(q - 9) * n + k] = s;
+    }
+    a.np = warp_sum(a.np);
+  } else {
+    double v[4] = {a.b0, a.b1, a.b2, 0};
+    const double s = warp_sums<4>(v, lane);
+    if ((lane & 7) == 0 && lane < 24) B[(lane >> 3) * n + k] = s;
+  }
+  if constexpr (FULL) {
+    if (lane == 0 && p.npairs) atomicAdd(p.npairs, (unsigned long long)a.np);
   }
 }
 

@@ -25,4 +25,9 @@ constexpr int kScatSeg = 64;
 // over this many threads (by chunk), reduced in a fixed order.
 constexpr int kScatterParts = 4;
 
+// Tables of the FP64 pair terms: intervals of width 1/128 in alpha r (beyond
+// them the library functions), and exp(-k/64) up to the same alpha r.
+constexpr int kGIntervals = 768;
+constexpr int kEEntries = 36 * 64 + 2;
+
 }  // namespace md

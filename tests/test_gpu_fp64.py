@@ -1,0 +1,49 @@
+"""FP64 path against the FP64 oracle at the edges of its kernels: particle
+counts around the blocks, k cut-offs around the tasks of four |nx|, an
+alpha r beyond the tables of the pair terms, coating potentials, cores in
+contact.  Both sides sum ~n terms of the same size in another order, so the
+contact-normalised differences stay far below TOL_FP64 = 1e-10."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import TOL_FP64, gpu_system, oracle_system, random_system, scales
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,kc,rc_frac,alpha_rc", [
+    (2, 2, 0.45, None), (31, 3, 0.5, None), (33, 4, 0.4, None), (130, 7, 0.3, None), (257, 8, 0.35, None),
+    (96, 15, 0.25, None), (40, 31, 0.2, None), (64, 96, 0.3, None), (150, 5, 0.5, 9.0)])
+def test_interactions_against_oracle(n, kc, rc_frac, alpha_rc):
+    ini, g = random_system(n, seed=10 * n + kc, rc_frac=rc_frac, lognormal=n % 2 == 0)
+    g["kc"] = kc
+    if alpha_rc:  # the cut-off reaches beyond the tables (alpha r = 6)
+        g["alpha"] = alpha_rc / g["rc"]
+    fAl, bAl, _ = scales(ini, g)
+    sim, orc = gpu_system(ini, g, 0), oracle_system(ini, g)
+    B, F, P = sim.CompInteractions()
+    Bo, Fo, Po = orc.compute_interactions()
+    assert O.rms_rel(B, Bo, bAl) < TOL_FP64
+    assert O.rms_rel(F, Fo, fAl) < TOL_FP64
+    np.testing.assert_allclose(P, Po, rtol=0, atol=1e-10 * fAl * g["rc"] * n)
+    rng = np.random.default_rng(n)
+    mm = rng.standard_normal((3, n))
+    mm /= np.linalg.norm(mm, axis=0)
+    assert O.rms_rel(sim.CompDemagField(mm), orc.compute_field(mm), bAl) < TOL_FP64
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.35])
+def test_contact_distances(scale):
+    """Positions pulled together until cores touch or overlap: the clamped
+    distance and the push follow the reference."""
+    n = 96
+    ini, g = random_system(n, seed=3, rc_frac=0.4)
+    g["pos"] = np.ascontiguousarray(g["pos"] * scale)
+    fAl, bAl, _ = scales(ini, g)
+    sim, orc = gpu_system(ini, g, 0), oracle_system(ini, g)
+    B, F, _ = sim.CompInteractions()
+    Bo, Fo, _ = orc.compute_interactions()
+    assert O.rms_rel(B, Bo, bAl) < TOL_FP64
+    assert O.rms_rel(F, Fo, fAl) < TOL_FP64
+    np.testing.assert_allclose(sim.get_state()[0], orc.get_state()[0], rtol=0, atol=1e-12 * g["lBox"])
