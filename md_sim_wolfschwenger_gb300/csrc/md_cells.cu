@@ -41,6 +41,16 @@ __device__ __forceinline__ double wrap_box(double x, double invL) {
   return xb - floor(xb + 0.5);
 }
 
+// round(x_box 2^32) as a wrapping 32-bit integer (the fold by whole boxes drops
+// out mod 2^32): adding 1.5 2^52 leaves the rounded integer in the low word, two
+// FP64 instructions for |x| < 2^17 box lengths.
+__device__ __forceinline__ int fixed_box(double x, double invL) {
+  const double t = x * (invL * 4294967296.0);
+  if ((__double2hiint(t) & 0x7fffffff) < 0x43000000)  // |t| < 2^49
+    return __double2loint(t + 6755399441055744.0);
+  return (int)(unsigned)(long long)llrint(wrap_box(x, invL) * 4294967296.0);
+}
+
 __device__ __forceinline__ bool skip(const StepFlags* f) { return f && !f->rebuild; }
 
 // Start of a step: rebuild the cell order and the neighbour list if the host
@@ -173,14 +183,12 @@ __device__ __forceinline__ void sorted_fill(const CellParams& p, int bx) {
       p.xbuild[2 * n + i] = pz;
     }
   }
-  const double x = wrap_box(px, p.invL), y = wrap_box(py, p.invL), z = wrap_box(pz, p.invL);
   const double rm = p.rMag_u[i];
-  s.xf[k] = make_float4((float)x, (float)y, (float)z, (float)rm);
   if constexpr (std::is_same<T, float>::value) {
-    const double sc = 4294967296.0;
-    s.xi[k] = make_int4((int)(unsigned)(long long)llrint(x * sc), (int)(unsigned)(long long)llrint(y * sc),
-                        (int)(unsigned)(long long)llrint(z * sc), i);
+    s.xi[k] = make_int4(fixed_box(px, p.invL), fixed_box(py, p.invL), fixed_box(pz, p.invL), i);
   } else {
+    const double x = wrap_box(px, p.invL), y = wrap_box(py, p.invL), z = wrap_box(pz, p.invL);
+    s.xf[k] = make_float4((float)x, (float)y, (float)z, (float)rm);
     s.xd[k] = make_double4_32a(x, y, z, rm);
   }
   const double mu = p.magMom_u[i];

@@ -230,6 +230,7 @@ struct StrongView {
     }
     if (!usable() || !a) return false;
     const int e0 = max(off[r], 0), e1 = (int)min((long long)off[r + 1], cap);
+    if (e0 >= e1) return false;
     for (int e = e0; e < e1; e = (e & ~31) + 32) {
 #pragma unroll
       for (int q = 0; q < 3; q++) {
@@ -320,12 +321,14 @@ struct IntParams {
   // particle constants (orig order)
   const double* magMom_u;    // |mu_i| / mu_u
   const double* rMag_u;      // rMag / L
-  const double* invZt;       // 1 / zeta_trans
-  const double* velEa1;
-  const double* velEa2;
-  const double* sT;          // thermal torque scale (DefThermFluct)
-  const double* sB;          // thermal field scale
-  const double* sF;          // thermal force scale
+  // per-particle constants in T (k_int_consts), T4 each: thermal torque, field
+  // and force scale (DefThermFluct), 1 / zeta_trans; velEa1, velEa2, |mu| /
+  // mu_u, rMag / L
+  const void *cA, *cB;
+  // the scalars above as T = float sees them
+  struct F32 {
+    float dt, L, iL, B_unit, F_unit, cself, csurf, anisConst, velMmConst, magDamp;
+  } f;
   // work arrays (orig order, T)
   void *k1m, *k1e, *m2, *e2, *th;   // th: [9][n] scaled noise
   // stage outputs (sorted order, T)
@@ -411,37 +414,82 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1
   return c;
 }
 
-// Nine standard normals of particle i at step s (torque xyz, field xyz,
-// force xyz), Box-Muller on uniforms (x + 0.5) 2^-32.
+// Standard normals of particle i at step s (torque xyz, field xyz, force xyz,
+// three spare): Box-Muller on uniforms (x + 0.5) 2^-32 of Philox blocks {i, b,
+// step}; pair j of block j / 2 gives normals 2 j and 2 j + 1.
+template <typename T>
+__device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, T z[2]) {
+  if constexpr (std::is_same<T, float>::value) {
+    const float u1 = ((float)a + 0.5f) * 2.3283064365386963e-10f;
+    const float u2 = ((float)b + 0.5f) * 2.3283064365386963e-10f;
+    float rr = sqrtf(-2.0f * logf(u1)), s, c;
+    sincospif(2.0f * u2, &s, &c);
+    z[0] = rr * c;
+    z[1] = rr * s;
+  } else {
+    const double u1 = ((double)a + 0.5) * 2.3283064365386963e-10;
+    const double u2 = ((double)b + 0.5) * 2.3283064365386963e-10;
+    double rr = sqrt(-2.0 * log(u1)), s, c;
+    sincospi(2.0 * u2, &s, &c);
+    z[0] = rr * c;
+    z[1] = rr * s;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void philox_pair(uint64_t seed, uint64_t step, uint32_t i, int j, T z[2]) {
+  const uint4 r = philox4x32_10(make_uint4(i, (uint32_t)j >> 1, (uint32_t)step, (uint32_t)(step >> 32)),
+                                (uint32_t)seed, (uint32_t)(seed >> 32));
+  (j & 1) ? box_muller<T>(r.z, r.w, z) : box_muller<T>(r.x, r.y, z);
+}
 template <typename T>
 __device__ __forceinline__ void philox_normals9(uint64_t seed, uint64_t step, uint32_t i, T z[9]) {
-  T w[12];
 #pragma unroll
   for (uint32_t b = 0; b < 3; b++) {
-    uint4 r = philox4x32_10(make_uint4(i, b, (uint32_t)step, (uint32_t)(step >> 32)), (uint32_t)seed,
-                            (uint32_t)(seed >> 32));
-    uint32_t u[4] = {r.x, r.y, r.z, r.w};
+    const uint4 r = philox4x32_10(make_uint4(i, b, (uint32_t)step, (uint32_t)(step >> 32)), (uint32_t)seed,
+                                  (uint32_t)(seed >> 32));
+    T w[4];
+    box_muller<T>(r.x, r.y, w);
+    box_muller<T>(r.z, r.w, w + 2);
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if constexpr (std::is_same<T, float>::value) {
-        float u1 = ((float)u[2 * h] + 0.5f) * 2.3283064365386963e-10f;
-        float u2 = ((float)u[2 * h + 1] + 0.5f) * 2.3283064365386963e-10f;
-        float rr = sqrtf(-2.0f * logf(u1)), s, c;
-        sincospif(2.0f * u2, &s, &c);
-        w[4 * b + 2 * h] = rr * c;
-        w[4 * b + 2 * h + 1] = rr * s;
-      } else {
-        double u1 = ((double)u[2 * h] + 0.5) * 2.3283064365386963e-10;
-        double u2 = ((double)u[2 * h + 1] + 0.5) * 2.3283064365386963e-10;
-        double rr = sqrt(-2.0 * log(u1)), s, c;
-        sincospi(2.0 * u2, &s, &c);
-        w[4 * b + 2 * h] = rr * c;
-        w[4 * b + 2 * h + 1] = rr * s;
-      }
+    for (int h = 0; h < 4; h++)
+      if (4 * b + h < 9) z[4 * b + h] = w[h];
+  }
+}
+
+// Sums of W values (a power of two) over the warp with W - 1 + log2(32 / W)
+// additions per lane instead of 5 W (FP64 additions: 64 cycles each): each
+// butterfly step halves the values a lane carries.  Returns the sum of value
+// (lane / (32 / W)).
+template <int W>
+__device__ __forceinline__ double warp_sums(double (&v)[W], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = W / 2; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < h; q++) {
+      const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(kFull, give, o);
     }
   }
-#pragma unroll
-  for (int k = 0; k < 9; k++) z[k] = w[k];
+  double s = v[0];
+  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s;
+}
+
+// FP64 <-> FP32 in integer operations (the FP64 pipe takes 64 cycles per warp
+// instruction): widening is exact, narrowing truncates; zeros, subnormals,
+// infinities and NaN (and what FP32 cannot hold) take the conversion
+// instructions.
+__device__ __forceinline__ double widen(float v) {
+  const unsigned b = __float_as_uint(v);
+  if (((b >> 23) & 255u) - 1u >= 254u) return (double)v;
+  return __hiloint2double((int)((((b & 0x7fffffffu) >> 3) + (896u << 20)) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  if (((hi >> 20) & 0x7ffu) - 897u >= 254u) return (float)v;
+  return __uint_as_float((hi & 0x80000000u) | ((((hi & 0x7fffffffu) - (896u << 20)) << 3) | (lo >> 29)));
 }
 
 template <typename T>

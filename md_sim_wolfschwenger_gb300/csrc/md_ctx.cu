@@ -317,12 +317,10 @@ IntParams int_params(md_ctx* c, double dt, const void* Br, const void* Bk) {
   p.posRef = c->posRef;
   p.magMom_u = c->magMom_u;
   p.rMag_u = c->rMag_u;
-  p.invZt = c->invZt;
-  p.velEa1 = c->velEa1;
-  p.velEa2 = c->velEa2;
-  p.sT = c->sT;
-  p.sB = c->sB;
-  p.sF = c->sF;
+  p.cA = c->cA;
+  p.cB = c->cB;
+  p.f = IntParams::F32{(float)p.dt,     (float)p.L,     1.0f / (float)p.L,   (float)p.B_unit,     (float)p.F_unit,
+                       (float)p.cself, (float)p.csurf, (float)p.anisConst, (float)p.velMmConst, (float)p.magDamp};
   p.k1m = c->k1m;
   p.k1e = c->k1e;
   p.m2 = c->m2;
@@ -392,7 +390,8 @@ static int fork_join(md_ctx* c, int q, int seg_real, int seg_k, RP&& real_prep, 
 }
 
 // Field + force evaluation on the current master state (no integrator).
-static int issue_interactions(md_ctx* c) {
+// dt >= 0: the step's noise is drawn beside it.
+static int issue_interactions(md_ctx* c, double dt = -1.0) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
   const CellParams cp = cell_params(c);
@@ -401,7 +400,11 @@ static int issue_interactions(md_ctx* c) {
   cudaMemsetAsync(&c->sc->pairs, 0, sizeof(unsigned long long), c->stream);
   l += fork_join(
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,
-      [&](cudaStream_t st) { return launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), &c->sc->flags, fp64(c)); },
+      [&](cudaStream_t st) {
+        int l = launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), &c->sc->flags, fp64(c));
+        if (dt >= 0) l += launch_noise(st, int_params(c, dt, nullptr, nullptr), fp64(c));
+        return l;
+      },
       [&](cudaStream_t st) { return launch_real(st, real_params(c, c->Br, c->Fr, c->ov), true, fp64(c)); },
       [&](cudaStream_t st) { return launch_phase_tables(st, k_params(c, nullptr, nullptr), fp64(c)); },
       [&](cudaStream_t st) {
@@ -427,7 +430,7 @@ static int issue_field(md_ctx* c) {
 }
 
 static int issue_step(md_ctx* c, double dt) {
-  int l = issue_interactions(c);
+  int l = issue_interactions(c, dt);
   mark(c, MD_SEG_HEUN1);
   l += launch_heun1(c->stream, int_params(c, dt, c->Br, c->Bk), fp64(c));
   l += issue_field(c);
@@ -827,7 +830,7 @@ int md_ctx_create(const md_config* cfg, int64_t n, int precision, md_ctx** out) 
   for (auto p : d3)
     if ((st = dalloc(c, p, 24 * N))) return fail(st);
   if ((st = dalloc(c, &c->xi, 72 * N))) return fail(st);
-  double** d1[] = {&c->magMom_u, &c->rMag_u, &c->invZt, &c->velEa1, &c->velEa2, &c->sT, &c->sB, &c->sF};
+  double** d1[] = {&c->magMom_u, &c->rMag_u, &c->invZt, &c->velEa1, &c->velEa2, &c->zetaR, &c->zetaT, &c->invVol};
   for (auto p : d1)
     if ((st = dalloc(c, p, 8 * N))) return fail(st);
   int** i1[] = {&c->cellOf, &c->tmp, &c->perm, &c->rank, &c->scell};
@@ -840,6 +843,7 @@ int md_ctx_create(const md_config* cfg, int64_t n, int precision, md_ctx** out) 
     if ((st = dalloc(c, &c->xi4, 16 * N))) return fail(st);
   }
   if ((st = dalloc(c, &c->mu, 4 * T * N))) return fail(st);
+  if ((st = dalloc(c, &c->cA, 4 * T * N)) || (st = dalloc(c, &c->cB, 4 * T * N))) return fail(st);
   void** t3[] = {&c->Br, &c->Fr, &c->ov, &c->Bk, &c->Fk, &c->Br2, &c->Bk2, &c->k1m, &c->k1e, &c->m2, &c->e2};
   for (auto p : t3)
     if ((st = dalloc(c, p, 3 * T * N))) return fail(st);
@@ -915,17 +919,21 @@ int md_set_particles(md_ctx* c, const double* rMag, const double* rHydr) {
   c->props = p;
   c->L = p.lBox;
   const size_t N = (size_t)c->n;
-  std::vector<double> mu(N), rm(N), izt(N);
+  std::vector<double> mu(N), rm(N), izt(N), ivol(N);
   for (size_t i = 0; i < N; i++) {
     mu[i] = p.magMom[i] / p.muMax;
     rm[i] = p.rMag[i] / c->L;
     izt[i] = 1.0 / p.zetaTrans[i];
+    ivol[i] = 1.0 / p.volMag[i];
   }
   CK(c, cudaMemcpyAsync(c->magMom_u, mu.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaMemcpyAsync(c->rMag_u, rm.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaMemcpyAsync(c->invZt, izt.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaMemcpyAsync(c->velEa1, p.velEa1.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaMemcpyAsync(c->velEa2, p.velEa2.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
+  CK(c, cudaMemcpyAsync(c->zetaR, p.zetaRot.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
+  CK(c, cudaMemcpyAsync(c->zetaT, p.zetaTrans.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
+  CK(c, cudaMemcpyAsync(c->invVol, ivol.data(), 8 * N, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
   c->have_particles = true;
   c->have_ewald = false;
@@ -948,6 +956,7 @@ int md_set_box(md_ctx* c, double lBox) {
   std::vector<double> rm(c->n);
   for (int64_t i = 0; i < c->n; i++) rm[i] = c->props.rMag[i] / lBox;
   CK(c, cudaMemcpy(c->rMag_u, rm.data(), 8 * c->n, cudaMemcpyHostToDevice));
+  c->cur_dt = -1;  // the integrator's constants hold rMag / L
   c->have_ewald = false;
   c->list_valid = false;
   invalidate_graph(c);
@@ -1378,15 +1387,19 @@ int ensure_records(md_ctx* c, int64_t extra) {
   return MD_OK;
 }
 
+// DefThermFluct prefactors (src/simulation.cpp:563-603) and the other
+// per-particle constants of the integrator, computed on the device for this
+// dt (queued on the stream; the adaptive solvers change dt every step).
 int prepare_dt(md_ctx* c, double dt) {
   if (dt == c->cur_dt) return MD_OK;
-  std::vector<double> a, b, d;
-  mdh::noise_scales(c->cfg, c->props, dt, &a, &b, &d);
-  const size_t N8 = 8 * (size_t)c->n;
-  CK(c, cudaMemcpyAsync(c->sT, a.data(), N8, cudaMemcpyHostToDevice, c->stream));
-  CK(c, cudaMemcpyAsync(c->sB, b.data(), N8, cudaMemcpyHostToDevice, c->stream));
-  CK(c, cudaMemcpyAsync(c->sF, d.data(), N8, cudaMemcpyHostToDevice, c->stream));
-  CK(c, cudaStreamSynchronize(c->stream));
+  const md_config& g = c->cfg;
+  const double kt = 2.0 * g.kB * g.temp / dt;
+  const double kb = 2.0 * g.kB * g.temp * g.magDamp / (g.gyroMr * g.satMag * dt);
+  cudaGetLastError();  // an earlier call's error was reported there
+  launch_int_consts(c->stream, (int)c->n, g.ENABLE_THERM_TORQUE ? kt : 0.0, g.ENABLE_THERM_FIELD ? kb : 0.0,
+                    g.ENABLE_THERM_FORCE ? kt : 0.0, c->zetaR, c->zetaT, c->invVol, c->invZt, c->velEa1, c->velEa2,
+                    c->magMom_u, c->rMag_u, c->cA, c->cB, fp64(c));
+  CK(c, cudaGetLastError());
   c->cur_dt = dt;
   invalidate_graph(c);
   return MD_OK;
@@ -1535,7 +1548,7 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
     if (c->noise == MD_NOISE_UPLOADED)
       CK(c, cudaMemcpyAsync(c->xi, xi + (size_t)done * 9 * c->n, 72 * (size_t)c->n, cudaMemcpyHostToDevice,
                             c->stream));
-    c->launches += issue_interactions(c);
+    c->launches += issue_interactions(c, dt0);
     bool cond = true, noFailed = true, first = true;
     double nf = 1.0, used = dt0;
     while (cond) {

@@ -79,7 +79,8 @@ struct md_ctx {
   double *pos = nullptr, *mm = nullptr, *ea = nullptr, *truePos = nullptr, *posRef = nullptr;
   double *xi = nullptr, *tmpmm = nullptr, *Bout = nullptr, *Fout = nullptr;
   double *magMom_u = nullptr, *rMag_u = nullptr, *invZt = nullptr, *velEa1 = nullptr, *velEa2 = nullptr;
-  double *sT = nullptr, *sB = nullptr, *sF = nullptr;
+  double *zetaR = nullptr, *zetaT = nullptr, *invVol = nullptr;
+  void *cA = nullptr, *cB = nullptr;  // the integrator's constants in T (k_int_consts)
   // cells and sorted views
   int *cellOf = nullptr, *tmp = nullptr, *perm = nullptr, *rank = nullptr, *scell = nullptr;
   int *count = nullptr, *cell_start = nullptr;

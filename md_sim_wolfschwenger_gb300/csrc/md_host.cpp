@@ -335,20 +335,6 @@ int make_props(const md_config& c, const double* rMag, const double* rHydr, int6
   return MD_OK;
 }
 
-void noise_scales(const md_config& c, const Props& p, double dt, std::vector<double>* sT, std::vector<double>* sB,
-                  std::vector<double>* sF) {
-  const size_t n = p.rMag.size();
-  sT->assign(n, 0.0);
-  sB->assign(n, 0.0);
-  sF->assign(n, 0.0);
-  for (size_t i = 0; i < n; i++) {
-    if (c.ENABLE_THERM_TORQUE) (*sT)[i] = std::sqrt((2.0 * c.kB * c.temp / dt) * p.zetaRot[i]);
-    if (c.ENABLE_THERM_FIELD)
-      (*sB)[i] = std::sqrt(2.0 * c.kB * c.temp * c.magDamp / (c.gyroMr * c.satMag * dt) * (1.0 / p.volMag[i]));
-    if (c.ENABLE_THERM_FORCE) (*sF)[i] = std::sqrt((2.0 * c.kB * c.temp / dt) * p.zetaTrans[i]);
-  }
-}
-
 // ================================================================== Ewald
 
 EwaldModel ewald_model(const md_config& c, const Props& p) {

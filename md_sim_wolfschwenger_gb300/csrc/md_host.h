@@ -31,9 +31,6 @@ struct Props {
 int make_props(const md_config& c, const double* rMag, const double* rHydr, int64_t n, Props* p,
                std::string* err);
 double integral_eff_diameter(const md_config& c, double dMag);
-// DefThermFluct scale factors for a step dt.
-void noise_scales(const md_config& c, const Props& p, double dt, std::vector<double>* sT,
-                  std::vector<double>* sB, std::vector<double>* sF);
 
 // ------------------------------------------------------------ Ewald
 struct EwaldModel {

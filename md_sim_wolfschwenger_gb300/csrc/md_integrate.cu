@@ -20,8 +20,14 @@
 // Precision: T = float (mixed) or double.  Positions, the master copies of
 // m and n, the self/surface Ewald terms and all reductions are FP64.
 //
-// Roofline: HBM/L2 bound, tiny; per particle and step ~250 B of algorithmic
-// traffic (state 72 B read + 72 B written, stage outputs, work arrays).
+// Roofline: ~250 B of algorithmic traffic per particle and step (state 72 B
+// read + 72 B written, stage outputs, work arrays); what bounds these launches
+// is latency: their loads and, on the mixed path, the FP64 instructions of a
+// thread, each 64 cycles of an SM quarter whatever the occupancy.  So the
+// noise is drawn by a launch of its own beside the field evaluation
+// (k_noise), constants are kept per particle in T (k_int_consts), exact
+// conversions are integer operations (widen, narrow), and FP64 work whose
+// result is known (no overlap push, no wrap, no strong pairs) is skipped.
 #include "md_common.cuh"
 #include "md_kernels.h"
 
@@ -37,6 +43,15 @@ __device__ __forceinline__ double ext_field_z(const IntParams& p, double t) {
   return t < p.tMag ? p.magFluxDens : 0.0;
 }
 
+// A scalar parameter in T (no conversion instruction in the kernel).
+template <typename T>
+__device__ __forceinline__ T scalar(double d, float f) {
+  if constexpr (std::is_same<T, float>::value)
+    return f;
+  else
+    return d;
+}
+
 // RKCoeffs: Beff = ext + demag + anisConst (m.n) n + B_th;
 // dn/dt = velEa1 (m.n)(m - (m.n) n) + velEa2 (tau_th x n);
 // dm/dt = -velMmConst (m x Beff + magDamp m x (m x Beff)).
@@ -44,7 +59,7 @@ template <typename T>
 __device__ __forceinline__ void rk(const IntParams& p, const T m[3], const T e[3], const T bd[3], T bz_ext,
                                    const T bth[3], const T tau[3], T v1, T v2, T km[3], T ke[3]) {
   const T dot = m[0] * e[0] + m[1] * e[1] + m[2] * e[2];
-  const T ac = (T)p.anisConst;
+  const T ac = scalar<T>(p.anisConst, p.f.anisConst);
   T be[3];
   be[0] = bd[0] + ac * (e[0] * dot) + bth[0];
   be[1] = bd[1] + ac * (e[1] * dot) + bth[1];
@@ -66,7 +81,7 @@ __device__ __forceinline__ void rk(const IntParams& p, const T m[3], const T e[3
   const T y0 = m[1] * x2 - m[2] * x1;
   const T y1 = m[2] * x0 - m[0] * x2;
   const T y2 = m[0] * x1 - m[1] * x0;
-  const T vm = (T)p.velMmConst, md = (T)p.magDamp;
+  const T vm = scalar<T>(p.velMmConst, p.f.velMmConst), md = scalar<T>(p.magDamp, p.f.magDamp);
   km[0] = -vm * (x0 + md * y0);
   km[1] = -vm * (x1 + md * y1);
   km[2] = -vm * (x2 + md * y2);
@@ -75,9 +90,11 @@ __device__ __forceinline__ void rk(const IntParams& p, const T m[3], const T e[3
 // Demagnetising field of particle i (sorted slot r) in SI: the real- and
 // k-space sums and the self and surface terms combined in FP64, then
 // returned in the integrator's type T.
-// sbs: the strong-pair field sums of slot r when the caller has them already.
+// sbs: the strong-pair field sums of slot r when the caller has looked them
+// up already (has: there are any).
 template <typename T, typename R = T>
-__device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], const double* sbs = nullptr) {
+__device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], const double* sbs = nullptr,
+                                         bool has = false) {
   using T4 = typename V4<T>::t;
   const int n = p.n;
   const T* Br = (const T*)p.Br;
@@ -88,7 +105,7 @@ __device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], cons
     sb[0] = sbs[0];
     sb[1] = sbs[1];
     sb[2] = sbs[2];
-    hs = true;
+    hs = has;
   } else {
     hs = p.sv.sum3(p.sv.B, r, sb);
   }
@@ -98,7 +115,7 @@ __device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], cons
     // at ~1/64 of the FP32 rate on GB300; the self term that cancels the
     // k-space self field is small against the pair fields, so the FP32 sum
     // loses nothing measurable)
-    const float cs = (float)p.cself, cu = (float)p.csurf, bu = (float)p.B_unit;
+    const float cs = p.f.cself, cu = p.f.csurf, bu = p.f.B_unit;
     const float mu3[3] = {(float)mu.x, (float)mu.y, (float)mu.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -133,44 +150,105 @@ __device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], cons
   }
 }
 
+// Thermal torque, field and force of the step: unit normals (drawn, uploaded
+// or zero) times the particle's scales, into th.  Independent of the fields,
+// so the launch runs beside their evaluation.
+// Thread = one Box-Muller pair (j of five) of one particle.
 template <typename T>
+__global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
+  const int i = blockIdx.x * kIntOne + threadIdx.x, j = blockIdx.y, n = p.n;
+  if (i >= n) return;
+  T z[2] = {0, 0};
+  if (p.noise == 2) {
+    philox_pair<T>(p.seed, (uint64_t)*p.stepno, (uint32_t)i, j, z);
+  } else if (p.noise == 1) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int q = 2 * j + h;
+      if (q < 9) z[h] = (T)p.xi[q * n + i];
+    }
+  }
+  using T4 = typename V4<T>::t;
+  const T4 c = ((const T4*)p.cA)[i];
+  T* th = (T*)p.th;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int q = 2 * j + h;
+    if (q < 9) th[q * n + i] = (q < 3 ? c.x : (q < 6 ? c.y : c.z)) * z[h];
+  }
+}
+
+// Per-particle constants of the integrator in T for the step dt: ct, cb, cf
+// are the DefThermFluct prefactors under the square roots (0: switched off).
+template <typename T>
+__global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf,
+                                                            const double* __restrict__ zr, const double* __restrict__ zt,
+                                                            const double* __restrict__ ivol,
+                                                            const double* __restrict__ izt,
+                                                            const double* __restrict__ v1, const double* __restrict__ v2,
+                                                            const double* __restrict__ mu, const double* __restrict__ rm,
+                                                            void* cA, void* cB) {
+  using T4 = typename V4<T>::t;
+  const int i = blockIdx.x * kIntThreads + threadIdx.x;
+  if (i >= n) return;
+  T4 a, b;
+  a.x = (T)sqrt(ct * zr[i]);
+  a.y = (T)sqrt(cb * ivol[i]);
+  a.z = (T)sqrt(cf * zt[i]);
+  a.w = (T)izt[i];
+  b.x = (T)v1[i];
+  b.y = (T)v2[i];
+  b.z = (T)mu[i];
+  b.w = (T)rm[i];
+  ((T4*)cA)[i] = a;
+  ((T4*)cB)[i] = b;
+}
+
+// DRAW: the noise is drawn here (packed batches) and not by k_noise.
+template <typename T, bool DRAW>
 __device__ __forceinline__ void heun1(const IntParams& p, int bx) {
   using T4 = typename V4<T>::t;
   const int i = bx * (int)blockDim.x + threadIdx.x;
   const int n = p.n;
   if (i >= n) return;
   const int r = p.s.rank[i];
-  T m[3], e[3], bd[3], z[9];
+  const T4 cb = ((const T4*)p.cB)[i];
+  T m[3], e[3], bd[3], tau[3], bth[3];
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     m[a] = (T)p.mm[a * n + i];
     e[a] = (T)p.ea[a * n + i];
   }
-  demag_si<T>(p, r, bd);
-  if (p.noise == 2) {
-    philox_normals9<T>(p.seed, (uint64_t)*p.stepno, (uint32_t)i, z);
-  } else if (p.noise == 1) {
+  if constexpr (DRAW) {
+    const T4 ca = ((const T4*)p.cA)[i];
+    T z[9];
+    if (p.noise == 2) {
+      philox_normals9<T>(p.seed, (uint64_t)*p.stepno, (uint32_t)i, z);
+    } else {
 #pragma unroll
-    for (int q = 0; q < 9; q++) z[q] = (T)p.xi[(q / 3) * 3 * n + (q % 3) * n + i];
+      for (int q = 0; q < 9; q++) z[q] = 0;
+    }
+    T* th = (T*)p.th;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      tau[a] = ca.x * z[a];
+      bth[a] = ca.y * z[3 + a];
+      th[a * n + i] = tau[a];
+      th[(3 + a) * n + i] = bth[a];
+      th[(6 + a) * n + i] = ca.z * z[6 + a];
+    }
   } else {
 #pragma unroll
-    for (int q = 0; q < 9; q++) z[q] = 0;
+    for (int a = 0; a < 3; a++) {
+      tau[a] = ((const T*)p.th)[a * n + i];
+      bth[a] = ((const T*)p.th)[(3 + a) * n + i];
+    }
   }
-  const T sT = (T)p.sT[i], sB = (T)p.sB[i], sF = (T)p.sF[i];
-  T tau[3], bth[3];
-  T* th = (T*)p.th;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    tau[a] = sT * z[a];
-    bth[a] = sB * z[3 + a];
-    th[a * n + i] = tau[a];
-    th[(3 + a) * n + i] = bth[a];
-    th[(6 + a) * n + i] = sF * z[6 + a];
-  }
+  demag_si<T>(p, r, bd);
   const T bz = (T)ext_field_z(p, *p.time);
   T km[3], ke[3];
-  rk<T>(p, m, e, bd, bz, bth, tau, (T)p.velEa1[i], (T)p.velEa2[i], km, ke);
-  const T dt = (T)p.dt;
+  rk<T>(p, m, e, bd, bz, bth, tau, cb.x, cb.y, km, ke);
+  const T dt = scalar<T>(p.dt, p.f.dt);
   T* k1m = (T*)p.k1m;
   T* k1e = (T*)p.k1e;
   T* m2 = (T*)p.m2;
@@ -184,12 +262,11 @@ __device__ __forceinline__ void heun1(const IntParams& p, int bx) {
     mm2[a] = m[a] + dt * km[a];
     m2[a * n + i] = mm2[a];
   }
-  const T mu = (T)p.magMom_u[i];
   T4 v;
-  v.x = mm2[0] * mu;
-  v.y = mm2[1] * mu;
-  v.z = mm2[2] * mu;
-  v.w = (T)p.rMag_u[i];
+  v.x = mm2[0] * cb.z;
+  v.y = mm2[1] * cb.z;
+  v.z = mm2[2] * cb.z;
+  v.w = cb.w;
   ((T4*)p.s.mu)[r] = v;
 }
 
@@ -206,11 +283,11 @@ __device__ __forceinline__ void heun1(const IntParams& p, int bx) {
 // round(.../L) of the reference; the displacement since the list build only
 // feeds the rebuild test and is FP32.
 // sfp: the strong-pair force and pressure sums of slot r (6 values) when the
-// caller has them already.
+// caller has looked them up already (has: there are any).
 template <typename T>
 __device__ __forceinline__ void finish_particle(const IntParams& p, int i, int r, const T mn[3], const T en[3],
-                                                const T fth[3], double acc[7], float& disp2,
-                                                const double* sfp = nullptr) {
+                                                const T fth[3], T izt, double acc[7], float& disp2,
+                                                const double* sfp = nullptr, bool has = false) {
   const int n = p.n;
   acc[4] = p.Ppart[3 * i];
   acc[5] = p.Ppart[3 * i + 1];
@@ -223,82 +300,93 @@ __device__ __forceinline__ void finish_particle(const IntParams& p, int i, int r
       sf[q] = sfp[q];
       sp[q] = sfp[3 + q];
     }
-    hs = true;
+    hs = has;
   } else {
     hs = p.sv.sums(r, p.sv.F, sf, nullptr, nullptr, p.sv.P, sp);
   }
-  acc[4] += sp[0];
-  acc[5] += sp[1];
-  acc[6] += sp[2];
+  if (hs) {
+    acc[4] += sp[0];
+    acc[5] += sp[1];
+    acc[6] += sp[2];
+  }
   const T nm = sqrt(mn[0] * mn[0] + mn[1] * mn[1] + mn[2] * mn[2]);
   const T ne = sqrt(en[0] * en[0] + en[1] * en[1] + en[2] * en[2]);
   const T* Fr = (const T*)p.Fr;
   const T* Fk = (const T*)p.Fk;
   const T* ov = (const T*)p.ov;
   const double L = p.L, half = 0.5 * L, dtd = p.dt;
-  const float Lf = (float)L, iLf = 1.0f / Lf;
-  const T izt = (T)p.invZt[i];
+  const int half_hi = __double2hiint(half) - 1;  // |x| below this in the high word: inside the box
+  const float Lf = p.f.L, iLf = p.f.iL;
+  const T fu = scalar<T>(p.F_unit, p.f.F_unit);
   bool bad = false;
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     const T mf = mn[a] / nm, ef = en[a] / ne;
-    p.mm[a * n + i] = (double)mf;
-    p.ea[a * n + i] = (double)ef;
-    T f;
     const T fr = hs ? Fr[a * n + r] + (T)sf[a] : Fr[a * n + r];
-    if constexpr (std::is_same<T, float>::value)
-      f = (fr + Fk[a * n + r]) * (float)p.F_unit + fth[a];
-    else
-      f = (fr + Fk[a * n + r]) * p.F_unit + fth[a];
-    double x = p.pos[a * n + i] + (double)ov[a * n + r] * L + dtd * (double)(f * izt);
-    if (x > half) x -= L;
-    if (x < -half) x += L;
+    const T f = (fr + Fk[a * n + r]) * fu + fth[a], o = ov[a * n + r];
+    double x = p.pos[a * n + i];
+    if (o != (T)0) x += (double)o * L;
+    if constexpr (std::is_same<T, float>::value) {
+      p.mm[a * n + i] = widen(mf);
+      p.ea[a * n + i] = widen(ef);
+      x += dtd * widen(f * izt);
+      bad |= !isfinite(mf) || !isfinite(ef);
+    } else {
+      p.mm[a * n + i] = mf;
+      p.ea[a * n + i] = ef;
+      x += dtd * (f * izt);
+      bad |= !isfinite(mf) || !isfinite(ef);
+    }
+    if ((__double2hiint(x) & 0x7fffffff) >= half_hi) {
+      bad |= !isfinite(x);
+      if (x > half) x -= L;
+      if (x < -half) x += L;
+    }
     p.pos[a * n + i] = x;
     if (p.xbuild) {
-      float db = (float)(x - p.xbuild[a * n + i]);
+      float db = narrow(x - p.xbuild[a * n + i]);
       db -= Lf * rintf(db * iLf);
       disp2 += db * db;
     }
     double tp = p.truePos[a * n + i];
-    const float wraps = rintf((float)(tp - x) * iLf);
-    tp = x + (double)wraps * L;
+    const float wraps = rintf(narrow(tp - x) * iLf);
+    tp = wraps != 0.f ? x + (double)wraps * L : x;
     p.truePos[a * n + i] = tp;
     const double d = tp - p.posRef[a * n + i];
     acc[a] = d * d;
-    bad |= !isfinite(x) || !isfinite((double)mf) || !isfinite((double)ef);
+    if (a == 2) acc[3] = (double)mf;
   }
-  acc[3] = p.mm[2 * n + i];
   if (bad) atomicOr(p.err, kErrNonFinite);
 }
 
 // Block sums of the step records and the largest displacement since the
 // last list build (every thread of the block calls this; blocks of up to
-// kIntThreads threads).  The seven sums go through shared memory: a warp
-// adds a record's column of values with one FP64 addition per warp of the
-// block and five butterfly steps per lane (a butterfly per record and warp
-// would take 7 x 5 per warp).
+// kIntThreads threads): per warp the seven sums by halving butterflies, then
+// one thread per record over the warps (12 dependent FP64 additions in a
+// 128-thread block).
 __device__ __forceinline__ void step_block_sums(const IntParams& p, int bx, const double acc[7], float disp2) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
   if (p.flags) {
-    float d = sqrtf(disp2) * (1.0f / (float)p.L);
+    float d = sqrtf(disp2) * p.f.iL;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d = fmaxf(d, __shfl_xor_sync(kFull, d, o));
-    if ((threadIdx.x & 31) == 0 && d > 0.f) atomicMax(&p.flags->maxdisp, __float_as_uint(d));
+    if (lane == 0 && d > 0.f) atomicMax(&p.flags->maxdisp, __float_as_uint(d));
   }
-  __shared__ double red[7][kIntThreads];
-#pragma unroll
-  for (int q = 0; q < 7; q++) red[q][threadIdx.x] = acc[q];
+  __shared__ double red[kIntThreads / 32][8];
+  double v[8] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], 0.0};
+  const double s = warp_sums<8>(v, lane);
+  if ((lane & 3) == 0) red[w][lane >> 2] = s;
   __syncthreads();
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (int)blockDim.x >> 5;
-  for (int q = w; q < 7; q += nw) {
-    double s = red[q][l];
-    for (int k = 1; k < nw; k++) s += red[q][l + 32 * k];
-    s = warp_sum(s);
-    if (l == 0) p.obs_part[7 * bx + q] = s;
+  if (threadIdx.x < 7) {
+    double t = red[0][threadIdx.x];
+    for (int k = 1; k < nw; k++) t += red[k][threadIdx.x];
+    p.obs_part[7 * bx + threadIdx.x] = t;
   }
 }
 
 template <typename T>
 __device__ __forceinline__ void heun2(const IntParams& p, int bx) {
+  using T4 = typename V4<T>::t;
   const int i = bx * (int)blockDim.x + threadIdx.x;
   const int n = p.n;
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -306,6 +394,8 @@ __device__ __forceinline__ void heun2(const IntParams& p, int bx) {
   if (i < n) {
     const int r = p.s.rank[i];
     const T* th = (const T*)p.th;
+    const T4 cb = ((const T4*)p.cB)[i];
+    const T izt = ((const T4*)p.cA)[i].w;
     T m[3], e[3], m2[3], e2[3], bd[3], tau[3], bth[3], k1m[3], k1e[3], fth[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -323,60 +413,55 @@ __device__ __forceinline__ void heun2(const IntParams& p, int bx) {
     // force and pressure of the step's full evaluation, in one pass
     double sb[3], sfp[6];
     const bool hs = p.sv.sums(r, p.sv.B, sb, p.sv.F, sfp, p.sv.P, sfp + 3);
-    demag_si<T>(p, r, bd, hs ? sb : nullptr);
+    demag_si<T>(p, r, bd, sb, hs);
     const T bz = (T)ext_field_z(p, *p.time);
     T km[3], ke[3];
-    rk<T>(p, m2, e2, bd, bz, bth, tau, (T)p.velEa1[i], (T)p.velEa2[i], km, ke);
-    const T dt = (T)p.dt, h = (T)0.5;
+    rk<T>(p, m2, e2, bd, bz, bth, tau, cb.x, cb.y, km, ke);
+    const T dt = scalar<T>(p.dt, p.f.dt), h = (T)0.5;
     T mn[3], en[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       en[a] = e[a] + dt * (h * k1e[a] + h * ke[a]);
       mn[a] = m[a] + dt * (h * k1m[a] + h * km[a]);
     }
-    finish_particle<T>(p, i, r, mn, en, fth, acc, disp2, hs ? sfp : nullptr);
+    finish_particle<T>(p, i, r, mn, en, fth, izt, acc, disp2, sfp, hs);
   }
   step_block_sums(p, bx, acc, disp2);
 }
 
+// Step records from the blocks' partials: thread = (record t & 7, every
+// (blockDim / 8)-th block), added in a fixed order; then the clock.
 __device__ __forceinline__ void obs(const ObsParams& p) {
-  __shared__ double red[7][8];
-  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < p.nblk_int; b += blockDim.x)
-    for (int q = 0; q < 7; q++) acc[q] += __ldcg(p.obs_part + 7 * b + q);
-  for (int q = 0; q < 7; q++) {
-    const double v = warp_sum(acc[q]);
-    if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = v;
-  }
+  __shared__ double red[kIntThreads / 32][8];
+  const int q = threadIdx.x & 7, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  double s = 0.0;
+  if (q < 7)
+    for (int b = threadIdx.x >> 3; b < p.nblk_int; b += (int)blockDim.x >> 3) s += __ldcg(p.obs_part + 7 * b + q);
+  s += __shfl_xor_sync(kFull, s, 8);
+  s += __shfl_xor_sync(kFull, s, 16);
+  if (lane < 8) red[w][lane] = s;
+  const long long k = *p.nrec;
+  const double time = *p.time;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s[7];
-    for (int q = 0; q < 7; q++) {
-      s[q] = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) s[q] += red[q][w];
-    }
-    const long long k = *p.nrec;
+  if (threadIdx.x < 8) {
     if (k < p.cap) {
-      double* o = p.records + 8 * k;
-      o[0] = *p.time;
-      o[1] = s[3] * p.inv_n;
-      o[2] = s[0] * p.inv_n;
-      o[3] = s[1] * p.inv_n;
-      o[4] = s[2] * p.inv_n;
-      o[5] = s[4] * p.p_scale;
-      o[6] = s[5] * p.p_scale;
-      o[7] = s[6] * p.p_scale;
-      *p.nrec = k + 1;
+      for (int g = 1; g < nw; g++) s += red[g][q];
+      // record: t, m_z, MSD x, y, z, P xy, xz, yz (q = MSD x, y, z, m_z, P .., 7: t)
+      const int at = q < 3 ? q + 2 : (q == 3 ? 1 : (q < 7 ? q + 1 : 0));
+      p.records[8 * k + at] = q == 7 ? time : s * (q < 4 ? p.inv_n : p.p_scale);
     }
-    *p.time += p.dt;
-    *p.stepno += 1;
-    if (p.status) *p.status = *p.err | (p.flags->overflow ? 4 : 0);
+    if (threadIdx.x == 0) {
+      if (k < p.cap) *p.nrec = k + 1;
+      *p.time = time + p.dt;
+      *p.stepno += 1;
+      if (p.status) *p.status = *p.err | (p.flags->overflow ? 4 : 0);
+    }
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kIntThreads) k_heun1(IntParams p) {
-  heun1<T>(p, blockIdx.x);
+  heun1<T, false>(p, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_obs(ObsParams p) { obs(p); }
 
@@ -403,7 +488,7 @@ __global__ void __launch_bounds__(kIntOne) k_heun2_obs(IntParams p, ObsParams o,
 __global__ void __launch_bounds__(kIntThreads, 4) k_heun1_packed(const IntParams* __restrict__ ps,
                                                              const Task* __restrict__ tk, int ntask, WorkQ* wq) {
   for_tasks<false>(tk, ntask, wq, [&](const Task& t) {
-      heun1<float>(ps[t.rep], t.blk);
+      heun1<float, true>(ps[t.rep], t.blk);
   });
 }
 __global__ void __launch_bounds__(kIntThreads, 4) k_heun2_packed(const IntParams* __restrict__ ps,
@@ -477,20 +562,6 @@ int launch_real_part(cudaStream_t st, const IntParams& p, double* Bout, double* 
 // (AdjustTimeStep) and launches the accept kernel with the step used.
 
 template <typename T>
-__device__ __forceinline__ void noise9(const IntParams& p, int i, T z[9]) {
-  const int n = p.n;
-  if (p.noise == 2) {
-    philox_normals9<T>(p.seed, (uint64_t)*p.stepno, (uint32_t)i, z);
-  } else if (p.noise == 1) {
-#pragma unroll
-    for (int q = 0; q < 9; q++) z[q] = (T)p.xi[(q / 3) * 3 * n + (q % 3) * n + i];
-  } else {
-#pragma unroll
-    for (int q = 0; q < 9; q++) z[q] = 0;
-  }
-}
-
-template <typename T>
 __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
   using T4 = typename V4<T>::t;
   const IntParams& p = q.p;
@@ -499,23 +570,23 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
   double err = 0.0;
   if (i < n) {
     const int r = p.s.rank[i];
-    T m[3], e[3], bd[3], z[9], tau[3], bth[3];
+    const T4 cb = ((const T4*)p.cB)[i];
+    T m[3], e[3], bd[3], tau[3], bth[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       m[a] = q.s == 0 ? (T)p.mm[a * n + i] : ((const T*)q.cm)[a * n + i];
       e[a] = q.s == 0 ? (T)p.ea[a * n + i] : ((const T*)q.ce)[a * n + i];
     }
     demag_si<T>(p, r, bd);
-    noise9<T>(p, i, z);
-    const T sT = (T)(p.sT[i] * q.nf), sB = (T)(p.sB[i] * q.nf);
+    const T nf = (T)q.nf;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      tau[a] = sT * z[a];
-      bth[a] = sB * z[3 + a];
+      tau[a] = nf * ((const T*)p.th)[a * n + i];
+      bth[a] = nf * ((const T*)p.th)[(3 + a) * n + i];
     }
     const T bz = (T)ext_field_z(p, *p.time);
     T km[3], ke[3];
-    rk<T>(p, m, e, bd, bz, bth, tau, (T)p.velEa1[i], (T)p.velEa2[i], km, ke);
+    rk<T>(p, m, e, bd, bz, bth, tau, cb.x, cb.y, km, ke);
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       ((T*)q.km[q.s])[a * n + i] = km[a];
@@ -539,12 +610,11 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
         nm[a] = (T)(p.mm[a * n + i] + p.dt * sm);
         ((T*)q.cm)[a * n + i] = nm[a];
       }
-      const T mu = (T)p.magMom_u[i];
       T4 v;
-      v.x = nm[0] * mu;
-      v.y = nm[1] * mu;
-      v.z = nm[2] * mu;
-      v.w = (T)p.rMag_u[i];
+      v.x = nm[0] * cb.z;
+      v.y = nm[1] * cb.z;
+      v.z = nm[2] * cb.z;
+      v.w = cb.w;
       ((T4*)p.s.mu)[r] = v;
     } else {
       double ev[3];
@@ -579,7 +649,7 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_accept(RKStage q) {
   float disp2 = 0;
   if (i < n) {
     const int r = p.s.rank[i];
-    T mn[3], en[3], z[9], fth[3];
+    T mn[3], en[3], fth[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       if (q.last) {  // Bogacki-Shampine: the last stage's coordinates
@@ -598,11 +668,9 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_accept(RKStage q) {
     }
     // the thermal force at the scale of the step's first trial (the
     // reference rescales it on rejections only after it entered the force)
-    noise9<T>(p, i, z);
-    const T sF = (T)p.sF[i];
 #pragma unroll
-    for (int a = 0; a < 3; a++) fth[a] = sF * z[6 + a];
-    finish_particle<T>(p, i, r, mn, en, fth, acc, disp2);
+    for (int a = 0; a < 3; a++) fth[a] = ((const T*)p.th)[(6 + a) * n + i];
+    finish_particle<T>(p, i, r, mn, en, fth, ((const typename V4<T>::t*)p.cA)[i].w, acc, disp2);
   }
   step_block_sums(p, blockIdx.x, acc, disp2);
 }
@@ -627,6 +695,26 @@ int launch_rk_accept(cudaStream_t st, const RKStage& q, bool fp64) {
 
 int int_blocks(int n) { return (n + kIntThreads - 1) / kIntThreads; }
 int int_blocks_one(int n) { return (n + kIntOne - 1) / kIntOne; }
+
+int launch_noise(cudaStream_t st, const IntParams& p, bool fp64) {
+  const dim3 g(int_blocks_one(p.n), 5);
+  if (fp64)
+    k_noise<double><<<g, kIntOne, 0, st>>>(p);
+  else
+    k_noise<float><<<g, kIntOne, 0, st>>>(p);
+  return 1;
+}
+
+int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, const double* zr, const double* zt,
+                      const double* ivol, const double* izt, const double* v1, const double* v2, const double* mu,
+                      const double* rm, void* cA, void* cB, bool fp64) {
+  const int g = int_blocks(n);
+  if (fp64)
+    k_int_consts<double><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+  else
+    k_int_consts<float><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+  return 1;
+}
 
 int launch_heun1(cudaStream_t st, const IntParams& p, bool fp64) {
   if (fp64)

@@ -183,17 +183,6 @@ __device__ __forceinline__ void pair_terms(const RealParams& p, float dx, float 
 // 78 FP64 instructions per pair (field, force and pressure), 50 for the field
 // alone, against ~230 / ~170 with the library's erfc, exp and rsqrt.
 
-// FP64 <-> FP32 in integer operations: widening is exact for normal numbers,
-// narrowing truncates (both arguments are normal, positive here).
-__device__ __forceinline__ double widen(float v) {
-  const unsigned b = __float_as_uint(v);
-  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + (896u << 20) | (b & 0x80000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ float narrow(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  return __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
-}
-
 // Minimum-image difference b - a of box coordinates, with the reference's
 // fold (d > 1/2 -> d - 1, d < -1/2 -> d + 1); af, bf: their float copies.
 __device__ __forceinline__ double fold64(double a, double b, float af, float bf) {
@@ -313,26 +302,6 @@ __device__ __forceinline__ void pair64(const RealParams& p, const double4_32a& d
     a.p1 = fma(dx, vz, a.p1);
     a.p2 = fma(dy, vz, a.p2);
   }
-}
-
-// Sums of W values (a power of two) over the warp with W - 1 + log2(32 / W)
-// FP64 additions per lane instead of 5 W: each butterfly step halves the
-// values a lane carries.  Returns the sum of value (lane / (32 / W)).
-template <int W>
-__device__ __forceinline__ double warp_sums(double (&v)[W], int lane) {
-  int o = 16;
-#pragma unroll
-  for (int h = W / 2; h >= 1; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int q = 0; q < h; q++) {
-      const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
-      v[q] = keep + __shfl_xor_sync(kFull, give, o);
-    }
-  }
-  double s = v[0];
-  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-  return s;
 }
 
 // ------------------------------------------------- packed pair terms (FP32)

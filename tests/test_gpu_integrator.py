@@ -1,0 +1,48 @@
+"""Edges of the integrator kernels and of the fixed-point coordinates."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import TOL_MIXED, gpu_system, oracle_system, random_system, scales
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("boxes", [1, 3000, 1 << 18])
+def test_positions_outside_the_box(boxes):
+    """Positions some boxes away are the same periodic system (the fold of the
+    fixed-point coordinates, below and above its fast range).  Adding 2^18
+    boxes moves a position by <= 2^18 2^-53 box lengths, ~1e-9 of a pair
+    distance: far below the mixed path's budget."""
+    ini, g = random_system(33, seed=8, rc_frac=0.4)
+    fAl, bAl, _ = scales(ini, g)
+    B0, F0, _ = gpu_system(ini, g, 1).CompInteractions()
+    k = np.random.default_rng(1).choice([-boxes, 0, boxes], size=g["pos"].shape)
+    g["pos"] = np.ascontiguousarray(g["pos"] + k * g["lBox"])
+    B, F, _ = gpu_system(ini, g, 1).CompInteractions()
+    assert O.rms_rel(B, B0, bAl) < TOL_MIXED and O.rms_rel(F, F0, fAl) < TOL_MIXED
+
+
+@pytest.mark.parametrize("n", [2, 31, 128, 129, 300])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_records_and_state_at_block_edges(n, precision):
+    """State, m_z and MSD of drawn-noise steps for particle counts around the
+    warps and blocks of the step kernels, against the oracle's Philox steps
+    (mixed: increments of ~1e-2 in FP32, 3 steps)."""
+    ini, g = random_system(n, seed=n, rc_frac=0.4, noise=True)
+    sim = gpu_system(ini, g, precision, noise=2, seed=77)
+    orc = oracle_system(ini, g)
+    sim.step(3, g["dt"])
+    for _ in range(3):
+        orc.step(g["dt"], 2, seed=77)
+    p, m, e = sim.get_state()
+    po, mo, eo, _ = orc.get_state()
+    tol = 1e-10 if precision == 0 else 2e-6
+    assert np.abs(m - mo).max() < tol and np.abs(e - eo).max() < tol
+    assert np.abs(p - po).max() < (1e-13 if precision == 0 else 1e-9) * g["lBox"]
+    r = sim.records()
+    d = po - g["pos"]
+    d -= g["lBox"] * np.round(d / g["lBox"])
+    np.testing.assert_allclose(r[-1, 1], mo[2].mean(), rtol=0, atol=tol)
+    np.testing.assert_allclose(r[-1, 2:5], (d * d).mean(axis=1), rtol=1e-10 if precision == 0 else 1e-4)
+    assert r.shape == (3, 8) and np.allclose(r[:, 0], np.arange(3) * g["dt"])
