@@ -198,7 +198,10 @@ int md_set_ewald(md_ctx* ctx, double alpha, double rc, int64_t kc);
  * tensor-core kernels' shared memory (kc <= 25).  Applies to the current
  * and later Ewald parameters. */
 int md_set_kspace_engine(md_ctx* ctx, int engine);
-/* *tensor_cores = 1 when the current Ewald parameters use the tensor cores. */
+/* *tensor_cores = 1 when the current Ewald parameters are those of the tensor
+ * cores.  With MD_KSPACE_AUTO and the default tiling, systems too small to
+ * fill them (about 3e6 k vectors x particles) evaluate the same k rows on the
+ * CUDA cores under that setting; MD_KSPACE_TC always takes the tensor cores. */
 int md_kspace_engine_active(const md_ctx* ctx, int* tensor_cores);
 /* Tiling of the tensor-core structure factor (no counterpart in the
  * reference; the autotuner's knobs): ring = the operand-ring option (0..5,

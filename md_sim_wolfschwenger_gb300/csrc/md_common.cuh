@@ -290,15 +290,15 @@ struct KParams {
   int tc_scat_smem;      // dynamic shared memory of the scatter launch
   int tc_yz;             // the scatter stages the Y, Z phases in shared memory
   int tc_sfa, tc_sfb;    // structure-factor ring slots (generated, copied)
-  // FP64 path (md_kspace64.cu): tasks of four |nx| of one row
-  int k64_T, k64_R;          // tasks, rows
-  int k64_nblk, k64_threads; // structure factor: task blocks, threads per block
-  int k64_chunk, k64_nchunk; // particles per chunk, chunks
-  const int4* k64_task;      // [T] row, ny, nz, first |nx|
-  const int* k64_kidx;       // [T][4][+, -] sorted k index, or -1
-  const double2* k64_row;    // [R] (ny, nz)
-  const int2* k64_rowt;      // [R] first task, tasks
-  double2* k64_ad;           // [T][4][A, D]
+  // k space by rows (md_krows.cu; rw_T = 0: off): tasks of four |nx| of one row
+  int rw_T, rw_R;          // tasks, rows
+  int rw_nblk, rw_threads; // structure factor: task blocks, threads per block
+  int rw_chunk, rw_nchunk; // particles per chunk, chunks
+  const int4* rw_task;      // [T] row, ny, nz, first |nx|
+  const int* rw_kidx;       // [T][4][+, -] sorted k index, or -1
+  const double2* rw_row;    // [R] (ny, nz)
+  const int2* rw_rowt;      // [R] first task, tasks
+  void* rw_ad;              // [T][4] T4 (A, D)
   long long tc_wait;     // SM clock cycles after which an mbarrier wait gives up
   int* err;              // device error word (kErrTcWait on a wait that gave up)
 };

@@ -271,17 +271,17 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.tc_yz = c->tcs.yz;
   p.tc_sfa = c->tcs.sfa;
   p.tc_sfb = c->tcs.sfb;
-  p.k64_T = c->k64_T;
-  p.k64_R = c->k64_R;
-  p.k64_nblk = c->k64s.nblk;
-  p.k64_threads = c->k64s.threads;
-  p.k64_chunk = c->k64s.chunk;
-  p.k64_nchunk = c->k64s.nchunk;
-  p.k64_task = c->k64_task;
-  p.k64_kidx = c->k64_kidx;
-  p.k64_row = c->k64_row;
-  p.k64_rowt = c->k64_rowt;
-  p.k64_ad = c->k64_ad;
+  p.rw_T = c->rw_T;
+  p.rw_R = c->rw_R;
+  p.rw_nblk = c->rws.nblk;
+  p.rw_threads = c->rws.threads;
+  p.rw_chunk = c->rws.chunk;
+  p.rw_nchunk = c->rws.nchunk;
+  p.rw_task = c->rw_task;
+  p.rw_kidx = c->rw_kidx;
+  p.rw_row = c->rw_row;
+  p.rw_rowt = c->rw_rowt;
+  p.rw_ad = c->rw_ad;
   p.tc_wait = c->tc_wait;
   p.err = &c->sc->err;
   return p;
@@ -659,9 +659,25 @@ static int setup_tc(md_ctx* c) {
   return MD_OK;
 }
 
-// FP64 k space: tasks of four consecutive |nx| of one k row, rows by nz then
-// ny, and the buffers of the launches (md_kspace64.cu).
-static int setup_k64(md_ctx* c) {
+// Whether the mixed path's default engine takes the row kernels (md_krows.cu)
+// instead of the tensor cores: systems of up to 3e6 (k, particle) terms, whose
+// tensor-core launches are mostly set-up.  Measured step times, rows against
+// tensor cores: N = 512, kc = 7 (0.4e6 terms) 66 / 84 us, N = 1000, kc = 7 (0.7e6)
+// 80 / 86, N = 2048, kc = 8 (2.2e6) 90 / 94; N = 4096, kc = 9 (6.3e6) 120 / 105,
+// N = 3001, kc = 11 (8.4e6) 130 / 119.  An engine or a tensor-core tiling that
+// the caller chose is kept.
+static bool krows_wanted(const md_ctx* c) {
+  const double nk = 2.0943951 * (double)c->kc * (double)c->kc * (double)c->kc;  // half space
+  return c->kengine == MD_KSPACE_AUTO && c->tc_ring < 0 && c->tc_waves == 1 && md::kspace_tc_supported((int)c->kc) &&
+         nk * (double)c->n <= 3e6;
+}
+
+// k space by rows: tasks of four consecutive |nx| of one k row, rows by nz
+// then ny, and the buffers of the launches (md_krows.cu).  Always on the FP64
+// path, on the mixed path for the systems of krows_wanted.
+static int setup_rows(md_ctx* c) {
+  c->rw_T = c->rw_R = 0;
+  if (!fp64(c) && !krows_wanted(c)) return MD_OK;
   const int kc = (int)c->kc, nk = c->klist.nk;
   std::map<std::pair<int, int>, std::vector<std::pair<int, int>>> byrow;  // (nz, ny) -> (nx, k)
   for (int k = 0; k < nk; k++)
@@ -687,22 +703,21 @@ static int setup_k64(md_ctx* c) {
   const int T = (int)task.size(), R = (int)row.size();
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const md::K64Shape sh = md::kspace64_shape(kc, (int)c->n, T, nsm);
-  void* old[] = {c->k64_task, c->k64_kidx, c->k64_row, c->k64_rowt, c->k64_ad};
+  const md::RowShape sh = md::krows_shape(kc, (int)c->n, T, nsm, fp64(c));
+  void* old[] = {c->rw_task, c->rw_kidx, c->rw_row, c->rw_rowt, c->rw_ad};
   for (void* q : old) dfree(c, q);
-  c->k64_task = nullptr;
-  c->k64_kidx = nullptr;
-  c->k64_row = nullptr;
-  c->k64_rowt = nullptr;
-  c->k64_ad = nullptr;
-  c->k64_T = 0;
+  c->rw_task = nullptr;
+  c->rw_kidx = nullptr;
+  c->rw_row = nullptr;
+  c->rw_rowt = nullptr;
+  c->rw_ad = nullptr;
   int st;
-  if ((st = dalloc(c, &c->k64_task, sizeof(int4) * (size_t)T))) return st;
-  if ((st = dalloc(c, &c->k64_kidx, sizeof(int) * kidx.size()))) return st;
-  if ((st = dalloc(c, &c->k64_row, sizeof(double2) * (size_t)R))) return st;
-  if ((st = dalloc(c, &c->k64_rowt, sizeof(int2) * (size_t)R))) return st;
-  if ((st = dalloc(c, &c->k64_ad, 8 * sizeof(double2) * (size_t)T))) return st;
-  const size_t sp = 8 * (size_t)T * (size_t)sh.nchunk;
+  if ((st = dalloc(c, &c->rw_task, sizeof(int4) * (size_t)T))) return st;
+  if ((st = dalloc(c, &c->rw_kidx, sizeof(int) * kidx.size()))) return st;
+  if ((st = dalloc(c, &c->rw_row, sizeof(double2) * (size_t)R))) return st;
+  if ((st = dalloc(c, &c->rw_rowt, sizeof(int2) * (size_t)R))) return st;
+  if ((st = dalloc(c, &c->rw_ad, 16 * tsz(c) * (size_t)T))) return st;
+  const size_t sp = tsz(c) * (size_t)T * (size_t)sh.nchunk;  // 16 T per task and chunk, in double2
   if (sp > c->spart_cap) {
     dfree(c, c->Spart);
     c->Spart = nullptr;
@@ -717,14 +732,20 @@ static int setup_k64(md_ctx* c) {
     if ((st = dalloc(c, &c->musum_part, 24 * (size_t)sh.nchunk))) return st;
     c->musum_cap = sh.nchunk;
   }
-  CK(c, cudaMemcpy(c->k64_task, task.data(), sizeof(int4) * (size_t)T, cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->k64_kidx, kidx.data(), sizeof(int) * kidx.size(), cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->k64_row, row.data(), sizeof(double2) * (size_t)R, cudaMemcpyHostToDevice));
-  CK(c, cudaMemcpy(c->k64_rowt, rowt.data(), sizeof(int2) * (size_t)R, cudaMemcpyHostToDevice));
-  c->k64s = sh;
-  c->k64_T = T;
-  c->k64_R = R;
+  CK(c, cudaMemcpy(c->rw_task, task.data(), sizeof(int4) * (size_t)T, cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->rw_kidx, kidx.data(), sizeof(int) * kidx.size(), cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->rw_row, row.data(), sizeof(double2) * (size_t)R, cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->rw_rowt, rowt.data(), sizeof(int2) * (size_t)R, cudaMemcpyHostToDevice));
+  c->rws = sh;
+  c->rw_T = T;
+  c->rw_R = R;
   return MD_OK;
+}
+
+// The k-space engine of the current parameters.
+static int setup_engine(md_ctx* c) {
+  const int st = setup_tc(c);
+  return st ? st : setup_rows(c);
 }
 
 extern "C" {
@@ -1200,10 +1221,8 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
     // the padding entries of the scatter layout are never written: zero
     CK(c, cudaMemset(c->eS, 0, 8 * nks));
     CK(c, cudaMemcpy(c->chunks, c->klist.chunks.data(), sizeof(int) * c->klist.chunks.size(), cudaMemcpyHostToDevice));
-  } else if (int st = setup_k64(c)) {
-    return st;
   }
-  if (int st = setup_tc(c)) return st;
+  if (int st = setup_engine(c)) return st;
   {
     // k-space self-interaction: B_i holds -cflux sum_k e(k) (n . mu_i) n of
     // each particle's own moment (the k list's e(k) covers the half space)
@@ -1248,8 +1267,7 @@ int md_set_kspace_engine(md_ctx* c, int engine) {
   c->kengine = engine;
   // the per-step operand images of a newly chosen engine come with the next full evaluation
   c->have_geometry = false;
-  if (c->have_ewald) return setup_tc(c);
-  return MD_OK;
+  return c->have_ewald ? setup_engine(c) : MD_OK;
 }
 
 int md_kspace_engine_active(const md_ctx* c, int* tensor_cores) {
@@ -1265,8 +1283,7 @@ int md_set_kspace_tiling(md_ctx* c, int ring, int waves) {
   c->tc_ring = ring;
   c->tc_waves = waves;
   c->have_geometry = false;  // the per-step operands come with the next full evaluation
-  if (c->have_ewald) return setup_tc(c);
-  return MD_OK;
+  return c->have_ewald ? setup_engine(c) : MD_OK;
 }
 
 int md_get_kspace_tiling(const md_ctx* c, int* ring, int* waves, int* chunk) {
@@ -2007,7 +2024,7 @@ int md_autotune_ewald(md_ctx* c, int ncand, double* alpha_out, double* rc_out, i
       c->kengine = cd.engine;
       c->tc_ring = cd.ring;
       c->tc_waves = cd.waves;
-      if (setup_tc(c) != MD_OK) continue;
+      if (setup_engine(c) != MD_OK) continue;
       invalidate_graph(c);
       const double ms = time_evaluations(c, e0, e1, flush, flush_bytes);
       if (q == 0) bms0 = ms;
@@ -2019,7 +2036,7 @@ int md_autotune_ewald(md_ctx* c, int ncand, double* alpha_out, double* rc_out, i
     c->kengine = bc.engine;
     c->tc_ring = bc.ring;
     c->tc_waves = bc.waves;
-    if ((st = setup_tc(c))) return done(st);
+    if ((st = setup_engine(c))) return done(st);
     invalidate_graph(c);
     c->have_geometry = false;
     if (bms < 1e300) best = std::min(best, bms);

@@ -117,14 +117,14 @@ struct md_ctx {
   size_t ptab_cap = 0;
   size_t ksize_cap = 0, spart_cap = 0;
   int musum_cap = 0;
-  // FP64 k space (md_kspace64.cu)
-  int k64_T = 0, k64_R = 0;
-  K64Shape k64s{};
-  int4* k64_task = nullptr;
-  int* k64_kidx = nullptr;
-  double2* k64_row = nullptr;
-  int2* k64_rowt = nullptr;
-  double2* k64_ad = nullptr;
+  // k space by rows (md_krows.cu; rw_T = 0 while it is off)
+  int rw_T = 0, rw_R = 0;
+  RowShape rws{};
+  int4* rw_task = nullptr;
+  int* rw_kidx = nullptr;
+  double2* rw_row = nullptr;
+  int2* rw_rowt = nullptr;
+  void* rw_ad = nullptr;
   // tensor-core k space (mixed path; md_ktc.cu): engine choice, k rows and
   // their buffers (tc_rows = 0 while the engine is off)
   int kengine = MD_KSPACE_AUTO;

@@ -118,14 +118,15 @@ int launch_kspace_tc_packed(cudaStream_t st, const KParams* ps, const Packed& sf
 // One warp waits on an mbarrier that gets an arrival only when `arrive` is
 // set; a wait that gives up after `limit` cycles sets kErrTcWait in *err.
 int launch_tc_wait_probe(cudaStream_t st, int* err, int arrive, long long limit);
-// FP64 k space (md_kspace64.cu): launch shape for kc, n particles and the
-// given number of tasks.
-struct K64Shape {
+// k space by rows on the CUDA cores (md_krows.cu): the FP64 path, and on the
+// mixed path the systems of krows_wanted; launch shape for kc, n particles and
+// the given number of tasks.
+struct RowShape {
   int nblk, threads, chunk, nchunk;
 };
-K64Shape kspace64_shape(int kc, int n, int tasks, int nsm);
-int launch_phase64(cudaStream_t st, const KParams& p);
-int launch_kspace64(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev);
+RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
+int launch_phase_rows(cudaStream_t st, const KParams& p, bool fp64);
+int launch_krows(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaEvent_t* ev);
 // Per-particle phase tables (once per step; positions are frozen across the
 // two Heun stages).
 int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64);

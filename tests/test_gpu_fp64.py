@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from helpers import TOL_FP64, gpu_system, oracle_system, random_system, scales
+from helpers import TOL_FP64, TOL_MIXED, gpu_system, oracle_system, random_system, scales
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +31,26 @@ def test_interactions_against_oracle(n, kc, rc_frac, alpha_rc):
     mm = rng.standard_normal((3, n))
     mm /= np.linalg.norm(mm, axis=0)
     assert O.rms_rel(sim.CompDemagField(mm), orc.compute_field(mm), bAl) < TOL_FP64
+
+
+@pytest.mark.parametrize("n,kc", [(2, 2), (9, 3), (33, 4), (130, 7), (257, 8), (513, 11), (100, 24), (2500, 5)])
+def test_small_mixed_systems_by_rows(n, kc):
+    """The default mixed engine takes the same k rows in FP32 for systems this
+    small: against the FP64 path and the tensor cores, with the tolerances the
+    engines are compared by elsewhere (FP32 rounding of the k-space sums)."""
+    ini, g = random_system(n, seed=7 * n + kc, rc_frac=0.4, lognormal=n % 2 == 1)
+    g["kc"] = kc
+    fAl, bAl, _ = scales(ini, g)
+    ref, rows, tc = (gpu_system(ini, g, p) for p in (0, 1, 1))
+    tc.set_kspace_engine("tc")
+    out = [s.CompInteractions()[:2] for s in (ref, rows, tc)]
+    for q, al in ((0, bAl), (1, fAl)):
+        assert O.rms_rel(out[1][q], out[0][q], al) < TOL_MIXED
+        assert O.rms_rel(out[1][q], out[2][q], al) < 5e-6
+    S0, S1 = ref.debug_structure_factor()[:, 3:], rows.debug_structure_factor()[:, 3:]
+    assert np.sqrt(np.mean((S1 - S0) ** 2) / np.mean(S0 ** 2)) < 1e-6
+    mm = g["mm"][:, ::-1].copy()
+    assert O.rms_rel(rows.CompDemagField(mm), ref.CompDemagField(mm), bAl) < TOL_MIXED
 
 
 @pytest.mark.parametrize("scale", [1.0, 0.35])
