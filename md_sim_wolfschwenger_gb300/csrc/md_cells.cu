@@ -35,22 +35,6 @@ __device__ __forceinline__ int cell_coord(double xb, int ncx) {
   return c < 0 ? 0 : (c >= ncx ? ncx - 1 : c);
 }
 
-// Box coordinate wrapped to [-0.5, 0.5).
-__device__ __forceinline__ double wrap_box(double x, double invL) {
-  double xb = x * invL;
-  return xb - floor(xb + 0.5);
-}
-
-// round(x_box 2^32) as a wrapping 32-bit integer (the fold by whole boxes drops
-// out mod 2^32): adding 1.5 2^52 leaves the rounded integer in the low word, two
-// FP64 instructions for |x| < 2^17 box lengths.
-__device__ __forceinline__ int fixed_box(double x, double invL) {
-  const double t = x * (invL * 4294967296.0);
-  if ((__double2hiint(t) & 0x7fffffff) < 0x43000000)  // |t| < 2^49
-    return __double2loint(t + 6755399441055744.0);
-  return (int)(unsigned)(long long)llrint(wrap_box(x, invL) * 4294967296.0);
-}
-
 __device__ __forceinline__ bool skip(const StepFlags* f) { return f && !f->rebuild; }
 
 // Start of a step: rebuild the cell order and the neighbour list if the host

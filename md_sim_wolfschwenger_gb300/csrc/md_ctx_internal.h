@@ -95,6 +95,9 @@ struct md_ctx {
   // stage outputs (T)
   void *Br = nullptr, *Fr = nullptr, *ov = nullptr, *Bk = nullptr, *Fk = nullptr, *Br2 = nullptr, *Bk2 = nullptr;
   void *k1m = nullptr, *k1e = nullptr, *m2 = nullptr, *e2 = nullptr, *th = nullptr;
+  // md_rdf's workspace (allocated on first use)
+  void* rdf_ws = nullptr;
+  size_t rdf_cap = 0;
   // adaptive solvers (allocated on first use): stage slopes and coordinates
   void *rk_km[7] = {}, *rk_ke[7] = {}, *rk_cm = nullptr, *rk_ce = nullptr;
   double *Ppart = nullptr, *obs_part = nullptr;

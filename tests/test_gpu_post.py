@@ -26,3 +26,27 @@ def test_rdf_matches_script(n, lognormal, include_last):
     mismatch = np.abs(gd - gr) > 1e-12 * gr.max()
     assert mismatch.sum() <= 2
     assert cnt.sum() > 0
+
+
+@pytest.mark.parametrize("n,phi,bins,range_mag,shift", [
+    (33, 0.02, 1, 9.0, 0), (257, 0.02, 7, 7.0, 0), (700, 0.02, 500, 8.0, 0), (2000, 0.05, 8192, 6.0, 0),
+    (2000, 0.05, 500, 8.0, 2), (600, 0.1, 64, 20.0, 0)])
+def test_rdf_routes(n, phi, bins, range_mag, shift):
+    """The cell route at block edges, one bin, the most bins (where many pairs
+    take the FP64 expression), particles some boxes outside (one wrap per
+    axis only), and a long range (all pairs): counts as the script's, up to
+    the pairs within rounding of a bin edge."""
+    ini, g = random_system(n, seed=n + bins, rc_frac=0.3, phi=phi)
+    pos = g["pos"].copy()
+    if shift:
+        pos[:, ::5] += shift * g["lBox"]
+        pos[0, 1::7] += 0.3 * g["lBox"]
+    g["pos"] = pos
+    sim = gpu_system(ini, g, 1)
+    r0 = float(g["rMag"][0])
+    _, gd, cnt = sim.rdf(bins=bins, range_mag=range_mag, r_mag0=r0)
+    _, gr = analysis.radial_distribution(pos, g["lBox"], r0, bins=bins, range_mag=range_mag)
+    bw = range_mag * r0 / bins
+    ref = np.rint(gr * (np.arange(bins) + 0.5) ** 2 * (2 * np.pi * bw ** 3 * n * n) / g["lBox"] ** 3).astype(np.int64)
+    assert (np.abs(cnt.astype(np.int64) - ref) > 0).sum() <= 2
+    assert np.abs(cnt.astype(np.int64).sum() - ref.sum()) <= 1 and ref.sum() > 0
