@@ -1299,48 +1299,30 @@ int md_compute_interactions(md_ctx* c, double* B, double* F, double* P3) {
   int st = check_ready(c, true);
   if (st) return st;
   if ((st = force_rebuild(c))) return st;
-  c->launches = issue_interactions(c);
-  if (strong_active(c)) {
-    // a strong list that did not fit its estimate: grown, built again and
-    // evaluated again, so the returned result has its strong pairs in FP64
-    StepFlags f0;
-    CK(c, cudaMemcpyAsync(&f0, &c->sc->flags, sizeof f0, cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    if (f0.soverflow && !f0.overflow) {
-      if ((st = handle_overflow(c, f0))) return st;
-      c->launches = issue_interactions(c);
-    }
-  }
-  IntParams ip = int_params(c, 0.0, c->Br, c->Bk);
-  if (!fp64(c)) ip.mexact = c->mm;
-  c->launches += launch_combine(c->stream, ip, c->Bout, c->Fout, 1, fp64(c));
-  CK(c, cudaGetLastError());
   const size_t Bz = 24 * (size_t)c->n;
-  if (B) CK(c, cudaMemcpyAsync(B, c->Bout, Bz, cudaMemcpyDeviceToHost, c->stream));
-  if (F) CK(c, cudaMemcpyAsync(F, c->Fout, Bz, cudaMemcpyDeviceToHost, c->stream));
-  std::vector<double> pp(3 * (size_t)c->n);
-  CK(c, cudaMemcpyAsync(pp.data(), c->Ppart, 8 * pp.size(), cudaMemcpyDeviceToHost, c->stream));
-  StepFlags fl{};
-  int stotal = 0;
-  if (strong_active(c)) {
-    CK(c, cudaMemcpyAsync(&fl, &c->sc->flags, sizeof fl, cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaMemcpyAsync(&stotal, c->snbr_off + c->n, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  const int nb = int_blocks((int)c->n);
+  std::vector<double> pp(3 * (size_t)nb);
+  DevScalars h;
+  c->launches = 0;
+  // evaluated again when the strong list did not fit its estimate: grown and
+  // built anew, so the returned result has its strong pairs in FP64
+  for (int pass = 0; pass < 2; pass++) {
+    c->launches += issue_interactions(c);
+    IntParams ip = int_params(c, 0.0, c->Br, c->Bk);
+    if (!fp64(c)) ip.mexact = c->mm;
+    c->launches += launch_combine(c->stream, ip, c->Bout, c->Fout, c->obs_part, 1 + pass, fp64(c));
+    CK(c, cudaGetLastError());
+    CK(c, cudaMemcpyAsync(&h, c->sc, sizeof h, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemcpyAsync(pp.data(), c->obs_part, 8 * pp.size(), cudaMemcpyDeviceToHost, c->stream));
+    if (B) CK(c, cudaMemcpyAsync(B, c->Bout, Bz, cudaMemcpyDeviceToHost, c->stream));
+    if (F) CK(c, cudaMemcpyAsync(F, c->Fout, Bz, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    const bool again = pass == 0 && strong_active(c) && h.flags.soverflow && !h.flags.overflow;
+    if ((st = handle_overflow(c, h.flags))) return st;
+    if (!again) break;
   }
-  CK(c, cudaStreamSynchronize(c->stream));
-  // pressure of the strong pairs: the FP64 partial of each 32-entry chunk
-  // (stored at the chunk's first entry), summed here
-  double sp3[3] = {0, 0, 0};
-  if (strong_active(c) && !fl.overflow && !fl.soverflow && stotal > 0 && stotal <= c->scap) {
-    std::vector<double> sp(3 * (size_t)stotal);
-    for (int q = 0; q < 3; q++)
-      CK(c, cudaMemcpy(sp.data() + (size_t)q * stotal, c->svals + (6 + q) * c->scap, 8 * (size_t)stotal,
-                       cudaMemcpyDeviceToHost));
-    for (int q = 0; q < 3; q++)
-      for (int e = 0; e < stotal; e += 32) sp3[q] += sp[(size_t)q * stotal + e];
-  }
-  if ((st = check_overflow(c))) return st;
   if (P3) {
-    double s[3] = {sp3[0], sp3[1], sp3[2]};
+    double s[3] = {0.0, 0.0, 0.0};
     for (size_t b = 0; b < pp.size() / 3; b++)
       for (int q = 0; q < 3; q++) s[q] += pp[3 * b + q];
     const double sc = c->L * F_unit(c) / 2.0;
@@ -1361,7 +1343,7 @@ int md_compute_field(md_ctx* c, const double* mm, double* B) {
   c->launches += issue_field(c);
   IntParams ip = int_params(c, 0.0, c->Br2, c->Bk2);
   if (!fp64(c)) ip.mexact = c->tmpmm;
-  c->launches += launch_combine(c->stream, ip, c->Bout, nullptr, 0, fp64(c));
+  c->launches += launch_combine(c->stream, ip, c->Bout, nullptr, nullptr, 0, fp64(c));
   CK(c, cudaGetLastError());
   if (B) CK(c, cudaMemcpyAsync(B, c->Bout, 24 * (size_t)c->n, cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));

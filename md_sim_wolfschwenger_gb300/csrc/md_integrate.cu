@@ -506,23 +506,41 @@ __global__ void __launch_bounds__(256) k_obs_packed(const ObsParams* __restrict_
 }
 
 // B and F in SI, particle order; optional overlap push of the positions
-// (CompInteractVecs moves the positions, src/interaction.cpp:126-127).
+// (CompInteractVecs moves the positions, src/interaction.cpp:126-127), left out
+// at apply_overlap = 1 while the strong list overflowed (the caller then grows
+// it and evaluates again).  Ppart_out (may be null): the block's pressure sums [grid][3].
 template <typename T>
-__global__ void k_combine(IntParams p, double* Bout, double* Fout, int apply_overlap) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kIntThreads) k_combine(IntParams p, double* Bout, double* Fout, double* Ppart_out,
+                                                         int apply_overlap) {
+  const int i = blockIdx.x * kIntThreads + threadIdx.x;
   const int n = p.n;
-  if (i >= n) return;
-  const int r = p.s.rank[i];
-  double b[3];  // reported field: no rounding to the integrator's type
-  demag_si<T, double>(p, r, b);
-  double sf[3];
-  p.sv.sum3(p.sv.F, r, sf);
+  double pr[4] = {0.0, 0.0, 0.0, 0.0};
+  if (i < n) {
+    const int r = p.s.rank[i];
+    double sb[3], sf[3];
+    const bool hs = p.sv.sums(r, p.sv.B, sb, Fout ? p.sv.F : nullptr, sf, Ppart_out ? p.sv.P : nullptr, pr);
+    double b[3];  // reported field: no rounding to the integrator's type
+    demag_si<T, double>(p, r, b, sb, hs);
+    if (apply_overlap == 1 && p.sv.off && p.flags->soverflow && !p.flags->overflow) apply_overlap = 0;
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
-    if (Bout) Bout[a * n + i] = b[a];
-    if (Fout) Fout[a * n + i] = ((double)((const T*)p.Fr)[a * n + r] + sf[a] + (double)((const T*)p.Fk)[a * n + r]) *
-                                p.F_unit;
-    if (apply_overlap) p.pos[a * n + i] += (double)((const T*)p.ov)[a * n + r] * p.L;
+    for (int a = 0; a < 3; a++) {
+      if (Bout) Bout[a * n + i] = b[a];
+      if (Fout) Fout[a * n + i] = ((double)((const T*)p.Fr)[a * n + r] + sf[a] + (double)((const T*)p.Fk)[a * n + r]) *
+                                  p.F_unit;
+      if (apply_overlap) p.pos[a * n + i] += (double)((const T*)p.ov)[a * n + r] * p.L;
+      if (Ppart_out) pr[a] += p.Ppart[3 * i + a];
+    }
+  }
+  if (!Ppart_out) return;
+  __shared__ double red[kIntThreads / 32][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double s = warp_sums<4>(pr, lane);
+  if ((lane & 7) == 0) red[w][lane >> 3] = s;
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int g = 0; g < kIntThreads / 32; g++) t += red[g][threadIdx.x];
+    Ppart_out[3 * blockIdx.x + threadIdx.x] = t;
   }
 }
 
@@ -757,11 +775,13 @@ int launch_obs_packed(cudaStream_t st, const ObsParams* ps, int R, unsigned* any
   return 1;
 }
 
-int launch_combine(cudaStream_t st, const IntParams& p, double* Bout, double* Fout, int apply_overlap, bool fp64) {
+int launch_combine(cudaStream_t st, const IntParams& p, double* Bout, double* Fout, double* Ppart_out,
+                   int apply_overlap, bool fp64) {
+  const int g = int_blocks(p.n);
   if (fp64)
-    k_combine<double><<<(p.n + 255) / 256, 256, 0, st>>>(p, Bout, Fout, apply_overlap);
+    k_combine<double><<<g, kIntThreads, 0, st>>>(p, Bout, Fout, Ppart_out, apply_overlap);
   else
-    k_combine<float><<<(p.n + 255) / 256, 256, 0, st>>>(p, Bout, Fout, apply_overlap);
+    k_combine<float><<<g, kIntThreads, 0, st>>>(p, Bout, Fout, Ppart_out, apply_overlap);
   return 1;
 }
 

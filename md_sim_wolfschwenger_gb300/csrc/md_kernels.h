@@ -149,13 +149,14 @@ int launch_heun2_obs(cudaStream_t st, const IntParams& p, const ObsParams& o, un
 int launch_heun1_packed(cudaStream_t st, const IntParams* ps, const Packed& n256);
 int launch_heun2_packed(cudaStream_t st, const IntParams* ps, const Packed& n256);
 int launch_obs_packed(cudaStream_t st, const ObsParams* ps, int R, unsigned* anyrb);
-// B, F in SI (orig order, double) from the stage outputs; optional overlap push.
 // Real-space field and force alone of the last full evaluation (test hook).
 int launch_real_part(cudaStream_t st, const IntParams& p, double* Bout, double* Fout, bool fp64);
 // Adaptive Runge-Kutta stage / accept kernels (md_integrate.cu).
 int launch_rk_stage(cudaStream_t st, const RKStage& q, bool fp64);
 int launch_rk_accept(cudaStream_t st, const RKStage& q, bool fp64);
-int launch_combine(cudaStream_t st, const IntParams& p, double* Bout, double* Fout, int apply_overlap,
-                   bool fp64);
+// B, F in SI (orig order, double) from the stage outputs; optional overlap push
+// and per-block pressure sums [int_blocks(n)][3].
+int launch_combine(cudaStream_t st, const IntParams& p, double* Bout, double* Fout, double* Ppart_out,
+                   int apply_overlap, bool fp64);
 
 }  // namespace md

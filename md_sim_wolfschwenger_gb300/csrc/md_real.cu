@@ -525,11 +525,14 @@ __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, 
     if (s >= e) return;
     if constexpr (F32) {
       const float sc = 2.3283064365386963e-10f;
-      int4 nxt = s + lane < e ? p.s.xi[s + lane] : make_int4(0, 0, 0, 0);
+      // two batches of 32 candidates loaded ahead
+      const int4 z4 = make_int4(0, 0, 0, 0);
+      int4 n0 = s + lane < e ? p.s.xi[s + lane] : z4, n1 = s + 32 + lane < e ? p.s.xi[s + 32 + lane] : z4;
       for (int j0 = s; j0 < e; j0 += 32) {
         const int j = j0 + lane;
-        const int4 sj = nxt;
-        if (j0 + 32 + lane < e) nxt = p.s.xi[j0 + 32 + lane];
+        const int4 sj = n0;
+        n0 = n1;
+        if (j0 + 64 + lane < e) n1 = p.s.xi[j0 + 64 + lane];
         const float dx = (float)(sj.x - me.si.x), dy = (float)(sj.y - me.si.y), dz = (float)(sj.z - me.si.z);
         const bool in = j < e && j != k && dx * dx + dy * dy + dz * dz < r2fix;
         visit(in, j, dx * sc, dy * sc, dz * sc);
@@ -616,10 +619,11 @@ __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   constexpr bool F32 = std::is_same<T, float>::value;
   const bool cls = F32 && p.strong;
   const float4* gmu = (const float4*)p.s.mu;
-  float mi2 = 0.f;
+  float mi2 = 0.f, near8 = 0.f;
   if (cls) {
     const float4 m = gmu[k];
     mi2 = m.x * m.x + m.y * m.y + m.z * m.z;
+    near8 = mi2 * 1.0001f;  // |mu_j| <= mu_max = 1: farther pairs cannot be strong
   }
   const bool sfill = FILL && cls && !p.flags->soverflow;
   int cnt = 0, scnt = 0;
@@ -627,13 +631,20 @@ __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   int2* sout = sfill ? p.snbr + p.snbr_off[k] : nullptr;
   scan_rows<T>(p, k, lane, me, p.rl2, [&](bool in, int j, float dx, float dy, float dz) {
     bool st = false;
-    if (cls && in) {
-      const float4 mj = gmu[j];
-      const float r2 = dx * dx + dy * dy + dz * dz, r4 = r2 * r2;
-      st = mi2 * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > p.strong_w4sq * (r4 * r4);
+    unsigned smask = 0;
+    if (cls) {
+      // the moment is fetched only for pairs near enough (a few per cent), so
+      // the candidate loop does not wait on a gather
+      const float r2 = dx * dx + dy * dy + dz * dz, r4 = r2 * r2, w8 = p.strong_w4sq * (r4 * r4);
+      if (__any_sync(kFull, in && w8 < near8)) {
+        if (in && w8 < near8) {
+          const float4 mj = gmu[j];
+          st = mi2 * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > w8;
+        }
+        smask = __ballot_sync(kFull, st);
+      }
     }
     const unsigned mask = __ballot_sync(kFull, in);
-    const unsigned smask = __ballot_sync(kFull, st);
     if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = (sfill && st) ? (int)((unsigned)j | 0x80000000u) : j;
     if (sfill && st) sout[scnt + __popc(smask & lanemask_lt())] = make_int2(k, j);
     cnt += __popc(mask);
@@ -645,64 +656,66 @@ __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   }
 }
 
-// Exclusive scan of cnt[0, n) into off[0, n] by one block (every thread
-// calls it); returns the total to every thread.  Offsets saturate at
-// INT_MAX (the list is then flagged as overflowing).
+// Exclusive scan of cnt[0, n) into off[0, n] by one block of 1024 threads;
+// returns the total to every thread.  Offsets saturate at INT_MAX (the list is
+// then flagged as overflowing).  Each warp takes a contiguous 32nd, 32
+// coalesced values at a time (a run of n / 1024 values per thread touched a
+// cache line per thread and load: 28 us at n = 20011).
 __device__ __forceinline__ long long block_scan_counts(const int* cnt, int* off, int n) {
-  __shared__ long long wsum[32];
-  __shared__ long long total;
-  const int t = threadIdx.x, nt = blockDim.x;
-  const int per = (n + nt - 1) / nt;
-  const int b = t * per, e = min(n, b + per);
+  __shared__ long long wsum[33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per = ((n + 31) / 32 + 31) & ~31;
+  const int b = min(w * per, n), e = min(b + per, n);
   long long local = 0;
-  for (int i = b; i < e; i++) local += cnt[i];
-  const int lane = t & 31, w = t >> 5;
-  long long incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long v = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) wsum[w] = incl;
+#pragma unroll 4
+  for (int i = b + lane; i < e; i += 32) local += cnt[i];
+  local = warp_sum(local);
+  if (lane == 0) wsum[w] = local;
   __syncthreads();
   if (w == 0) {
-    const long long v = lane < (nt >> 5) ? wsum[lane] : 0;
-    long long inc2 = v;
+    const long long v = wsum[lane];
+    long long incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long u = __shfl_up_sync(kFull, inc2, o);
-      if (lane >= o) inc2 += u;
+      const long long u = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += u;
     }
-    wsum[lane] = inc2 - v;
+    wsum[lane] = incl - v;
+    if (lane == 31) wsum[32] = incl;
   }
   __syncthreads();
-  long long run = wsum[w] + incl - local;
-  for (int i = b; i < e; i++) {
-    off[i] = (int)min(run, (long long)0x7fffffff);
-    run += cnt[i];
+  long long run = wsum[w];
+  int nxt = b + lane < e ? cnt[b + lane] : 0;
+  for (int i0 = b; i0 < e; i0 += 32) {
+    const int v = nxt;
+    if (i0 + 32 + lane < e) nxt = cnt[i0 + 32 + lane];
+    int incl = i0 + lane < e ? v : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (i0 + lane < e) off[i0 + lane] = (int)min(run + incl - v, (long long)0x7fffffff);
+    run += __shfl_sync(kFull, incl, 31);
   }
-  if (t == nt - 1) {
-    off[n] = (int)min(run, (long long)0x7fffffff);
-    total = run;
-  }
-  __syncthreads();
-  const long long r = total;
-  __syncthreads();  // the shared scratch is reused by a second call
-  return r;
+  const long long total = wsum[32];
+  if (threadIdx.x == 0) off[n] = (int)min(total, (long long)0x7fffffff);
+  return total;
 }
 
-// Offsets of the Verlet list (and of the strong list); flags overflow.
-__device__ __forceinline__ void nbr_scan(const RealParams& p) {
+// Offsets of the Verlet list (block half 0) and of the strong list (half 1);
+// flags overflow.
+__device__ __forceinline__ void nbr_scan(const RealParams& p, int half) {
   StepFlags* flags = p.flags;
   if (!flags->rebuild) return;
-  const long long tot = block_scan_counts(p.nbr_cnt, p.nbr_off, p.n);
-  long long stot = 0;
-  if (p.strong) stot = block_scan_counts(p.snbr_cnt, p.snbr_off, p.n);
-  if (threadIdx.x == 0) {
-    flags->overflow = tot > p.nbr_cap ? 1 : 0;
+  if (half == 0) {
+    const long long tot = block_scan_counts(p.nbr_cnt, p.nbr_off, p.n);
+    if (threadIdx.x == 0) flags->overflow = tot > p.nbr_cap ? 1 : 0;
+  } else {
     // a build that did not classify leaves the strong list unusable until the
     // next build that does (the FP64 kernels then contribute nothing)
-    flags->soverflow = p.strong ? (stot > p.scap ? 1 : 0) : 1;
+    const long long stot = p.strong ? block_scan_counts(p.snbr_cnt, p.snbr_off, p.n) : 0;
+    if (threadIdx.x == 0) flags->soverflow = p.strong ? (stot > p.scap ? 1 : 0) : 1;
   }
 }
 
@@ -1068,7 +1081,7 @@ __global__ void __launch_bounds__(kRealWarps * 32) k_nbr_build(RealParams p, int
   if (!p.flags->rebuild) return;
   for (int bx = blockIdx.x; bx < nblk; bx += gridDim.x) nbr_build<T, FILL>(p, bx);
 }
-__global__ void __launch_bounds__(1024) k_nbr_scan(RealParams p) { nbr_scan(p); }
+__global__ void __launch_bounds__(1024) k_nbr_scan(RealParams p) { nbr_scan(p, blockIdx.x); }
 // The FP32 passes without coating keep the occupancy of their pair loops
 // (field: 9 blocks of 4 warps per SM, 56 registers; field + force: 7 blocks,
 // 72 registers): the FP64 strong-pair code in the same kernel must not
@@ -1092,7 +1105,7 @@ __global__ void __launch_bounds__(kRealWarps * 32) k_nbr_build_packed(const Real
 }
 __global__ void __launch_bounds__(1024) k_nbr_scan_packed(const RealParams* __restrict__ ps) {
   const RealParams p = ps[blockIdx.x];
-  nbr_scan(p);
+  nbr_scan(p, blockIdx.y);
 }
 // the block shape of the single-system passes (k_real): 8 warps with
 // coating in the field + force pass, otherwise 4; 6 (field + force) or 7
@@ -1119,7 +1132,7 @@ int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64
   else
     k_nbr_build<float, false><<<grid, block, 0, st>>>(p, nblk);
   (void)flags;
-  k_nbr_scan<<<1, 1024, 0, st>>>(p);
+  k_nbr_scan<<<2, 1024, 0, st>>>(p);
   if (fp64)
     k_nbr_build<double, true><<<grid, block, 0, st>>>(p, nblk);
   else
@@ -1151,7 +1164,7 @@ int launch_nbr_packed(cudaStream_t st, const RealParams* ps, int R, const Packed
   if (real.n)
     k_nbr_build_packed<false><<<persistent_grid((const void*)k_nbr_build_packed<false>, th, 0, real.n), th, 0, st>>>(
         ps, real.tasks, real.n, real.wq, anyrb);
-  k_nbr_scan_packed<<<R, 1024, 0, st>>>(ps);
+  k_nbr_scan_packed<<<dim3(R, 2), 1024, 0, st>>>(ps);
   if (real.n)
     k_nbr_build_packed<true><<<persistent_grid((const void*)k_nbr_build_packed<true>, th, 0, real.n), th, 0, st>>>(
         ps, real.tasks, real.n, real.wq, anyrb);
