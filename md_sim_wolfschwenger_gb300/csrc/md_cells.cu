@@ -169,7 +169,12 @@ __device__ __forceinline__ void sorted_fill(const CellParams& p, int bx) {
   }
   const double rm = p.rMag_u[i];
   if constexpr (std::is_same<T, float>::value) {
-    s.xi[k] = make_int4(fixed_box(px, p.invL), fixed_box(py, p.invL), fixed_box(pz, p.invL), i);
+    const int4 q = make_int4(fixed_box(px, p.invL), fixed_box(py, p.invL), fixed_box(pz, p.invL), i);
+    s.xi[k] = q;
+    // float copies for the cell scans (list builds, and every evaluation while
+    // the list does not fit)
+    const float sc = 2.3283064365386963e-10f;
+    if (rb || p.flags->overflow) s.xf[k] = make_float4((float)q.x * sc, (float)q.y * sc, (float)q.z * sc, (float)rm);
   } else {
     const double x = wrap_box(px, p.invL), y = wrap_box(py, p.invL), z = wrap_box(pz, p.invL);
     s.xf[k] = make_float4((float)x, (float)y, (float)z, (float)rm);

@@ -18,7 +18,7 @@
 // against rc like the reference.  Build: one warp per particle walks the rows
 // of its cell stencil; lane r computes row r's cell range, culled to the
 // cells that intersect the search sphere; lanes test 32 candidates at a time
-// (next 32 prefetched) and a ballot compacts the hits (count pass, prefix
+// (the next 64 prefetched) and a ballot compacts the hits (count pass, prefix
 // sum, fill pass).  If the list does not fit its capacity the evaluation
 // falls back to that scan directly, with in-range pairs compacted into a
 // per-warp shared-memory queue (correct, slower); the host then grows the
@@ -488,7 +488,7 @@ __device__ __forceinline__ Self<T> load_self(const RealParams& p, int k) {
   if constexpr (std::is_same<T, float>::value) {
     s.si = p.s.xi[k];
     const float sc = 2.3283064365386963e-10f;
-    s.x = (float)s.si.x * sc;
+    s.x = (float)s.si.x * sc;  // of the cells' scan only
     s.y = (float)s.si.y * sc;
     s.z = (float)s.si.z * sc;
     s.w = 0.f;
@@ -505,56 +505,53 @@ __device__ __forceinline__ Self<T> load_self(const RealParams& p, int k) {
   return s;
 }
 
-// Walks the cell-stencil rows of particle k and calls visit(in, j, dx, dy, dz)
-// for every batch of 32 candidates (warp-synchronous; `in` marks candidates
-// within the search radius; dx.. is the pair vector on the mixed path).
-template <typename T, typename V>
+// Walks the cell-stencil rows of particle k and calls visit(in, j, r2) for
+// every batch of 32 candidates (warp-synchronous).  `in` marks the candidates
+// within the search radius by their float coordinates, with a margin above
+// the rounding of those (a superset: list entries beyond rc carry no weight
+// and the direct scan tests each pair again); r2 in box units.  FRESH: the
+// cells are those of the coordinates (a build), so the image of a row's cells
+// is the image of its particles and the shift is applied to the own position
+// once per row; otherwise (the direct scan between builds) and on the one-cell
+// grid each difference is folded.
+template <bool FRESH, typename T, typename V>
 __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, const Self<T>& me, double r2box,
                                           V&& visit) {
-  constexpr bool F32 = std::is_same<T, float>::value;
   const int ncx = p.grid.ncx, m = p.grid.reach, side = 2 * m + 1, R = side * side;
   const int cell = p.s.cell[k];
   const int cx = cell % ncx, cy = (cell / ncx) % ncx, cz = cell / (ncx * ncx);
   const float inv = 1.0f / (float)ncx;
-  const double rr = sqrt(r2box);
-  const float rt = (float)(rr * (1.0 + 1e-6) + 2e-7);
-  const float rct2 = rt * rt;                                          // culling / FP64 pre-test
-  const float r2fix = (float)(r2box * 18446744073709551616.0);         // (r / (L 2^-32))^2
+  const float rt = (float)(sqrt(r2box) * (1.0 + 1e-6) + 2e-7);
+  const float rct2 = rt * rt;
   const int* cs = p.s.cell_start;
-  auto scan = [&](int s, int e) {
+  const float4* xf = p.s.xf;
+  auto scan = [&](int s, int e, float mx, float my, float mz) {
     if (s >= e) return;
-    if constexpr (F32) {
-      const float sc = 2.3283064365386963e-10f;
-      // two batches of 32 candidates loaded ahead
-      const int4 z4 = make_int4(0, 0, 0, 0);
-      int4 n0 = s + lane < e ? p.s.xi[s + lane] : z4, n1 = s + 32 + lane < e ? p.s.xi[s + 32 + lane] : z4;
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const int j = j0 + lane;
-        const int4 sj = n0;
-        n0 = n1;
-        if (j0 + 64 + lane < e) n1 = p.s.xi[j0 + 64 + lane];
-        const float dx = (float)(sj.x - me.si.x), dy = (float)(sj.y - me.si.y), dz = (float)(sj.z - me.si.z);
-        const bool in = j < e && j != k && dx * dx + dy * dy + dz * dz < r2fix;
-        visit(in, j, dx * sc, dy * sc, dz * sc);
-      }
-    } else {
-      float4 nxt = s + lane < e ? p.s.xf[s + lane] : make_float4(0, 0, 0, 0);
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const int j = j0 + lane;
-        const float4 xj = nxt;
-        if (j0 + 32 + lane < e) nxt = p.s.xf[j0 + 32 + lane];
-        float dx = xj.x - me.x, dy = xj.y - me.y, dz = xj.z - me.z;
+    // two batches of 32 candidates per turn, the next two loaded ahead
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 n0 = s + lane < e ? xf[s + lane] : z4, n1 = s + 32 + lane < e ? xf[s + 32 + lane] : z4;
+    auto test = [&](int j, const float4& q) {
+      float dx = q.x - mx, dy = q.y - my, dz = q.z - mz;
+      if constexpr (!FRESH) {
         dx -= rintf(dx);
         dy -= rintf(dy);
         dz -= rintf(dz);
-        const bool in = j < e && j != k && dx * dx + dy * dy + dz * dz < rct2;
-        visit(in, j, 0.f, 0.f, 0.f);
       }
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      visit(j < e && j != k && r2 < rct2, j, r2);
+    };
+    for (int j = s + lane; j - lane < e; j += 64) {
+      const float4 q0 = n0, q1 = n1;
+      if (j + 64 < e) n0 = xf[j + 64];
+      if (j + 96 < e) n1 = xf[j + 96];
+      test(j, q0);
+      if (j - lane + 32 < e) test(j + 32, q1);
     }
   };
   for (int rb = 0; rb < R; rb += 32) {
     const int r = rb + lane;
     int a0 = 0, b0 = 0, a1 = 0, b1 = 0;
+    int code = 0;  // images (+1) of the first and second x segment, of y and of z, two bits each
     if (r < R) {
       const int dy = r % side - m, dz = r / side - m;
       const int uy = cy + dy, uz = cz + dz;
@@ -575,28 +572,37 @@ __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, 
       if (ok && xlo <= xhi) {
         const int wy = (uy + ncx) % ncx, wz = (uz + ncx) % ncx;
         const int base = (wz * ncx + wy) * ncx;
+        const int iy = uy < 0 ? 0 : (uy >= ncx ? 2 : 1), iz = uz < 0 ? 0 : (uz >= ncx ? 2 : 1);
+        int i0 = 1, i1 = 1;
         if (xlo < 0) {
           a0 = cs[base + xlo + ncx];
           b0 = cs[base + ncx];
           a1 = cs[base];
           b1 = cs[base + xhi + 1];
+          i0 = 0;
         } else if (xhi >= ncx) {
           a0 = cs[base + xlo];
           b0 = cs[base + ncx];
           a1 = cs[base];
           b1 = cs[base + xhi - ncx + 1];
+          i1 = 2;
         } else {
           a0 = cs[base + xlo];
           b0 = cs[base + xhi + 1];
         }
+        code = i0 | i1 << 2 | iy << 4 | iz << 6;
       }
     }
     const int nr = min(32, R - rb);
     for (int q = 0; q < nr; q++) {
       const int s0 = __shfl_sync(kFull, a0, q), e0 = __shfl_sync(kFull, b0, q);
       const int s1 = __shfl_sync(kFull, a1, q), e1 = __shfl_sync(kFull, b1, q);
-      scan(s0, e0);
-      scan(s1, e1);
+      const int cd = __shfl_sync(kFull, code, q);
+      // a row of image i holds particles whose periodic copies lie i - 1 boxes on
+      const float my = FRESH ? me.y + (float)(1 - (cd >> 4 & 3)) : me.y;
+      const float mz = FRESH ? me.z + (float)(1 - (cd >> 6 & 3)) : me.z;
+      scan(s0, e0, FRESH ? me.x + (float)(1 - (cd & 3)) : me.x, my, mz);
+      scan(s1, e1, FRESH ? me.x + (float)(1 - (cd >> 2 & 3)) : me.x, my, mz);
     }
   }
 }
@@ -608,6 +614,12 @@ __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, 
 // (|mu_k|^2 |mu_j|^2 > strong_w4sq r^8 at this build): strong entries carry
 // the sign bit in the Verlet list and are copied, as (k, j), into the
 // strong list (unless that list overflowed in the count).
+//
+// Bound: instruction issue (84 % issue active before, ~84 instructions per 32
+// candidates in fixed-point arithmetic; the float test with the row's image
+// shift takes ~22).  A pair is classified, with its moment and fixed-point
+// distance fetched, only when it is near enough for the largest moment to
+// make it strong (a few per cent of the candidates).
 template <typename T, bool FILL>
 __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   if (!p.flags->rebuild) return;
@@ -619,37 +631,47 @@ __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   constexpr bool F32 = std::is_same<T, float>::value;
   const bool cls = F32 && p.strong;
   const float4* gmu = (const float4*)p.s.mu;
-  float mi2 = 0.f, near8 = 0.f;
+  float mi2 = 0.f, near2 = -1.f;
   if (cls) {
     const float4 m = gmu[k];
     mi2 = m.x * m.x + m.y * m.y + m.z * m.z;
-    near8 = mi2 * 1.0001f;  // |mu_j| <= mu_max = 1: farther pairs cannot be strong
+    near2 = sqrtf(sqrtf(mi2 / p.strong_w4sq)) * 1.001f;  // |mu_j| <= mu_max = 1
   }
   const bool sfill = FILL && cls && !p.flags->soverflow;
   int cnt = 0, scnt = 0;
   int* out = FILL ? p.nbr + p.nbr_off[k] : nullptr;
   int2* sout = sfill ? p.snbr + p.snbr_off[k] : nullptr;
-  scan_rows<T>(p, k, lane, me, p.rl2, [&](bool in, int j, float dx, float dy, float dz) {
-    bool st = false;
-    unsigned smask = 0;
-    if (cls) {
-      // the moment is fetched only for pairs near enough (a few per cent), so
-      // the candidate loop does not wait on a gather
-      const float r2 = dx * dx + dy * dy + dz * dz, r4 = r2 * r2, w8 = p.strong_w4sq * (r4 * r4);
-      if (__any_sync(kFull, in && w8 < near8)) {
-        if (in && w8 < near8) {
+  auto visit = [&](bool in, int j, float r2) {
+    const unsigned mask = __ballot_sync(kFull, in);
+    unsigned jv = (unsigned)j;
+    if constexpr (F32) {
+      const bool near = in && r2 < near2;
+      if (__any_sync(kFull, near)) {
+        bool st = false;
+        if (near) {
           const float4 mj = gmu[j];
-          st = mi2 * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > w8;
+          const int4 sj = p.s.xi[j];
+          const float sc = 2.3283064365386963e-10f;
+          const float dx = (float)(sj.x - me.si.x) * sc, dy = (float)(sj.y - me.si.y) * sc,
+                      dz = (float)(sj.z - me.si.z) * sc;
+          const float q2 = dx * dx + dy * dy + dz * dz, q4 = q2 * q2;
+          st = mi2 * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > p.strong_w4sq * (q4 * q4);
         }
-        smask = __ballot_sync(kFull, st);
+        const unsigned smask = __ballot_sync(kFull, st);
+        if (sfill && st) {
+          sout[scnt + __popc(smask & lanemask_lt())] = make_int2(k, j);
+          jv |= 0x80000000u;
+        }
+        scnt += __popc(smask);
       }
     }
-    const unsigned mask = __ballot_sync(kFull, in);
-    if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = (sfill && st) ? (int)((unsigned)j | 0x80000000u) : j;
-    if (sfill && st) sout[scnt + __popc(smask & lanemask_lt())] = make_int2(k, j);
+    if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = (int)jv;
     cnt += __popc(mask);
-    scnt += __popc(smask);
-  });
+  };
+  if (p.grid.ncx > 1)
+    scan_rows<true, T>(p, k, lane, me, p.rl2, visit);
+  else
+    scan_rows<false, T>(p, k, lane, me, p.rl2, visit);
   if (!FILL && lane == 0) {
     p.nbr_cnt[k] = cnt;
     if (cls) p.snbr_cnt[k] = scnt;
@@ -985,7 +1007,7 @@ __device__ __forceinline__ void real_eval(const RealParams& p, int bx) {
       head += cnt;
       if (lane < cnt) eval(__float_as_int(e.w));
     };
-    scan_rows<T>(p, k, lane, me, p.rc2, [&](bool in, int j, float, float, float) {
+    scan_rows<false, T>(p, k, lane, me, p.rc2, [&](bool in, int j, float) {
       const unsigned mask = __ballot_sync(kFull, in);
       if (in) q[wib][(tail + __popc(mask & lanemask_lt())) & 63] = make_float4(0, 0, 0, __int_as_float(j));
       tail += __popc(mask);
