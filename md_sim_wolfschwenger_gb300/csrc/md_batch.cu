@@ -116,7 +116,6 @@ int upload_params(md_batch* b) {
     md_ctx* c = s.ctx;
     cell[r] = cell_params(c);
     rfull[r] = real_params(c, c->Br, c->Fr, c->ov);
-    rfull[r].npairs = nullptr;
     rfield[r] = real_params(c, c->Br2, nullptr, nullptr);
     kfull[r] = k_params(c, c->Bk, c->Fk);
     kfield[r] = k_params(c, c->Bk2, nullptr);

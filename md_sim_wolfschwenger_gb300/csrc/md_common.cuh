@@ -122,27 +122,47 @@ __device__ __forceinline__ void for_tasks(const Task* __restrict__ tk, int ntask
 // d_fix = 2^32 d, r2f = 2^64 r^2; the unit scale and the exp -> 2^x
 // conversion are folded into the factors.
 struct PairK {
-  float ke;     // -alpha^2 log2(e) 2^-64: exp(-alpha^2 r^2) = 2^(ke r2f)
-  float kz;     // alpha 2^-32 / 2: erfc denominator 1 + alpha r / 2 = 1 + kz r_fix
-  float c2a;    // 2 alpha / sqrt(pi)
-  float ka2n;   // -3 2^-64 and -2 alpha^2 2^-64: field-pass a2 r^2 from a1, t
-  float kt2n;   //   with the pair weight negated
-  float al2x2;  // 2 alpha^2
-  float al4x4;  // 4 alpha^4
-  float eps;    // contact offset
-  float rc2f;   // rc^2 2^64: the cutoff test on r2f
+  float ke;          // -alpha^2 log2(e): exp(-alpha^2 r^2) = 2^(ke r^2)
+  float kz;          // 0.42 alpha: the erfcx fit's denominator 1 + kz r
+  float c2an;        // -2 alpha / sqrt(pi)
+  float a2a, a2t;    // a2 2^-32 = a2a (-a1) / r^2 + a2t (-t), t the Gaussian term
+  float a3a, a3t;    // -a3 2^-96 = a3a (a2 2^-32) / r^2 + a3t (-t)
+  float a2fa, a2ft;  // a2 2^-64 of the field-only pass
+  float eps;         // contact offset
+  float rc2f;        // rc^2 2^64: the cutoff test on r2f
 };
+
+// erfcx(z) = exp(z^2) erfc(z) on the mixed path: t Q(t) with t = 1 / (1 + 0.42 z)
+// and Q of degree 7, a minimax fit (weighted least squares on Chebyshev nodes,
+// Lawson's iteration) over 0 <= z <= 5: relative error 3.2e-8 there, 5e-7 at
+// z = 8 (where exp(-z^2) is 1e-28).  One polynomial and no second exponential:
+// Numerical Recipes' erfcc = t exp(-z^2 + P(t)), used before, is of degree 9
+// with an error of 1.0e-7.
+constexpr float kErfcxA = 0.42f;
+__host__ __device__ constexpr float erfcx_c(int k) {
+  return k == 0   ? 0.2367379418f
+         : k == 1 ? 0.240826718f
+         : k == 2 ? 0.1874095252f
+         : k == 3 ? 0.2917243134f
+         : k == 4 ? -0.1721644463f
+         : k == 5 ? 0.4843077908f
+         : k == 6 ? -0.34481585f
+                  : 0.07597403895f;
+}
+
 inline PairK make_pair_consts(double alpha, double c2a, double cont_eps, double rc2) {
-  const double s64 = 5.421010862427522e-20;  // 2^-64
+  const double s32 = 2.3283064365386963e-10, s64 = s32 * s32;  // 2^-32, 2^-64
   const double al2 = alpha * alpha;
   PairK k;
-  k.ke = (float)(-al2 * 1.4426950408889634 * s64);
-  k.kz = (float)(0.5 * alpha * 2.3283064365386963e-10);
-  k.c2a = (float)c2a;
-  k.ka2n = (float)(-3.0 * s64);
-  k.kt2n = (float)(-2.0 * al2 * s64);
-  k.al2x2 = (float)(2.0 * al2);
-  k.al4x4 = (float)(4.0 * al2 * al2);
+  k.ke = (float)(-al2 * 1.4426950408889634);
+  k.kz = (float)((double)kErfcxA * alpha);
+  k.c2an = (float)-c2a;
+  k.a2a = (float)(-3.0 * s32);
+  k.a2t = (float)(-2.0 * al2 * s32);
+  k.a3a = (float)(-5.0 * s64);
+  k.a3t = (float)(4.0 * al2 * al2 * s32 * s64);
+  k.a2fa = (float)(-3.0 * s64);
+  k.a2ft = (float)(-2.0 * al2 * s64);
   k.eps = (float)cont_eps;
   k.rc2f = (float)(rc2 * 18446744073709551616.0);
   return k;
@@ -170,7 +190,6 @@ struct RealParams {
   void* F;      // [3][n] T, sorted order (FULL only)
   void* ov;     // [3][n] T, overlap displacement, box units (FULL only)
   double* Ppart;  // [n][3] per-particle pressure sums (FULL only)
-  unsigned long long* npairs;  // in-range ordered pairs (FULL only, may be null)
   int* err;       // device error word
   // Verlet neighbour list (sorted indices) with a skin: rebuilt when a
   // particle has moved more than skin/2 since the last build.
@@ -460,19 +479,19 @@ __device__ __forceinline__ void philox_normals9(uint64_t seed, uint64_t step, ui
 // additions per lane instead of 5 W (FP64 additions: 64 cycles each): each
 // butterfly step halves the values a lane carries.  Returns the sum of value
 // (lane / (32 / W)).
-template <int W>
-__device__ __forceinline__ double warp_sums(double (&v)[W], int lane) {
+template <int W, typename T>
+__device__ __forceinline__ T warp_sums(T (&v)[W], int lane) {
   int o = 16;
 #pragma unroll
   for (int h = W / 2; h >= 1; h >>= 1, o >>= 1) {
     const bool up = lane & o;
 #pragma unroll
     for (int q = 0; q < h; q++) {
-      const double give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      const T give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
       v[q] = keep + __shfl_xor_sync(kFull, give, o);
     }
   }
-  double s = v[0];
+  T s = v[0];
   for (; o >= 1; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
   return s;
 }

@@ -162,7 +162,6 @@ RealParams real_params(md_ctx* c, void* B, void* F, void* ov) {
   p.F = F;
   p.ov = ov;
   p.Ppart = c->Ppart;
-  p.npairs = F ? &c->sc->pairs : nullptr;
   p.err = &c->sc->err;
   const double rl = rcb * (1.0 + c->skin_frac);
   p.rl2 = rl * rl;
@@ -397,7 +396,6 @@ static int issue_interactions(md_ctx* c, double dt = -1.0) {
   const CellParams cp = cell_params(c);
   l += launch_step_begin(c->stream, cp.flags, cp.half_skin);
   l += launch_cells(c->stream, cp, fp64(c));
-  cudaMemsetAsync(&c->sc->pairs, 0, sizeof(unsigned long long), c->stream);
   l += fork_join(
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,
       [&](cudaStream_t st) {
@@ -439,6 +437,19 @@ static int issue_step(md_ctx* c, double dt) {
   mark(c, MD_SEG_OBS);  // the records are taken inside the stage-2 launch
   mark(c, MD_NSEG);
   return l;
+}
+
+// In-range pairs of the last evaluation, counted while its list is still there
+// (before new particles, box, cut-off or skin) and on request.
+static int count_pairs(md_ctx* c) {
+  if (!c->list_valid) return MD_OK;
+  unsigned long long v = 0;
+  CK(c, cudaMemsetAsync(&c->sc->pairs, 0, sizeof v, c->stream));
+  launch_count_pairs(c->stream, real_params(c, nullptr, nullptr, nullptr), &c->sc->pairs, fp64(c));
+  CK(c, cudaMemcpyAsync(&v, &c->sc->pairs, sizeof v, cudaMemcpyDeviceToHost, c->stream));
+  CK(c, cudaStreamSynchronize(c->stream));
+  c->pairs = (int64_t)(v / 2);
+  return MD_OK;
 }
 
 // Asks the device to rebuild the cell order and the neighbour list at the
@@ -937,6 +948,7 @@ int md_set_particles(md_ctx* c, const double* rMag, const double* rHydr) {
   mdh::Props p;
   int st = mdh::make_props(c->cfg, rMag, rHydr, c->n, &p, &e);
   if (st) return set_err(c, st, "%s", e.c_str());
+  if ((st = count_pairs(c))) return st;
   c->props = p;
   c->L = p.lBox;
   const size_t N = (size_t)c->n;
@@ -972,6 +984,7 @@ int md_get_box(const md_ctx* c, double* lBox) {
 
 int md_set_box(md_ctx* c, double lBox) {
   if (!c || !(lBox > 0) || !c->have_particles) return set_err(c, MD_ERR_INVALID, "bad box or particles not set");
+  if (int st = count_pairs(c)) return st;
   c->L = lBox;
   c->props.lBox = lBox;
   std::vector<double> rm(c->n);
@@ -1128,6 +1141,7 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
   if (!fp64(c) && kscatter_smem((int)kc) == 0) return set_err(c, MD_ERR_UNSUPPORTED, "kc too large for shared memory");
   invalidate_graph(c);
   CK(c, cudaStreamSynchronize(c->stream));
+  if (int st = count_pairs(c)) return st;
   c->alpha = alpha;
   c->rc = rc;
   c->kc = kc;
@@ -1135,7 +1149,13 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
   const double ab = alpha * c->L;
   const double w = std::pow(c->cfg.my_pi / ab, 2.0);
   c->klist = mdh::build_klist((int)kc, w);
-  c->grid = mdh::choose_grid(rc / c->L, c->n, 2);
+  // cells: a stencil of +-2 on the FP64 path; on the mixed path ~4 particles
+  // each, which keeps the two consecutive sorted particles whose lists one
+  // warp builds close together and fits the cells to the search sphere
+  int reach = 2;
+  if (!fp64(c))
+    reach = (int)std::lround(rc / c->L * std::cbrt(0.25 * (double)c->n));
+  c->grid = mdh::choose_grid(rc / c->L, c->n, std::max(2, std::min(reach, 12)));
   if (!fp64(c)) {
     // structure-factor grid (segment blocks x particle chunks): the fewest
     // whole waves of resident blocks that keep every FP32 chunk sum within 512
@@ -1753,16 +1773,14 @@ int md_debug_launches(const md_ctx* c, int64_t* launches) {
 
 int md_debug_pairs(md_ctx* c, int64_t* pairs) {
   if (!c || !pairs) return set_err(c, MD_ERR_INVALID, "null argument");
-  unsigned long long v = 0;
-  CK(c, cudaStreamSynchronize(c->stream));
-  CK(c, cudaMemcpy(&v, &c->sc->pairs, sizeof v, cudaMemcpyDeviceToHost));
-  *pairs = (int64_t)(v / 2);
+  if (int st = count_pairs(c)) return st;
+  *pairs = c->pairs;
   return MD_OK;
 }
 
 int md_set_neighbor_skin(md_ctx* c, double skin_frac) {
   if (!c || !(skin_frac >= 0) || skin_frac > 1) return set_err(c, MD_ERR_INVALID, "skin fraction must be in [0, 1]");
-  CK(c, cudaStreamSynchronize(c->stream));
+  if (int st = count_pairs(c)) return st;
   c->skin_frac = skin_frac;
   c->list_valid = false;
   invalidate_graph(c);

@@ -151,6 +151,7 @@ struct md_ctx {
   // particle ~5 pm at dt = 1e-12 s, so even a 0.5 % skin (1 nm at rc = 400
   // nm) is crossed only after ~1e4 steps and rebuilds stay rare.
   double skin_frac = 0.005;
+  int64_t pairs = 0;        // in-range pairs of the last evaluation, as last counted
   bool list_valid = false;  // a build for the current particles, grid and skin exists
   // Strong pairs (mixed path, md_real.cu): list entries whose force weight
   // (|mu_i| |mu_j| / mu_min^2) (2 rHydr_min / r)^4 exceeds strong_theta are

@@ -15,18 +15,17 @@
 // last build; it is rebuilt (on the device, inside the step) when some
 // particle has moved more than skin/2 since then, so every pair that is now
 // within rc is in the list.  Each evaluation tests the exact distance
-// against rc like the reference.  Build: one warp per particle walks the rows
-// of its cell stencil; lane r computes row r's cell range, culled to the
-// cells that intersect the search sphere; lanes test 32 candidates at a time
-// (the next 64 prefetched) and a ballot compacts the hits (count pass, prefix
-// sum, fill pass).  If the list does not fit its capacity the evaluation
-// falls back to that scan directly, with in-range pairs compacted into a
-// per-warp shared-memory queue (correct, slower); the host then grows the
-// list.
+// against rc like the reference.  Build: FP64 path one warp per particle
+// (nbr_build64), mixed path one warp per two (nbr_build2); a warp walks the rows
+// of its cell stencil, culled to the cells that intersect the search sphere,
+// and a ballot compacts the hits (count pass, prefix sum, fill pass).  If the
+// list does not fit its capacity the evaluation scans the cells directly, with
+// in-range pairs compacted into a per-warp shared-memory queue (correct,
+// slower); the host then grows the list.
 //
-// Evaluation: one warp per particle; lanes take list entries 32 at a time,
-// gather the neighbour's coordinates and moment, and run the pair maths
-// (erfc, exp, ~90 flops).  Per-lane sums are reduced with warp shuffles.
+// Evaluation: one warp per particle; lanes take list entries 32 at a time (mixed
+// path 64), gather the neighbour's coordinates and moment, and run the pair
+// maths (erfc, exp, ~90 flops).  Per-lane sums are reduced with warp shuffles.
 //
 // Geometry (mixed path): 32-bit fixed-point coordinates (2^32 per box
 // length); their wrapping difference is the exact minimum image, converted
@@ -34,11 +33,9 @@
 // uses FP64 box coordinates and the reference's fold (d > L/2 -> d - L,
 // d < -L/2 -> d + L), with an FP32 pre-test that has a small margin.
 //
-// erfc on the mixed path: the Chebyshev fit erfcc of Numerical Recipes
-// (Press et al., 2nd ed., section 6.2), relative error < 1.2e-7 for x >= 0,
-// written as t exp(-x^2) exp(P(t)) so that exp(-x^2) is shared with the
-// Gaussian term; exponentials with __expf.  The FP64 path takes both from
-// tables of polynomials (ewald64).
+// erfc: exp(-x^2), shared with the Gaussian term, times erfcx from a fit
+// (erfcx32) on the mixed path and from tables of polynomials on the FP64 path
+// (ewald64).
 //
 // Overlap push: CompInteractVecs moves cores apart in place while it walks
 // the pairs, so later pairs see moved positions.  Here every overlap is
@@ -65,23 +62,15 @@ constexpr int kFieldWarps = 4;
 template <typename T>
 struct Acc {
   T b0 = 0, b1 = 0, b2 = 0, f0 = 0, f1 = 0, f2 = 0, o0 = 0, o1 = 0, o2 = 0, p0 = 0, p1 = 0, p2 = 0;
-  int np = 0;  // in-range pairs seen by this lane
 };
 
-// Numerical Recipes erfcc: erfc(z) = t exp(-z^2 + P(t)), t = 1/(1 + z/2).
-__device__ __forceinline__ float erfc_nr(float z, float ez2) {
-  const float t = __fdividef(1.0f, fmaf(0.5f, z, 1.0f));
-  float q = 0.17087277f;
-  q = fmaf(q, t, -0.82215223f);
-  q = fmaf(q, t, 1.48851587f);
-  q = fmaf(q, t, -1.13520398f);
-  q = fmaf(q, t, 0.27886807f);
-  q = fmaf(q, t, -0.18628806f);
-  q = fmaf(q, t, 0.09678418f);
-  q = fmaf(q, t, 0.37409196f);
-  q = fmaf(q, t, 1.00002368f);
-  q = fmaf(q, t, -1.26551223f);
-  return t * ez2 * __expf(q);
+// The erfcx fit in scalar code.
+__device__ __forceinline__ float erfcx32(float z) {
+  const float t = __fdividef(1.0f, fmaf(kErfcxA, z, 1.0f));
+  float q = erfcx_c(7);
+#pragma unroll
+  for (int k = 6; k >= 0; k--) q = fmaf(q, t, erfcx_c(k));
+  return t * q;
 }
 
 // Coating potentials of a pair inside rCutSR (CompSterRep,
@@ -109,7 +98,6 @@ __device__ __forceinline__ double coat_force(const RealParams& p, double rd, int
 template <bool FULL, bool COAT>
 __device__ __forceinline__ void pair_terms(const RealParams& p, float dx, float dy, float dz, float r2, const float4& mi,
                                            const float4& mj, int oi, int oj, Acc<float>& a) {
-  a.np++;
   const float ir0 = rsqrtf(r2), r0 = r2 * ir0;
   const float ux = dx * ir0, uy = dy * ir0, uz = dz * ir0;
   float r = r0, ire = ir0;
@@ -126,7 +114,7 @@ __device__ __forceinline__ void pair_terms(const RealParams& p, float dx, float 
   }
   const float ire2 = ire * ire;
   const float re2 = r * r;
-  const float e = __expf(-(float)p.al2 * re2), erfcv = erfc_nr((float)p.alpha * r, e);
+  const float e = __expf(-(float)p.al2 * re2), erfcv = e * erfcx32((float)p.alpha * r);
   const float t = (float)p.c2a * e * ire2;
   const float a1 = erfcv * ire2 * ire + t;
   const float a2 = 3.0f * a1 * ire2 + 2.0f * (float)p.al2 * t;
@@ -240,7 +228,6 @@ __device__ __forceinline__ void pair64(const RealParams& p, const double4_32a& d
   double dx = fold64(di.x, dj.x, fi.x, fj.x), dy = fold64(di.y, dj.y, fi.y, fj.y), dz = fold64(di.z, dj.z, fi.z, fj.z);
   double r2 = dx * dx + dy * dy + dz * dz;
   if (!(r2 < p.rc2)) return;
-  a.np++;
   bool sr = false;
   if constexpr (FULL && COAT) sr = r2 < p.rcut_sr2;
   double ire;
@@ -306,20 +293,22 @@ __device__ __forceinline__ void pair64(const RealParams& p, const double4_32a& d
 
 // ------------------------------------------------- packed pair terms (FP32)
 // Two pairs at once in the halves of float2 operations (Blackwell's packed
-// FP32 instructions: one issue slot for two FMAs, the FMA rate unchanged), for
-// the mixed path's list loop, which gathers two neighbours per lane and
-// iteration.  The per-pair arithmetic is the one of pair_terms (same
-// operations and rounding per half); special functions stay scalar.
+// FP32 instructions: one issue slot for two FMAs, the FMA rate unchanged): two
+// neighbours of the warp's particle.  Special functions stay scalar.
 __device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 pk1(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// Sums of the list loop.  Field only: b.  Field + force: b of the a1 terms, d
+// times 2^32 of the a2 terms, e of a2 (mj.d), f of the force with the opposite sign
+// without its terms along mi, p of the pressure's radial terms times 2^32
+// (the end of the loop puts them together).
 struct Acc2 {
-  float2 b0 = {0.f, 0.f}, b1 = {0.f, 0.f}, b2 = {0.f, 0.f}, f0 = {0.f, 0.f}, f1 = {0.f, 0.f}, f2 = {0.f, 0.f};
-  float2 p0 = {0.f, 0.f}, p1 = {0.f, 0.f}, p2 = {0.f, 0.f};
+  float2 b0 = {0.f, 0.f}, b1 = {0.f, 0.f}, b2 = {0.f, 0.f};
+  float f0 = 0.f, f1 = 0.f, f2 = 0.f, p0 = 0.f, p1 = 0.f, p2 = 0.f;
+  float d0 = 0.f, d1 = 0.f, d2 = 0.f, e = 0.f;
 };
 
 // Single-instruction approximations (PTX ex2/rsqrt/rcp .approx.ftz); their
@@ -340,134 +329,109 @@ __device__ __forceinline__ float rcp_ftz(float x) {
   return y;
 }
 
-// erfc polynomial of Numerical Recipes' erfcc (the one of erfc_nr) times
-// log2(e), so that 2^q replaces exp(q); the coefficients stay below 2 in
-// magnitude, so the scaling costs no precision.
-__host__ __device__ constexpr float erfc_c(double c) { return (float)(c * 1.4426950408889634); }
-
-// Pairs A and B: fixed-point pair vectors (dxf..), r2f = |d_fix|^2, the
-// neighbour moments ma, mb; inA, inB: the pair is within rc.  Pairs outside
-// get a harmless distance and weight 0.  wA, wB: the pair's Ewald field,
-// force and pressure go into the sums (in range and not a strong pair, whose
-// terms the FP64 kernels add; the overlap push follows inA, inB).  Same
-// formulas as pair_terms, with the field sums of the field-only pass as two
-// FMAs per component.
+// Neighbours A and B: fixed-point pair vectors (dxf..), r2f = |d_fix|^2,
+// moments ma, mb; inA, inB: the pair is within rc; stA, stB: it is a strong pair
+// (its terms are added in FP64; it still pushes).  A pair that adds nothing
+// gets a distance at which exp(-alpha^2 r^2) is zero, and with it every
+// coefficient: no weights.  Same formulas as pair_terms; the pair vector stays
+// in fixed-point units, their powers of 2^-32 folded into the constants, and
+// the coefficients are negated (the fit's sign), which saves the sign of the
+// field's second term.  push: the lane's overlap push in shared memory ([3][32]),
+// rare.
+//
+// Field + force: with e1 = a2 (mi.d), e2 = a2 (mj.d), t1 = a2 m12 - a3 (mi.d)(mj.d)
+//   F_ij = t1 d + e2 mi + e1 mj,  P_ab = sum over ordered pairs of d_a F_b.
+// mi is the same for the whole list, so e2 mi is summed as e2.  In P the terms
+// d_a e2 mi_b and d_a e1 mj_b turn into each other when the pair is taken in the
+// other order, which the other particle's list holds, so the total takes
+// 2 mi_b sum d_a e2, and that sum is the field's (d): per pair the pressure
+// costs the five operations of t1 d_a d_b.  (A particle's own share of P is then
+// not the sum over its list; only the total is ever used.)
+//
+// Bound: FP32 issue and the FMA pipe: 35 packed operations per two pairs for
+// the field, 28 packed and 64 scalar with the force (43 and 36 + 90 with
+// erfcc, pair weights, a scaled pair vector and P from F_ij).
 template <bool FULL>
 __device__ __forceinline__ void pair_terms2(const PairK& K, float wdc, float2 dxf, float2 dyf, float2 dzf, float2 r2f,
-                                            bool inA, bool inB, bool wA, bool wB, float rc2_fix, const float4& mi,
-                                            const float4& ma, const float4& mb, Acc<float>& a, Acc2& a2) {
-  const float sc = 2.3283064365386963e-10f;  // 2^-32 (exact scaling)
-  r2f = pk(inA ? r2f.x : rc2_fix, inB ? r2f.y : rc2_fix);
-  a.np += (int)inA + (int)inB;
-  float2 irf = pk(rsqrt_ftz(r2f.x), rsqrt_ftz(r2f.y));  // 1 / r_fix
-  float2 rfx = mul2(r2f, irf);  // r_fix
-  float2 r = mul2(rfx, pk1(sc));
+                                            bool inA, bool inB, bool stA, bool stB, const float4& mi,
+                                            const float4& ma, const float4& mb, Acc2& s, float* push) {
+  const float far2 = 1.8446744e23f;  // (100 box lengths)^2 in fixed units
+  float2 r2 = mul2(pk(inA ? r2f.x : far2, inB ? r2f.y : far2), pk1(5.421010862427522e-20f));  // 2^-64
+  float2 ire = pk(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));  // 1 / r
+  float2 r = mul2(r2, ire);
   const float2 dcont = pk(wdc + ma.w, wdc + mb.w);
-  const bool ovA = inA && r.x < dcont.x, ovB = inB && r.y < dcont.y;
-  if (ovA || ovB) {  // rare: clamp overlapping pairs to contact
-    const float s32 = 4294967296.0f;
-    // push along the unit vector d / r; then the pair vector itself is
-    // rescaled to the contact length, which the assembly below uses
-    if (ovA) {
+  float2 r2e = r2;  // distance of the exponential
+  if (r.x < dcont.x || r.y < dcont.y || stA || stB) {  // rare
+    auto clamp = [&](float& rr, float& ir, float& re, float dc, float& x, float& y, float& z) {
+      // overlapping cores: pushed apart, the pair vector rescaled to the contact length
       if constexpr (FULL) {
-        const float h = 0.5f * (dcont.x - r.x) * irf.x;
-        a.o0 -= h * dxf.x;
-        a.o1 -= h * dyf.x;
-        a.o2 -= h * dzf.x;
+        const float h = 0.5f * (dc - rr) * ir * 2.3283064365386963e-10f;
+        push[0] -= h * x;
+        push[32] -= h * y;
+        push[64] -= h * z;
       }
-      const float g = dcont.x * s32 * irf.x;
-      dxf.x *= g;
-      dyf.x *= g;
-      dzf.x *= g;
-      r.x = dcont.x;
-      rfx.x = dcont.x * s32;
-      irf.x = rcp_ftz(rfx.x);
-      r2f.x = rfx.x * rfx.x;
-    }
-    if (ovB) {
-      if constexpr (FULL) {
-        const float h = 0.5f * (dcont.y - r.y) * irf.y;
-        a.o0 -= h * dxf.y;
-        a.o1 -= h * dyf.y;
-        a.o2 -= h * dzf.y;
-      }
-      const float g = dcont.y * s32 * irf.y;
-      dxf.y *= g;
-      dyf.y *= g;
-      dzf.y *= g;
-      r.y = dcont.y;
-      rfx.y = dcont.y * s32;
-      irf.y = rcp_ftz(rfx.y);
-      r2f.y = rfx.y * rfx.y;
-    }
+      const float g = dc * ir;
+      x *= g;
+      y *= g;
+      z *= g;
+      rr = dc;
+      ir = rcp_ftz(dc);
+      re = dc * dc;
+    };
+    if (r.x < dcont.x) clamp(r.x, ire.x, r2e.x, dcont.x, dxf.x, dyf.x, dzf.x);
+    if (r.y < dcont.y) clamp(r.y, ire.y, r2e.y, dcont.y, dxf.y, dyf.y, dzf.y);
+    if (stA) r2e.x = 1e4f;
+    if (stB) r2e.y = 1e4f;
   }
-  const float2 ire = mul2(irf, pk1(4294967296.0f));  // 1 / r
   const float2 ire2 = mul2(ire, ire);
-  const float2 ee = mul2(pk1(K.ke), r2f);
+  const float2 ee = mul2(r2e, pk1(K.ke));
   const float2 e = pk(ex2_ftz(ee.x), ex2_ftz(ee.y));  // exp(-alpha^2 r^2)
-  const float2 den = fma2(pk1(K.kz), rfx, pk1(1.0f));
-  const float2 tt = pk(rcp_ftz(den.x), rcp_ftz(den.y));
-  float2 q = pk1(erfc_c(0.17087277));
-  q = fma2(q, tt, pk1(erfc_c(-0.82215223)));
-  q = fma2(q, tt, pk1(erfc_c(1.48851587)));
-  q = fma2(q, tt, pk1(erfc_c(-1.13520398)));
-  q = fma2(q, tt, pk1(erfc_c(0.27886807)));
-  q = fma2(q, tt, pk1(erfc_c(-0.18628806)));
-  q = fma2(q, tt, pk1(erfc_c(0.09678418)));
-  q = fma2(q, tt, pk1(erfc_c(0.37409196)));
-  q = fma2(q, tt, pk1(erfc_c(1.00002368)));
-  q = fma2(q, tt, pk1(erfc_c(-1.26551223)));
-  const float2 erfcv = mul2(mul2(tt, e), pk(ex2_ftz(q.x), ex2_ftz(q.y)));
-  const float2 t = mul2(mul2(pk1(K.c2a), e), ire2);
+  const float2 den = fma2(r, pk1(K.kz), pk1(1.0f));
+  const float2 t = pk(rcp_ftz(den.x), rcp_ftz(den.y));  // 1 / (1 + 0.42 alpha r)
+  float2 q = pk1(-erfcx_c(7));
+#pragma unroll
+  for (int k = 6; k >= 0; k--) q = fma2(q, t, pk1(-erfcx_c(k)));
+  const float2 erfcn = mul2(mul2(t, e), q);              // -erfc(alpha r)
+  const float2 tn = mul2(mul2(e, pk1(K.c2an)), ire2);    // minus the Gaussian term
+  const float2 a1n = fma2(mul2(erfcn, ire2), ire, tn);   // -a1
   if constexpr (FULL) {
-    // field + force: packed coefficients, then each pair assembled in scalar
-    // code (as pair_terms), which keeps fewer values live.  The assembly uses
-    // the pair vector d = r u itself: B = a2 (mj.d) d - a1 mj, F_ij = (a2 m12
-    // - a3 (mi.d)(mj.d)) d + a2 ((mj.d) mi + (mi.d) mj), P += d_x F_y, ...
-    // (no normalisation, fewer products of r)
-    const float2 w = pk(wA ? 1.f : 0.f, wB ? 1.f : 0.f);
-    const float2 a1 = mul2(fma2(mul2(erfcv, ire2), ire, t), w);
-    const float2 tw = mul2(t, w);
-    const float2 a2c = fma2(mul2(pk1(3.f), a1), ire2, mul2(pk1(K.al2x2), tw));
-    const float2 a3 = fma2(mul2(pk1(5.f), a2c), ire2, mul2(pk1(K.al4x4), tw));
-    const float2 dvx = mul2(dxf, pk1(sc)), dvy = mul2(dyf, pk1(sc)), dvz = mul2(dzf, pk1(sc));  // box units
+    // packed coefficients, then each pair in scalar code: packed, the sums take
+    // twice the registers, and at 6 blocks per SM the pass took 261 us
+    // instead of 250 at 7 (N = 32768)
+    const float2 a2 = fma2(mul2(a1n, pk1(K.a2a)), ire2, mul2(tn, pk1(K.a2t)));   // a2 2^-32
+    const float2 a3n = fma2(mul2(a2, pk1(K.a3a)), ire2, mul2(tn, pk1(K.a3t)));   // -a3 2^-96
     auto assemble = [&](float a1s, float a2s, float a3s, float dx, float dy, float dz, const float4& mj) {
-      // dot products in scalar code: packed, they would first pair up the
-      // two neighbours' moment components
       const float D1 = fmaf(mi.z, dz, fmaf(mi.y, dy, mi.x * dx));
       const float D2 = fmaf(mj.z, dz, fmaf(mj.y, dy, mj.x * dx));
-      const float e2 = a2s * D2;
-      a.b0 = fmaf(e2, dx, fmaf(-a1s, mj.x, a.b0));
-      a.b1 = fmaf(e2, dy, fmaf(-a1s, mj.y, a.b1));
-      a.b2 = fmaf(e2, dz, fmaf(-a1s, mj.z, a.b2));
       const float m12 = fmaf(mi.z, mj.z, fmaf(mi.y, mj.y, mi.x * mj.x));
-      const float t1 = fmaf(-a3s * D1, D2, a2s * m12);
-      const float e1 = a2s * D1;
-      const float vx = fmaf(t1, dx, fmaf(e2, mi.x, e1 * mj.x));
-      const float vy = fmaf(t1, dy, fmaf(e2, mi.y, e1 * mj.y));
-      const float vz = fmaf(t1, dz, fmaf(e2, mi.z, e1 * mj.z));
-      a.f0 -= vx;
-      a.f1 -= vy;
-      a.f2 -= vz;
-      a.p0 = fmaf(dx, vy, a.p0);
-      a.p1 = fmaf(dx, vz, a.p1);
-      a.p2 = fmaf(dy, vz, a.p2);
+      const float e2 = a2s * D2, e1 = a2s * D1;
+      s.b0.x = fmaf(a1s, mj.x, s.b0.x);
+      s.b1.x = fmaf(a1s, mj.y, s.b1.x);
+      s.b2.x = fmaf(a1s, mj.z, s.b2.x);
+      s.d0 = fmaf(e2, dx, s.d0);
+      s.d1 = fmaf(e2, dy, s.d1);
+      s.d2 = fmaf(e2, dz, s.d2);
+      s.e += e2;
+      const float t1 = fmaf(a3s * D1, D2, a2s * m12);
+      s.f0 = fmaf(t1, dx, fmaf(e1, mj.x, s.f0));
+      s.f1 = fmaf(t1, dy, fmaf(e1, mj.y, s.f1));
+      s.f2 = fmaf(t1, dz, fmaf(e1, mj.z, s.f2));
+      const float tx = t1 * dx, ty = t1 * dy;
+      s.p0 = fmaf(tx, dy, s.p0);
+      s.p1 = fmaf(tx, dz, s.p1);
+      s.p2 = fmaf(ty, dz, s.p2);
     };
-    assemble(a1.x, a2c.x, a3.x, dvx.x, dvy.x, dvz.x, ma);
-    assemble(a1.y, a2c.y, a3.y, dvx.y, dvy.y, dvz.y, mb);
+    assemble(a1n.x, a2.x, a3n.x, dxf.x, dyf.x, dzf.x, ma);
+    assemble(a1n.y, a2.y, a3n.y, dxf.y, dyf.y, dzf.y, mb);
   } else {
-    // B += a2 (mj.d) d - a1 mj with d the pair vector in fixed-point units
-    // (a2 (mj.u) r^2 u), the weight negated (wn = -w): a1n = -a1, and the
-    // 2^-64 of the fixed-point units folded into a2s
+    // B += a2 (mj.d) d - a1 mj
     const float2 mjx = pk(ma.x, mb.x), mjy = pk(ma.y, mb.y), mjz = pk(ma.z, mb.z);
-    const float2 d2 = fma2(mjz, dzf, fma2(mjy, dyf, mul2(mjx, dxf)));
-    const float2 wn = pk(wA ? -1.f : 0.f, wB ? -1.f : 0.f);
-    const float2 a1n = mul2(fma2(mul2(erfcv, ire2), ire, t), wn);
-    const float2 a2s = fma2(mul2(pk1(K.ka2n), a1n), ire2, mul2(pk1(K.kt2n), mul2(t, wn)));
-    const float2 c1 = mul2(a2s, d2);
-    a2.b0 = fma2(c1, dxf, fma2(a1n, mjx, a2.b0));
-    a2.b1 = fma2(c1, dyf, fma2(a1n, mjy, a2.b1));
-    a2.b2 = fma2(c1, dzf, fma2(a1n, mjz, a2.b2));
+    const float2 D2 = fma2(mjz, dzf, fma2(mjy, dyf, mul2(mjx, dxf)));
+    const float2 a2 = fma2(mul2(a1n, pk1(K.a2fa)), ire2, mul2(tn, pk1(K.a2ft)));  // a2 2^-64
+    const float2 c1 = mul2(a2, D2);
+    s.b0 = fma2(c1, dxf, fma2(a1n, mjx, s.b0));
+    s.b1 = fma2(c1, dyf, fma2(a1n, mjy, s.b1));
+    s.b2 = fma2(c1, dzf, fma2(a1n, mjz, s.b2));
   }
 }
 
@@ -609,73 +573,218 @@ __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, 
 
 // ------------------------------------------------------- neighbour list
 
-// Count (FILL = false) or write (FILL = true) the neighbours within rc + skin.
-// On the mixed path with strong pairs on, each neighbour is also classified
-// (|mu_k|^2 |mu_j|^2 > strong_w4sq r^8 at this build): strong entries carry
-// the sign bit in the Verlet list and are copied, as (k, j), into the
-// strong list (unless that list overflowed in the count).
-//
-// Bound: instruction issue (84 % issue active before, ~84 instructions per 32
-// candidates in fixed-point arithmetic; the float test with the row's image
-// shift takes ~22).  A pair is classified, with its moment and fixed-point
-// distance fetched, only when it is near enough for the largest moment to
-// make it strong (a few per cent of the candidates).
-template <typename T, bool FILL>
-__device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
-  if (!p.flags->rebuild) return;
+// FP64 path: count (FILL = false) or write (FILL = true) the neighbours of
+// each particle within rc + skin, one warp per particle.
+template <bool FILL>
+__device__ __forceinline__ void nbr_build64(const RealParams& p, int bx) {
   if (FILL && p.flags->overflow) return;
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k = bx * kRealWarps + wib;
+  const int lane = threadIdx.x & 31, k = bx * kRealWarps + (threadIdx.x >> 5);
   if (k >= p.n) return;
-  const Self<T> me = load_self<T, false>(p, k);
-  constexpr bool F32 = std::is_same<T, float>::value;
-  const bool cls = F32 && p.strong;
-  const float4* gmu = (const float4*)p.s.mu;
-  float mi2 = 0.f, near2 = -1.f;
-  if (cls) {
-    const float4 m = gmu[k];
-    mi2 = m.x * m.x + m.y * m.y + m.z * m.z;
-    near2 = sqrtf(sqrtf(mi2 / p.strong_w4sq)) * 1.001f;  // |mu_j| <= mu_max = 1
-  }
-  const bool sfill = FILL && cls && !p.flags->soverflow;
-  int cnt = 0, scnt = 0;
+  const Self<double> me = load_self<double, false>(p, k);
+  int cnt = 0;
   int* out = FILL ? p.nbr + p.nbr_off[k] : nullptr;
-  int2* sout = sfill ? p.snbr + p.snbr_off[k] : nullptr;
-  auto visit = [&](bool in, int j, float r2) {
+  auto visit = [&](bool in, int j, float) {
     const unsigned mask = __ballot_sync(kFull, in);
-    unsigned jv = (unsigned)j;
-    if constexpr (F32) {
-      const bool near = in && r2 < near2;
-      if (__any_sync(kFull, near)) {
-        bool st = false;
-        if (near) {
-          const float4 mj = gmu[j];
-          const int4 sj = p.s.xi[j];
-          const float sc = 2.3283064365386963e-10f;
-          const float dx = (float)(sj.x - me.si.x) * sc, dy = (float)(sj.y - me.si.y) * sc,
-                      dz = (float)(sj.z - me.si.z) * sc;
-          const float q2 = dx * dx + dy * dy + dz * dz, q4 = q2 * q2;
-          st = mi2 * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > p.strong_w4sq * (q4 * q4);
-        }
-        const unsigned smask = __ballot_sync(kFull, st);
-        if (sfill && st) {
-          sout[scnt + __popc(smask & lanemask_lt())] = make_int2(k, j);
-          jv |= 0x80000000u;
-        }
-        scnt += __popc(smask);
-      }
-    }
-    if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = (int)jv;
+    if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = j;
     cnt += __popc(mask);
   };
   if (p.grid.ncx > 1)
-    scan_rows<true, T>(p, k, lane, me, p.rl2, visit);
+    scan_rows<true, double>(p, k, lane, me, p.rl2, visit);
   else
-    scan_rows<false, T>(p, k, lane, me, p.rl2, visit);
-  if (!FILL && lane == 0) {
-    p.nbr_cnt[k] = cnt;
-    if (cls) p.snbr_cnt[k] = scnt;
+    scan_rows<false, double>(p, k, lane, me, p.rl2, visit);
+  if (!FILL && lane == 0) p.nbr_cnt[k] = cnt;
+}
+
+// Mixed path: one warp builds the lists of two consecutive sorted particles
+// (2 w, 2 w + 1), which are close (the cells hold ~4 particles; periodic images
+// across the ends of a row): the rows are set up and the candidates loaded
+// once for both.
+//
+// Search.  The pair's bounding box, grown by the list radius, gives the rows of
+// cells and per row the x range; 32 rows are set up at a time, one per lane,
+// and then taken four at a time by eight lanes each (rows hold ~40 particles),
+// the shift to a row's periodic image applied to the own positions.  Where the
+// box does not fit into the periodic cell (few cells, or two particles far
+// apart), and on the one-cell grid, all particles are tested with a fold.
+//
+// With strong pairs on, each neighbour is also classified per particle
+// (|mu_i|^2 |mu_j|^2 > strong_w4sq r^8 at this build): strong entries carry the
+// sign bit in the list and are copied, as (i, j), into the strong list (unless
+// that list overflowed in the count).  A pair is classified, with its
+// moment and fixed-point distance fetched, only when it is near enough for
+// the largest moment to make it strong.
+constexpr unsigned kStrong = 0x80000000u;
+constexpr int kNbrIndex = 0x7fffffff;
+
+template <bool FILL>
+__device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
+  if (FILL && p.flags->overflow) return;
+  const int lane = threadIdx.x & 31, w = bx * kRealWarps + (threadIdx.x >> 5);
+  const int n = p.n, k1 = 2 * w, k2 = min(k1 + 1, n - 1);
+  if (k1 >= n) return;
+  const float4* xf = p.s.xf;
+  const float4 f1 = xf[k1], f2 = xf[k2];
+  float ex = f2.x - f1.x, ey = f2.y - f1.y, ez = f2.z - f1.z;  // the second particle's nearest image
+  ex -= rintf(ex);
+  ey -= rintf(ey);
+  ez -= rintf(ez);
+  const bool cls = p.strong;
+  const float4* gmu = (const float4*)p.s.mu;
+  float m1 = 0.f, m2 = 0.f, near1 = -1.f, near2 = -1.f;
+  if (cls) {
+    const float4 u = gmu[k1], v = gmu[k2];
+    m1 = u.x * u.x + u.y * u.y + u.z * u.z;
+    m2 = v.x * v.x + v.y * v.y + v.z * v.z;
+    near1 = sqrtf(sqrtf(m1 / p.strong_w4sq)) * 1.001f;  // |mu_j| <= mu_max = 1
+    near2 = sqrtf(sqrtf(m2 / p.strong_w4sq)) * 1.001f;
   }
+  const bool sfill = FILL && cls && !p.flags->soverflow;
+  int c1 = 0, c2 = 0, sc1 = 0, sc2 = 0;
+  int *out1 = nullptr, *out2 = nullptr;
+  if (FILL) {
+    out1 = p.nbr + p.nbr_off[k1];
+    out2 = p.nbr + p.nbr_off[k2];
+  }
+  int2 *so1 = nullptr, *so2 = nullptr;
+  if (sfill) {
+    so1 = p.snbr + p.snbr_off[k1];
+    so2 = p.snbr + p.snbr_off[k2];
+  }
+  const float rt = (float)(sqrt(p.rl2) * (1.0 + 1e-6) + 2e-7), rt2 = rt * rt;
+  auto strong = [&](int k, int j, float mk) {
+    const float4 mj = gmu[j];
+    const int4 si = p.s.xi[k], sj = p.s.xi[j];
+    const float sc = 2.3283064365386963e-10f;
+    const float dx = (float)(sj.x - si.x) * sc, dy = (float)(sj.y - si.y) * sc, dz = (float)(sj.z - si.z) * sc;
+    const float q2 = dx * dx + dy * dy + dz * dz, q4 = q2 * q2;
+    return mk * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > p.strong_w4sq * (q4 * q4);
+  };
+  const bool two = k2 > k1;
+  auto visit = [&](bool valid, int j, float ra, float rb) {
+    const bool in1 = valid && ra < rt2 && j != k1, in2 = valid && rb < rt2 && j != k2 && two;
+    const unsigned ma = __ballot_sync(kFull, in1), mb = __ballot_sync(kFull, in2);
+    unsigned j1 = (unsigned)j, j2 = (unsigned)j;
+    const bool n1 = in1 && ra < near1, n2 = in2 && rb < near2;
+    if (__any_sync(kFull, n1 || n2)) {
+      const bool s1 = n1 && strong(k1, j, m1), s2 = n2 && strong(k2, j, m2);
+      const unsigned sa = __ballot_sync(kFull, s1), sb = __ballot_sync(kFull, s2);
+      if (sfill && s1) {
+        so1[sc1 + __popc(sa & lanemask_lt())] = make_int2(k1, j);
+        j1 |= kStrong;
+      }
+      if (sfill && s2) {
+        so2[sc2 + __popc(sb & lanemask_lt())] = make_int2(k2, j);
+        j2 |= kStrong;
+      }
+      sc1 += __popc(sa);
+      sc2 += __popc(sb);
+    }
+    if (FILL) {
+      if (in1) out1[c1 + __popc(ma & lanemask_lt())] = (int)j1;
+      if (in2) out2[c2 + __popc(mb & lanemask_lt())] = (int)j2;
+    }
+    c1 += __popc(ma);
+    c2 += __popc(mb);
+  };
+  const int ncx = p.grid.ncx;
+  const float inv = 1.0f / (float)ncx;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (ncx > 1 && fmaxf(fmaxf(fabsf(ex), fabsf(ey)), fabsf(ez)) + 2.f * rt < 1.f - 2.f * inv) {
+    const float xlo = f1.x + fminf(ex, 0.f), xhi = f1.x + fmaxf(ex, 0.f);
+    const float ylo = f1.y + fminf(ey, 0.f), yhi = f1.y + fmaxf(ey, 0.f);
+    const float zlo = f1.z + fminf(ez, 0.f), zhi = f1.z + fmaxf(ez, 0.f);
+    auto cell = [&](float x) { return (int)floorf((x + 0.5f) * (float)ncx); };
+    const int cy0 = cell(ylo - rt), ny = cell(yhi + rt) - cy0 + 1, cz0 = cell(zlo - rt), nz = cell(zhi + rt) - cz0 + 1;
+    const int* cs = p.s.cell_start;
+    for (int rb = 0; rb < ny * nz; rb += 32) {
+      // lane: one row; a0, l0 / a1, l1: its x range, split at the box's end
+      const int r = rb + lane;
+      int a0 = 0, l0 = 0, a1 = 0, l1 = 0;
+      int code = 0;  // images (+1): x of the two segments, y, z, two bits each
+      if (r < ny * nz) {
+        const int uy = cy0 + r % ny, uz = cz0 + r / ny;
+        const float yc = uy * inv - 0.5f, zc = uz * inv - 0.5f;
+        const float dy = fmaxf(0.f, fmaxf(yc - yhi, ylo - yc - inv)), dz = fmaxf(0.f, fmaxf(zc - zhi, zlo - zc - inv));
+        const float d2 = dy * dy + dz * dz;
+        if (d2 < rt2) {
+          const float h = sqrtf(rt2 - d2);
+          const int x0 = cell(xlo - h), x1 = cell(xhi + h);
+          const int iy = uy < 0 ? 0 : (uy >= ncx ? 2 : 1), iz = uz < 0 ? 0 : (uz >= ncx ? 2 : 1);
+          const int* row = cs + ((uz - (iz - 1) * ncx) * ncx + (uy - (iy - 1) * ncx)) * ncx;
+          int i0 = 1, i1 = 1;
+          if (x0 < 0) {
+            a0 = row[x0 + ncx];
+            l0 = row[ncx] - a0;
+            a1 = row[0];
+            l1 = row[x1 + 1] - a1;
+            i0 = 0;
+          } else if (x1 >= ncx) {
+            a0 = row[x0];
+            l0 = row[ncx] - a0;
+            a1 = row[0];
+            l1 = row[x1 - ncx + 1] - a1;
+            i1 = 2;
+          } else {
+            a0 = row[x0];
+            l0 = row[x1 + 1] - a0;
+          }
+          code = i0 | i1 << 2 | iy << 4 | iz << 6;
+        }
+      }
+      const int nr = min(32, ny * nz - rb);
+      for (int q = 0; q < nr; q += 4) {
+        const int src = q + (lane >> 3);  // lanes past the last row hold empty ranges
+        const int b0 = __shfl_sync(kFull, a0, src), n0 = __shfl_sync(kFull, l0, src);
+        const int b1 = __shfl_sync(kFull, a1, src) - n0, len = n0 + __shfl_sync(kFull, l1, src);
+        const int cd = __shfl_sync(kFull, code, src);
+        const int top = __reduce_max_sync(kFull, len);
+        // a row of image i holds particles whose periodic copies lie i - 1 boxes on
+        const float xa = f1.x + (float)(1 - (cd & 3)), xb = f1.x + (float)(1 - (cd >> 2 & 3));
+        const float y = f1.y + (float)(1 - (cd >> 4 & 3)), z = f1.z + (float)(1 - (cd >> 6 & 3));
+        int t = lane & 7;
+        float4 nxt = t < len ? xf[(t < n0 ? b0 : b1) + t] : z4;
+        for (int t0 = 0; t0 < top; t0 += 8, t += 8) {
+          const float4 c = nxt;
+          const int j = (t < n0 ? b0 : b1) + t;
+          if (t + 8 < len) nxt = xf[(t + 8 < n0 ? b0 : b1) + t + 8];
+          const float dx = c.x - (t < n0 ? xa : xb), dy = c.y - y, dz = c.z - z;
+          const float gx = dx - ex, gy = dy - ey, gz = dz - ez;
+          visit(t < len, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
+        }
+      }
+    }
+  } else {
+    for (int j0 = 0; j0 < n; j0 += 32) {
+      const int j = j0 + lane;
+      const float4 c = j < n ? xf[j] : z4;
+      float dx = c.x - f1.x, dy = c.y - f1.y, dz = c.z - f1.z;
+      dx -= rintf(dx);
+      dy -= rintf(dy);
+      dz -= rintf(dz);
+      float gx = c.x - f2.x, gy = c.y - f2.y, gz = c.z - f2.z;
+      gx -= rintf(gx);
+      gy -= rintf(gy);
+      gz -= rintf(gz);
+      visit(j < n, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
+    }
+  }
+  if (!FILL && lane == 0) {
+    p.nbr_cnt[k1] = c1;
+    if (two) p.nbr_cnt[k2] = c2;
+    if (cls) {
+      p.snbr_cnt[k1] = sc1;
+      if (two) p.snbr_cnt[k2] = sc2;
+    }
+  }
+}
+
+template <typename T, bool FILL>
+__device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
+  if (!p.flags->rebuild) return;
+  if constexpr (std::is_same<T, float>::value)
+    nbr_build2<FILL>(p, bx);
+  else
+    nbr_build64<FILL>(p, bx);
 }
 
 // Exclusive scan of cnt[0, n) into off[0, n] by one block of 1024 threads;
@@ -909,176 +1018,207 @@ __device__ __forceinline__ void strong_chunks(const RealParams& p, int k, int la
 
 // ------------------------------------------------------------ evaluation
 
-template <typename T, bool FULL, bool COAT, int NW = kRealWarps>
-__device__ __forceinline__ void real_eval(const RealParams& p, int bx) {
-  using T4 = typename V4<T>::t;
-  constexpr bool F32 = std::is_same<T, float>::value;
-  __shared__ float4 q[NW][64];
+// Direct scan of particle k's cells when the list did not fit: in-range
+// candidates are compacted through the warp's queue q, eval(j) for each.
+template <typename T, typename E>
+__device__ __forceinline__ void direct_scan(const RealParams& p, int k, int lane, const Self<T>& me, int* q, E&& eval) {
+  int head = 0, tail = 0;
+  auto flush = [&](int cnt) {
+    __syncwarp();
+    const int j = lane < cnt ? q[(head + lane) & 63] : 0;
+    __syncwarp();
+    head += cnt;
+    if (lane < cnt) eval(j);
+  };
+  scan_rows<false, T>(p, k, lane, me, p.rc2, [&](bool in, int j, float) {
+    const unsigned mask = __ballot_sync(kFull, in);
+    if (in) q[(tail + __popc(mask & lanemask_lt())) & 63] = j;
+    tail += __popc(mask);
+    if (tail - head >= 32) flush(32);
+  });
+  if (tail - head > 0) flush(tail - head);
+}
+
+// FP64 path: one warp per particle, lanes take list entries.
+template <bool FULL, bool COAT, int NW>
+__device__ __forceinline__ void real_eval64(const RealParams& p, int bx) {
+  __shared__ int q[NW][64];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = bx * NW + wib;
   if (k >= p.n) return;  // whole warp; no block-level synchronisation below
-  if constexpr (F32 && !COAT) {
-    if (p.strong && !p.flags->overflow) strong_chunks<FULL>(p, k, lane);
-  }
-  Acc<T> a;
-  Acc2 a2;  // packed sums (mixed path list loop)
-  const T4 mi = ((const T4*)p.s.mu)[k];
-  const Self<T> me = load_self<T, COAT>(p, k);
-  const float rc2_fix = p.pk.rc2f;  // (rc / (L 2^-32))^2
-  const float wdc = (float)mi.w + p.pk.eps;  // own core radius + contact offset
-
-  // pair terms with the neighbour's loaded coordinates and moment (mixed path)
-  auto eval_loaded = [&](const int4& sj, const T4& mj) {
-    if constexpr (F32) {
-      // wrapping 32-bit differences are the exact minimum image
-      const float dxf = (float)(sj.x - me.si.x), dyf = (float)(sj.y - me.si.y), dzf = (float)(sj.z - me.si.z);
-      if (dxf * dxf + dyf * dyf + dzf * dzf < rc2_fix) {
-        const float sc = 2.3283064365386963e-10f;  // 2^-32
-        const float dx = dxf * sc, dy = dyf * sc, dz = dzf * sc;
-        pair_terms<FULL, COAT>(p, dx, dy, dz, dx * dx + dy * dy + dz * dz, mi, mj, me.oi, COAT ? sj.w : 0, a);
-      }
-    }
-  };
-  // pair terms of sorted particle j, with the in-range test
-  auto eval = [&](int j) {
-    if constexpr (F32) {
-      eval_loaded(p.s.xi[j], ((const T4*)p.s.mu)[j]);
-    } else {
-      pair64<FULL, COAT>(p, me.di, make_float4(me.x, me.y, me.z, me.w), mi, me.oi, j, a);
-    }
-  };
-
+  Acc<double> a;
+  const double4_32a mi = ((const double4_32a*)p.s.mu)[k];
+  const Self<double> me = load_self<double, COAT>(p, k);
+  const float4 mf = make_float4(me.x, me.y, me.z, me.w);
+  auto eval = [&](int j) { pair64<FULL, COAT>(p, me.di, mf, mi, me.oi, j, a); };
   if (!p.flags->overflow) {
-    // Verlet list of this particle
     const int* lst = p.nbr + p.nbr_off[k];
-    const int cnt = p.nbr_off[k + 1] - p.nbr_off[k];
-    if constexpr (F32) {
-      // two batches of 32 entries per iteration, all gathers issued first;
-      // the list indices of the next iteration are loaded one ahead, so a
-      // gather waits on one memory round trip instead of two
-      // entries with the sign bit set are strong pairs (FP64 kernels) when
-      // the context evaluates them there, ordinary ones otherwise
-      const int sflag = p.strong ? (int)0x80000000u : 0;
-      // the list is streamed once per pass: evict-first loads leave L1 to the
-      // neighbour gathers (0.3-0.9 % per step)
-      int ja_n = lane < cnt ? __ldcs(lst + lane) : k, jb_n = 32 + lane < cnt ? __ldcs(lst + 32 + lane) : k;
-      for (int t0 = 0; t0 < cnt; t0 += 64) {
-        const int ta = t0 + lane, tb = t0 + 32 + lane;
-        const bool va = ta < cnt, vb = tb < cnt;
-        const bool sta = (ja_n & sflag) != 0, stb = (jb_n & sflag) != 0;
-        const int ja = ja_n & 0x7fffffff, jb = jb_n & 0x7fffffff;
-        ja_n = ta + 64 < cnt ? __ldcs(lst + ta + 64) : k;
-        jb_n = tb + 64 < cnt ? __ldcs(lst + tb + 64) : k;
-        const int4 sa = p.s.xi[ja], sb = p.s.xi[jb];
-        const T4 ma = ((const T4*)p.s.mu)[ja], mb = ((const T4*)p.s.mu)[jb];
-        if constexpr (!COAT) {
-          // both neighbours in the halves of packed FP32 operations (the
-          // field + force pass assembles each pair in scalar code)
-          const float2 dxf = pk((float)(sa.x - me.si.x), (float)(sb.x - me.si.x));
-          const float2 dyf = pk((float)(sa.y - me.si.y), (float)(sb.y - me.si.y));
-          const float2 dzf = pk((float)(sa.z - me.si.z), (float)(sb.z - me.si.z));
-          const float2 r2f = fma2(dzf, dzf, fma2(dyf, dyf, mul2(dxf, dxf)));
-          const bool inA = va && r2f.x < rc2_fix, inB = vb && r2f.y < rc2_fix;
-          // unconditional: nearly every iteration has a pair in range, and
-          // entries out of range carry weight 0
-          pair_terms2<FULL>(p.pk, wdc, dxf, dyf, dzf, r2f, inA, inB, inA && !sta, inB && !stb, rc2_fix, mi, ma,
-                            mb, a, a2);
-        } else {
-          if (va) eval_loaded(sa, ma);
-          if (vb) eval_loaded(sb, mb);
-        }
-      }
-    } else {
-      int jn = lane < cnt ? lst[lane] : 0;
-      for (int t0 = 0; t0 < cnt; t0 += 32) {
-        const int j = jn & 0x7fffffff;
-        const bool valid = t0 + lane < cnt;
-        if (t0 + 32 + lane < cnt) jn = lst[t0 + 32 + lane];
-        if (valid) eval(j);
-      }
+    const int cnt = p.nbr_cnt[k];
+    int jn = lane < cnt ? lst[lane] : 0;
+    for (int t0 = 0; t0 < cnt; t0 += 32) {
+      const int j = jn;
+      const bool valid = t0 + lane < cnt;
+      if (t0 + 32 + lane < cnt) jn = lst[t0 + 32 + lane];
+      if (valid) eval(j);
     }
   } else {
-    // fallback: scan the cells; in-range candidates through the warp queue
-    int head = 0, tail = 0;
-    auto flush = [&](int cnt) {
-      __syncwarp();
-      const float4 e = lane < cnt ? q[wib][(head + lane) & 63] : make_float4(0, 0, 0, 0);
-      __syncwarp();
-      head += cnt;
-      if (lane < cnt) eval(__float_as_int(e.w));
-    };
-    scan_rows<false, T>(p, k, lane, me, p.rc2, [&](bool in, int j, float) {
-      const unsigned mask = __ballot_sync(kFull, in);
-      if (in) q[wib][(tail + __popc(mask & lanemask_lt())) & 63] = make_float4(0, 0, 0, __int_as_float(j));
-      tail += __popc(mask);
-      if (tail - head >= 32) flush(32);
-    });
-    if (tail - head > 0) flush(tail - head);
+    direct_scan<double>(p, k, lane, me, q[wib], eval);
   }
-
-  if constexpr (F32 && !FULL && !COAT) {
-    a.b0 += a2.b0.x + a2.b0.y;
-    a.b1 += a2.b1.x + a2.b1.y;
-    a.b2 += a2.b2.x + a2.b2.y;
-  }
-  T* B = (T*)p.B;
-  T* F = (T*)p.F;
-  T* O = (T*)p.ov;
+  double *B = (double*)p.B, *F = (double*)p.F, *O = (double*)p.ov;
   const int n = p.n;
-  if constexpr (F32) {
-    a.b0 = warp_sum(a.b0);
-    a.b1 = warp_sum(a.b1);
-    a.b2 = warp_sum(a.b2);
-    if constexpr (FULL) {
-      a.f0 = warp_sum(a.f0);
-      a.f1 = warp_sum(a.f1);
-      a.f2 = warp_sum(a.f2);
-      a.o0 = warp_sum(a.o0);
-      a.o1 = warp_sum(a.o1);
-      a.o2 = warp_sum(a.o2);
-      a.p0 = warp_sum(a.p0);
-      a.p1 = warp_sum(a.p1);
-      a.p2 = warp_sum(a.p2);
-      a.np = warp_sum(a.np);
-    }
-    if (lane == 0) {
-      B[k] = a.b0;
-      B[n + k] = a.b1;
-      B[2 * n + k] = a.b2;
-      if constexpr (FULL) {
-        F[k] = a.f0;
-        F[n + k] = a.f1;
-        F[2 * n + k] = a.f2;
-        O[k] = a.o0;
-        O[n + k] = a.o1;
-        O[2 * n + k] = a.o2;
-        p.Ppart[3 * k] = (double)a.p0;
-        p.Ppart[3 * k + 1] = (double)a.p1;
-        p.Ppart[3 * k + 2] = (double)a.p2;
-      }
-    }
-  } else if constexpr (FULL) {
+  if constexpr (FULL) {
     double v[16] = {a.b0, a.b1, a.b2, a.f0, a.f1, a.f2, a.p0, a.p1, a.p2, a.o0, a.o1, a.o2, 0, 0, 0, 0};
     const double s = warp_sums<16>(v, lane);
-    const int q = lane >> 1;
-    if ((lane & 1) == 0 && q < 12) {
-      if (q < 3)
-        B[q * n + k] = s;
-      else if (q < 6)
-        F[(q - 3) * n + k] = s;
-      else if (q < 9)
-        p.Ppart[3 * k + q - 6] = s;
+    const int c = lane >> 1;
+    if ((lane & 1) == 0 && c < 12) {
+      if (c < 3)
+        B[c * n + k] = s;
+      else if (c < 6)
+        F[(c - 3) * n + k] = s;
+      else if (c < 9)
+        p.Ppart[3 * k + c - 6] = s;
       else
-        O[(q - 9) * n + k] = s;
+        O[(c - 9) * n + k] = s;
     }
-    a.np = warp_sum(a.np);
   } else {
     double v[4] = {a.b0, a.b1, a.b2, 0};
     const double s = warp_sums<4>(v, lane);
     if ((lane & 7) == 0 && lane < 24) B[(lane >> 3) * n + k] = s;
   }
+}
+
+// Mixed path: one warp per particle, lanes take two list entries at a time in
+// the halves of packed FP32 operations.
+//
+// Bound: FP32 issue and the FMA pipe (see pair_terms2); 250 / 188 us for field +
+// force / field at N = 32768, 7.5e7 ordered pairs (273 / 193 with the arithmetic
+// before).  The list comes from DRAM, ~1 us away, longer than an iteration of a
+// warp, so its entries are loaded two iterations (128) ahead.
+//
+// A list per two particles (the union of their neighbours, each neighbour in
+// both halves: gathers and list bytes shared, everything packed) took 293 /
+// 182 us: the union is 14 % longer than one list, and the field + force pass
+// needs 96 registers.
+template <bool FULL, bool COAT, int NW>
+__device__ __forceinline__ void real_eval32(const RealParams& p, int bx) {
+  __shared__ int q[NW][64];
+  __shared__ float pushes[FULL ? NW : 1][3][32];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = bx * NW + wib;
+  if (k >= p.n) return;  // whole warp; no block-level synchronisation below
+  float* push = FULL ? &pushes[wib][0][lane] : nullptr;
+  if constexpr (FULL) push[0] = push[32] = push[64] = 0.f;
+  if constexpr (!COAT) {
+    if (p.strong && !p.flags->overflow) strong_chunks<FULL>(p, k, lane);
+  }
+  const int n = p.n;
+  const float4* gmu = (const float4*)p.s.mu;
+  const float4 mi = gmu[k];
+  Acc2 s;
+  if (!COAT && !p.flags->overflow) {
+    const int4 si = p.s.xi[k];
+    const float rc2_fix = p.pk.rc2f;  // (rc / (L 2^-32))^2
+    const float wdc = mi.w + p.pk.eps;  // own core radius + contact offset
+    const int* lst = p.nbr + p.nbr_off[k];
+    const int cnt = p.nbr_cnt[k];
+    // flags count only when the context evaluates the strong pairs in FP64
+    const unsigned fs = p.strong ? kStrong : 0u;
+    // the list is streamed once per pass: evict-first loads leave L1 to the gathers
+    auto entry = [&](int t) { return t < cnt ? (unsigned)__ldcs(lst + t) : (unsigned)k; };
+    auto process = [&](unsigned ea, unsigned eb, int t) {
+      const int ja = (int)(ea & kNbrIndex), jb = (int)(eb & kNbrIndex);
+      const int4 sa = p.s.xi[ja], sb = p.s.xi[jb];
+      const float4 ma = gmu[ja], mb = gmu[jb];
+      // wrapping 32-bit differences are the exact minimum image
+      const float2 dxf = pk((float)(sa.x - si.x), (float)(sb.x - si.x));
+      const float2 dyf = pk((float)(sa.y - si.y), (float)(sb.y - si.y));
+      const float2 dzf = pk((float)(sa.z - si.z), (float)(sb.z - si.z));
+      const float2 r2f = fma2(dzf, dzf, fma2(dyf, dyf, mul2(dxf, dxf)));
+      const bool inA = t < cnt && r2f.x < rc2_fix, inB = t + 32 < cnt && r2f.y < rc2_fix;
+      pair_terms2<FULL>(p.pk, wdc, dxf, dyf, dzf, r2f, inA, inB, inA && (ea & fs), inB && (eb & fs), mi, ma, mb, s,
+                        push);
+    };
+    unsigned n0 = entry(lane), n1 = entry(32 + lane), n2 = entry(64 + lane), n3 = entry(96 + lane);
+    for (int t = lane; t - lane < cnt; t += 128) {
+      const unsigned c0 = n0, c1 = n1, c2 = n2, c3 = n3;
+      n0 = entry(t + 128);
+      n1 = entry(t + 160);
+      n2 = entry(t + 192);
+      n3 = entry(t + 224);
+      process(c0, c1, t);
+      if (t - lane + 64 < cnt) process(c2, c3, t + 64);
+    }
+    if constexpr (FULL) {
+      s.f0 = fmaf(s.e, mi.x, s.f0);
+      s.f1 = fmaf(s.e, mi.y, s.f1);
+      s.f2 = fmaf(s.e, mi.z, s.f2);
+      s.p0 = fmaf(2.f * s.d0, mi.y, s.p0);
+      s.p1 = fmaf(2.f * s.d0, mi.z, s.p1);
+      s.p2 = fmaf(2.f * s.d1, mi.z, s.p2);
+      s.b0.x = fmaf(s.d0, 2.3283064365386963e-10f, s.b0.x);
+      s.b1.x = fmaf(s.d1, 2.3283064365386963e-10f, s.b1.x);
+      s.b2.x = fmaf(s.d2, 2.3283064365386963e-10f, s.b2.x);
+    }
+  } else {
+    // coating potentials, or the direct scan: scalar
+    const Self<float> me = load_self<float, COAT>(p, k);
+    Acc<float> a;
+    auto eval = [&](int j) {
+      const int4 sj = p.s.xi[j];
+      const float4 mj = gmu[j];
+      const float dxf = (float)(sj.x - me.si.x), dyf = (float)(sj.y - me.si.y), dzf = (float)(sj.z - me.si.z);
+      if (dxf * dxf + dyf * dyf + dzf * dzf < p.pk.rc2f) {
+        const float sc = 2.3283064365386963e-10f;  // 2^-32
+        const float dx = dxf * sc, dy = dyf * sc, dz = dzf * sc;
+        pair_terms<FULL, COAT>(p, dx, dy, dz, dx * dx + dy * dy + dz * dz, mi, mj, me.oi, COAT ? sj.w : 0, a);
+      }
+    };
+    if (!p.flags->overflow) {
+      const int* lst = p.nbr + p.nbr_off[k];
+      const int cnt = p.nbr_cnt[k];
+      int jn = lane < cnt ? lst[lane] : 0;
+      for (int t = lane; t < cnt; t += 32) {
+        const int j = jn & kNbrIndex;
+        if (t + 32 < cnt) jn = lst[t + 32];
+        eval(j);
+      }
+    } else {
+      direct_scan<float>(p, k, lane, me, q[wib], eval);
+    }
+    s.b0.x = a.b0;
+    s.b1.x = a.b1;
+    s.b2.x = a.b2;
+    if constexpr (FULL) {
+      s.f0 = -a.f0;
+      s.f1 = -a.f1;
+      s.f2 = -a.f2;
+      s.p0 = a.p0 * 4294967296.f;
+      s.p1 = a.p1 * 4294967296.f;
+      s.p2 = a.p2 * 4294967296.f;
+      push[0] = a.o0;
+      push[32] = a.o1;
+      push[64] = a.o2;
+    }
+  }
+  float *B = (float*)p.B, *F = (float*)p.F, *O = (float*)p.ov;
   if constexpr (FULL) {
-    if (lane == 0 && p.npairs) atomicAdd(p.npairs, (unsigned long long)a.np);
+    float v[16] = {s.b0.x, s.b1.x, s.b2.x, s.f0, s.f1, s.f2, s.p0, s.p1, s.p2, push[0], push[32], push[64], 0, 0, 0, 0};
+    const float t = warp_sums<16>(v, lane);
+    const int c = lane >> 1;
+    if ((lane & 1) == 0 && c < 12) {
+      if (c < 3)
+        B[c * n + k] = t;
+      else if (c < 6)
+        F[(c - 3) * n + k] = -t;
+      else if (c < 9)
+        p.Ppart[3 * k + c - 6] = (double)(t * 2.3283064365386963e-10f);
+      else
+        O[(c - 9) * n + k] = t;
+    }
+  } else {
+    float v[4] = {s.b0.x + s.b0.y, s.b1.x + s.b1.y, s.b2.x + s.b2.y, 0.f};
+    const float t = warp_sums<4>(v, lane);
+    if ((lane & 7) == 0 && lane < 24) B[(lane >> 3) * n + k] = t;
   }
 }
 
@@ -1093,7 +1233,6 @@ static int num_sms() {
   return nsm;
 }
 
-
 // ------------------------------------------------------------ entry points
 
 // Grid-stride over the particle blocks: most steps do not rebuild, and a
@@ -1105,13 +1244,49 @@ __global__ void __launch_bounds__(kRealWarps * 32) k_nbr_build(RealParams p, int
 }
 __global__ void __launch_bounds__(1024) k_nbr_scan(RealParams p) { nbr_scan(p, blockIdx.x); }
 // The FP32 passes without coating keep the occupancy of their pair loops
-// (field: 9 blocks of 4 warps per SM, 56 registers; field + force: 7 blocks,
+// (field: 8 blocks of 4 warps per SM, 64 registers; field + force: 7 blocks,
 // 72 registers): the FP64 strong-pair code in the same kernel must not
-// raise the register count.
+// raise the register count.  Measured at N = 32768: field + force 250 us at 7,
+// 259 at 6; field 186 at 8, 188 at 9, 246 at 10 (spills).
 template <typename T, bool FULL, bool COAT>
 __global__ void __launch_bounds__(((FULL && COAT) ? kRealWarps : kFieldWarps) * 32,
-                                  (std::is_same<T, float>::value && !COAT) ? (FULL ? 7 : 9) : 1) k_real(RealParams p) {
-  real_eval<T, FULL, COAT, (FULL && COAT) ? kRealWarps : kFieldWarps>(p, blockIdx.x);
+                                  (std::is_same<T, float>::value && !COAT) ? (FULL ? 7 : 8) : 1) k_real(RealParams p) {
+  constexpr int NW = (FULL && COAT) ? kRealWarps : kFieldWarps;
+  if constexpr (std::is_same<T, float>::value)
+    real_eval32<FULL, COAT, NW>(p, blockIdx.x);
+  else
+    real_eval64<FULL, COAT, NW>(p, blockIdx.x);
+}
+
+// In-range ordered pairs of the last evaluation's geometry.
+template <typename T>
+__global__ void __launch_bounds__(kRealWarps * 32) k_count_pairs(RealParams p, unsigned long long* out) {
+  __shared__ int q[kRealWarps][64];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, k = blockIdx.x * kRealWarps + wib;
+  if (k >= p.n) return;
+  int np = 0;
+  const Self<T> me = load_self<T, false>(p, k);
+  auto eval = [&](int j) {
+    if constexpr (std::is_same<T, float>::value) {
+      const int4 s = p.s.xi[j];
+      const float dx = (float)(s.x - me.si.x), dy = (float)(s.y - me.si.y), dz = (float)(s.z - me.si.z);
+      np += fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < p.pk.rc2f;
+    } else {
+      const double4_32a s = p.s.xd[j];
+      const float4 f = p.s.xf[j];
+      const double dx = fold64(me.di.x, s.x, me.x, f.x), dy = fold64(me.di.y, s.y, me.y, f.y),
+                   dz = fold64(me.di.z, s.z, me.z, f.z);
+      np += dx * dx + dy * dy + dz * dz < p.rc2;
+    }
+  };
+  if (!p.flags->overflow) {
+    const int b = p.nbr_off[k], e = b + p.nbr_cnt[k];
+    for (int t = b + lane; t < e; t += 32) eval(p.nbr[t] & kNbrIndex);
+  } else {
+    direct_scan<T>(p, k, lane, me, q[wib], eval);
+  }
+  np = __reduce_add_sync(kFull, np);
+  if (lane == 0) atomicAdd(out, (unsigned long long)np);
 }
 
 // persistent: blocks stride over the task table (see md_cells.cu); the
@@ -1130,24 +1305,36 @@ __global__ void __launch_bounds__(1024) k_nbr_scan_packed(const RealParams* __re
   nbr_scan(p, blockIdx.y);
 }
 // the block shape of the single-system passes (k_real): 8 warps with
-// coating in the field + force pass, otherwise 4; 6 (field + force) or 7
-// (field) blocks per SM, one fewer than k_real's 7 / 9: the task loop
-// around the pair loop needs the registers (at 7 / 9 both spilled, and the
-// field sweep ran 1.1 % slower)
+// coating in the field + force pass, otherwise 4; 6 (field + force) or 8
+// (field) blocks per SM (32 systems of 500 to 4000 particles: 6.85 ms per five
+// steps; 6.92 at 6 / 7, 6.97 at 5 / 7)
 template <bool FULL, bool COAT>
-__global__ void __launch_bounds__(((FULL && COAT) ? kRealWarps : kFieldWarps) * 32, COAT ? 2 : (FULL ? 6 : 7))
+__global__ void __launch_bounds__(((FULL && COAT) ? kRealWarps : kFieldWarps) * 32, COAT ? 2 : (FULL ? 6 : 8))
     k_real_packed(const RealParams* __restrict__ ps, const Task* __restrict__ tk, int ntask, WorkQ* wq) {
   for_tasks<false>(tk, ntask, wq, [&](const Task& t) {
-      real_eval<float, FULL, COAT, (FULL && COAT) ? kRealWarps : kFieldWarps>(ps[t.rep], t.blk);
+      real_eval32<FULL, COAT, (FULL && COAT) ? kRealWarps : kFieldWarps>(ps[t.rep], t.blk);
   });
+}
+
+// Share of an SM's 228 KB that the FP32 passes ask for as shared memory, in
+// percent; the rest is the L1 cache, which serves their gathers (85 % of
+// its throughput in the field pass).  They need 25 KB.  Left to itself the driver
+// widens the shared part for the k-space kernels on the other stream, and the
+// two run each other down: per step at N = 32768 (131072) 779 us (5.07 ms),
+// slower than one after the other (715 us, 4.33 ms); at 16 % 672 us (4.27 ms), at
+// 60 % 769 us (4.96 ms); 32 small systems together 7.35 -> 6.85 ms per five steps.
+constexpr int kRealCarveout = 16;
+static void keep_l1(const void* kern) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, kRealCarveout);
 }
 
 int real_blocks(int n) { return (n + kRealWarps - 1) / kRealWarps; }
 int real_pass_blocks(int n) { return (n + kFieldWarps - 1) / kFieldWarps; }
+int nbr_blocks(int n, bool fp64) { return real_blocks(fp64 ? n : (n + 1) / 2); }
 
 int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64) {
   const int nsm = num_sms();
-  const int nblk = real_blocks(p.n);
+  const int nblk = nbr_blocks(p.n, fp64);
   dim3 grid(std::min(nblk, 8 * nsm)), block(kRealWarps * 32);
   if (fp64)
     k_nbr_build<double, false><<<grid, block, 0, st>>>(p, nblk);
@@ -1162,6 +1349,13 @@ int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64
   return 3;
 }
 
+void launch_count_pairs(cudaStream_t st, const RealParams& p, unsigned long long* out, bool fp64) {
+  if (fp64)
+    k_count_pairs<double><<<real_blocks(p.n), kRealWarps * 32, 0, st>>>(p, out);
+  else
+    k_count_pairs<float><<<real_blocks(p.n), kRealWarps * 32, 0, st>>>(p, out);
+}
+
 int launch_real(cudaStream_t st, const RealParams& p, bool full, bool fp64) {
   const int nw = (full && p.coat) ? kRealWarps : kFieldWarps;
   dim3 grid((p.n + nw - 1) / nw), block(nw * 32);
@@ -1172,6 +1366,8 @@ int launch_real(cudaStream_t st, const RealParams& p, bool full, bool fp64) {
     else
       k_real<double, false, false><<<grid, block, 0, st>>>(p);
   } else {
+    keep_l1((const void*)k_real<float, true, false>);
+    keep_l1((const void*)k_real<float, false, false>);
     if (full)
       p.coat ? k_real<float, true, true><<<grid, block, 0, st>>>(p)
              : k_real<float, true, false><<<grid, block, 0, st>>>(p);
@@ -1195,6 +1391,8 @@ int launch_nbr_packed(cudaStream_t st, const RealParams* ps, int R, const Packed
 
 int launch_real_packed(cudaStream_t st, const RealParams* ps, const Packed& real, const Packed& pass, bool full,
                        bool coat) {
+  keep_l1((const void*)k_real_packed<true, false>);
+  keep_l1((const void*)k_real_packed<false, false>);
   auto go = [&](auto kern, const Packed& tb, int th) {
     kern<<<persistent_grid((const void*)kern, th, 0, tb.n), th, 0, st>>>(ps, tb.tasks, tb.n, tb.wq);
   };

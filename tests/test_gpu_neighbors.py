@@ -50,3 +50,30 @@ def test_list_overflow_falls_back_to_cell_scan(prec, tol):
     assert sim.neighbor_capacity() == used
     assert O.rms_rel(B2, Bo, bAl) < tol and O.rms_rel(F2, Fo, fAl) < tol
     assert O.rms_rel(B0, Bo, bAl) < tol
+
+
+@pytest.mark.parametrize("n,rc_frac", [(2, 0.45), (3, 0.4), (33, 0.5), (64, 0.25), (257, 0.35), (1001, 0.3),
+                                       (2999, 0.2), (4096, 0.12)])
+def test_lists_built_for_two_particles_at_once(n, rc_frac):
+    """Mixed path: one warp lists the neighbours of two consecutive sorted
+    particles (odd counts, one-cell grids, boxes that do not fit the periodic
+    cell and fine grids).  Every pair within rc is found, on either path, and
+    the pressure, whose terms along the own moment are taken from the field's
+    sums, equals the oracle's (TOL_MIXED of a contact force times rc per
+    particle)."""
+    ini, g = random_system(n, seed=53 + n, rc_frac=rc_frac, lognormal=n % 2 == 1)
+    fAl, bAl, _ = scales(ini, g)
+    x = g["pos"]
+    want = 0
+    for i in range(n):
+        d = x[:, i + 1:] - x[:, i:i + 1]
+        d -= g["lBox"] * np.rint(d / g["lBox"])
+        want += int(((d ** 2).sum(0) < g["rc"] ** 2).sum())
+    Bo, Fo, Po = oracle_system(ini, g).compute_interactions()
+    for prec in (0, 1):
+        sim = gpu_system(ini, g, prec)
+        B, F, P = sim.CompInteractions()
+        assert sim.pairs() == want
+        tol = TOL_MIXED if prec else TOL_FP64
+        assert O.rms_rel(B, Bo, bAl) < tol and O.rms_rel(F, Fo, fAl) < tol
+        np.testing.assert_allclose(P, Po, rtol=0, atol=tol * fAl * g["rc"] * n)
