@@ -58,7 +58,7 @@ enum {
 
 /* Reciprocal-space engine of the mixed path (md_set_kspace_engine). */
 enum {
-  MD_KSPACE_AUTO = 0, /* tensor cores when kc allows, else the FP32 kernels   */
+  MD_KSPACE_AUTO = 0, /* by size: see md_kspace_engine_active                  */
   MD_KSPACE_SIMT = 1, /* FP32 CUDA-core kernels (row segments, phase recurrences) */
   MD_KSPACE_TC = 2    /* tensor cores (3-pass TF32 matrix products over k rows) */
 };
@@ -201,7 +201,8 @@ int md_set_kspace_engine(md_ctx* ctx, int engine);
 /* *tensor_cores = 1 when the current Ewald parameters are those of the tensor
  * cores.  With MD_KSPACE_AUTO and the default tiling, systems too small to
  * fill them (about 3e6 k vectors x particles) evaluate the same k rows on the
- * CUDA cores under that setting; MD_KSPACE_TC always takes the tensor cores. */
+ * CUDA cores under that setting, and systems of 1e8 and more take the same sums
+ * through a mesh; MD_KSPACE_TC always takes the tensor cores. */
 int md_kspace_engine_active(const md_ctx* ctx, int* tensor_cores);
 /* Tiling of the tensor-core structure factor (no counterpart in the
  * reference; the autotuner's knobs): ring = the operand-ring option (0..5,

@@ -20,7 +20,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(OUT, "libmd_gb300.so")
 EXE = os.path.join(OUT, "md_run")
 
-CUDA_SOURCES = ["md_cells.cu", "md_real.cu", "md_kspace.cu", "md_krows.cu", "md_integrate.cu", "md_ctx.cu", "md_batch.cu",
+CUDA_SOURCES = ["md_cells.cu", "md_real.cu", "md_kspace.cu", "md_krows.cu", "md_kmesh.cu", "md_integrate.cu", "md_ctx.cu", "md_batch.cu",
                 "md_noalloc.cu", "md_post.cu", "md_ktc.cu",
                 "md_place.cu"]
 HOST_SOURCES = ["md_host.cpp", "md_serve.cpp", "md_io.cpp"]

@@ -318,6 +318,17 @@ struct KParams {
   const double2* rw_row;    // [R] (ny, nz)
   const int2* rw_rowt;      // [R] first task, tasks
   void* rw_ad;              // [T][4] T4 (A, D)
+  // k space through a mesh (md_kmesh.cu; gm_M = 0: off)
+  int gm_M, gm_nbrick;     // mesh points per axis, bricks of the spread
+  int gm_ncx;              // cells per axis of the sorted view
+  float gm_reach;          // distance a particle may be from the cell it is filed in, box units
+  const float* gm_coef;    // [kMeshW][kMeshDeg + 1] window polynomials, lowest order first
+  const float2* gm_fac;    // [R][2 kc + 1] e(n) / omega^6(n), 1 / omega^3(n) of the rows' k vectors
+  const float2* gm_tw;     // [M] exp(2 pi i j / M)
+  float* gm_part;          // [bricks][3][padded brick]
+  float2* gm_z;            // [3][kc + 1][M][M] after the z axis
+  float4 *gm_y, *gm_t;     // [kc + 1][2 kc + 1][M] rows before and after the x axis
+  float4* gm_b;            // [M][M][M] field mesh
   long long tc_wait;     // SM clock cycles after which an mbarrier wait gives up
   int* err;              // device error word (kErrTcWait on a wait that gave up)
 };

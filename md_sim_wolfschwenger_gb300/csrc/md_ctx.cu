@@ -281,6 +281,19 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.rw_row = c->rw_row;
   p.rw_rowt = c->rw_rowt;
   p.rw_ad = c->rw_ad;
+  p.gm_M = c->gm_M;
+  if (c->gm_M > 0) p.gm_nbrick = md::mesh_bricks(c->gm_M);
+  p.gm_ncx = c->grid.ncx;
+  // half the skin since the build, and rounding
+  p.gm_reach = (float)(0.5 * c->skin_frac * c->rc / c->L * (1.0 + 1e-5) + 2e-6);
+  p.gm_coef = c->gm_coef;
+  p.gm_fac = c->gm_fac;
+  p.gm_tw = c->gm_tw;
+  p.gm_part = c->gm_part;
+  p.gm_z = c->gm_z;
+  p.gm_y = c->gm_y;
+  p.gm_t = c->gm_t;
+  p.gm_b = c->gm_b;
   p.tc_wait = c->tc_wait;
   p.err = &c->sc->err;
   return p;
@@ -753,10 +766,82 @@ static int setup_rows(md_ctx* c) {
   return MD_OK;
 }
 
+// Whether the mixed path's default engine goes through a mesh (md_kmesh.cu)
+// instead of the tensor cores: systems of 1e8 (k, particle) terms and more, whose
+// products outweigh the mesh's six dependent launches.  Measured step times, mesh
+// against tensor cores: N = 12000, kc = 12 (0.4e8 terms) 214 / 187 us, N = 20011,
+// kc = 15 (1.4e8) 348 / 387, N = 32768, kc = 15 (2.3e8) 614 / 662, N = 131072,
+// kc = 20 (2.2e9) 3159 / 4186.  Errors of the k-space part against FP64 (rms,
+// N = 32768): field 1.5e-7 / 1.2e-6, force 2.8e-7 / 1.3e-6.  An engine or a
+// tensor-core tiling that the caller chose is kept.
+static bool mesh_wanted(const md_ctx* c) {
+  const double nk = 2.0943951 * (double)c->kc * (double)c->kc * (double)c->kc;  // half space
+  return !fp64(c) && c->kengine == MD_KSPACE_AUTO && c->tc_ring < 0 && c->tc_waves == 1 && c->tc_rows > 0 &&
+         c->kc >= md::kMeshMinKc && nk * (double)c->n >= 1e8;
+}
+
+// k space through a mesh: window tables and the mesh in its stages (md_kmesh.cu).
+static int setup_mesh(md_ctx* c) {
+  c->gm_M = 0;
+  if (!mesh_wanted(c)) return MD_OK;
+  const int kc = (int)c->kc, M = md::mesh_points(kc), nb = md::mesh_bricks(M);
+  const size_t kc1 = (size_t)kc + 1, rows = kc1 * (2 * (size_t)kc + 1), M2 = (size_t)M * M;
+  const mdh::MeshTables t = mdh::mesh_tables(kc, M);
+  // factors in the layout of tc_kmap: row, nx
+  const int Q = 2 * kc + 1;
+  std::map<std::pair<int, int>, int> rowid;
+  for (int k = 0; k < c->klist.nk; k++)
+    if (c->klist.kreal[k]) rowid[{c->klist.kz[k], c->klist.ky[k]}] = 0;
+  int nr = 0;
+  for (auto& e : rowid) e.second = nr++;
+  std::vector<float2> fac((size_t)nr * Q, make_float2(0.f, 0.f));
+  for (int k = 0; k < c->klist.nk; k++)
+    if (c->klist.kreal[k]) {
+      const int nx = c->klist.kx[k], ny = c->klist.ky[k], nz = c->klist.kz[k];
+      const double d = t.dec[std::abs(nx)] * t.dec[std::abs(ny)] * t.dec[nz];
+      fac[(size_t)rowid[{nz, ny}] * Q + nx + kc] = make_float2((float)(c->klist.ek[k] * d * d), (float)d);
+    }
+  std::vector<float2> tw(M);
+  for (int j = 0; j < M; j++) {
+    const double a = 2.0 * std::acos(-1.0) * j / M;
+    tw[j] = make_float2((float)std::cos(a), (float)std::sin(a));
+  }
+  void* old[] = {c->gm_coef, c->gm_fac, c->gm_tw, c->gm_part, c->gm_z, c->gm_y, c->gm_t, c->gm_b};
+  for (void* q : old) dfree(c, q);
+  c->gm_coef = nullptr;
+  c->gm_fac = nullptr;
+  c->gm_tw = nullptr;
+  c->gm_part = nullptr;
+  c->gm_z = nullptr;
+  c->gm_y = c->gm_t = c->gm_b = nullptr;
+  int st;
+  if ((st = dalloc(c, &c->gm_coef, sizeof(float) * t.coef.size()))) return st;
+  if ((st = dalloc(c, &c->gm_fac, sizeof(float2) * fac.size()))) return st;
+  if ((st = dalloc(c, &c->gm_tw, sizeof(float2) * (size_t)M))) return st;
+  if ((st = dalloc(c, &c->gm_part, sizeof(float) * md::mesh_part_floats(M)))) return st;
+  if ((st = dalloc(c, &c->gm_z, sizeof(float2) * 3 * kc1 * M2))) return st;
+  if ((st = dalloc(c, &c->gm_y, sizeof(float4) * rows * M))) return st;
+  if ((st = dalloc(c, &c->gm_t, sizeof(float4) * rows * M))) return st;
+  if ((st = dalloc(c, &c->gm_b, sizeof(float4) * M2 * M))) return st;
+  if (nb > c->musum_cap) {
+    dfree(c, c->musum_part);
+    c->musum_part = nullptr;
+    c->musum_cap = 0;
+    if ((st = dalloc(c, &c->musum_part, 24 * (size_t)nb))) return st;
+    c->musum_cap = nb;
+  }
+  CK(c, cudaMemcpy(c->gm_coef, t.coef.data(), sizeof(float) * t.coef.size(), cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->gm_fac, fac.data(), sizeof(float2) * fac.size(), cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->gm_tw, tw.data(), sizeof(float2) * (size_t)M, cudaMemcpyHostToDevice));
+  c->gm_M = M;
+  return MD_OK;
+}
+
 // The k-space engine of the current parameters.
 static int setup_engine(md_ctx* c) {
-  const int st = setup_tc(c);
-  return st ? st : setup_rows(c);
+  int st = setup_tc(c);
+  if (!st) st = setup_rows(c);
+  return st ? st : setup_mesh(c);
 }
 
 extern "C" {

@@ -128,6 +128,14 @@ struct md_ctx {
   double2* rw_row = nullptr;
   int2* rw_rowt = nullptr;
   void* rw_ad = nullptr;
+  // k space through a mesh (md_kmesh.cu; gm_M = 0 while it is off)
+  int gm_M = 0;
+  float* gm_coef = nullptr;
+  float2* gm_fac = nullptr;
+  float2* gm_tw = nullptr;
+  float* gm_part = nullptr;
+  float2* gm_z = nullptr;
+  float4 *gm_y = nullptr, *gm_t = nullptr, *gm_b = nullptr;
   // tensor-core k space (mixed path; md_ktc.cu): engine choice, k rows and
   // their buffers (tc_rows = 0 while the engine is off)
   int kengine = MD_KSPACE_AUTO;

@@ -629,6 +629,52 @@ RealTables real_tables64(double irPi) {
   return r;
 }
 
+// ====================================================== window of the mesh
+
+MeshTables mesh_tables(int kc, int M) {
+  const double pi = std::acos(-1.0);  // of the discrete transform itself
+  constexpr int W = md::kMeshW, D = md::kMeshDeg, N = D + 1;
+  const double beta = 2.3 * W;
+  auto omega = [&](double z) {
+    const double t = 2.0 * z / W, q = 1.0 - t * t;
+    return std::exp(beta * (std::sqrt(q > 0 ? q : 0.0) - 1.0));
+  };
+  MeshTables r;
+  r.dec.assign(kc + 1, 0.0);
+  for (int j = 0; j < W; j++) {
+    // Chebyshev interpolation on the interval, then powers of s
+    double c[N] = {}, pw[N] = {};
+    for (int k = 0; k < N; k++)
+      for (int i = 0; i < N; i++) {
+        const double th = pi * (i + 0.5) / N;
+        c[k] += (k ? 2.0 : 1.0) / N * std::cos(k * th) * omega(-0.5 * W + j + 0.5 * (std::cos(th) + 1.0));
+      }
+    double t0[N] = {1.0}, t1[N] = {0.0, 1.0};  // T_{k-1}, T_k
+    for (int q = 0; q < N; q++) pw[q] = c[0] * t0[q] + c[1] * t1[q];
+    for (int k = 2; k < N; k++) {
+      double t2[N];
+      for (int q = 0; q < N; q++) t2[q] = (q ? 2.0 * t1[q - 1] : 0.0) - t0[q];
+      for (int q = 0; q < N; q++) {
+        pw[q] += c[k] * t2[q];
+        t0[q] = t1[q];
+        t1[q] = t2[q];
+      }
+    }
+    for (int q = 0; q < N; q++) r.coef.push_back((float)pw[q]);
+    // transform of the FP32 polynomial: Simpson's rule, 256 intervals of 1 / 256
+    const float* f = &r.coef[(size_t)j * N];
+    for (int i = 0; i <= 256; i++) {
+      const double s = i / 128.0 - 1.0, z = -0.5 * W + j + i / 256.0;
+      double v = 0.0;
+      for (int q = D; q >= 0; q--) v = v * s + f[q];
+      v *= (i == 0 || i == 256 ? 1.0 : (i % 2 ? 4.0 : 2.0)) / 768.0;
+      for (int n = 0; n <= kc; n++) r.dec[n] += v * std::cos(2.0 * pi * n * z / M);
+    }
+  }
+  for (double& v : r.dec) v = 1.0 / v;
+  return r;
+}
+
 // ============================================================ cell grid
 
 // Cells of edge >= rc / reach; a stencil of +-reach cells must not wrap onto

@@ -82,6 +82,15 @@ struct RealTables {
 };
 RealTables real_tables64(double irPi);
 
+// Window of the k-space mesh (md_kmesh.cu): coef, its polynomial on each unit
+// interval in s = 2 frac - 1 [kMeshW][kMeshDeg + 1], lowest order first; dec, one
+// over its Fourier transform at n / M for n = 0 .. kc.
+struct MeshTables {
+  std::vector<float> coef;
+  std::vector<double> dec;
+};
+MeshTables mesh_tables(int kc, int M);
+
 // ----------------------------------------------------------- cell grid
 md::CellGrid choose_grid(double rc_box, int64_t n, int reach);
 

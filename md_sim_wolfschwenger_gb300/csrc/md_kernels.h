@@ -129,6 +129,13 @@ struct RowShape {
 };
 RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
 int launch_phase_rows(cudaStream_t st, const KParams& p, bool fp64);
+// k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks and
+// partial-mesh floats of the spread.
+constexpr int kMeshMinKc = 5;  // M >= 24: a window and its neighbour bricks do not wrap onto themselves
+inline int mesh_points(int kc) { return 8 * ((kc + 1) / 2); }
+int mesh_bricks(int M);
+size_t mesh_part_floats(int M);
+int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev);
 int launch_krows(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaEvent_t* ev);
 // Per-particle phase tables (once per step; positions are frozen across the
 // two Heun stages).

@@ -447,6 +447,7 @@ static void scatter_launch(cudaStream_t st, const KParams& p, bool full, size_t 
 
 int launch_kspace(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaEvent_t* ev) {
   if (p.rw_T > 0) return launch_krows(st, p, full, fp64, ev);
+  if (p.gm_M > 0) return launch_kmesh(st, p, full, ev);
   if (p.tc_rows > 0) return launch_kspace_tc(st, p, full, ev);
   const size_t sm1 = ksf_smem(p.kc);
   cudaFuncSetAttribute(k_sk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
@@ -465,6 +466,7 @@ int launch_kspace(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaE
 
 int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64) {
   if (p.rw_T > 0) return launch_phase_rows(st, p, fp64);
+  if (p.gm_M > 0) return 0;  // the mesh takes the coordinates themselves
   k_phase_tables<<<phase_blocks(p.n), kPhaseThreads, 0, st>>>(p);
   if (p.tc_rows > 0) return 1 + launch_kspace_tc_prep(st, p);
   return 1;

@@ -30,4 +30,8 @@ constexpr int kScatterParts = 4;
 constexpr int kGIntervals = 768;
 constexpr int kEEntries = 36 * 64 + 2;
 
+// k space through a mesh (md_kmesh.cu): window width in mesh points, degree of
+// its polynomials
+constexpr int kMeshW = 9, kMeshDeg = 12;
+
 }  // namespace md

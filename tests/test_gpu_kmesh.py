@@ -1,0 +1,61 @@
+"""k space of large mixed systems through a mesh (md_kmesh.cu) against the FP64
+path: the same CompDipInteractEwaldF / CompDipFieldEwaldF sums
+(src/interaction.cpp:429-514, 588-672)."""
+import numpy as np
+import pytest
+
+from helpers import gpu_system, random_system
+from test_gpu_parity import random_system_fast
+
+pytestmark = pytest.mark.gpu
+
+# The window's error is 4e-9 (field) and 2.4e-7 (force) of the k-space part, the
+# FP32 sums of ~100 terms add ~3e-7.
+TOL = 1e-6
+
+
+def k_part(sim, mm):
+    B, F, _ = sim.CompInteractions()
+    Br, Fr = sim.debug_real_part()
+    k = sim.debug_structure_factor()
+    return B - Br, F - Fr, k[:, 3] + 1j * k[:, 4], sim.CompDemagField(mm)
+
+
+def rms(a, b):
+    return np.sqrt(np.mean(np.abs(a - b) ** 2) / np.mean(np.abs(b) ** 2))
+
+
+# sizes just above the engine's threshold (1e8 k vectors x particles), with meshes of
+# whole and partial bricks (M = 104, 88, 72, 64, 48, 32), a one-cell grid (3101), odd
+# counts
+@pytest.mark.parametrize("n,kc,rc_frac", [(3101, 25, 0.45), (5000, 22, 0.3), (8501, 18, 0.25), (12000, 16, 0.2),
+                                          (47001, 11, 0.12), (100000, 8, 0.1)])
+def test_k_part_against_fp64(n, kc, rc_frac):
+    ini, g = random_system_fast(n, seed=n, phi=0.10, B0=0.02)
+    g["rc"], g["kc"] = rc_frac * g["lBox"], kc
+    g["alpha"] = 3.5 / g["rc"]
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref = k_part(gpu_system(ini, g, 0), mm)
+    sim = gpu_system(ini, g, 1)
+    sim.set_strong_pairs(0.0)  # their FP64 terms are not in the real part that is taken off
+    got = k_part(sim, mm)
+    assert rms(got[0], ref[0]) < TOL
+    assert rms(got[1], ref[1]) < TOL
+    assert rms(got[2], ref[2]) < TOL
+    assert rms(got[3], ref[3]) < TOL
+    again = k_part(sim, mm)
+    assert all(np.array_equal(a, b) for a, b in zip(got, again))
+
+
+def test_particles_far_from_their_cells():
+    """A skin of rc: the bricks' particles come from all cells they may have
+    drifted from; the result stays that of a fresh sort."""
+    n = 20011
+    ini, g = random_system_fast(n, seed=5, phi=0.10, B0=0.02)
+    sim = gpu_system(ini, g, 1)
+    mm = np.roll(g["mm"], 1, axis=1)
+    a = k_part(sim, mm)
+    sim.set_neighbor_skin(1.0)
+    b = k_part(sim, mm)
+    for q in (2, 3):
+        assert rms(b[q], a[q]) < TOL
