@@ -51,6 +51,7 @@ struct StepFlags {
   int overflow;       // the neighbour list did not fit: real space scans cells
   int force;          // host request: rebuild on the next step
   unsigned maxdisp;   // float bits of the largest displacement since the build (box units)
+  int refill;         // a neighbour list was longer than its share: the lists lie one after another
   int soverflow;      // the strong-pair list did not fit: every pair stays on the FP32 path
 };
 
@@ -198,6 +199,7 @@ struct RealParams {
   int* nbr_cnt;               // [n]
   int* nbr_off;               // [n + 1]
   long long nbr_cap;
+  int nbr_share;              // entries per list while every list fits that many (nbr_cap / n)
   StepFlags* flags;           // rebuild / overflow
   // Strong pairs (mixed path): list entries with |mu_i|^2 |mu_j|^2 >
   // strong_w4sq r^8 at the build (box units, moments in mu_max) carry the

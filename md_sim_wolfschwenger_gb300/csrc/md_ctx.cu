@@ -169,6 +169,7 @@ RealParams real_params(md_ctx* c, void* B, void* F, void* ov) {
   p.nbr_cnt = c->nbr_cnt;
   p.nbr_off = c->nbr_off;
   p.nbr_cap = c->nbr_cap;
+  p.nbr_share = (int)(std::min<long long>(c->nbr_cap, 0x7fffffff) / c->n);
   p.flags = &c->sc->flags;
   if (strong_active(c)) {
     p.strong = 1;

@@ -18,7 +18,8 @@
 // against rc like the reference.  Build: FP64 path one warp per particle
 // (nbr_build64), mixed path one warp per two (nbr_build2); a warp walks the rows
 // of its cell stencil, culled to the cells that intersect the search sphere,
-// and a ballot compacts the hits (count pass, prefix sum, fill pass).  If the
+// and a ballot compacts the hits (a pass into equal shares of the list's memory; a
+// second one, after a prefix sum, when a share was too small).  If the
 // list does not fit its capacity the evaluation scans the cells directly, with
 // in-range pairs compacted into a per-warp shared-memory queue (correct,
 // slower); the host then grows the list.
@@ -573,26 +574,32 @@ __device__ __forceinline__ void scan_rows(const RealParams& p, int k, int lane, 
 
 // ------------------------------------------------------- neighbour list
 
-// FP64 path: count (FILL = false) or write (FILL = true) the neighbours of
-// each particle within rc + skin, one warp per particle.
-template <bool FILL>
+// FP64 path: the neighbours of each particle within rc + skin, one warp per
+// particle, into its share of the list's memory, or (SECOND) anew when one was
+// longer than that (see nbr_build2).
+template <bool SECOND>
 __device__ __forceinline__ void nbr_build64(const RealParams& p, int bx) {
-  if (FILL && p.flags->overflow) return;
+  if (SECOND && (p.flags->overflow || !p.flags->refill)) return;
   const int lane = threadIdx.x & 31, k = bx * kRealWarps + (threadIdx.x >> 5);
   if (k >= p.n) return;
   const Self<double> me = load_self<double, false>(p, k);
+  const int off = SECOND ? p.nbr_off[k] : k * p.nbr_share, room = SECOND ? 0x7fffffff : p.nbr_share;
   int cnt = 0;
-  int* out = FILL ? p.nbr + p.nbr_off[k] : nullptr;
+  int* out = p.nbr + off;
   auto visit = [&](bool in, int j, float) {
     const unsigned mask = __ballot_sync(kFull, in);
-    if (FILL && in) out[cnt + __popc(mask & lanemask_lt())] = j;
+    const int at = cnt + __popc(mask & lanemask_lt());
+    if (in && at < room) out[at] = j;
     cnt += __popc(mask);
   };
   if (p.grid.ncx > 1)
     scan_rows<true, double>(p, k, lane, me, p.rl2, visit);
   else
     scan_rows<false, double>(p, k, lane, me, p.rl2, visit);
-  if (!FILL && lane == 0) p.nbr_cnt[k] = cnt;
+  if (!SECOND && lane == 0) {
+    p.nbr_cnt[k] = cnt;
+    p.nbr_off[k] = off;
+  }
 }
 
 // Mixed path: one warp builds the lists of two consecutive sorted particles
@@ -609,26 +616,33 @@ __device__ __forceinline__ void nbr_build64(const RealParams& p, int bx) {
 //
 // With strong pairs on, each neighbour is also classified per particle
 // (|mu_i|^2 |mu_j|^2 > strong_w4sq r^8 at this build): strong entries carry the
-// sign bit in the list and are copied, as (i, j), into the strong list (unless
-// that list overflowed in the count).  A pair is classified, with its
-// moment and fixed-point distance fetched, only when it is near enough for
-// the largest moment to make it strong.
+// sign bit in the list and are copied, as (i, j), into the strong list.  A pair is
+// classified, with its moment and fixed-point distance fetched, only when it is
+// near enough for the largest moment to make it strong.
+//
+// The first pass writes each list into an equal share of the capacity (1.3 times
+// the mean and 64 entries, where the system is uniform) and counts; the second
+// fills the strong list, from the near pairs alone, and writes the lists again,
+// one after another, when one did not fit its share.  Counting first and filling
+// after the scan took 119 + 161 us at N = 20011, this 150 + 36.
 constexpr unsigned kStrong = 0x80000000u;
 constexpr int kNbrIndex = 0x7fffffff;
 
-template <bool FILL>
+template <bool SECOND>
 __device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
-  if (FILL && p.flags->overflow) return;
+  const bool refill = SECOND && p.flags->refill, cls = p.strong, sfill = SECOND && cls && !p.flags->soverflow;
+  if (SECOND && (p.flags->overflow || !(refill || sfill))) return;
   const int lane = threadIdx.x & 31, w = bx * kRealWarps + (threadIdx.x >> 5);
   const int n = p.n, k1 = 2 * w, k2 = min(k1 + 1, n - 1);
   if (k1 >= n) return;
+  const bool two = k2 > k1;
+  if (SECOND && !refill && p.snbr_cnt[k1] + (two ? p.snbr_cnt[k2] : 0) == 0) return;
   const float4* xf = p.s.xf;
   const float4 f1 = xf[k1], f2 = xf[k2];
   float ex = f2.x - f1.x, ey = f2.y - f1.y, ez = f2.z - f1.z;  // the second particle's nearest image
   ex -= rintf(ex);
   ey -= rintf(ey);
   ez -= rintf(ez);
-  const bool cls = p.strong;
   const float4* gmu = (const float4*)p.s.mu;
   float m1 = 0.f, m2 = 0.f, near1 = -1.f, near2 = -1.f;
   if (cls) {
@@ -638,19 +652,16 @@ __device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
     near1 = sqrtf(sqrtf(m1 / p.strong_w4sq)) * 1.001f;  // |mu_j| <= mu_max = 1
     near2 = sqrtf(sqrtf(m2 / p.strong_w4sq)) * 1.001f;
   }
-  const bool sfill = FILL && cls && !p.flags->soverflow;
   int c1 = 0, c2 = 0, sc1 = 0, sc2 = 0;
-  int *out1 = nullptr, *out2 = nullptr;
-  if (FILL) {
-    out1 = p.nbr + p.nbr_off[k1];
-    out2 = p.nbr + p.nbr_off[k2];
-  }
+  const int o1 = SECOND ? p.nbr_off[k1] : k1 * p.nbr_share, o2 = SECOND ? p.nbr_off[k2] : k2 * p.nbr_share;
+  const int room = SECOND ? 0x7fffffff : p.nbr_share;
+  int *out1 = p.nbr + o1, *out2 = p.nbr + o2;
   int2 *so1 = nullptr, *so2 = nullptr;
   if (sfill) {
     so1 = p.snbr + p.snbr_off[k1];
     so2 = p.snbr + p.snbr_off[k2];
   }
-  const float rt = (float)(sqrt(p.rl2) * (1.0 + 1e-6) + 2e-7), rt2 = rt * rt;
+  const float rl = (float)(sqrt(p.rl2) * (1.0 + 1e-6) + 2e-7), rl2 = rl * rl;
   auto strong = [&](int k, int j, float mk) {
     const float4 mj = gmu[j];
     const int4 si = p.s.xi[k], sj = p.s.xi[j];
@@ -659,29 +670,25 @@ __device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
     const float q2 = dx * dx + dy * dy + dz * dz, q4 = q2 * q2;
     return mk * (mj.x * mj.x + mj.y * mj.y + mj.z * mj.z) > p.strong_w4sq * (q4 * q4);
   };
-  const bool two = k2 > k1;
-  auto visit = [&](bool valid, int j, float ra, float rb) {
-    const bool in1 = valid && ra < rt2 && j != k1, in2 = valid && rb < rt2 && j != k2 && two;
+  auto visit = [&](bool lists, bool strongs, bool valid, int j, float ra, float rb) {
+    const bool in1 = valid && ra < rl2 && j != k1, in2 = valid && rb < rl2 && j != k2 && two;
     const unsigned ma = __ballot_sync(kFull, in1), mb = __ballot_sync(kFull, in2);
     unsigned j1 = (unsigned)j, j2 = (unsigned)j;
     const bool n1 = in1 && ra < near1, n2 = in2 && rb < near2;
     if (__any_sync(kFull, n1 || n2)) {
       const bool s1 = n1 && strong(k1, j, m1), s2 = n2 && strong(k2, j, m2);
       const unsigned sa = __ballot_sync(kFull, s1), sb = __ballot_sync(kFull, s2);
-      if (sfill && s1) {
-        so1[sc1 + __popc(sa & lanemask_lt())] = make_int2(k1, j);
-        j1 |= kStrong;
-      }
-      if (sfill && s2) {
-        so2[sc2 + __popc(sb & lanemask_lt())] = make_int2(k2, j);
-        j2 |= kStrong;
-      }
+      if (strongs && s1) so1[sc1 + __popc(sa & lanemask_lt())] = make_int2(k1, j);
+      if (strongs && s2) so2[sc2 + __popc(sb & lanemask_lt())] = make_int2(k2, j);
+      if (s1) j1 |= kStrong;
+      if (s2) j2 |= kStrong;
       sc1 += __popc(sa);
       sc2 += __popc(sb);
     }
-    if (FILL) {
-      if (in1) out1[c1 + __popc(ma & lanemask_lt())] = (int)j1;
-      if (in2) out2[c2 + __popc(mb & lanemask_lt())] = (int)j2;
+    if (lists) {
+      const int a = c1 + __popc(ma & lanemask_lt()), b = c2 + __popc(mb & lanemask_lt());
+      if (in1 && a < room) out1[a] = (int)j1;
+      if (in2 && b < room) out2[b] = (int)j2;
     }
     c1 += __popc(ma);
     c2 += __popc(mb);
@@ -689,88 +696,104 @@ __device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
   const int ncx = p.grid.ncx;
   const float inv = 1.0f / (float)ncx;
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (ncx > 1 && fmaxf(fmaxf(fabsf(ex), fabsf(ey)), fabsf(ez)) + 2.f * rt < 1.f - 2.f * inv) {
-    const float xlo = f1.x + fminf(ex, 0.f), xhi = f1.x + fmaxf(ex, 0.f);
-    const float ylo = f1.y + fminf(ey, 0.f), yhi = f1.y + fmaxf(ey, 0.f);
-    const float zlo = f1.z + fminf(ez, 0.f), zhi = f1.z + fmaxf(ez, 0.f);
-    auto cell = [&](float x) { return (int)floorf((x + 0.5f) * (float)ncx); };
-    const int cy0 = cell(ylo - rt), ny = cell(yhi + rt) - cy0 + 1, cz0 = cell(zlo - rt), nz = cell(zhi + rt) - cz0 + 1;
-    const int* cs = p.s.cell_start;
-    for (int rb = 0; rb < ny * nz; rb += 32) {
-      // lane: one row; a0, l0 / a1, l1: its x range, split at the box's end
-      const int r = rb + lane;
-      int a0 = 0, l0 = 0, a1 = 0, l1 = 0;
-      int code = 0;  // images (+1): x of the two segments, y, z, two bits each
-      if (r < ny * nz) {
-        const int uy = cy0 + r % ny, uz = cz0 + r / ny;
-        const float yc = uy * inv - 0.5f, zc = uz * inv - 0.5f;
-        const float dy = fmaxf(0.f, fmaxf(yc - yhi, ylo - yc - inv)), dz = fmaxf(0.f, fmaxf(zc - zhi, zlo - zc - inv));
-        const float d2 = dy * dy + dz * dz;
-        if (d2 < rt2) {
-          const float h = sqrtf(rt2 - d2);
-          const int x0 = cell(xlo - h), x1 = cell(xhi + h);
-          const int iy = uy < 0 ? 0 : (uy >= ncx ? 2 : 1), iz = uz < 0 ? 0 : (uz >= ncx ? 2 : 1);
-          const int* row = cs + ((uz - (iz - 1) * ncx) * ncx + (uy - (iy - 1) * ncx)) * ncx;
-          int i0 = 1, i1 = 1;
-          if (x0 < 0) {
-            a0 = row[x0 + ncx];
-            l0 = row[ncx] - a0;
-            a1 = row[0];
-            l1 = row[x1 + 1] - a1;
-            i0 = 0;
-          } else if (x1 >= ncx) {
-            a0 = row[x0];
-            l0 = row[ncx] - a0;
-            a1 = row[0];
-            l1 = row[x1 - ncx + 1] - a1;
-            i1 = 2;
-          } else {
-            a0 = row[x0];
-            l0 = row[x1 + 1] - a0;
+  auto search = [&](float rt, bool lists, bool strongs) {
+    const float rt2 = rt * rt;
+    if (ncx > 1 && fmaxf(fmaxf(fabsf(ex), fabsf(ey)), fabsf(ez)) + 2.f * rt < 1.f - 2.f * inv) {
+      const float xlo = f1.x + fminf(ex, 0.f), xhi = f1.x + fmaxf(ex, 0.f);
+      const float ylo = f1.y + fminf(ey, 0.f), yhi = f1.y + fmaxf(ey, 0.f);
+      const float zlo = f1.z + fminf(ez, 0.f), zhi = f1.z + fmaxf(ez, 0.f);
+      auto cell = [&](float x) { return (int)floorf((x + 0.5f) * (float)ncx); };
+      const int cy0 = cell(ylo - rt), ny = cell(yhi + rt) - cy0 + 1, cz0 = cell(zlo - rt), nz = cell(zhi + rt) - cz0 + 1;
+      const int* cs = p.s.cell_start;
+      for (int rb = 0; rb < ny * nz; rb += 32) {
+        // lane: one row; a0, l0 / a1, l1: its x range, split at the box's end
+        const int r = rb + lane;
+        int a0 = 0, l0 = 0, a1 = 0, l1 = 0;
+        int code = 0;  // images (+1): x of the two segments, y, z, two bits each
+        if (r < ny * nz) {
+          const int uy = cy0 + r % ny, uz = cz0 + r / ny;
+          const float yc = uy * inv - 0.5f, zc = uz * inv - 0.5f;
+          const float dy = fmaxf(0.f, fmaxf(yc - yhi, ylo - yc - inv)), dz = fmaxf(0.f, fmaxf(zc - zhi, zlo - zc - inv));
+          const float d2 = dy * dy + dz * dz;
+          if (d2 < rt2) {
+            const float h = sqrtf(rt2 - d2);
+            const int x0 = cell(xlo - h), x1 = cell(xhi + h);
+            const int iy = uy < 0 ? 0 : (uy >= ncx ? 2 : 1), iz = uz < 0 ? 0 : (uz >= ncx ? 2 : 1);
+            const int* row = cs + ((uz - (iz - 1) * ncx) * ncx + (uy - (iy - 1) * ncx)) * ncx;
+            int i0 = 1, i1 = 1;
+            if (x0 < 0) {
+              a0 = row[x0 + ncx];
+              l0 = row[ncx] - a0;
+              a1 = row[0];
+              l1 = row[x1 + 1] - a1;
+              i0 = 0;
+            } else if (x1 >= ncx) {
+              a0 = row[x0];
+              l0 = row[ncx] - a0;
+              a1 = row[0];
+              l1 = row[x1 - ncx + 1] - a1;
+              i1 = 2;
+            } else {
+              a0 = row[x0];
+              l0 = row[x1 + 1] - a0;
+            }
+            code = i0 | i1 << 2 | iy << 4 | iz << 6;
           }
-          code = i0 | i1 << 2 | iy << 4 | iz << 6;
+        }
+        const int nr = min(32, ny * nz - rb);
+        for (int q = 0; q < nr; q += 4) {
+          const int src = q + (lane >> 3);  // lanes past the last row hold empty ranges
+          const int b0 = __shfl_sync(kFull, a0, src), n0 = __shfl_sync(kFull, l0, src);
+          const int b1 = __shfl_sync(kFull, a1, src) - n0, len = n0 + __shfl_sync(kFull, l1, src);
+          const int cd = __shfl_sync(kFull, code, src);
+          const int top = __reduce_max_sync(kFull, len);
+          // a row of image i holds particles whose periodic copies lie i - 1 boxes on
+          const float xa = f1.x + (float)(1 - (cd & 3)), xb = f1.x + (float)(1 - (cd >> 2 & 3));
+          const float y = f1.y + (float)(1 - (cd >> 4 & 3)), z = f1.z + (float)(1 - (cd >> 6 & 3));
+          int t = lane & 7;
+          float4 nxt = t < len ? xf[(t < n0 ? b0 : b1) + t] : z4;
+          for (int t0 = 0; t0 < top; t0 += 8, t += 8) {
+            const float4 c = nxt;
+            const int j = (t < n0 ? b0 : b1) + t;
+            if (t + 8 < len) nxt = xf[(t + 8 < n0 ? b0 : b1) + t + 8];
+            const float dx = c.x - (t < n0 ? xa : xb), dy = c.y - y, dz = c.z - z;
+            const float gx = dx - ex, gy = dy - ey, gz = dz - ez;
+            visit(lists, strongs, t < len, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
+          }
         }
       }
-      const int nr = min(32, ny * nz - rb);
-      for (int q = 0; q < nr; q += 4) {
-        const int src = q + (lane >> 3);  // lanes past the last row hold empty ranges
-        const int b0 = __shfl_sync(kFull, a0, src), n0 = __shfl_sync(kFull, l0, src);
-        const int b1 = __shfl_sync(kFull, a1, src) - n0, len = n0 + __shfl_sync(kFull, l1, src);
-        const int cd = __shfl_sync(kFull, code, src);
-        const int top = __reduce_max_sync(kFull, len);
-        // a row of image i holds particles whose periodic copies lie i - 1 boxes on
-        const float xa = f1.x + (float)(1 - (cd & 3)), xb = f1.x + (float)(1 - (cd >> 2 & 3));
-        const float y = f1.y + (float)(1 - (cd >> 4 & 3)), z = f1.z + (float)(1 - (cd >> 6 & 3));
-        int t = lane & 7;
-        float4 nxt = t < len ? xf[(t < n0 ? b0 : b1) + t] : z4;
-        for (int t0 = 0; t0 < top; t0 += 8, t += 8) {
-          const float4 c = nxt;
-          const int j = (t < n0 ? b0 : b1) + t;
-          if (t + 8 < len) nxt = xf[(t + 8 < n0 ? b0 : b1) + t + 8];
-          const float dx = c.x - (t < n0 ? xa : xb), dy = c.y - y, dz = c.z - z;
-          const float gx = dx - ex, gy = dy - ey, gz = dz - ez;
-          visit(t < len, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
-        }
+    } else {
+      for (int j0 = 0; j0 < n; j0 += 32) {
+        const int j = j0 + lane;
+        const float4 c = j < n ? xf[j] : z4;
+        float dx = c.x - f1.x, dy = c.y - f1.y, dz = c.z - f1.z;
+        dx -= rintf(dx);
+        dy -= rintf(dy);
+        dz -= rintf(dz);
+        float gx = c.x - f2.x, gy = c.y - f2.y, gz = c.z - f2.z;
+        gx -= rintf(gx);
+        gy -= rintf(gy);
+        gz -= rintf(gz);
+        visit(lists, strongs, j < n, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
       }
     }
-  } else {
-    for (int j0 = 0; j0 < n; j0 += 32) {
-      const int j = j0 + lane;
-      const float4 c = j < n ? xf[j] : z4;
-      float dx = c.x - f1.x, dy = c.y - f1.y, dz = c.z - f1.z;
-      dx -= rintf(dx);
-      dy -= rintf(dy);
-      dz -= rintf(dz);
-      float gx = c.x - f2.x, gy = c.y - f2.y, gz = c.z - f2.z;
-      gx -= rintf(gx);
-      gy -= rintf(gy);
-      gz -= rintf(gz);
-      visit(j < n, j, dx * dx + dy * dy + dz * dz, gx * gx + gy * gy + gz * gz);
-    }
+  };
+  if (!SECOND || refill) search(rl, true, false);
+  if (sfill) {
+    // only the near pairs: well inside the list radius (near1 and near2 hold a
+    // margin over the classification, so both passes find the same strong pairs), or
+    // the whole of it
+    const float nr = fmaxf(near1, near2);
+    sc1 = sc2 = 0;
+    search(nr < 0.98f * rl2 ? sqrtf(nr) * 1.0001f + 2e-7f : rl, false, true);
   }
-  if (!FILL && lane == 0) {
+  if (!SECOND && lane == 0) {
     p.nbr_cnt[k1] = c1;
-    if (two) p.nbr_cnt[k2] = c2;
+    p.nbr_off[k1] = o1;
+    if (two) {
+      p.nbr_cnt[k2] = c2;
+      p.nbr_off[k2] = o2;
+    }
     if (cls) {
       p.snbr_cnt[k1] = sc1;
       if (two) p.snbr_cnt[k2] = sc2;
@@ -778,13 +801,13 @@ __device__ __forceinline__ void nbr_build2(const RealParams& p, int bx) {
   }
 }
 
-template <typename T, bool FILL>
+template <typename T, bool SECOND>
 __device__ __forceinline__ void nbr_build(const RealParams& p, int bx) {
   if (!p.flags->rebuild) return;
   if constexpr (std::is_same<T, float>::value)
-    nbr_build2<FILL>(p, bx);
+    nbr_build2<SECOND>(p, bx);
   else
-    nbr_build64<FILL>(p, bx);
+    nbr_build64<SECOND>(p, bx);
 }
 
 // Exclusive scan of cnt[0, n) into off[0, n] by one block of 1024 threads;
@@ -840,8 +863,36 @@ __device__ __forceinline__ void nbr_scan(const RealParams& p, int half) {
   StepFlags* flags = p.flags;
   if (!flags->rebuild) return;
   if (half == 0) {
-    const long long tot = block_scan_counts(p.nbr_cnt, p.nbr_off, p.n);
-    if (threadIdx.x == 0) flags->overflow = tot > p.nbr_cap ? 1 : 0;
+    // the lists lie in their shares unless one is longer
+    int top = 0;
+    long long tot = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < p.n; i += 1024) {
+      const int c = p.nbr_cnt[i];
+      top = max(top, c);
+      tot += c;
+    }
+    __shared__ long long wsum[32];
+    __shared__ int wtop[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    tot = warp_sum(tot);
+    top = __reduce_max_sync(kFull, top);
+    if (lane == 0) {
+      wsum[w] = tot;
+      wtop[w] = top;
+    }
+    __syncthreads();
+    tot = warp_sum(wsum[lane]);
+    top = __reduce_max_sync(kFull, wtop[lane]);
+    const bool refill = top > p.nbr_share;
+    if (refill)
+      block_scan_counts(p.nbr_cnt, p.nbr_off, p.n);
+    else if (threadIdx.x == 0)
+      p.nbr_off[p.n] = (int)min(tot, (long long)0x7fffffff);
+    if (threadIdx.x == 0) {
+      flags->refill = refill;
+      flags->overflow = refill && tot > p.nbr_cap ? 1 : 0;
+    }
   } else {
     // a build that did not classify leaves the strong list unusable until the
     // next build that does (the FP64 kernels then contribute nothing)
@@ -1122,7 +1173,7 @@ __device__ __forceinline__ void real_eval32(const RealParams& p, int bx) {
     const int* lst = p.nbr + p.nbr_off[k];
     const int cnt = p.nbr_cnt[k];
     // flags count only when the context evaluates the strong pairs in FP64
-    const unsigned fs = p.strong ? kStrong : 0u;
+    const unsigned fs = p.strong && !p.flags->soverflow ? kStrong : 0u;
     // the list is streamed once per pass: evict-first loads leave L1 to the gathers
     auto entry = [&](int t) { return t < cnt ? (unsigned)__ldcs(lst + t) : (unsigned)k; };
     auto process = [&](unsigned ea, unsigned eb, int t) {
@@ -1237,10 +1288,10 @@ static int num_sms() {
 
 // Grid-stride over the particle blocks: most steps do not rebuild, and a
 // grid of a few blocks per SM then costs one flag read per block.
-template <typename T, bool FILL>
+template <typename T, bool SECOND>
 __global__ void __launch_bounds__(kRealWarps * 32) k_nbr_build(RealParams p, int nblk) {
   if (!p.flags->rebuild) return;
-  for (int bx = blockIdx.x; bx < nblk; bx += gridDim.x) nbr_build<T, FILL>(p, bx);
+  for (int bx = blockIdx.x; bx < nblk; bx += gridDim.x) nbr_build<T, SECOND>(p, bx);
 }
 __global__ void __launch_bounds__(1024) k_nbr_scan(RealParams p) { nbr_scan(p, blockIdx.x); }
 // The FP32 passes without coating keep the occupancy of their pair loops
@@ -1291,13 +1342,13 @@ __global__ void __launch_bounds__(kRealWarps * 32) k_count_pairs(RealParams p, u
 
 // persistent: blocks stride over the task table (see md_cells.cu); the
 // list build and the pair loop are warp-private (no block barrier)
-template <bool FILL>
+template <bool SECOND>
 __global__ void __launch_bounds__(kRealWarps * 32) k_nbr_build_packed(const RealParams* __restrict__ ps,
                                                                       const Task* __restrict__ tk, int ntask, WorkQ* wq,
                                                                       const unsigned* anyrb) {
   if (!__ldcg(anyrb)) return;  // the whole grid: no system rebuilds this step
   for_tasks<false>(tk, ntask, wq, [&](const Task& t) {
-      nbr_build<float, FILL>(ps[t.rep], t.blk);
+      nbr_build<float, SECOND>(ps[t.rep], t.blk);
   });
 }
 __global__ void __launch_bounds__(1024) k_nbr_scan_packed(const RealParams* __restrict__ ps) {

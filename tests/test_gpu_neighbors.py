@@ -77,3 +77,21 @@ def test_lists_built_for_two_particles_at_once(n, rc_frac):
         tol = TOL_MIXED if prec else TOL_FP64
         assert O.rms_rel(B, Bo, bAl) < tol and O.rms_rel(F, Fo, fAl) < tol
         np.testing.assert_allclose(P, Po, rtol=0, atol=tol * fAl * g["rc"] * n)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("n,rc_frac", [(65, 0.4), (1001, 0.3), (2000, 0.25)])
+def test_lists_beyond_their_share(prec, n, rc_frac):
+    """A capacity of exactly the entries in use: some list is longer than an equal
+    share of it, and the lists are written again one after another; the entries
+    and their order, strong pairs included, are the same."""
+    ini, g = random_system(n, seed=n, rc_frac=rc_frac, lognormal=True)
+    sim = gpu_system(ini, g, prec)
+    a = sim.CompInteractions()
+    used = sim.neighbor_capacity()
+    sim.neighbor_capacity(cap=used)
+    sim.set_state(g["pos"], g["mm"], g["ea"])
+    b = sim.CompInteractions()
+    assert sim.neighbor_capacity() == used
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
