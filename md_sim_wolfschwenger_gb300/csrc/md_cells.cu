@@ -50,11 +50,8 @@ __device__ __forceinline__ void step_begin(StepFlags* f, float half_skin) {
 }
 
 // Cell of each particle (all-pairs grid: identity order, one cell).
-__device__ __forceinline__ void cell_assign(const CellParams& p, int bx) {
-  if (skip(p.flags)) return;
-  const int i = bx * kCellThreads + threadIdx.x, n = p.n;
-  if (i >= n) return;
-  const int ncx = p.grid.ncx;
+__device__ __forceinline__ void assign_one(const CellParams& p, int i) {
+  const int n = p.n, ncx = p.grid.ncx;
   if (ncx == 1) {
     p.s.perm[i] = i;
     p.cellOf[i] = 0;
@@ -67,11 +64,14 @@ __device__ __forceinline__ void cell_assign(const CellParams& p, int bx) {
   p.cellOf[i] = c;
   atomicAdd(&p.count[c], 1);
 }
+__device__ __forceinline__ void cell_assign(const CellParams& p, int bx) {
+  const int i = bx * kCellThreads + threadIdx.x;
+  if (!skip(p.flags) && i < p.n) assign_one(p, i);
+}
 
 // Exclusive scan of count[0..ncell) -> start[0..ncell]; count is zeroed so it
 // can serve as the fill counter of the scatter.  One block of 1024 threads.
-__device__ __forceinline__ void cell_scan(const CellParams& p) {
-  if (skip(p.flags) || p.grid.ncx == 1) return;
+__device__ __forceinline__ void scan_cells(const CellParams& p) {
   __shared__ int wsum[32];
   const int ncell = p.grid.ncell;
   int* count = p.count;
@@ -110,23 +110,23 @@ __device__ __forceinline__ void cell_scan(const CellParams& p) {
   }
   if (t == nt - 1) start[ncell] = run;
 }
+__device__ __forceinline__ void cell_scan(const CellParams& p) {
+  if (!skip(p.flags) && p.grid.ncx > 1) scan_cells(p);
+}
 
-__device__ __forceinline__ void cell_scatter(const CellParams& p, int bx) {
-  if (skip(p.flags) || p.grid.ncx == 1) return;
-  const int i = bx * kCellThreads + threadIdx.x;
-  if (i >= p.n) return;
+__device__ __forceinline__ void scatter_one(const CellParams& p, int i) {
   const int c = p.cellOf[i];
   p.tmp[p.s.cell_start[c] + atomicAdd(&p.count[c], 1)] = i;
+}
+__device__ __forceinline__ void cell_scatter(const CellParams& p, int bx) {
+  const int i = bx * kCellThreads + threadIdx.x;
+  if (!skip(p.flags) && p.grid.ncx > 1 && i < p.n) scatter_one(p, i);
 }
 
 // One warp per cell: rank of each element = number of smaller indices in the
 // segment (indices are distinct), so perm is the segment sorted ascending.
 // The cell's fill counter is zeroed for the next build.
-__device__ __forceinline__ void cell_sort(const CellParams& p, int bx) {
-  if (skip(p.flags) || p.grid.ncx == 1) return;
-  const int c = (bx * kCellThreads + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= p.grid.ncell) return;
+__device__ __forceinline__ void sort_cell(const CellParams& p, int c, int lane) {
   const int* tmp = p.tmp;
   int* perm = p.s.perm;
   const int s = p.s.cell_start[c], e = p.s.cell_start[c + 1], len = e - s;
@@ -143,6 +143,10 @@ __device__ __forceinline__ void cell_sort(const CellParams& p, int bx) {
     for (int b = 0; b < len; b++) r += tmp[s + b] < v;
     perm[s + r] = v;
   }
+}
+__device__ __forceinline__ void cell_sort(const CellParams& p, int bx) {
+  const int c = (bx * kCellThreads + threadIdx.x) >> 5;
+  if (!skip(p.flags) && p.grid.ncx > 1 && c < p.grid.ncell) sort_cell(p, c, threadIdx.x & 31);
 }
 
 // Sorted views.  Fixed point: x_fix = round(x_box * 2^32) as a wrapping
@@ -193,6 +197,34 @@ __device__ __forceinline__ void sorted_fill(const CellParams& p, int bx) {
 
 __global__ void k_step_begin(StepFlags* f, float half_skin) {
   if (threadIdx.x == 0 && blockIdx.x == 0) step_begin(f, half_skin);
+}
+
+// Small systems: the start of the step and the whole cell order in one launch, a
+// cluster of eight blocks with the cluster's barrier between the stages.  Most
+// steps rebuild nothing and paid a launch (~0.7 us in a graph) for each of the five
+// kernels: N = 1000 69.7 -> 67.3, N = 4096 109.8 -> 105.9, N = 8192 146.0 -> 142.3 us
+// per step.  Above kClusterCells particles the rebuild itself, on 8192 threads,
+// would cost more than the launches.
+constexpr int kClusterBlocks = 8, kClusterCells = 8192;
+__device__ __forceinline__ void cluster_sync() {
+  __threadfence();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(1024) k_cells_small(CellParams p) {
+  StepFlags* f = p.flags;
+  const int g = blockIdx.x * 1024 + threadIdx.x, G = kClusterBlocks * 1024;
+  const bool rb = *(volatile int*)&f->force || __uint_as_float(*(volatile unsigned*)&f->maxdisp) > p.half_skin;
+  cluster_sync();  // every thread has read the flags
+  if (g == 0) step_begin(f, p.half_skin);
+  if (!rb) return;
+  for (int i = g; i < p.n; i += G) assign_one(p, i);
+  if (p.grid.ncx == 1) return;
+  cluster_sync();
+  if (blockIdx.x == 0) scan_cells(p);
+  cluster_sync();
+  for (int i = g; i < p.n; i += G) scatter_one(p, i);
+  cluster_sync();
+  for (int c = g >> 5; c < p.grid.ncell; c += G >> 5) sort_cell(p, c, threadIdx.x & 31);
 }
 __global__ void __launch_bounds__(kCellThreads) k_cell_assign(CellParams p) { cell_assign(p, blockIdx.x); }
 __global__ void __launch_bounds__(1024) k_cell_scan(CellParams p) { cell_scan(p); }
@@ -382,20 +414,21 @@ int launch_disp_check(cudaStream_t st, int n, const double* pos, const double* x
   return 1;
 }
 
-int launch_step_begin(cudaStream_t st, StepFlags* flags, double half_skin) {
-  k_step_begin<<<1, 32, 0, st>>>(flags, (float)half_skin);
-  return 1;
-}
-
 int launch_cells(cudaStream_t st, const CellParams& p, bool fp64) {
   const int nb = cell_blocks(p.n);
   int launches = 1;
-  k_cell_assign<<<nb, kCellThreads, 0, st>>>(p);
-  if (p.grid.ncx > 1) {
-    k_cell_scan<<<1, 1024, 0, st>>>(p);
-    k_cell_scatter<<<nb, kCellThreads, 0, st>>>(p);
-    k_cell_sort<<<cell_sort_blocks(p.grid), kCellThreads, 0, st>>>(p);
-    launches += 3;
+  if (p.n <= kClusterCells) {
+    k_cells_small<<<kClusterBlocks, 1024, 0, st>>>(p);
+  } else {
+    k_step_begin<<<1, 32, 0, st>>>(p.flags, p.half_skin);
+    k_cell_assign<<<nb, kCellThreads, 0, st>>>(p);
+    launches++;
+    if (p.grid.ncx > 1) {
+      k_cell_scan<<<1, 1024, 0, st>>>(p);
+      k_cell_scatter<<<nb, kCellThreads, 0, st>>>(p);
+      k_cell_sort<<<cell_sort_blocks(p.grid), kCellThreads, 0, st>>>(p);
+      launches += 3;
+    }
   }
   if (fp64)
     k_sorted_fill<double><<<nb, kCellThreads, 0, st>>>(p);

@@ -408,7 +408,6 @@ static int issue_interactions(md_ctx* c, double dt = -1.0) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
   const CellParams cp = cell_params(c);
-  l += launch_step_begin(c->stream, cp.flags, cp.half_skin);
   l += launch_cells(c->stream, cp, fp64(c));
   l += fork_join(
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,

@@ -40,10 +40,9 @@ int scatter_blocks(const KParams& p, int np);
 int int_blocks(int n);
 int int_blocks_one(int n);        // single-system Heun launches (128-thread blocks)
 
-// Step start: decides whether this step rebuilds the cell order and the
-// neighbour list (host request, or a particle moved more than half_skin).
-int launch_step_begin(cudaStream_t st, StepFlags* flags, double half_skin);
-// anyrb: the batch's word "some system rebuilds its lists this step" (set here,
+// Step start of a batch: decides for each system whether this step rebuilds the
+// cell order and the neighbour list (host request, or a particle moved more than
+// half_skin).  anyrb: the batch's word "some system rebuilds its lists this step" (set here,
 // read by the packed list kernels, cleared by launch_obs_packed's kernel)
 int launch_step_begin_packed(cudaStream_t st, const CellParams* ps, int R, unsigned* anyrb);
 // Raises the displacement since the last build after new positions arrived.
@@ -55,7 +54,8 @@ int launch_state_in(cudaStream_t st, int n, const double* hpos, const double* hm
                     double* mm, double* ea, const double* xbuild, double L, StepFlags* flags);
 int launch_state_out(cudaStream_t st, int n, const double* pos, const double* mm, const double* ea, double* hpos,
                      double* hmm, double* hea);
-// Cell order (skipped unless the step rebuilds) and the sorted views.
+// Step start as above, cell order (skipped unless the step rebuilds) and the
+// sorted views.
 int launch_cells(cudaStream_t st, const CellParams& p, bool fp64);
 int launch_cells_packed(cudaStream_t st, const CellParams* ps, int R, const Packed& n256, const Packed& sort,
                         const unsigned* anyrb);

@@ -95,3 +95,21 @@ def test_lists_beyond_their_share(prec, n, rc_frac):
     assert sim.neighbor_capacity() == used
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,rc_frac", [(33, 0.4), (1025, 0.3), (8191, 0.2), (8192, 0.2), (8193, 0.2)])
+def test_cell_order_of_small_and_large_systems(n, rc_frac):
+    """Up to 8192 particles one cluster of blocks makes the whole cell order,
+    beyond them a kernel per stage: a stable counting sort either way, at the first
+    step and after one that moved nothing."""
+    ini, g = random_system(n, seed=n, rc_frac=rc_frac)
+    sim = gpu_system(ini, g, 1)
+    xb = g["pos"] / g["lBox"]
+    xb = xb - np.floor(xb + 0.5)
+    for _ in range(2):
+        sim.CompInteractions()
+        ncx, cs, perm = sim.debug_cells()
+        c = np.clip(((xb + 0.5) * ncx).astype(np.int64), 0, ncx - 1)
+        cell = (c[2] * ncx + c[1]) * ncx + c[0]
+        np.testing.assert_array_equal(perm, np.argsort(cell, kind="stable"))
+        np.testing.assert_array_equal(cs, np.concatenate([[0], np.cumsum(np.bincount(cell, minlength=ncx ** 3))]))
