@@ -73,6 +73,10 @@ struct md_ctx {
   bool graph_valid = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
+  // kGraphSteps steps in one graph, once kGraphAfter single steps were replayed
+  cudaGraph_t graph_n = nullptr;
+  cudaGraphExec_t gexec_n = nullptr;
+  int64_t replays = 0;
   int64_t launches = 0, launches_per_step = 0;
 
   // device: master state & particle constants

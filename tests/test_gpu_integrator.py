@@ -46,3 +46,17 @@ def test_records_and_state_at_block_edges(n, precision):
     np.testing.assert_allclose(r[-1, 1], mo[2].mean(), rtol=0, atol=tol)
     np.testing.assert_allclose(r[-1, 2:5], (d * d).mean(axis=1), rtol=1e-10 if precision == 0 else 1e-4)
     assert r.shape == (3, 8) and np.allclose(r[:, 0], np.arange(3) * g["dt"])
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_steps_in_one_graph_equal_single_steps(prec):
+    """A long run goes on in graphs of several steps: the same bits as one call per
+    step, with a change of dt and a remainder in between."""
+    ini, g = random_system(150, seed=8, rc_frac=0.35, noise=True)
+    a, b = (gpu_system(ini, g, prec, noise=2, seed=4) for _ in range(2))
+    for k, dt in ((300, g["dt"]), (13, 0.5 * g["dt"]), (203, g["dt"])):
+        a.step(k, dt)
+        for _ in range(k):
+            b.step(1, dt)
+        for x, y in zip(a.get_state(), b.get_state()):
+            np.testing.assert_array_equal(x, y)
