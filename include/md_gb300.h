@@ -201,8 +201,8 @@ int md_set_kspace_engine(md_ctx* ctx, int engine);
 /* *tensor_cores = 1 when the current Ewald parameters are those of the tensor
  * cores.  With MD_KSPACE_AUTO and the default tiling, systems too small to
  * fill them (about 3e6 k vectors x particles) evaluate the same k rows on the
- * CUDA cores under that setting, and systems of 1e8 and more take the same sums
- * through a mesh; MD_KSPACE_TC always takes the tensor cores. */
+ * CUDA cores under that setting, and systems of 6000 particles and more with
+ * kc >= 15 (32768: kc >= 13) take the same sums through a mesh; MD_KSPACE_TC always takes the tensor cores. */
 int md_kspace_engine_active(const md_ctx* ctx, int* tensor_cores);
 /* Tiling of the tensor-core structure factor (no counterpart in the
  * reference; the autotuner's knobs): ring = the operand-ring option (0..5,

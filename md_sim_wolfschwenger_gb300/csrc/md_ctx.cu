@@ -770,17 +770,21 @@ static int setup_rows(md_ctx* c) {
 }
 
 // Whether the mixed path's default engine goes through a mesh (md_kmesh.cu)
-// instead of the tensor cores: systems of 1e8 (k, particle) terms and more, whose
-// products outweigh the mesh's six dependent launches.  Measured step times, mesh
-// against tensor cores: N = 12000, kc = 12 (0.4e8 terms) 214 / 187 us, N = 20011,
-// kc = 15 (1.4e8) 348 / 387, N = 32768, kc = 15 (2.3e8) 614 / 662, N = 131072,
-// kc = 20 (2.2e9) 3159 / 4186.  Errors of the k-space part against FP64 (rms,
-// N = 32768): field 1.5e-7 / 1.2e-6, force 2.8e-7 / 1.3e-6.  An engine or a
-// tensor-core tiling that the caller chose is kept.
+// instead of the tensor cores.  The mesh's work per particle is that of ~6000 k
+// vectors (half space) on the tensor cores, ~4000 once its kernels fill the GPU;
+// its transforms, ~M^3, must not outweigh the particles.  Measured step times,
+// mesh / tensor cores, us: N = 6000, kc = 20 212 / 237, kc = 25 (M = 104) 377 / 322;
+// N = 8192, kc = 13 174 / 165, kc = 16 179 / 199, kc = 20 241 / 273, kc = 25 397 / 356;
+// N = 12000, kc = 14 236 / 227, kc = 16 237 / 265; N = 16384, kc = 13 286 / 267, kc = 15
+// 285 / 284..297; N = 20011, kc = 15 344 / 388; N = 32768, kc = 12 609 / 595, kc = 13
+// 621 / 626, kc = 15 599 / 664; N = 131072, kc = 13 3135 / 3286, kc = 20 3097 / 4186.
+// Errors of the k-space part against FP64 (rms, N = 32768): field 1.5e-7 / 1.2e-6,
+// force 2.8e-7 / 1.3e-6.  An engine or a tensor-core tiling that the caller chose is
+// kept.
 static bool mesh_wanted(const md_ctx* c) {
-  const double nk = 2.0943951 * (double)c->kc * (double)c->kc * (double)c->kc;  // half space
-  return !fp64(c) && c->kengine == MD_KSPACE_AUTO && c->tc_ring < 0 && c->tc_waves == 1 && c->tc_rows > 0 &&
-         c->kc >= md::kMeshMinKc && nk * (double)c->n >= 1e8;
+  if (fp64(c) || c->kengine != MD_KSPACE_AUTO || c->tc_ring >= 0 || c->tc_waves != 1 || c->tc_rows == 0) return false;
+  const double M = md::mesh_points((int)c->kc);
+  return c->n >= 6000 && (c->kc >= 15 || (c->kc >= 13 && c->n >= 32768)) && M * M * M <= 100.0 * (double)c->n;
 }
 
 // k space through a mesh: window tables and the mesh in its stages (md_kmesh.cu).

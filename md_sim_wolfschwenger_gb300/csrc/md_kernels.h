@@ -131,7 +131,7 @@ RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
 int launch_phase_rows(cudaStream_t st, const KParams& p, bool fp64);
 // k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks and
 // partial-mesh floats of the spread.
-constexpr int kMeshMinKc = 5;  // M >= 24: a window and its neighbour bricks do not wrap onto themselves
+// (kc >= 5: M >= 24, so that a window and its neighbour bricks do not wrap onto themselves)
 inline int mesh_points(int kc) { return 8 * ((kc + 1) / 2); }
 int mesh_bricks(int M);
 size_t mesh_part_floats(int M);

@@ -24,8 +24,8 @@
 // 2.4e-7 in F, the rest FP32 rounding of sums of ~100 terms.  All sums have a
 // fixed order: results are deterministic.
 //
-// Measured at N = 32768 (M = 64) / 131072 (M = 80), us: spread 39 / 113, the four
-// transforms 30 / 50, interpolation 41 / 123 with the force, 35 / 107 without;
+// Measured at N = 32768 (M = 64) / 131072 (M = 80), us: spread 29 / 79, the four
+// transforms 30 / 50, interpolation 41 / 124 with the force, 35 / 107 without;
 // the tensor cores' 135 / 850 and 120 / 700 for the same.
 #include "md_common.cuh"
 #include "md_kernels.h"
@@ -61,20 +61,24 @@ __device__ __forceinline__ int mesh_point(int x, int M, float& s) {
 // The spread and the interpolation work on bricks of 16 x 8 x 8 mesh points, a
 // block each, for the particles whose window starts there; with the window's
 // reach a brick has 24 x 16 x 16 points.
+template <int NT>
 struct BrickScan {
-  int pre[kBrThreads + 1];    // candidates before row t
-  int a0[kBrThreads], l0[kBrThreads], a1[kBrThreads];
-  int wcount[8][kBrWarps];    // [class][warp]
-  int start[9];               // first particle of each class, and their number
+  int pre[NT + 1];    // candidates before row t
+  int a0[NT], l0[NT], a1[NT];
+  int wsum[NT / 32];
+  int place[NT];      // [class][warp]: particles, then the first one's place
+  int start[33];      // first particle of each class, and their number
 };
 
-// Finds the particles of the brick at (x0, y0, z0), in cell order within each
-// class x / 2 of their window's start: the cells that reach into it, grown by the distance a particle may have moved since they were
-// filled.  put(k, j, start, s) stores the k-th of up to kBrThreads particles
+// Finds the particles of the brick at (x0, y0, z0): the cells that reach into it,
+// grown by the distance a particle may have moved since they were filled, are
+// searched NT candidates at a time.  put(k, j, start, s) stores a particle found
 // (sorted index, window start x | y << 8 | z << 16, arguments of the window's
-// polynomials); chunk(hits) is then called by the whole block, between barriers.
-template <typename P, typename C>
-__device__ __forceinline__ void brick_particles(const KParams& p, BrickScan& b, int x0, int y0, int z0, P&& put,
+// polynomials); k runs over the classes 4 (x / 2) + y / 2 of the start, and in cell
+// order within a class.  chunk(hits) is then called by the whole block, between
+// barriers.
+template <int NT, typename P, typename C>
+__device__ __forceinline__ void brick_particles(const KParams& p, BrickScan<NT>& b, int x0, int y0, int z0, P&& put,
                                                 C&& chunk) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int M = p.gm_M, wx = min(kBX, M - x0), ncx = p.gm_ncx;
@@ -94,7 +98,7 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan& b, 
   cells(x0, wx, cx, nx);
   cells(y0, kBY, cy, ny);
   cells(z0, kBZ, cz, nz);
-  for (int r0 = 0; r0 < ny * nz; r0 += kBrThreads) {
+  for (int r0 = 0; r0 < ny * nz; r0 += NT) {
     __syncthreads();
     {  // one row of cells per thread, split where it wraps
       const int r = r0 + tid;
@@ -118,18 +122,18 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan& b, 
         const int u = __shfl_up_sync(kFull, incl, o);
         if (lane >= o) incl += u;
       }
-      if (lane == 31) b.wcount[0][wid] = incl;
+      if (lane == 31) b.wsum[wid] = incl;
       b.a0[tid] = a0;
       b.l0[tid] = l0;
       b.a1[tid] = a1;
       __syncthreads();
-      for (int q = 0; q < wid; q++) incl += b.wcount[0][q];
+      for (int q = 0; q < wid; q++) incl += b.wsum[q];
       b.pre[tid + 1] = incl;
       if (tid == 0) b.pre[0] = 0;
     }
     __syncthreads();
-    const int total = b.pre[kBrThreads], nrow = min(kBrThreads, ny * nz - r0);
-    for (int t0 = 0; t0 < total; t0 += kBrThreads) {
+    const int total = b.pre[NT], nrow = min(NT, ny * nz - r0);
+    for (int t0 = 0; t0 < total; t0 += NT) {
       const int t = t0 + tid;
       bool in = false;
       int at = 0, j = 0;
@@ -153,32 +157,28 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan& b, 
         in = ix < wx && iy < kBY && iz < kBZ;
         at = ix | iy << 8 | iz << 16;
       }
-      // stable counting sort by the class x / 2
-      const int cls = in ? at >> 1 & 7 : 8;
-      unsigned mine = 0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const unsigned m = __ballot_sync(kFull, cls == q);
-        if (cls == q) mine = m;
-        if (lane == q) b.wcount[q][wid] = __popc(m);
-      }
+      // stable counting sort by the class
+      b.place[tid] = 0;
       __syncthreads();
-      if (wid == 0) {  // lane: two of the 64 counts in (class, warp) order
-        int* c = &b.wcount[0][0] + 2 * lane;
-        const int c0 = c[0], c1 = c[1];
-        int incl = c0 + c1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += u;
-        }
-        c[0] = incl - c0 - c1;
-        c[1] = incl - c1;
-        if ((lane & 3) == 0) b.start[lane >> 2] = incl - c0 - c1;
-        if (lane == 31) b.start[8] = incl;
-      }
+      const int cls = in ? (at >> 1 & 7) * 4 + (at >> 9 & 3) : 32;
+      const unsigned same = __match_any_sync(kFull, cls);
+      if (in && __ffs(same) - 1 == lane) b.place[cls * (NT / 32) + wid] = __popc(same);
       __syncthreads();
-      const int k = in ? b.wcount[cls][wid] + __popc(mine & lanemask_lt()) : 0, hits = b.start[8];
+      const int c = b.place[tid];
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += u;
+      }
+      if (lane == 31) b.wsum[wid] = incl;
+      __syncthreads();
+      for (int q = 0; q < wid; q++) incl += b.wsum[q];
+      b.place[tid] = incl - c;
+      if (tid % (NT / 32) == 0) b.start[tid / (NT / 32)] = incl - c;
+      if (tid == NT - 1) b.start[32] = incl;
+      __syncthreads();
+      const int k = in ? b.place[cls * (NT / 32) + wid] + __popc(same & lanemask_lt()) : 0, hits = b.start[32];
       if (in) put(k, j, at, s);
       __syncthreads();
       chunk(hits);
@@ -189,16 +189,18 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan& b, 
 // ---------------------------------------------------------------- spread
 //
 // A thread keeps the 24 points of its (y, z) in registers, as pairs along x, and
-// takes the particles one after another, sorted by the pair their window starts
-// at: it covers five aligned pairs, whose register indices are then constants.  The five of eight warps whose
-// rows y the window covers work.  The padded bricks go to global memory, where
+// takes the particles one after another, in classes by the place of their window:
+// it covers five aligned pairs along x, whose register indices are constants within
+// a class, and the rows y of five of the eight warps, each of which takes the
+// classes that reach its rows.  The padded bricks go to global memory, where
 // k_mesh_z adds the (up to eight) that overlap in a mesh point in a fixed order.
 //
-// Bound: latency of 16 warps per SM (128 registers a thread), and a last wave: 256
-// bricks on 152 SMs at M = 64.  (Adding to the brick in shared
-// memory, a lane per (x, y) column, was bound by the 729 x 3 read-modify-writes
-// per particle: 52 us at N = 32768, M = 64.)  16 x 8 x 8 rather than 8 x 8 x 8: the
-// padded bricks are 6 times the mesh instead of 8 (19 MB at M = 64).
+// Bound: latency of 16 warps per SM (128 registers a thread), and the last wave: 256
+// bricks on 152 SMs at M = 64; 29 us at N = 32768 (37 sorted by x only, with a test
+// per particle and warp; 52 adding to the brick in shared memory, a lane per
+// (x, y) column, bound by the 729 x 3 read-modify-writes per particle).  16 x 8 x 8
+// rather than 8 x 8 x 8: the padded bricks are 6 times the mesh instead of 8 (19 MB
+// at M = 64).
 constexpr int kNX2 = kPX / 2;                  // a thread's mesh points: float2 pairs along x
 constexpr int kSub = 128;                      // particles whose window values are in shared memory at a time
 // Window values of a particle in shared memory: x in five pairs aligned to even
@@ -211,7 +213,7 @@ struct SpreadSmem {
   int at[kBrThreads];
   float coef[kMW * kMC];
   double red[3][kBrWarps];
-  BrickScan scan;
+  BrickScan<kBrThreads> scan;
 };
 
 static_assert(kBX == 16 && kBX / 2 - 1 + 5 == kNX2, "eight classes of five pairs");
@@ -256,15 +258,17 @@ __global__ void __launch_bounds__(kBrThreads, 2) k_mesh_spread(KParams p) {
             if (v == 0) w[kWX + (odd ? 0 : kMW)] = 0.f;  // the pair's other half at the window's open end
           }
           __syncthreads();
+          // the classes whose rows y reach this warp's
+          const int f0 = max(wid - 4, 0), f1 = min(wid, 3) + 1;
 #pragma unroll
           for (int I = 0; I < 8; I++) {
-            const int e = min(sm.scan.start[I + 1] - h0, cnt);
-            for (int h = max(sm.scan.start[I] - h0, 0); h < e; h++) {
-              const int at = sm.at[h0 + h], iy = at >> 8 & 255, iz = at >> 16;
-              if ((unsigned)(2 * wid + 1 - iy) > (unsigned)kMW) continue;  // the window misses this warp's rows
+            const int e = min(sm.scan.start[4 * I + f1] - h0, cnt);
+#pragma unroll 2
+            for (int h = max(sm.scan.start[4 * I + f0] - h0, 0); h < e; h++) {
+              const int at = sm.at[h0 + h];
               const float* w = sm.w + h * kWS;
               const float4 mu = sm.mu[h0 + h];
-              const float v = w[kWY + kWPad + y - iy] * w[kWZ + kWPad + z - iz];
+              const float v = w[kWY + kWPad + y - (at >> 8 & 255)] * w[kWZ + kWPad + z - (at >> 16)];
               const float vx = v * mu.x, vy = v * mu.y, vz = v * mu.z;
               const float4 a = *(const float4*)(w + kWX), b = *(const float4*)(w + kWX + 4);
               const float2 x[5] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y),
@@ -635,24 +639,24 @@ __global__ void __launch_bounds__(256) k_mesh_yz(KParams p) {
 // (sums over the lanes for every particle).
 constexpr int kFY = 17;  // row stride: lane l's point lies in bank group l mod 8
 static_assert(kFY % 8 == kMW % 8 && kFY >= kPZ, "27 lanes in four wavefronts");
+constexpr int kInThreads = 384;
 struct InterpSmem {
   float4 f[kPX * kPY * kFY];
-  int j[kBrThreads];
-  BrickScan scan;
+  int j[kInThreads];
+  BrickScan<kInThreads> scan;
 };
 template <bool FULL>
-__global__ void __launch_bounds__(kBrThreads, 2) k_mesh_interp(KParams p) {
+__global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
   InterpSmem& sm = *(InterpSmem*)smem;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int M = p.gm_M, n = p.n, nbx = (M + kBX - 1) / kBX, nby = M / kBY;
   const int x0 = blockIdx.x % nbx * kBX, y0 = blockIdx.x / nbx % nby * kBY, z0 = blockIdx.x / (nbx * nby) * kBZ;
   auto fold = [&](int i) { return i >= M ? i - M : i; };
-  {
-    const int y = tid >> 4, z = tid & 15;
-    const float4* src = p.gm_b + (size_t)fold(y0 + y) * M + fold(z0 + z);
 #pragma unroll 8
-    for (int x = 0; x < kPX; x++) sm.f[(x * kPY + y) * kFY + z] = src[(size_t)fold(x0 + x) * M * M];
+  for (int e = tid; e < kPX * kPY * kPZ; e += kInThreads) {
+    const int x = e / (kPY * kPZ), y = e / kPZ % kPY, z = e % kPZ;
+    sm.f[(x * kPY + y) * kFY + z] = p.gm_b[((size_t)fold(x0 + x) * M + fold(y0 + y)) * M + fold(z0 + z)];
   }
   const int rr = min(lane / kMW, 2), pt = lane % kMW;  // also the axis of the window values
   const bool on = lane < 3 * kMW;
@@ -672,12 +676,12 @@ __global__ void __launch_bounds__(kBrThreads, 2) k_mesh_interp(KParams p) {
           xn = p.s.xi[kn];
           if (FULL) mn = ((const float4*)p.s.mu)[kn];
         }
-        for (int h = wid; h < hits; h += kBrWarps) {
+        for (int h = wid; h < hits; h += kInThreads / 32) {
           const int k = kn;
           const int4 xi = xn;
           const float4 mu = mn;
-          if (h + kBrWarps < hits) {  // the next particle
-            kn = sm.j[h + kBrWarps];
+          if (h + kInThreads / 32 < hits) {  // the next particle
+            kn = sm.j[h + kInThreads / 32];
             xn = p.s.xi[kn];
             if (FULL) mn = ((const float4*)p.s.mu)[kn];
           }
@@ -699,7 +703,7 @@ __global__ void __launch_bounds__(kBrThreads, 2) k_mesh_interp(KParams p) {
           // packed: (x, y) and (z, z) of a mesh point against the window value and, in
           // the other half or another sum, its derivative
           float2 gxy[3] = {}, gz[3] = {}, hxy[3] = {};
-#pragma unroll
+#pragma unroll 3
           for (int a = 0; a < kMW; a++) {
             const float xv = __shfl_sync(kFull, w, a), xd = FULL ? __shfl_sync(kFull, dw, a) : 0.f;
 #pragma unroll
@@ -771,9 +775,9 @@ int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) 
   const size_t smf = sizeof(InterpSmem);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
   if (full)
-    k_mesh_interp<true><<<p.gm_nbrick, kBrThreads, smf, st>>>(p);
+    k_mesh_interp<true><<<p.gm_nbrick, kInThreads, smf, st>>>(p);
   else
-    k_mesh_interp<false><<<p.gm_nbrick, kBrThreads, smf, st>>>(p);
+    k_mesh_interp<false><<<p.gm_nbrick, kInThreads, smf, st>>>(p);
   return 6;
 }
 

@@ -25,11 +25,10 @@ def rms(a, b):
     return np.sqrt(np.mean(np.abs(a - b) ** 2) / np.mean(np.abs(b) ** 2))
 
 
-# sizes just above the engine's threshold (1e8 k vectors x particles), with meshes of
-# whole and partial bricks (M = 104, 88, 72, 64, 48, 32), a one-cell grid (3101), odd
-# counts
-@pytest.mark.parametrize("n,kc,rc_frac", [(3101, 25, 0.45), (5000, 22, 0.3), (8501, 18, 0.25), (12000, 16, 0.2),
-                                          (47001, 11, 0.12), (100000, 8, 0.1)])
+# sizes near the engine's bounds, with meshes of whole and partial bricks (M = 104, 88,
+# 80, 72, 64, 56), a one-cell grid (rc = L / 2), odd counts
+@pytest.mark.parametrize("n,kc,rc_frac", [(6001, 20, 0.3), (8501, 22, 0.3), (8501, 18, 0.25), (11301, 25, 0.5),
+                                          (12000, 16, 0.2), (32771, 13, 0.12)])
 def test_k_part_against_fp64(n, kc, rc_frac):
     ini, g = random_system_fast(n, seed=n, phi=0.10, B0=0.02)
     g["rc"], g["kc"] = rc_frac * g["lBox"], kc
