@@ -67,3 +67,20 @@ def test_contact_distances(scale):
     assert O.rms_rel(B, Bo, bAl) < TOL_FP64
     assert O.rms_rel(F, Fo, fAl) < TOL_FP64
     np.testing.assert_allclose(sim.get_state()[0], orc.get_state()[0], rtol=0, atol=1e-12 * g["lBox"])
+
+
+@pytest.mark.parametrize("n,phi,errtol", [(9, 0.2, 1e-2), (65, 0.2, 1e-3), (300, 0.25, 1e-4), (1001, 0.25, 1e-4)])
+def test_coating_pairs_of_the_mixed_path(n, phi, errtol):
+    """Short-range cutoffs with none to ~110 coating pairs per particle (more than a
+    warp queues), particle counts beyond whole blocks, mixed against FP64: the
+    coating force itself is FP64 in both, so its sums differ by FP32 rounding."""
+    ini, g = random_system(n, seed=n, rc_frac=0.4, phi=phi, min_gap=5e-10)
+    ini["interactions"]["ENABLE_COATING_POT"] = "true"
+    ini["short_range_interactions"]["errTolSR"] = str(errtol)
+    fAl, bAl, _ = scales(ini, g)
+    B0, F0, P0 = gpu_system(ini, g, 0).CompInteractions()
+    B, F, P = gpu_system(ini, g, 1).CompInteractions()
+    al = max(fAl, np.sqrt(np.mean(F0 ** 2)))
+    assert O.rms_rel(B, B0, bAl) < TOL_MIXED
+    assert O.rms_rel(F, F0, al) < TOL_MIXED
+    np.testing.assert_allclose(P, P0, rtol=0, atol=TOL_MIXED * al * g["rc"] * n)
