@@ -224,7 +224,7 @@ int pack(md_batch* b) {
   table(b->sort, [](md_ctx* c) { return cell_sort_blocks(c->grid); });
   table(b->real, [](md_ctx* c) { return real_blocks((int)c->n); });
   table(b->pass, [](md_ctx* c) { return real_pass_blocks((int)c->n); });
-  table(b->phase, [](md_ctx* c) { return phase_blocks((int)c->n); });
+  table(b->phase, [&](md_ctx* c) { return on_tc(c) ? 0 : phase_blocks((int)c->n); });
   table(b->sk, [&](md_ctx* c) { return on_tc(c) ? 0 : sk_blocks(k_params(c, nullptr, nullptr)); });
   table(b->red, [&](md_ctx* c) { return on_tc(c) ? 0 : skred_blocks(k_params(c, nullptr, nullptr)); });
   const int np = b->np;

@@ -546,6 +546,14 @@ __device__ __forceinline__ void cmul(T ar, T ai, T br, T bi, T& cr, T& ci) {
   ci = ar * bi + ai * br;
 }
 
+// exp(2 pi i n x) evaluated directly, x in 2^-32 box lengths.
+__device__ __forceinline__ float2 phase_direct(int nn, unsigned sfix) {
+  const int ph = (int)((unsigned)nn * sfix);  // exact reduction mod one box length
+  float s, c;
+  sincospif(2.0f * ((float)ph * 2.3283064365386963e-10f), &s, &c);
+  return make_float2(c, s);
+}
+
 // Device error word bits.
 enum : int { kErrNonFinite = 1, kErrQueue = 2, kErrTcWait = 4 };
 

@@ -42,14 +42,6 @@ constexpr int kSkThreads = 128;
 constexpr int kSkTile = 64;
 constexpr int kSegMax = 16;
 
-// exp(2 pi i n x) evaluated directly, x in 2^-32 box lengths.
-__device__ __forceinline__ float2 phase_direct(int nn, unsigned sfix) {
-  const int ph = (int)((unsigned)nn * sfix);  // exact reduction mod one box length
-  float s, c;
-  sincospif(2.0f * ((float)ph * 2.3283064365386963e-10f), &s, &c);
-  return make_float2(c, s);
-}
-
 // ------------------------------------------------------------ phase tables
 
 constexpr int kPhaseThreads = 256;
@@ -467,8 +459,8 @@ int launch_kspace(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaE
 int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64) {
   if (p.rw_T > 0) return launch_phase_rows(st, p, fp64);
   if (p.gm_M > 0) return 0;  // the mesh takes the coordinates themselves
+  if (p.tc_rows > 0) return launch_kspace_tc_prep(st, p);
   k_phase_tables<<<phase_blocks(p.n), kPhaseThreads, 0, st>>>(p);
-  if (p.tc_rows > 0) return 1 + launch_kspace_tc_prep(st, p);
   return 1;
 }
 

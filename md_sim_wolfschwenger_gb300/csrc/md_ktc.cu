@@ -36,7 +36,7 @@
 //
 // Kernels:
 //   k_tc_prep    once per step (positions are frozen across the step's
-//                evaluations): the X operand tiles (hi, lo) of every stage
+//                evaluations): the phases, the X operand tiles (hi, lo) of every stage
 //                of 32 particles in the shared-memory layout of the
 //                structure factor, and their Y, Z phases in blocks.
 //   k_sf_tc      grid (M tiles, chunks); 16 warps generate the U, V operand
@@ -178,6 +178,35 @@ static size_t scat_smem(int kc, int nst, int /*rows*/, bool yz = false) {
 
 // ------------------------------------------------------ per-step operands
 
+// The phases of kSfSC particles, to p.tab (the scatter reads them from there) and
+// to ph [3][kc + 1][kSfSC]: an anchor every four n, products with n = 1 .. 3 between
+// (the values of k_phase_tables; a launch of its own before this one took 3.5 us at
+// N = 2744, 13.5 us for 32 systems of 256 to 8192 particles).
+__device__ __forceinline__ void tc_phases(const KParams& p, int j0, float2* ph) {
+  const int K1 = p.kc + 1, G = (K1 + 3) / 4, n = p.n;
+  float2* gtab = (float2*)p.tab;
+  for (int e = threadIdx.x; e < 3 * G * kSfSC; e += blockDim.x) {
+    const int jj = e % kSfSC, g = e / kSfSC % G, ax = e / (kSfSC * G), j = j0 + jj;
+    if (j >= n) continue;
+    const int4 xi = p.s.xi[j];
+    const unsigned sf = (unsigned)(ax == 0 ? xi.x : (ax == 1 ? xi.y : xi.z));
+    const float2 a = phase_direct(4 * g, sf);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int nn = 4 * g + q;
+      if (nn >= K1) break;
+      float2 v = a;
+      if (q > 0) {
+        const float2 d = phase_direct(q, sf);
+        if (g == 0) v = d;
+        else cmul<float>(a.x, a.y, d.x, d.y, v.x, v.y);
+      }
+      ph[(ax * K1 + nn) * kSfSC + jj] = v;
+      gtab[(size_t)(ax * K1 + nn) * n + j] = v;
+    }
+  }
+}
+
 // Block per stage of kSfSC particles: X operand rows 2q = (Re X, -Im X),
 // 2q + 1 = (Im X, Re X) per particle (q = nx + kc; zero beyond 2 kc and
 // beyond n) as FP16 hi, lo tiles [ns][2 kSfSC]; Y(|ny|), Z(nz) of the stage's
@@ -185,7 +214,9 @@ static size_t scat_smem(int kc, int nst, int /*rows*/, bool yz = false) {
 __device__ __forceinline__ void tc_prep_body(const KParams& p, int sb) {
   const int NS = p.tc_ns, kc = p.kc, K1 = kc + 1, n = p.n;
   const int j0 = sb * kSfSC;
-  const float2* gtab = (const float2*)p.tab;
+  __shared__ float2 ph[3 * (kTcMaxKc + 1) * kSfSC];
+  tc_phases(p, j0, ph);
+  __syncthreads();
   // FP16 tiles [hi, lo][NS][32]: 2 bytes per element
   unsigned char* bimg = (unsigned char*)p.tc_bimg + (size_t)sb * 2 * NS * kSfSK * 2;
   for (int e = threadIdx.x; e < NS * (kSfSK / 4); e += blockDim.x) {
@@ -199,7 +230,7 @@ __device__ __forceinline__ void tc_prep_body(const KParams& p, int sb) {
       for (int h = 0; h < 2; h++) {
         const int j = j0 + 2 * c + h;
         if (j < n) {
-          const float2 X = gtab[(size_t)ax * n + j];
+          const float2 X = ph[ax * kSfSC + j - j0];
           const float xr = X.x, xi = nx < 0 ? -X.y : X.y;
           v[2 * h] = par ? xi : xr;
           v[2 * h + 1] = par ? xr : -xi;
@@ -216,7 +247,7 @@ __device__ __forceinline__ void tc_prep_body(const KParams& p, int sb) {
   for (int e = threadIdx.x; e < 2 * K1 * kTabPad; e += blockDim.x) {
     const int row = e / kTabPad, jj = e - row * kTabPad;  // row = axis (Y, Z) * K1 + |n|
     const int j = j0 + jj;
-    tb[e] = (jj < kSfSC && j < n) ? gtab[(size_t)(K1 + row) * n + j] : make_float2(0.f, 0.f);
+    tb[e] = (jj < kSfSC && j < n) ? ph[(K1 + row) * kSfSC + jj] : make_float2(0.f, 0.f);
   }
 }
 
