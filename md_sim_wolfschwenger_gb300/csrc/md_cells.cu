@@ -149,48 +149,10 @@ __device__ __forceinline__ void cell_sort(const CellParams& p, int bx) {
   if (!skip(p.flags) && p.grid.ncx > 1 && c < p.grid.ncell) sort_cell(p, c, threadIdx.x & 31);
 }
 
-// Sorted views.  Fixed point: x_fix = round(x_box * 2^32) as a wrapping
-// 32-bit integer, so x_fix[j] - x_fix[i] (mod 2^32) is the minimum-image
-// difference in units of L / 2^32 (about 4e-16 m at L = 1.7 um).  On a
-// rebuild the particle positions are recorded as the list's reference.
 template <typename T>
 __device__ __forceinline__ void sorted_fill(const CellParams& p, int bx) {
-  using T4 = typename V4<T>::t;
-  const int k = bx * kCellThreads + threadIdx.x, n = p.n;
-  if (k >= n) return;
-  const SortedView& s = p.s;
-  const int i = s.perm[k];
-  const bool rb = !p.flags || p.flags->rebuild;
-  const double px = p.pos[i], py = p.pos[n + i], pz = p.pos[2 * n + i];
-  if (rb) {
-    s.rank[i] = k;
-    s.cell[k] = p.cellOf[i];
-    if (p.xbuild) {
-      p.xbuild[i] = px;
-      p.xbuild[n + i] = py;
-      p.xbuild[2 * n + i] = pz;
-    }
-  }
-  const double rm = p.rMag_u[i];
-  if constexpr (std::is_same<T, float>::value) {
-    const int4 q = make_int4(fixed_box(px, p.invL), fixed_box(py, p.invL), fixed_box(pz, p.invL), i);
-    s.xi[k] = q;
-    // float copies for the cell scans (list builds, and every evaluation while
-    // the list does not fit)
-    const float sc = 2.3283064365386963e-10f;
-    if (rb || p.flags->overflow) s.xf[k] = make_float4((float)q.x * sc, (float)q.y * sc, (float)q.z * sc, (float)rm);
-  } else {
-    const double x = wrap_box(px, p.invL), y = wrap_box(py, p.invL), z = wrap_box(pz, p.invL);
-    s.xf[k] = make_float4((float)x, (float)y, (float)z, (float)rm);
-    s.xd[k] = make_double4_32a(x, y, z, rm);
-  }
-  const double mu = p.magMom_u[i];
-  T4 m;
-  m.x = (T)(p.mm[i] * mu);
-  m.y = (T)(p.mm[n + i] * mu);
-  m.z = (T)(p.mm[2 * n + i] * mu);
-  m.w = (T)rm;
-  ((T4*)s.mu)[k] = m;
+  const int k = bx * kCellThreads + threadIdx.x;
+  if (k < p.n) fill_one<T>(p, k);
 }
 
 // ------------------------------------------------------------ one system
@@ -414,7 +376,7 @@ int launch_disp_check(cudaStream_t st, int n, const double* pos, const double* x
   return 1;
 }
 
-int launch_cells(cudaStream_t st, const CellParams& p, bool fp64) {
+int launch_cells(cudaStream_t st, const CellParams& p, bool fp64, bool fill) {
   const int nb = cell_blocks(p.n);
   int launches = 1;
   if (p.n <= kClusterCells) {
@@ -430,6 +392,7 @@ int launch_cells(cudaStream_t st, const CellParams& p, bool fp64) {
       launches += 3;
     }
   }
+  if (!fill) return launches;
   if (fp64)
     k_sorted_fill<double><<<nb, kCellThreads, 0, st>>>(p);
   else

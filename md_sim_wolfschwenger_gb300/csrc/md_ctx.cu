@@ -411,7 +411,10 @@ static int issue_interactions(md_ctx* c, double dt = -1.0) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
   const CellParams cp = cell_params(c);
-  l += launch_cells(c->stream, cp, fp64(c));
+  const KParams kp = k_params(c, nullptr, nullptr);
+  const bool fused = fill_phases_fused(kp);
+  l += launch_cells(c->stream, cp, fp64(c), !fused);
+  if (fused) l += launch_fill_phases(c->stream, cp, kp, fp64(c));
   l += fork_join(
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,
       [&](cudaStream_t st) {
@@ -420,7 +423,7 @@ static int issue_interactions(md_ctx* c, double dt = -1.0) {
         return l;
       },
       [&](cudaStream_t st) { return launch_real(st, real_params(c, c->Br, c->Fr, c->ov), true, fp64(c)); },
-      [&](cudaStream_t st) { return launch_phase_tables(st, k_params(c, nullptr, nullptr), fp64(c)); },
+      [&](cudaStream_t st) { return fused ? 0 : launch_phase_tables(st, kp); },
       [&](cudaStream_t st) {
         return launch_kspace(st, k_params(c, c->Bk, c->Fk), true, fp64(c),
                              c->prof ? &c->ev[MD_SEG_KRED_FULL] : nullptr);

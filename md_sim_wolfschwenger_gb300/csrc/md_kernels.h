@@ -55,8 +55,14 @@ int launch_state_in(cudaStream_t st, int n, const double* hpos, const double* hm
 int launch_state_out(cudaStream_t st, int n, const double* pos, const double* mm, const double* ea, double* hpos,
                      double* hmm, double* hea);
 // Step start as above, cell order (skipped unless the step rebuilds) and the
-// sorted views.
-int launch_cells(cudaStream_t st, const CellParams& p, bool fp64);
+// sorted views (fill; else launch_fill_phases follows).
+int launch_cells(cudaStream_t st, const CellParams& p, bool fp64, bool fill);
+// Sorted views and the phase tables of launch_phase_tables in one launch: whether
+// these parameters take it, and the launch.
+bool fill_phases_fused(const KParams& p);
+int launch_fill_phases(cudaStream_t st, const CellParams& c, const KParams& p, bool fp64);
+int launch_fill_phase_rows(cudaStream_t st, const CellParams& c, const KParams& p, bool fp64);
+int launch_fill_tc_prep(cudaStream_t st, const CellParams& c, const KParams& p);
 int launch_cells_packed(cudaStream_t st, const CellParams* ps, int R, const Packed& n256, const Packed& sort,
                         const unsigned* anyrb);
 // Neighbour list within rc + skin (count, scan, fill; skipped unless rebuilding).
@@ -128,7 +134,6 @@ struct RowShape {
   int nblk, threads, chunk, nchunk;
 };
 RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
-int launch_phase_rows(cudaStream_t st, const KParams& p, bool fp64);
 // k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks and
 // partial-mesh floats of the spread.
 // (kc >= 5: M >= 24, so that a window and its neighbour bricks do not wrap onto themselves)
@@ -139,7 +144,7 @@ int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev);
 int launch_krows(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaEvent_t* ev);
 // Per-particle phase tables (once per step; positions are frozen across the
 // two Heun stages).
-int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64);
+int launch_phase_tables(cudaStream_t st, const KParams& p);
 int launch_phase_tables_packed(cudaStream_t st, const KParams* ps, const Packed& phase);
 // FP32 FMA-chain calibration: returns FLOPs issued by one launch.
 double launch_fma_calibration(cudaStream_t st, float* out, int blocks, int threads);

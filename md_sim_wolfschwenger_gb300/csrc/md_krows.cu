@@ -46,13 +46,16 @@ constexpr int kRowPhase = 256;
 // warps take the directly evaluated phases (n < 4 and the multiples of 4) in
 // turn, then the products (the same values as one thread per particle and
 // axis gives, 20 us at N = 1000, in 1/8 of the chain).
-__global__ void __launch_bounds__(kRowPhase) k_phase64(KParams p) {
+__global__ void __launch_bounds__(kRowPhase) k_phase64(CellParams cp, KParams p) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
   double2* d = (double2*)smem_raw;  // [direct phases][32]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kRowPhase / 32;
   const int ax = blockIdx.y, k = blockIdx.x * 32 + lane, kk = min(k, p.n - 1);
-  const double4_32a q = p.s.xd[kk];
-  const double xb = ax == 0 ? q.x : (ax == 1 ? q.y : q.z);
+  if (ax == 3) {  // the sorted views
+    if (w == 0 && k < p.n) fill_one<double>(cp, k);
+    return;
+  }
+  const double xb = wrap_box(cp.pos[(size_t)ax * p.n + cp.s.perm[kk]], cp.invL);
   const int nd = p.kc < 4 ? p.kc + 1 : 4 + (p.kc >> 2);  // 0, 1, 2, 3, 4, 8, 12, ..
   for (int t = w; t < nd; t += nw) {
     const int nn = t < 4 ? t : 4 * (t - 3);
@@ -81,12 +84,15 @@ __global__ void __launch_bounds__(kRowPhase) k_phase64(KParams p) {
 
 // FP32: every phase directly, one thread each (the reduction mod one box
 // length is exact in the fixed-point coordinates).
-__global__ void __launch_bounds__(kRowPhase) k_phase32(KParams p) {
+__global__ void __launch_bounds__(kRowPhase) k_phase32(CellParams cp, KParams p) {
   const int k = blockIdx.x * kRowPhase + threadIdx.x, e = blockIdx.y, K1 = p.kc + 1;
   if (k >= p.n) return;
   const int ax = e / K1, nn = e - ax * K1;
-  const int4 q = p.s.xi[k];
-  const int ph = (int)((unsigned)nn * (unsigned)(ax == 0 ? q.x : (ax == 1 ? q.y : q.z)));
+  if (ax == 3) {  // the sorted views
+    fill_one<float>(cp, k);
+    return;
+  }
+  const int ph = (int)((unsigned)nn * (unsigned)fixed_box(cp.pos[(size_t)ax * p.n + cp.s.perm[k]], cp.invL));
   float s, c;
   sincospif(2.0f * ((float)ph * 2.3283064365386963e-10f), &s, &c);
   ((float2*)p.tab)[(size_t)e * p.n + k] = make_float2(c, s);
@@ -421,12 +427,12 @@ RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64) {
   return s;
 }
 
-int launch_phase_rows(cudaStream_t st, const KParams& p, bool fp64) {
+int launch_fill_phase_rows(cudaStream_t st, const CellParams& c, const KParams& p, bool fp64) {
   if (fp64) {
     const int nd = p.kc < 4 ? p.kc + 1 : 4 + (p.kc >> 2);
-    k_phase64<<<dim3((p.n + 31) / 32, 3), kRowPhase, 32 * sizeof(double2) * (size_t)nd, st>>>(p);
+    k_phase64<<<dim3((p.n + 31) / 32, 4), kRowPhase, 32 * sizeof(double2) * (size_t)nd, st>>>(c, p);
   } else {
-    k_phase32<<<dim3((p.n + kRowPhase - 1) / kRowPhase, 3 * (p.kc + 1)), kRowPhase, 0, st>>>(p);
+    k_phase32<<<dim3((p.n + kRowPhase - 1) / kRowPhase, 3 * (p.kc + 1) + 1), kRowPhase, 0, st>>>(c, p);
   }
   return 1;
 }

@@ -456,8 +456,20 @@ int launch_kspace(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaE
   return 3;
 }
 
-int launch_phase_tables(cudaStream_t st, const KParams& p, bool fp64) {
-  if (p.rw_T > 0) return launch_phase_rows(st, p, fp64);
+// The chain cells -> sorted views -> phases -> structure factor is what small
+// systems wait for: their views and phases take one launch, each thread computing
+// the coordinates it needs from the positions.  Step: N = 512 49.6 -> 48.2, N =
+// 3001 90.0 -> 87.6 us.  Beyond kFuseTc particles of the tensor-core engine the
+// real-space branch, which then is the longer one, would wait for the operands.
+constexpr int kFuseTc = 4096;
+bool fill_phases_fused(const KParams& p) {
+  return p.rw_T > 0 || (p.gm_M == 0 && p.tc_rows > 0 && p.n <= kFuseTc);
+}
+int launch_fill_phases(cudaStream_t st, const CellParams& c, const KParams& p, bool fp64) {
+  return p.rw_T > 0 ? launch_fill_phase_rows(st, c, p, fp64) : launch_fill_tc_prep(st, c, p);
+}
+
+int launch_phase_tables(cudaStream_t st, const KParams& p) {
   if (p.gm_M > 0) return 0;  // the mesh takes the coordinates themselves
   if (p.tc_rows > 0) return launch_kspace_tc_prep(st, p);
   k_phase_tables<<<phase_blocks(p.n), kPhaseThreads, 0, st>>>(p);

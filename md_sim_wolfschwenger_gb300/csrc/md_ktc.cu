@@ -182,14 +182,14 @@ static size_t scat_smem(int kc, int nst, int /*rows*/, bool yz = false) {
 // to ph [3][kc + 1][kSfSC]: an anchor every four n, products with n = 1 .. 3 between
 // (the values of k_phase_tables; a launch of its own before this one took 3.5 us at
 // N = 2744, 13.5 us for 32 systems of 256 to 8192 particles).
-__device__ __forceinline__ void tc_phases(const KParams& p, int j0, float2* ph) {
+template <typename X>
+__device__ __forceinline__ void tc_phases(const KParams& p, int j0, float2* ph, X&& coord) {
   const int K1 = p.kc + 1, G = (K1 + 3) / 4, n = p.n;
   float2* gtab = (float2*)p.tab;
   for (int e = threadIdx.x; e < 3 * G * kSfSC; e += blockDim.x) {
     const int jj = e % kSfSC, g = e / kSfSC % G, ax = e / (kSfSC * G), j = j0 + jj;
     if (j >= n) continue;
-    const int4 xi = p.s.xi[j];
-    const unsigned sf = (unsigned)(ax == 0 ? xi.x : (ax == 1 ? xi.y : xi.z));
+    const unsigned sf = (unsigned)coord(ax, j);
     const float2 a = phase_direct(4 * g, sf);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -211,11 +211,12 @@ __device__ __forceinline__ void tc_phases(const KParams& p, int j0, float2* ph) 
 // 2q + 1 = (Im X, Re X) per particle (q = nx + kc; zero beyond 2 kc and
 // beyond n) as FP16 hi, lo tiles [ns][2 kSfSC]; Y(|ny|), Z(nz) of the stage's
 // particles.
-__device__ __forceinline__ void tc_prep_body(const KParams& p, int sb) {
+template <typename X>
+__device__ __forceinline__ void tc_prep_body(const KParams& p, int sb, X&& coord) {
   const int NS = p.tc_ns, kc = p.kc, K1 = kc + 1, n = p.n;
   const int j0 = sb * kSfSC;
   __shared__ float2 ph[3 * (kTcMaxKc + 1) * kSfSC];
-  tc_phases(p, j0, ph);
+  tc_phases(p, j0, ph, coord);
   __syncthreads();
   // FP16 tiles [hi, lo][NS][32]: 2 bytes per element
   unsigned char* bimg = (unsigned char*)p.tc_bimg + (size_t)sb * 2 * NS * kSfSK * 2;
@@ -251,11 +252,25 @@ __device__ __forceinline__ void tc_prep_body(const KParams& p, int sb) {
   }
 }
 
-__global__ void __launch_bounds__(256) k_tc_prep(KParams p) { tc_prep_body(p, blockIdx.x); }
+__device__ __forceinline__ int sorted_coord(const KParams& p, int ax, int j) {
+  const int4 xi = p.s.xi[j];
+  return ax == 0 ? xi.x : (ax == 1 ? xi.y : xi.z);
+}
+__global__ void __launch_bounds__(256) k_tc_prep(KParams p) {
+  tc_prep_body(p, blockIdx.x, [&](int ax, int j) { return sorted_coord(p, ax, j); });
+}
+// With the sorted views of the block's particles.
+__global__ void __launch_bounds__(256) k_fill_tc_prep(CellParams c, KParams p) {
+  const int k = blockIdx.x * kSfSC + threadIdx.x;
+  if (threadIdx.x < kSfSC && k < p.n) fill_one<float>(c, k);
+  tc_prep_body(p, blockIdx.x,
+               [&](int ax, int j) { return fixed_box(c.pos[(size_t)ax * p.n + c.s.perm[j]], c.invL); });
+}
 // Packed systems: one block per task (system, stage block).
 __global__ void __launch_bounds__(256) k_tc_prep_packed(const KParams* __restrict__ ps, const Task* __restrict__ tk) {
   const Task t = tk[blockIdx.x];
-  tc_prep_body(ps[t.rep], t.blk);
+  const KParams& p = ps[t.rep];
+  tc_prep_body(p, t.blk, [&](int ax, int j) { return sorted_coord(p, ax, j); });
 }
 
 // ------------------------------------------------------ structure factor
@@ -1025,6 +1040,11 @@ void kspace_tc_row_desc(const int2* rows, int R, int kc, int n, bool yz, float4*
 size_t kspace_tc_image_floats(int kc, int nt) { return (size_t)nt * 2 * kScCols * tc_kp(kc); }
 size_t kspace_tc_bimg_floats(int kc, int nsb) { return (size_t)nsb * tc_ns(kc) * kSfSK; }  // FP16 hi, lo
 size_t kspace_tc_tblk_entries(int kc, int nsb) { return (size_t)nsb * 2 * (kc + 1) * kTabPad; }
+
+int launch_fill_tc_prep(cudaStream_t st, const CellParams& c, const KParams& p) {
+  k_fill_tc_prep<<<(p.n + kSfSC - 1) / kSfSC, 256, 0, st>>>(c, p);
+  return 1;
+}
 
 int launch_kspace_tc_prep(cudaStream_t st, const KParams& p) {
   k_tc_prep<<<(p.n + kSfSC - 1) / kSfSC, 256, 0, st>>>(p);
