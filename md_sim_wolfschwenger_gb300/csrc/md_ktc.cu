@@ -46,9 +46,10 @@
 //                dealt round-robin, one accumulator each, added in a fixed
 //                order at the end); mbarriers hand stages between the roles
 //                and tcgen05.commit releases the slots.
-//   k_sf_tc_reduce  exact sum of the chunk partials (TwoSum pairs, then
-//                FP64), S(n) = C_U + nx C_V and e(n) S(n) in FP64, and the scatter's W operand image (hi, lo) in
-//                the shared-memory layout the scatter copies in bulk.
+//   k_sf_tc_reduce  exact sum of the chunk partials (TwoSum pairs, then one
+//                FP64 addition), S(n) = C_U + nx C_V and e(n) S(n) in FP64, and
+//                the scatter's W operand image (hi, lo) in the shared-memory
+//                layout the scatter copies in bulk.
 //   k_kscat_tc   128 particles per block, their X phases (the A operand, hi
 //                and lo) in tensor memory; W tiles of 128 columns stream in
 //                by bulk copy (2-3 stages); two issuing warps alternate tiles
@@ -599,9 +600,9 @@ __device__ __forceinline__ void w_put(float* img, int kp, int row, int k, float 
 // <= 512 particles) are added exactly: within a group with error-free FP32
 // transformations (TwoSum: the running sum and its exact rounding errors;
 // GB300's FP64 rate is a small fraction of FP32, so a conversion and an FP64
-// addition per partial would cost more than the whole FP32 reduction), the
-// group sum (sum + compensation) and the groups in FP64, as are S(n) = C_U +
-// nx C_V and e(n) S(n); the W image is then split into its FP32 operands.
+// addition per partial would cost more than the whole FP32 reduction), and so
+// are the groups' pairs; sum + compensation, S(n) = C_U + nx C_V and e(n) S(n) are
+// FP64; the W image is then split into its FP32 operands.
 __device__ __forceinline__ void two_sum_acc(float& s, float& c, float v) {
   const float t = s + v;
   const float bp = t - s;
@@ -614,7 +615,7 @@ constexpr int kRedGroups = 8, kRedGroupsPacked = 2;
 template <bool FULL, int G>
 __device__ __forceinline__ void sf_reduce_body(const KParams& p, int bx) {
   using L = ScatLayout<FULL>;
-  __shared__ double red[G][4][64];  // [group][4 values][row]
+  __shared__ float2 red[G][4][64];  // [group][4 values][row]: sum, rounding errors
   const int Q = 2 * p.kc + 1;
   const int mtile = bx / Q, q = bx - mtile * Q;
   const int rl = threadIdx.x & 63, grp = threadIdx.x >> 6;
@@ -636,14 +637,23 @@ __device__ __forceinline__ void sf_reduce_body(const KParams& p, int bx) {
     two_sum_acc(su[3], cu[3], bc[(2 * q + 1) * 128 + 64 + rl]);
   }
 #pragma unroll
-  for (int v = 0; v < 4; v++) red[grp][v][rl] = (double)su[v] + (double)cu[v];
+  for (int v = 0; v < 4; v++) red[grp][v][rl] = make_float2(su[v], cu[v]);
   __syncthreads();
   if (grp != 0) return;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  // the groups' pairs the same way: 2^-48 of the sum, far below its terms' own
+  // errors (FP64 additions here were a chain of 64 cycles each: N = 3001 87.4 -> 82.8
+  // us per step, S unchanged to the digits shown, 3.3157e-7 of it off FP64)
 #pragma unroll
-  for (int g = 0; g < G; g++)
+  for (int g = 1; g < G; g++)
 #pragma unroll
-    for (int v = 0; v < 4; v++) acc[v] += red[g][v][rl];
+    for (int v = 0; v < 4; v++) {
+      const float2 q = red[g][v][rl];
+      two_sum_acc(su[v], cu[v], q.x);
+      cu[v] += q.y;
+    }
+  double acc[4];
+#pragma unroll
+  for (int v = 0; v < 4; v++) acc[v] = (double)su[v] + (double)cu[v];
   const int r = mtile * 64 + rl;
   if (r >= p.tc_rows) return;
   const int kk = p.tc_kmap[r * Q + q];
