@@ -406,8 +406,10 @@ static int fork_join(md_ctx* c, int q, int seg_real, int seg_k, RP&& real_prep, 
 }
 
 // Field + force evaluation on the current master state (no integrator).
-// dt >= 0: the step's noise is drawn beside it.
-static int issue_interactions(md_ctx* c, double dt = -1.0) {
+// dt >= 0: the step's noise is drawn beside it.  after_records: the step before left
+// its records to the side stream (issue_step); they come before the noise, and with
+// it the integrator.
+static int issue_interactions(md_ctx* c, double dt = -1.0, bool after_records = false) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
   const CellParams cp = cell_params(c);
@@ -419,6 +421,7 @@ static int issue_interactions(md_ctx* c, double dt = -1.0) {
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,
       [&](cudaStream_t st) {
         int l = launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), &c->sc->flags, fp64(c));
+        if (after_records) cudaStreamWaitEvent(st, c->join_ev[2], 0);
         if (dt >= 0) l += launch_noise(st, int_params(c, dt, nullptr, nullptr), fp64(c));
         return l;
       },
@@ -446,13 +449,26 @@ static int issue_field(md_ctx* c) {
       });
 }
 
-static int issue_step(md_ctx* c, double dt) {
-  int l = issue_interactions(c, dt);
+// leave_records: another step follows in the same graph, and the records of this
+// one are taken beside the start of that one (the kernel that ends with them in its
+// last block costs the chain of steps ~2 us more: N = 512 49.0 -> 46.8 us per step).
+static int issue_step(md_ctx* c, double dt, bool after_records = false, bool leave_records = false) {
+  int l = issue_interactions(c, dt, after_records);
   mark(c, MD_SEG_HEUN1);
   l += launch_heun1(c->stream, int_params(c, dt, c->Br, c->Bk), fp64(c));
   l += issue_field(c);
   mark(c, MD_SEG_HEUN2);
-  l += launch_heun2_obs(c->stream, int_params(c, dt, c->Br2, c->Bk2), obs_params(c, dt), &c->sc->done, fp64(c));
+  const IntParams ip = int_params(c, dt, c->Br2, c->Bk2);
+  const ObsParams op = obs_params(c, dt);
+  if (leave_records) {
+    l += launch_heun2(c->stream, ip, fp64(c));
+    cudaEventRecord(c->fork_ev[2], c->stream);
+    cudaStreamWaitEvent(c->side, c->fork_ev[2], 0);
+    l += launch_records(c->side, op, (int)c->n);
+    cudaEventRecord(c->join_ev[2], c->side);
+    return l;
+  }
+  l += launch_heun2_obs(c->stream, ip, op, &c->sc->done, fp64(c));
   mark(c, MD_SEG_OBS);  // the records are taken inside the stage-2 launch
   mark(c, MD_NSEG);
   return l;
@@ -948,7 +964,7 @@ int md_ctx_create(const md_config* cfg, int64_t n, int precision, md_ctx** out) 
       cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess)
     return fail(set_err(nullptr, MD_ERR_CUDA, "cudaStreamCreate failed"));
   pool_keep(c->device);
-  for (int q = 0; q < 2; q++)
+  for (int q = 0; q < 3; q++)
     if (cudaEventCreateWithFlags(&c->fork_ev[q], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->join_ev[q], cudaEventDisableTiming) != cudaSuccess)
       return fail(set_err(nullptr, MD_ERR_CUDA, "cudaEventCreate failed"));
@@ -1015,7 +1031,7 @@ int md_ctx_destroy(md_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->allocs.clear();
   c->alloc_bytes.clear();
-  for (int q = 0; q < 2; q++) {
+  for (int q = 0; q < 3; q++) {
     if (c->fork_ev[q]) cudaEventDestroy(c->fork_ev[q]);
     if (c->join_ev[q]) cudaEventDestroy(c->join_ev[q]);
   }
@@ -1522,7 +1538,7 @@ int prepare_dt(md_ctx* c, double dt) {
 // Captures k steps as one graph.
 static int capture_steps(md_ctx* c, int k, double dt, cudaGraph_t* graph, cudaGraphExec_t* exec, int* launches) {
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
-  for (int s = 0; s < k; s++) *launches = issue_step(c, dt);
+  for (int s = 0; s < k; s++) *launches = issue_step(c, dt, s > 0, s < k - 1);
   cudaError_t e = cudaStreamEndCapture(c->stream, graph);
   if (e != cudaSuccess) return set_err(c, MD_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
   CK(c, cudaGraphInstantiate(exec, *graph, 0));

@@ -52,7 +52,7 @@ struct md_ctx {
   // second stream of the step: the k-space branch runs on it concurrently
   // with the real-space branch (fork/join events; captured into the graph)
   cudaStream_t side = nullptr;
-  cudaEvent_t fork_ev[2] = {}, join_ev[2] = {};
+  cudaEvent_t fork_ev[3] = {}, join_ev[3] = {};  // full evaluation, field evaluation, records
   std::string err;
   int err_status = 0;
   std::vector<void*> allocs;

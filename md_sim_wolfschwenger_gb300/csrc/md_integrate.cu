@@ -471,6 +471,10 @@ __global__ void __launch_bounds__(256) k_obs(ObsParams p) { obs(p); }
 // Launched in blocks of kIntOne threads (bounded so: 72 registers and no
 // spills, where the bound of kIntThreads gave 64 and spilled).
 template <typename T>
+__global__ void __launch_bounds__(kIntOne) k_heun2(IntParams p) {
+  heun2<T>(p, blockIdx.x);
+}
+template <typename T>
 __global__ void __launch_bounds__(kIntOne) k_heun2_obs(IntParams p, ObsParams o, unsigned* done) {
   heun2<T>(p, blockIdx.x);
   __shared__ int last;
@@ -749,6 +753,21 @@ int launch_heun2_obs(cudaStream_t st, const IntParams& p, const ObsParams& o_in,
     k_heun2_obs<double><<<int_blocks_one(p.n), kIntOne, 0, st>>>(p, o, done);
   else
     k_heun2_obs<float><<<int_blocks_one(p.n), kIntOne, 0, st>>>(p, o, done);
+  return 1;
+}
+
+// Stage 2 and its records as two launches, with the same sums.
+int launch_heun2(cudaStream_t st, const IntParams& p, bool fp64) {
+  if (fp64)
+    k_heun2<double><<<int_blocks_one(p.n), kIntOne, 0, st>>>(p);
+  else
+    k_heun2<float><<<int_blocks_one(p.n), kIntOne, 0, st>>>(p);
+  return 1;
+}
+int launch_records(cudaStream_t st, const ObsParams& o_in, int n) {
+  ObsParams o = o_in;
+  o.nblk_int = int_blocks_one(n);
+  k_obs<<<1, kIntOne, 0, st>>>(o);
   return 1;
 }
 

@@ -160,6 +160,8 @@ int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, c
 int launch_heun1(cudaStream_t st, const IntParams& p, bool fp64);
 int launch_obs(cudaStream_t st, const ObsParams& p);
 // Stage 2 with the step records (k_obs) fused: done = a zeroed block counter.
+int launch_heun2(cudaStream_t st, const IntParams& p, bool fp64);
+int launch_records(cudaStream_t st, const ObsParams& o, int n);
 int launch_heun2_obs(cudaStream_t st, const IntParams& p, const ObsParams& o, unsigned* done, bool fp64);
 int launch_heun1_packed(cudaStream_t st, const IntParams* ps, const Packed& n256);
 int launch_heun2_packed(cudaStream_t st, const IntParams* ps, const Packed& n256);
