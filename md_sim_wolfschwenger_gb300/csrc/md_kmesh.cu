@@ -25,7 +25,7 @@
 // fixed order: results are deterministic.
 //
 // Measured at N = 32768 (M = 64) / 131072 (M = 80), us: spread 29 / 79, the four
-// transforms 30 / 50, interpolation 41 / 124 with the force, 35 / 107 without;
+// transforms 30 / 50, interpolation 36 / 104 with the force, 29 / 80 without;
 // the tensor cores' 135 / 850 and 120 / 700 for the same.
 #include "md_common.cuh"
 #include "md_kernels.h"
@@ -633,15 +633,19 @@ __global__ void __launch_bounds__(256) k_mesh_yz(KParams p) {
 // factors are applied at the end of their loops, so a mesh point costs six
 // multiply-adds (three without the force).
 //
-// Bound: shared-memory wavefronts (four per 27 mesh points, 27 times per particle)
-// and issue.  Reading the mesh from global memory took 46 / 37 us at N = 32768,
-// M = 64 (L1); the brick in the threads' registers, as in the spread, 68 / 53 us
-// (sums over the lanes for every particle).
-constexpr int kFY = 17;  // row stride: lane l's point lies in bank group l mod 8
-static_assert(kFY % 8 == kMW % 8 && kFY >= kPZ, "27 lanes in four wavefronts");
+// Bound: shared-memory wavefronts (three per 27 mesh points, 27 times per particle)
+// and issue: 36 / 29 us at N = 32768, M = 64 (41 / 35 with float4 points, four
+// wavefronts; 46 / 37 from global memory, L1; 68 / 53 with the brick in the threads'
+// registers, as in the spread, for its sums over the lanes).
+// (b_x, b_y) rows are rotated by 9 y, so that the points of 16 lanes on three rows of
+// nine lie in 16 pairs of banks; b_z rows are 21 apart (0 .. 8, 21 .. 29, 42 .. 50
+// are 27 banks): three wavefronts for 27 points, where float4 takes four.
+constexpr int kFZ = 21;
+static_assert(kMW == 9 && kPZ == 16 && kPY == 16, "rotation and stride of the brick's rows");
 constexpr int kInThreads = 384;
 struct InterpSmem {
-  float4 f[kPX * kPY * kFY];
+  float2 fxy[kPX * kPY * kPZ];
+  float fz[kPX * kPY * kFZ];
   int j[kInThreads];
   BrickScan<kInThreads> scan;
 };
@@ -656,7 +660,9 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
 #pragma unroll 8
   for (int e = tid; e < kPX * kPY * kPZ; e += kInThreads) {
     const int x = e / (kPY * kPZ), y = e / kPZ % kPY, z = e % kPZ;
-    sm.f[(x * kPY + y) * kFY + z] = p.gm_b[((size_t)fold(x0 + x) * M + fold(y0 + y)) * M + fold(z0 + z)];
+    const float4 v = p.gm_b[((size_t)fold(x0 + x) * M + fold(y0 + y)) * M + fold(z0 + z)];
+    sm.fxy[(x * kPY + y) * kPZ + ((z + kMW * y) & (kPZ - 1))] = make_float2(v.x, v.y);
+    sm.fz[(x * kPY + y) * kFZ + z] = v.z;
   }
   const int rr = min(lane / kMW, 2), pt = lane % kMW;  // also the axis of the window values
   const bool on = lane < 3 * kMW;
@@ -699,7 +705,13 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
             w = fmaf(w, s, cf[d]);
           }
           if (FULL) dw *= 2.f * (rr == 0 ? mu.x : (rr == 1 ? mu.y : mu.z));
-          const float4* f = sm.f + (ix * kPY + iy + rr) * kFY + iz + pt;
+          const float2* fxy[3];
+#pragma unroll
+          for (int t = 0; t < 3; t++) {
+            const int y = iy + 3 * t + rr;
+            fxy[t] = sm.fxy + (ix * kPY + y) * kPZ + ((iz + pt + kMW * y) & (kPZ - 1));
+          }
+          const float* fz = sm.fz + (ix * kPY + iy + rr) * kFZ + iz + pt;
           // packed: (x, y) and (z, z) of a mesh point against the window value and, in
           // the other half or another sum, its derivative
           float2 gxy[3] = {}, gz[3] = {}, hxy[3] = {};
@@ -708,13 +720,14 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
             const float xv = __shfl_sync(kFull, w, a), xd = FULL ? __shfl_sync(kFull, dw, a) : 0.f;
 #pragma unroll
             for (int t = 0; t < 3; t++) {
-              const float4 v = f[(a * kPY + 3 * t) * kFY];
-              gxy[t] = __ffma2_rn(make_float2(v.x, v.y), make_float2(xv, xv), gxy[t]);
+              const float2 v = fxy[t][a * kPY * kPZ];
+              const float z = fz[(a * kPY + 3 * t) * kFZ];
+              gxy[t] = __ffma2_rn(v, make_float2(xv, xv), gxy[t]);
               if (FULL) {
-                hxy[t] = __ffma2_rn(make_float2(v.x, v.y), make_float2(xd, xd), hxy[t]);
-                gz[t] = __ffma2_rn(make_float2(v.z, v.z), make_float2(xv, xd), gz[t]);
+                hxy[t] = __ffma2_rn(v, make_float2(xd, xd), hxy[t]);
+                gz[t] = __ffma2_rn(make_float2(z, z), make_float2(xv, xd), gz[t]);
               } else {
-                gz[t].x = fmaf(v.z, xv, gz[t].x);
+                gz[t].x = fmaf(z, xv, gz[t].x);
               }
             }
           }
