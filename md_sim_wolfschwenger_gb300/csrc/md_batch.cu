@@ -57,6 +57,7 @@ struct md_batch {
   int* d_toff = nullptr;    // per-system first-task offsets of every table
   size_t toff_cap = 0;
   Packed n256{}, sort{}, real{}, pass{}, phase{}, sk{}, red{}, sc{};
+  int pass_run = 1;  // groups of four particles per task of `pass`
   WorkQ* d_wq = nullptr;  // one work queue per task table (persistent packed launches)
   unsigned* d_anyrb = nullptr;  // some system rebuilds its lists this step (zeroed)
   // systems whose k space runs on the tensor cores (the context's engine):
@@ -167,6 +168,8 @@ __global__ void __launch_bounds__(256) k_expand_tasks(const int* __restrict__ to
   for (int q = q0 + (int)threadIdx.x; q < q1; q += blockDim.x) out[q] = Task{r, q - q0};
 }
 
+constexpr int64_t kPassTasks = 2500;  // real-space tasks below which groups are not joined
+
 // Task tables, parameters and the captured step for the current systems.
 int pack(md_batch* b) {
   drop_graph(b);
@@ -223,7 +226,15 @@ int pack(md_batch* b) {
   table(b->n256, [](md_ctx* c) { return cell_blocks((int)c->n); });
   table(b->sort, [](md_ctx* c) { return cell_sort_blocks(c->grid); });
   table(b->real, [](md_ctx* c) { return real_blocks((int)c->n); });
-  table(b->pass, [](md_ctx* c) { return real_pass_blocks((int)c->n); });
+  // A real-space task: up to eight groups of four particles, one after another,
+  // while two or three tasks per resident block remain.  A group takes ~7 us, a
+  // claim (an atomic's way to L2, two block barriers, the system's parameters) ~10 %
+  // of that: 32 systems of 256 to 8192 particles 897 -> 857 us per step, 8 of 256
+  // to 4000 188 -> 180 (at 4000 tasks 854 and 188).
+  int64_t groups = 0;
+  for (const Slot& s : b->slots) groups += real_pass_blocks((int)s.ctx->n, 1);
+  b->pass_run = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups / kPassTasks));
+  table(b->pass, [&](md_ctx* c) { return real_pass_blocks((int)c->n, b->pass_run); });
   table(b->phase, [&](md_ctx* c) { return on_tc(c) ? 0 : phase_blocks((int)c->n); });
   table(b->sk, [&](md_ctx* c) { return on_tc(c) ? 0 : sk_blocks(k_params(c, nullptr, nullptr)); });
   table(b->red, [&](md_ctx* c) { return on_tc(c) ? 0 : skred_blocks(k_params(c, nullptr, nullptr)); });
@@ -310,13 +321,13 @@ int pack(md_batch* b) {
   l += launch_kspace_packed(k, b->d_kfull, b->sk, b->red, b->sc, true, b->kcmax, b->np);
   l += launch_kspace_tc_packed(k, b->d_kfull, b->tsf, b->tred, b->tsc, true, b->tc_sf_smem, b->tc_sc_smem);
   l += launch_nbr_packed(s, b->d_rfull, R, b->real, b->d_anyrb);
-  l += launch_real_packed(s, b->d_rfull, b->real, b->pass, true, b->coat);
+  l += launch_real_packed(s, b->d_rfull, b->real, b->pass, b->pass_run, true, b->coat);
   join(0);
   l += launch_heun1_packed(s, b->d_i1, b->n256);
   fork(1);
   l += launch_kspace_packed(k, b->d_kfield, b->sk, b->red, b->sc, false, b->kcmax, b->np);
   l += launch_kspace_tc_packed(k, b->d_kfield, b->tsf, b->tred, b->tsc, false, b->tc_sf_smem, b->tc_sc_smem);
-  l += launch_real_packed(s, b->d_rfield, b->real, b->pass, false, false);
+  l += launch_real_packed(s, b->d_rfield, b->real, b->pass, b->pass_run, false, false);
   join(1);
   l += launch_heun2_packed(s, b->d_i2, b->n256);
   l += launch_obs_packed(s, b->d_obs, R, b->d_anyrb);

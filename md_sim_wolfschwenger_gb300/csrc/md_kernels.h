@@ -27,7 +27,7 @@ int persistent_grid(const void* fn, int threads, size_t smem, int ntask);
 int cell_blocks(int n);                 // cell assign/scatter/fill, integrator
 int cell_sort_blocks(const CellGrid& g);
 int real_blocks(int n);                 // real space (8-warp blocks)
-int real_pass_blocks(int n);            // real-space passes without coating (4-warp blocks)
+int real_pass_blocks(int n, int run);  // real-space passes without coating (run groups of 4 particles per block)
 int nbr_blocks(int n, bool fp64);       // neighbour-list build (mixed: a warp per two particles)
 int phase_blocks(int n);
 int sk_blocks(const KParams& p);
@@ -76,7 +76,7 @@ int launch_real(cudaStream_t st, const RealParams& p, bool full, bool fp64);
 // In-range ordered pairs of the last evaluation's geometry, added to *out.
 void launch_count_pairs(cudaStream_t st, const RealParams& p, unsigned long long* out, bool fp64);
 // pass: the 4-warp-block table (real_pass_blocks), used unless full && coat
-int launch_real_packed(cudaStream_t st, const RealParams* ps, const Packed& real, const Packed& pass, bool full,
+int launch_real_packed(cudaStream_t st, const RealParams* ps, const Packed& real, const Packed& pass, int run, bool full,
                        bool coat);
 
 // k space: structure factor partials, reduction, scatter (full or field only).

@@ -1419,9 +1419,15 @@ __global__ void __launch_bounds__(1024) k_nbr_scan_packed(const RealParams* __re
 // steps; 6.92 at 6 / 7, 6.97 at 5 / 7)
 template <bool FULL, bool COAT>
 __global__ void __launch_bounds__(((FULL && COAT) ? kRealWarps : kFieldWarps) * 32, COAT ? 2 : (FULL ? 6 : 8))
-    k_real_packed(const RealParams* __restrict__ ps, const Task* __restrict__ tk, int ntask, WorkQ* wq) {
+    k_real_packed(const RealParams* __restrict__ ps, const Task* __restrict__ tk, int ntask, WorkQ* wq, int run) {
   for_tasks<false>(tk, ntask, wq, [&](const Task& t) {
-      real_eval32<FULL, COAT, (FULL && COAT) ? kRealWarps : kFieldWarps>(ps[t.rep], t.blk);
+    const RealParams& p = ps[t.rep];
+    if constexpr (FULL && COAT) {
+      real_eval32<FULL, COAT, kRealWarps>(p, t.blk);
+    } else {
+#pragma unroll 1
+      for (int s = 0; s < run; s++) real_eval32<FULL, COAT, kFieldWarps>(p, run * t.blk + s);
+    }
   });
 }
 
@@ -1438,7 +1444,7 @@ static void keep_l1(const void* kern) {
 }
 
 int real_blocks(int n) { return (n + kRealWarps - 1) / kRealWarps; }
-int real_pass_blocks(int n) { return (n + kFieldWarps - 1) / kFieldWarps; }
+int real_pass_blocks(int n, int run) { return (n + kFieldWarps * run - 1) / (kFieldWarps * run); }
 int nbr_blocks(int n, bool fp64) { return real_blocks(fp64 ? n : (n + 1) / 2); }
 
 int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64) {
@@ -1498,12 +1504,12 @@ int launch_nbr_packed(cudaStream_t st, const RealParams* ps, int R, const Packed
   return 3;
 }
 
-int launch_real_packed(cudaStream_t st, const RealParams* ps, const Packed& real, const Packed& pass, bool full,
+int launch_real_packed(cudaStream_t st, const RealParams* ps, const Packed& real, const Packed& pass, int run, bool full,
                        bool coat) {
   keep_l1((const void*)k_real_packed<true, false>);
   keep_l1((const void*)k_real_packed<false, false>);
   auto go = [&](auto kern, const Packed& tb, int th) {
-    kern<<<persistent_grid((const void*)kern, th, 0, tb.n), th, 0, st>>>(ps, tb.tasks, tb.n, tb.wq);
+    kern<<<persistent_grid((const void*)kern, th, 0, tb.n), th, 0, st>>>(ps, tb.tasks, tb.n, tb.wq, run);
   };
   if (full && coat) {
     if (!real.n) return 0;
