@@ -58,3 +58,20 @@ def test_particles_far_from_their_cells():
     b = k_part(sim, mm)
     for q in (2, 3):
         assert rms(b[q], a[q]) < TOL
+
+
+@pytest.mark.parametrize("n,kc", [(8501, 18), (12000, 16)])
+def test_crowded_bricks(n, kc):
+    """Half of the particles in 1/64 of the box: bricks with many times the
+    particles that a block stages at once, and empty ones."""
+    ini, g = random_system_fast(n, seed=n + 1, phi=0.02, B0=0.02)
+    g["rc"], g["kc"] = 0.2 * g["lBox"], kc
+    g["alpha"] = 3.5 / g["rc"]
+    g["pos"][:, : n // 2] *= 0.25
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref = k_part(gpu_system(ini, g, 0), mm)
+    sim = gpu_system(ini, g, 1)
+    sim.set_strong_pairs(0.0)
+    got = k_part(sim, mm)
+    for q in range(3):
+        assert rms(got[q], ref[q]) < TOL
