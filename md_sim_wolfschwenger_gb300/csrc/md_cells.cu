@@ -30,9 +30,18 @@ namespace md {
 
 constexpr int kCellThreads = 256;
 
-__device__ __forceinline__ int cell_coord(double xb, int ncx) {
-  int c = (int)((xb + 0.5) * (double)ncx);
-  return c < 0 ? 0 : (c >= ncx ? ncx - 1 : c);
+// Cell along one axis.  The mixed path (FIXED) takes it from the fixed-point
+// coordinate that its sorted views hold: the list build finds a pair's image by
+// the cells, so a particle within 2^-33 of the upper face, whose fixed-point
+// coordinate has wrapped to the lower one, has to be filed there too.
+template <bool FIXED>
+__device__ __forceinline__ int cell_coord(double x, double invL, int ncx) {
+  if constexpr (FIXED) {
+    return (int)__umulhi((unsigned)fixed_box(x, invL) + 0x80000000u, (unsigned)ncx);
+  } else {
+    const int c = (int)((wrap_box(x, invL) + 0.5) * (double)ncx);
+    return c < 0 ? 0 : (c >= ncx ? ncx - 1 : c);
+  }
 }
 
 __device__ __forceinline__ bool skip(const StepFlags* f) { return f && !f->rebuild; }
@@ -50,6 +59,7 @@ __device__ __forceinline__ void step_begin(StepFlags* f, float half_skin) {
 }
 
 // Cell of each particle (all-pairs grid: identity order, one cell).
+template <bool FIXED>
 __device__ __forceinline__ void assign_one(const CellParams& p, int i) {
   const int n = p.n, ncx = p.grid.ncx;
   if (ncx == 1) {
@@ -57,16 +67,17 @@ __device__ __forceinline__ void assign_one(const CellParams& p, int i) {
     p.cellOf[i] = 0;
     return;
   }
-  const int cx = cell_coord(wrap_box(p.pos[i], p.invL), ncx);
-  const int cy = cell_coord(wrap_box(p.pos[n + i], p.invL), ncx);
-  const int cz = cell_coord(wrap_box(p.pos[2 * n + i], p.invL), ncx);
+  const int cx = cell_coord<FIXED>(p.pos[i], p.invL, ncx);
+  const int cy = cell_coord<FIXED>(p.pos[n + i], p.invL, ncx);
+  const int cz = cell_coord<FIXED>(p.pos[2 * n + i], p.invL, ncx);
   const int c = (cz * ncx + cy) * ncx + cx;
   p.cellOf[i] = c;
   atomicAdd(&p.count[c], 1);
 }
+template <bool FIXED>
 __device__ __forceinline__ void cell_assign(const CellParams& p, int bx) {
   const int i = bx * kCellThreads + threadIdx.x;
-  if (!skip(p.flags) && i < p.n) assign_one(p, i);
+  if (!skip(p.flags) && i < p.n) assign_one<FIXED>(p, i);
 }
 
 // Exclusive scan of count[0..ncell) -> start[0..ncell]; count is zeroed so it
@@ -172,6 +183,7 @@ __device__ __forceinline__ void cluster_sync() {
   __threadfence();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+template <bool FIXED>
 __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(1024) k_cells_small(CellParams p) {
   StepFlags* f = p.flags;
   const int g = blockIdx.x * 1024 + threadIdx.x, G = kClusterBlocks * 1024;
@@ -179,7 +191,7 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(1024) k
   cluster_sync();  // every thread has read the flags
   if (g == 0) step_begin(f, p.half_skin);
   if (!rb) return;
-  for (int i = g; i < p.n; i += G) assign_one(p, i);
+  for (int i = g; i < p.n; i += G) assign_one<FIXED>(p, i);
   if (p.grid.ncx == 1) return;
   cluster_sync();
   if (blockIdx.x == 0) scan_cells(p);
@@ -188,7 +200,8 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(1024) k
   cluster_sync();
   for (int c = g >> 5; c < p.grid.ncell; c += G >> 5) sort_cell(p, c, threadIdx.x & 31);
 }
-__global__ void __launch_bounds__(kCellThreads) k_cell_assign(CellParams p) { cell_assign(p, blockIdx.x); }
+template <bool FIXED>
+__global__ void __launch_bounds__(kCellThreads) k_cell_assign(CellParams p) { cell_assign<FIXED>(p, blockIdx.x); }
 __global__ void __launch_bounds__(1024) k_cell_scan(CellParams p) { cell_scan(p); }
 __global__ void __launch_bounds__(kCellThreads) k_cell_scatter(CellParams p) { cell_scatter(p, blockIdx.x); }
 __global__ void __launch_bounds__(kCellThreads) k_cell_sort(CellParams p) { cell_sort(p, blockIdx.x); }
@@ -218,7 +231,7 @@ __global__ void __launch_bounds__(kCellThreads) k_cell_assign_packed(const CellP
                                                                      const unsigned* anyrb) {
   if (!__ldcg(anyrb)) return;  // the whole grid: no system rebuilds this step
   for_tasks<true>(tk, ntask, wq, [&](const Task& t) {
-      cell_assign(ps[t.rep], t.blk);
+      cell_assign<true>(ps[t.rep], t.blk);  // packed systems are mixed
   });
 }
 __global__ void __launch_bounds__(1024) k_cell_scan_packed(const CellParams* __restrict__ ps) {
@@ -380,10 +393,10 @@ int launch_cells(cudaStream_t st, const CellParams& p, bool fp64, bool fill) {
   const int nb = cell_blocks(p.n);
   int launches = 1;
   if (p.n <= kClusterCells) {
-    k_cells_small<<<kClusterBlocks, 1024, 0, st>>>(p);
+    fp64 ? k_cells_small<false><<<kClusterBlocks, 1024, 0, st>>>(p) : k_cells_small<true><<<kClusterBlocks, 1024, 0, st>>>(p);
   } else {
     k_step_begin<<<1, 32, 0, st>>>(p.flags, p.half_skin);
-    k_cell_assign<<<nb, kCellThreads, 0, st>>>(p);
+    fp64 ? k_cell_assign<false><<<nb, kCellThreads, 0, st>>>(p) : k_cell_assign<true><<<nb, kCellThreads, 0, st>>>(p);
     launches++;
     if (p.grid.ncx > 1) {
       k_cell_scan<<<1, 1024, 0, st>>>(p);

@@ -113,3 +113,35 @@ def test_cell_order_of_small_and_large_systems(n, rc_frac):
         cell = (c[2] * ncx + c[1]) * ncx + c[0]
         np.testing.assert_array_equal(perm, np.argsort(cell, kind="stable"))
         np.testing.assert_array_equal(cs, np.concatenate([[0], np.cumsum(np.bincount(cell, minlength=ncx ** 3))]))
+
+
+@pytest.mark.parametrize("n,rc_frac", [(2001, 0.2), (8500, 0.15)])
+def test_particles_on_the_faces_of_the_box(n, rc_frac):
+    """Particles within the rounding of the fixed-point coordinates (2^-33 box
+    lengths) of a face, on each axis and both sides of it: whichever side their
+    coordinate is rounded to, their neighbours list them and they their neighbours
+    (one more of them on each side, well inside the range)."""
+    ini, g = random_system(n, seed=n, rc_frac=rc_frac, lognormal=True)
+    fAl, bAl, _ = scales(ini, g)
+    L, x = g["lBox"], g["pos"]
+    i = iter(np.random.default_rng(3).permutation(n))
+    for a in range(3):
+        for f in (0.5 - 1e-11, 0.5 * (1 - 1e-15), -(0.5 - 1e-11), 0.5 - 2.0 ** -34, 0.45, -0.45):
+            for _ in range(4):
+                x[a, next(i)] = f * L
+    ref = gpu_system(ini, g, 0)
+    B0, F0, P0 = ref.CompInteractions()
+    sim = gpu_system(ini, g, 1)
+    B, F, P = sim.CompInteractions()
+    want = 0
+    for k in range(n):
+        d = x[:, k + 1:] - x[:, k:k + 1]
+        d -= L * np.rint(d / L)
+        want += int(((d ** 2).sum(0) < g["rc"] ** 2).sum())
+    assert ref.pairs() == want
+    # a pair at the cut-off itself may fall on either side in FP32
+    assert abs(sim.pairs() - want) <= 2
+    assert O.rms_rel(B, B0, bAl) < TOL_MIXED and O.rms_rel(F, F0, fAl) < TOL_MIXED
+    # each particle: a missing neighbour is ~rc^-3 of a moment, far above FP32 rounding
+    assert np.abs(B - B0).max() < 1e-4 * np.abs(B0).max()
+    np.testing.assert_allclose(P, P0, rtol=0, atol=TOL_MIXED * fAl * g["rc"] * n)
