@@ -332,9 +332,10 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 
 // Neighbours A and B: fixed-point pair vectors (dxf..), r2f = |d_fix|^2,
 // moments ma, mb; inA, inB: the pair is within rc; stA, stB: it is a strong pair
-// (its terms are added in FP64; it still pushes).  A pair that adds nothing
-// gets a distance at which exp(-alpha^2 r^2) is zero, and with it every
-// coefficient: no weights.  Same formulas as pair_terms; the pair vector stays
+// (its terms are added in FP64; it still pushes).  A pair that adds nothing has no
+// weight: out of range it gets a distance of ~4e9 box lengths, where exp(-alpha^2
+// r^2) is zero and the coefficients are, for any alpha, below 1e-28; a strong pair
+// gets 1 / r = 0.  Same formulas as pair_terms; the pair vector stays
 // in fixed-point units, their powers of 2^-32 folded into the constants, and
 // the coefficients are negated (the fit's sign), which saves the sign of the
 // field's second term.  push: the lane's overlap push in shared memory ([3][32]),
@@ -356,7 +357,7 @@ template <bool FULL>
 __device__ __forceinline__ void pair_terms2(const PairK& K, float wdc, float2 dxf, float2 dyf, float2 dzf, float2 r2f,
                                             bool inA, bool inB, bool stA, bool stB, const float4& mi,
                                             const float4& ma, const float4& mb, Acc2& s, float* push) {
-  const float far2 = 1.8446744e23f;  // (100 box lengths)^2 in fixed units
+  const float far2 = 3e38f;  // in fixed units
   float2 r2 = mul2(pk(inA ? r2f.x : far2, inB ? r2f.y : far2), pk1(5.421010862427522e-20f));  // 2^-64
   float2 ire = pk(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));  // 1 / r
   float2 r = mul2(r2, ire);
@@ -381,8 +382,9 @@ __device__ __forceinline__ void pair_terms2(const PairK& K, float wdc, float2 dx
     };
     if (r.x < dcont.x) clamp(r.x, ire.x, r2e.x, dcont.x, dxf.x, dyf.x, dzf.x);
     if (r.y < dcont.y) clamp(r.y, ire.y, r2e.y, dcont.y, dxf.y, dyf.y, dzf.y);
-    if (stA) r2e.x = 1e4f;
-    if (stB) r2e.y = 1e4f;
+    // a strong pair adds nothing here: every coefficient has a factor 1 / r^2
+    if (stA) ire.x = 0.f;
+    if (stB) ire.y = 0.f;
   }
   const float2 ire2 = mul2(ire, ire);
   const float2 ee = mul2(r2e, pk1(K.ke));

@@ -102,3 +102,26 @@ def test_monodisperse_has_no_strong_pairs():
     err, _ = workloads.mixed_vs_fp64(cfg, rMag, rHydr, pos, mm, ea, ewald)
     assert err["strong_entries"] == 0
     assert err["B"] < TOL_MIXED and err["F"] < TOL_MIXED and err["torque"] < TOL_MIXED, err
+
+
+@pytest.mark.parametrize("alpha", [1e-6, 1e-3, 0.01, 0.03, 0.1, 1.0])
+@pytest.mark.parametrize("n", [257, 1001])
+def test_strong_pairs_count_once_at_any_splitting(n, alpha):
+    """alpha L down to a bare cut-off sum, where exp(-alpha^2 r^2) is 1 over many
+    boxes: strong pairs come from the FP64 list alone, and list entries out of range
+    add nothing."""
+    from helpers import gpu_system, random_system, scales
+    ini, g = random_system(n, seed=n, rc_frac=0.4, lognormal=True)
+    fAl, bAl, _ = scales(ini, g)
+    g["alpha"], g["kc"] = alpha / g["lBox"], 6
+    B0, F0, P0 = gpu_system(ini, g, 0).CompInteractions()
+    sim = gpu_system(ini, g, 1)
+    sim.set_neighbor_skin(0.2)
+    B, F, P = sim.CompInteractions()
+    assert sim.strong_pairs() > 0
+    assert O.rms_rel(B, B0, bAl) < TOL_MIXED and O.rms_rel(F, F0, fAl) < TOL_MIXED
+    np.testing.assert_allclose(P, P0, rtol=0, atol=TOL_MIXED * fAl * g["rc"] * n)
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref = gpu_system(ini, g, 0)
+    ref.CompInteractions()
+    assert O.rms_rel(sim.CompDemagField(mm), ref.CompDemagField(mm), bAl) < TOL_MIXED
