@@ -531,7 +531,12 @@ __global__ void __launch_bounds__(kIntThreads) k_combine(IntParams p, double* Bo
       if (Bout) Bout[a * n + i] = b[a];
       if (Fout) Fout[a * n + i] = ((double)((const T*)p.Fr)[a * n + r] + sf[a] + (double)((const T*)p.Fk)[a * n + r]) *
                                   p.F_unit;
-      if (apply_overlap) p.pos[a * n + i] += (double)((const T*)p.ov)[a * n + r] * p.L;
+      if (apply_overlap) {
+        const T o = ((const T*)p.ov)[a * n + r];
+        p.pos[a * n + i] += (double)o * p.L;
+        // the particle may have left its cell: the next evaluation sorts anew
+        if (o != (T)0) p.flags->force = 1;
+      }
       if (Ppart_out) pr[a] += p.Ppart[3 * i + a];
     }
   }
