@@ -289,7 +289,7 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   if (c->gm_M > 0) p.gm_nbrick = md::mesh_bricks(c->gm_M);
   p.gm_ncx = c->grid.ncx;
   // half the skin since the build, and rounding
-  p.gm_reach = (float)(0.5 * c->skin_frac * c->rc / c->L * (1.0 + 1e-5) + 2e-6);
+  p.gm_reach = (float)(0.5 * c->cell_skin * c->rc / c->L * (1.0 + 1e-5) + 2e-6);
   p.gm_coef = c->gm_coef;
   p.gm_fac = c->gm_fac;
   p.gm_tw = c->gm_tw;
@@ -412,6 +412,7 @@ static int fork_join(md_ctx* c, int q, int seg_real, int seg_k, RP&& real_prep, 
 static int issue_interactions(md_ctx* c, double dt = -1.0, bool after_records = false) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
+  if (!c->list_valid) c->cell_skin = c->skin_frac;  // this evaluation sorts anew
   const CellParams cp = cell_params(c);
   const KParams kp = k_params(c, nullptr, nullptr);
   const bool fused = fill_phases_fused(kp);
@@ -495,14 +496,27 @@ int force_rebuild(md_ctx* c) {
   return MD_OK;
 }
 
-int alloc_nbr(md_ctx* c, long long cap) {
+// Capacity of the neighbour list.  keep: the current list stays (field evaluations
+// at the last geometry still read it), unless there is no memory for both.
+int alloc_nbr(md_ctx* c, long long cap, bool keep) {
   cap = std::min<long long>(cap, 0x7ffffffeLL);
   if (cap <= c->nbr_cap) return MD_OK;
+  int* list = nullptr;
+  if (keep && c->have_geometry && c->nbr) {
+    const size_t at = (size_t)(std::find(c->allocs.begin(), c->allocs.end(), (void*)c->nbr) - c->allocs.begin());
+    const size_t held = std::min(c->alloc_bytes[at], 4 * (size_t)cap);
+    if (dalloc(c, &list, 4 * (size_t)cap) == MD_OK) {
+      CK(c, cudaMemcpyAsync(list, c->nbr, held, cudaMemcpyDeviceToDevice, c->stream));
+    } else {
+      cudaGetLastError();
+      c->have_geometry = false;
+    }
+  }
   dfree(c, c->nbr);
-  c->nbr = nullptr;
+  c->nbr = list;
   c->nbr_cap = 0;
-  int st = dalloc(c, &c->nbr, 4 * (size_t)cap);
-  if (st) return st;
+  if (!list)
+    if (int st = dalloc(c, &c->nbr, 4 * (size_t)cap)) return st;
   c->nbr_cap = cap;
   invalidate_graph(c);
   return MD_OK;
@@ -1919,13 +1933,14 @@ int md_set_neighbor_skin(md_ctx* c, double skin_frac) {
   if (!c || !(skin_frac >= 0) || skin_frac > 1) return set_err(c, MD_ERR_INVALID, "skin fraction must be in [0, 1]");
   if (int st = count_pairs(c)) return st;
   c->skin_frac = skin_frac;
+  c->cell_skin = std::max(c->cell_skin, skin_frac);
   c->list_valid = false;
   invalidate_graph(c);
   if (c->have_ewald) {
     const double rlb = c->rc / c->L * (1.0 + c->skin_frac);
     double est = (double)c->n * (double)c->n * 4.0 / 3.0 * 3.141592653589793 * rlb * rlb * rlb;
     est = std::min(est, (double)c->n * (double)(c->n - 1));
-    if (int st = alloc_nbr(c, (long long)(1.3 * est) + 64LL * c->n)) return st;
+    if (int st = alloc_nbr(c, (long long)(1.3 * est) + 64LL * c->n, true)) return st;
   }
   return force_rebuild(c);
 }

@@ -163,6 +163,9 @@ struct md_ctx {
   // particle ~5 pm at dt = 1e-12 s, so even a 0.5 % skin (1 nm at rc = 400
   // nm) is crossed only after ~1e4 steps and rebuilds stay rare.
   double skin_frac = 0.005;
+  // skin that the particles in the current cells may have used (larger than skin_frac
+  // between md_set_neighbor_skin and the next full evaluation)
+  double cell_skin = 0.005;
   int64_t pairs = 0;        // in-range pairs of the last evaluation, as last counted
   bool list_valid = false;  // a build for the current particles, grid and skin exists
   // Strong pairs (mixed path, md_real.cu): list entries whose force weight
@@ -214,7 +217,7 @@ md::IntParams int_params(md_ctx* c, double dt, const void* Br, const void* Bk);
 md::ObsParams obs_params(md_ctx* c, double dt);
 int check_ready(md_ctx* c, bool need_state);
 int force_rebuild(md_ctx* c);
-int alloc_nbr(md_ctx* c, long long cap);
+int alloc_nbr(md_ctx* c, long long cap, bool keep = false);
 // Strong-pair path: on for the mixed path without coating potentials and
 // with a finite threshold; alloc_strong grows the strong list.
 bool strong_active(const md_ctx* c);

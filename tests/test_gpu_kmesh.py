@@ -96,3 +96,27 @@ def test_step_after_overlaps_were_pushed(prec):
     tol = 1e-11 if prec == 0 else 2e-6
     for x, y, s in zip(a.get_state(), b.get_state(), (g["lBox"], 1.0, 1.0)):
         assert np.abs(x - y).max() < tol * s
+
+
+@pytest.mark.parametrize("skin", [1e-9, 0.9])
+def test_field_after_the_skin_was_changed(skin):
+    """A new skin holds from the next full evaluation on: a field at the last
+    geometry still finds the particles that moved out of their cells within the old
+    skin, and the list that was built for it."""
+    n = 8501
+    ini, g = random_system_fast(n, seed=17, phi=0.10, B0=0.02)
+    g["rc"], g["kc"] = 0.25 * g["lBox"], 18
+    g["alpha"] = 3.5 / g["rc"]
+    sim = gpu_system(ini, g, 1)
+    sim.set_neighbor_skin(0.3)
+    sim.CompInteractions()
+    perm = sim.debug_cells()[2]
+    sim.set_state(g["pos"] + 0.08 * g["rc"], g["mm"], g["ea"])  # 0.14 rc, all together
+    sim.step(1, 1e-14)
+    np.testing.assert_array_equal(sim.debug_cells()[2], perm)  # not sorted anew
+    mm = np.roll(g["mm"], 1, axis=1)
+    a = sim.CompDemagField(mm)
+    sim.set_neighbor_skin(skin)
+    assert rms(sim.CompDemagField(mm), a) < TOL
+    sim.CompInteractions()
+    assert rms(sim.CompDemagField(mm), a) < TOL
