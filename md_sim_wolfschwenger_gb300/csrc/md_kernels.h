@@ -23,6 +23,10 @@ struct Packed {
 // over the task table.
 int persistent_grid(const void* fn, int threads, size_t smem, int ntask);
 
+// Raises a kernel's dynamic shared memory limit to what the device allows, once per
+// device: a launch's own size must not depend on what another host thread set last.
+void allow_smem(const void* fn);
+
 // Blocks of one system per kernel shape (task-table construction).
 int cell_blocks(int n);                 // cell assign/scatter/fill, integrator
 int cell_sort_blocks(const CellGrid& g);

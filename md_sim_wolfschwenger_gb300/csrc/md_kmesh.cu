@@ -774,19 +774,19 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
 
 int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) {
   const int M = p.gm_M, kc1 = p.kc + 1, Q = 2 * p.kc + 1;
-  cudaFuncSetAttribute(k_mesh_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpreadSmem));
+  allow_smem((const void*)k_mesh_spread);
   k_mesh_spread<<<p.gm_nbrick, kBrThreads, sizeof(SpreadSmem), st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_mesh_z<<<dim3(M, M / kMZLines), 256, sizeof(float) * (2 * M + 3 * kMZLines * (M + 1)), st>>>(p);
   k_mesh_y<<<dim3(kc1, M / kMYLines), (16 * kc1 + 31) / 32 * 32, sizeof(float2) * (M + 3 * kMYLines * (M + 2)), st>>>(p);
   k_mesh_x<<<p.tc_rows, kMXThreads, sizeof(float) * (6 * M + 4 * kc1 + 8 * kMXThreads), st>>>(p);
   const size_t smi = sizeof(float4) * kc1 * Q * kMIx + sizeof(float2) * (M + kMIx * kMIy * kc1 * 3);
-  cudaFuncSetAttribute(k_mesh_yz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smi);
+  allow_smem((const void*)k_mesh_yz);
   k_mesh_yz<<<dim3(M / kMIx, M / kMIy), 256, smi, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal);
   const void* kern = full ? (const void*)k_mesh_interp<true> : (const void*)k_mesh_interp<false>;
   const size_t smf = sizeof(InterpSmem);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
+  allow_smem(kern);
   if (full)
     k_mesh_interp<true><<<p.gm_nbrick, kInThreads, smf, st>>>(p);
   else

@@ -274,7 +274,7 @@ extern "C" int md_rdf(md_ctx* c, int64_t bins, double range, double r_mag0, int 
         (int)std::floor(rb.rcont * rb.inv_bw), jmax, d_counts);
   } else {
     const size_t smem = (sizeof(double) + sizeof(float)) * 3 * md::kRdfThreads + sizeof(unsigned int) * (size_t)bins;
-    cudaFuncSetAttribute(md::k_rdf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    md::allow_smem((const void*)md::k_rdf);
     md::k_rdf<<<dim3(nt, nt), md::kRdfThreads, smem, c->stream>>>(n, c->pos, rb, (float)(rbox * rbox), jmax, d_counts);
   }
   std::vector<unsigned long long> h((size_t)bins);
