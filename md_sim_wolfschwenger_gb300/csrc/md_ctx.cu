@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -569,10 +570,10 @@ void update_strong(md_ctx* c) {
 // shell between contact and the distance where the weight falls to theta
 // (2 * 1.25e5 entries estimated vs 1.22e5 built for N = 32768, log-normal
 // sigma 0.2).
-double strong_estimate(const md_ctx* c) {
-  const std::vector<double>& m = c->props.magMom;
-  const std::vector<double>& rh = c->props.rHydr;
-  if (m.empty() || !(c->strong_theta > 0)) return 0;
+static double strong_estimate(const mdh::Props& p, double L, double rl, double theta) {
+  const std::vector<double>& m = p.magMom;
+  const std::vector<double>& rh = p.rHydr;
+  if (m.empty() || !(theta > 0)) return 0;
   double mmin = 1e300, mmax = 0, rhmin = 1e300;
   for (size_t i = 0; i < m.size(); i++) {
     mmin = std::min(mmin, m[i]);
@@ -588,16 +589,20 @@ double strong_estimate(const md_ctx* c) {
     mb[b] = std::max(mb[b], m[i]);
     rb[b] = std::min(rb[b], rh[i]);
   }
-  const double pi = 3.141592653589793, V = c->L * c->L * c->L, dmin = 2.0 * rhmin;
+  const double pi = 3.141592653589793, V = L * L * L, dmin = 2.0 * rhmin;
   double tot = 0;
   for (int a = 0; a < nb; a++)
     for (int b = 0; b < nb; b++) {
       if (cnt[a] == 0 || cnt[b] == 0) continue;
-      const double rs = dmin * std::pow(mb[a] * mb[b] / (mmin * mmin * c->strong_theta), 0.25);
-      const double rc = std::min(rs, c->rc * (1.0 + c->skin_frac)), cont = rb[a] + rb[b];
+      const double rs = dmin * std::pow(mb[a] * mb[b] / (mmin * mmin * theta), 0.25);
+      const double rc = std::min(rs, rl), cont = rb[a] + rb[b];
       if (rc > cont) tot += cnt[a] * cnt[b] * 4.0 / 3.0 * pi * (rc * rc * rc - cont * cont * cont) / V;
     }
   return tot;
+}
+
+static long long strong_entries(const md_ctx* c) {
+  return 4096 + (long long)(2.0 * strong_estimate(c->props, c->L, c->rc * (1.0 + c->skin_frac), c->strong_theta));
 }
 
 // After work on the stream: a neighbour list that did not fit was replaced by
@@ -657,6 +662,36 @@ static int tc_kc_bound(const md_ctx* c) {
   return (fp64(c) || c->kengine == MD_KSPACE_SIMT) ? 0 : md::kspace_tc_max_kc();
 }
 
+static int num_sms(int device) {
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  return nsm;
+}
+
+// Cells: a stencil of +-2 on the FP64 path; on the mixed path ~4 particles
+// each, which keeps the two consecutive sorted particles whose lists one
+// warp builds close together and fits the cells to the search sphere.
+static CellGrid cell_grid(double rc_box, int64_t n, bool f64) {
+  const int reach = f64 ? 2 : (int)std::lround(rc_box * std::cbrt(0.25 * (double)n));
+  return mdh::choose_grid(rc_box, n, std::max(2, std::min(reach, 12)));
+}
+
+// Structure-factor grid of the row segments (segment blocks x particle chunks): the
+// fewest whole waves of resident blocks that keep every FP32 chunk sum within 512
+// particles, with the chunk count chosen to fill those waves.
+static void segment_chunks(const mdh::KList& k, int64_t n, int kc, int nsm, int* chunk, int* nchunk) {
+  const int nsegb = (int)((k.seg.size() + md::sk_threads() - 1) / md::sk_threads());
+  const int64_t slots = (int64_t)nsm * md::sk_resident_blocks(kc);
+  const int64_t nch_min = std::max<int64_t>(1, (n + 511) / 512);
+  const int64_t waves = std::max<int64_t>(1, (nsegb * nch_min + slots - 1) / slots);
+  int64_t nch = std::max<int64_t>(nch_min, waves * slots / nsegb);
+  nch = std::min<int64_t>(nch, (n + 31) / 32);
+  *chunk = (int)(((n + nch - 1) / nch + 31) / 32 * 32);
+  *nchunk = (int)((n + *chunk - 1) / *chunk);
+}
+
+void ctx_packed_only(md_ctx* c) { c->packed_only = true; }
+
 // Tensor-core k space: the k rows (ny, nz) of the half-space k list, ordered
 // by nz then ny, the k index of each (row, nx), and the buffers of the
 // launches (md_ktc.cu).  Off (tc_rows = 0) on the FP64 path, when the
@@ -678,9 +713,7 @@ static int setup_tc(md_ctx* c) {
   std::vector<int> kmap((size_t)R * Q, -1);
   for (int k = 0; k < nk; k++)
     if (c->klist.kreal[k]) kmap[(size_t)rowid[{c->klist.kz[k], c->klist.ky[k]}] * Q + c->klist.kx[k] + kc] = k;
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const md::TcShape t = md::kspace_tc_shape(kc, (int)c->n, R, nsm, c->tc_ring, c->tc_waves);
+  const md::TcShape t = md::kspace_tc_shape(kc, (int)c->n, R, num_sms(c->device), c->tc_ring, c->tc_waves);
   void* old[] = {c->tc_row, c->tc_rowd, c->tc_kmap, c->tc_part, c->tc_wfull, c->tc_wfield, c->tc_bimg, c->tc_tblk};
   for (void* q : old) dfree(c, q);
   c->tc_row = nullptr;
@@ -728,8 +761,8 @@ static int setup_tc(md_ctx* c) {
 // the caller chose is kept.
 static bool krows_wanted(const md_ctx* c) {
   const double nk = 2.0943951 * (double)c->kc * (double)c->kc * (double)c->kc;  // half space
-  return c->kengine == MD_KSPACE_AUTO && c->tc_ring < 0 && c->tc_waves == 1 && md::kspace_tc_supported((int)c->kc) &&
-         nk * (double)c->n <= 3e6;
+  return c->kengine == MD_KSPACE_AUTO && !c->packed_only && c->tc_ring < 0 && c->tc_waves == 1 &&
+         md::kspace_tc_supported((int)c->kc) && nk * (double)c->n <= 3e6;
 }
 
 // k space by rows: tasks of four consecutive |nx| of one k row, rows by nz
@@ -761,9 +794,7 @@ static int setup_rows(md_ctx* c) {
     rowt.push_back(make_int2(t0, nt));
   }
   const int T = (int)task.size(), R = (int)row.size();
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const md::RowShape sh = md::krows_shape(kc, (int)c->n, T, nsm, fp64(c));
+  const md::RowShape sh = md::krows_shape(kc, (int)c->n, T, num_sms(c->device), fp64(c));
   void* old[] = {c->rw_task, c->rw_kidx, c->rw_row, c->rw_rowt, c->rw_ad};
   for (void* q : old) dfree(c, q);
   c->rw_task = nullptr;
@@ -816,7 +847,7 @@ static int setup_rows(md_ctx* c) {
 // force 2.8e-7 / 1.3e-6.  An engine or a tensor-core tiling that the caller chose is
 // kept.
 static bool mesh_wanted(const md_ctx* c) {
-  if (fp64(c) || c->kengine != MD_KSPACE_AUTO || c->tc_ring >= 0 || c->tc_waves != 1 || c->tc_rows == 0) return false;
+  if (fp64(c) || c->kengine != MD_KSPACE_AUTO || c->packed_only || c->tc_ring >= 0 || c->tc_waves != 1 || c->tc_rows == 0) return false;
   const double M = md::mesh_points((int)c->kc);
   return c->n >= 6000 && (c->kc >= 15 || (c->kc >= 13 && c->n >= 32768)) && M * M * M <= 100.0 * (double)c->n;
 }
@@ -1275,28 +1306,8 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
   const double ab = alpha * c->L;
   const double w = std::pow(c->cfg.my_pi / ab, 2.0);
   c->klist = mdh::build_klist((int)kc, w);
-  // cells: a stencil of +-2 on the FP64 path; on the mixed path ~4 particles
-  // each, which keeps the two consecutive sorted particles whose lists one
-  // warp builds close together and fits the cells to the search sphere
-  int reach = 2;
-  if (!fp64(c))
-    reach = (int)std::lround(rc / c->L * std::cbrt(0.25 * (double)c->n));
-  c->grid = mdh::choose_grid(rc / c->L, c->n, std::max(2, std::min(reach, 12)));
-  if (!fp64(c)) {
-    // structure-factor grid (segment blocks x particle chunks): the fewest
-    // whole waves of resident blocks that keep every FP32 chunk sum within 512
-    // particles, with the chunk count chosen to fill those waves
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-    const int nsegb = (int)((c->klist.seg.size() + md::sk_threads() - 1) / md::sk_threads());
-    const int64_t slots = (int64_t)nsm * md::sk_resident_blocks((int)kc);
-    const int64_t nch_min = std::max<int64_t>(1, (c->n + 511) / 512);
-    const int64_t waves = std::max<int64_t>(1, (nsegb * nch_min + slots - 1) / slots);
-    int64_t nch = std::max<int64_t>(nch_min, waves * slots / nsegb);
-    nch = std::min<int64_t>(nch, (c->n + 31) / 32);
-    c->chunk = (int)(((c->n + nch - 1) / nch + 31) / 32 * 32);
-    c->nchunk = (int)((c->n + c->chunk - 1) / c->chunk);
-  }
+  c->grid = cell_grid(rc / c->L, c->n, fp64(c));
+  if (!fp64(c)) segment_chunks(c->klist, c->n, (int)kc, num_sms(c->device), &c->chunk, &c->nchunk);
   // (re)allocate Ewald-sized buffers
   const int ncell = c->grid.ncell;
   if (ncell + 1 > c->ncell_cap) {
@@ -1386,20 +1397,53 @@ int md_set_ewald(md_ctx* c, double alpha, double rc, int64_t kc) {
     for (int q = 0; q < 6; q++) c->kself[q] = 4.0 * c->cfg.my_pi * K[q];
   }
   {
-    // neighbour-list capacity: uniform-density estimate + margin (grown on overflow)
-    const double rlb = rc / c->L * (1.0 + c->skin_frac);
-    double est = (double)c->n * (double)c->n * 4.0 / 3.0 * 3.141592653589793 * rlb * rlb * rlb;
-    est = std::min(est, (double)c->n * (double)(c->n - 1));
-    int st = alloc_nbr(c, (long long)(1.3 * est) + 64LL * c->n);
+    int st = alloc_nbr(c, mdh::list_entries(c->n, rc / c->L * (1.0 + c->skin_frac)));
     if (st) return st;
   }
   update_strong(c);
   if (c->strong_w4sq > 0.f && !c->cfg.ENABLE_COATING_POT)
-    if (int st = alloc_strong(c, 4096 + (long long)(2.0 * strong_estimate(c)))) return st;
+    if (int st = alloc_strong(c, strong_entries(c))) return st;
   if (int st = force_rebuild(c)) return st;
   c->have_ewald = true;
   c->have_geometry = false;
   return MD_OK;
+}
+
+// The allocations of md_ctx_create and md_set_ewald, and of the records.
+double mdi_packed_ctx_bytes(const md_config* cfg, int64_t n, const double* rMag, double alpha, double rc,
+                                       int64_t kc, int64_t steps) {
+  mdh::Props p;
+  std::string e;
+  if (mdh::make_props(*cfg, rMag, nullptr, n, &p, &e)) return -1.0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int nsm = num_sms(dev);
+  const double N = (double)n, L = p.lBox, rl = rc * (1.0 + kSkinFrac);
+  const mdh::KList k = mdh::build_klist((int)kc, std::pow(cfg->my_pi / (alpha * L), 2.0));
+  const size_t ks = std::max(std::max((size_t)k.nk, k.seg.size()), std::max((size_t)k.nk_scat, k.rseg.size())) + 2;
+  int chunk = 0, nchunk = 0;
+  segment_chunks(k, n, (int)kc, nsm, &chunk, &nchunk);
+  double b = 661.0 * N + 4096;                                        // state, stages and work arrays
+  b += 8.0 * (cell_grid(rc / L, n, false).ncell + 1);                 // cells
+  b += 4.0 * (double)mdh::list_entries(n, rl / L);                    // neighbour list
+  if (!cfg->ENABLE_COATING_POT)                                       // strong list and its sums
+    b += (sizeof(int2) + 96.0) * (4096 + 2.0 * strong_estimate(p, L, rl, kStrongTheta));
+  b += (48.0 + 2 * sizeof(KSeg)) * (double)ks + 16.0 * (double)k.nk * nchunk + 24.0 * (kc + 1) * N;  // k vectors, phases
+  if (md::kspace_tc_supported((int)kc)) {
+    std::set<std::pair<int, int>> rows;
+    for (int q = 0; q < k.nk; q++)
+      if (k.kreal[q]) rows.insert({k.kz[q], k.ky[q]});
+    const int R = (int)rows.size();
+    const md::TcShape t = md::kspace_tc_shape((int)kc, (int)n, R, nsm, -1, 1);
+    b += 8.0 * R + 16.0 * md::kspace_tc_rows_pad(R) + 4.0 * R * (2 * kc + 1);
+    b += 4.0 * ((double)t.nchunk * t.mt * t.ns * 128 + (double)md::kspace_tc_image_floats((int)kc, t.nt_full) +
+                (double)md::kspace_tc_image_floats((int)kc, t.nt_field) +
+                (double)md::kspace_tc_bimg_floats((int)kc, t.nsb)) +
+         8.0 * (double)md::kspace_tc_tblk_entries((int)kc, t.nsb);
+    nchunk = std::max(nchunk, t.nchunk);
+  }
+  b += 24.0 * nchunk;
+  return b + 64.0 * (steps + 1024);
 }
 
 int md_set_kspace_engine(md_ctx* c, int engine) {
@@ -1937,10 +1981,8 @@ int md_set_neighbor_skin(md_ctx* c, double skin_frac) {
   c->list_valid = false;
   invalidate_graph(c);
   if (c->have_ewald) {
-    const double rlb = c->rc / c->L * (1.0 + c->skin_frac);
-    double est = (double)c->n * (double)c->n * 4.0 / 3.0 * 3.141592653589793 * rlb * rlb * rlb;
-    est = std::min(est, (double)c->n * (double)(c->n - 1));
-    if (int st = alloc_nbr(c, (long long)(1.3 * est) + 64LL * c->n, true)) return st;
+    const int64_t cap = mdh::list_entries(c->n, c->rc / c->L * (1.0 + c->skin_frac));
+    if (int st = alloc_nbr(c, cap, true)) return st;
   }
   return force_rebuild(c);
 }
@@ -1953,7 +1995,7 @@ int md_set_strong_pairs(md_ctx* c, double theta) {
   if (!c->have_ewald) return MD_OK;
   update_strong(c);
   if (c->strong_w4sq > 0.f && !c->cfg.ENABLE_COATING_POT)
-    if (int st = alloc_strong(c, 4096 + (long long)(2.0 * strong_estimate(c)))) return st;
+    if (int st = alloc_strong(c, strong_entries(c))) return st;
   return force_rebuild(c);
 }
 

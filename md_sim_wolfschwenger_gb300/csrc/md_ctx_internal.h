@@ -43,6 +43,9 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+constexpr double kStrongTheta = 3.0;   // default threshold of the strong pairs
+constexpr double kSkinFrac = 0.005;    // default skin of the neighbour list
+
 struct md_ctx {
   md_config cfg{};
   int64_t n = 0;
@@ -124,6 +127,8 @@ struct md_ctx {
   size_t ptab_cap = 0;
   size_t ksize_cap = 0, spart_cap = 0;
   int musum_cap = 0;
+  // steps in batches only (ctx_packed_only): no engine that only md_step's kernels have
+  bool packed_only = false;
   // k space by rows (md_krows.cu; rw_T = 0 while it is off)
   int rw_T = 0, rw_R = 0;
   RowShape rws{};
@@ -162,10 +167,10 @@ struct md_ctx {
   // each in both passes (~3 skin of the list); a Brownian step moves a
   // particle ~5 pm at dt = 1e-12 s, so even a 0.5 % skin (1 nm at rc = 400
   // nm) is crossed only after ~1e4 steps and rebuilds stay rare.
-  double skin_frac = 0.005;
+  double skin_frac = kSkinFrac;
   // skin that the particles in the current cells may have used (larger than skin_frac
   // between md_set_neighbor_skin and the next full evaluation)
-  double cell_skin = 0.005;
+  double cell_skin = kSkinFrac;
   int64_t pairs = 0;        // in-range pairs of the last evaluation, as last counted
   bool list_valid = false;  // a build for the current particles, grid and skin exists
   // Strong pairs (mixed path, md_real.cu): list entries whose force weight
@@ -173,7 +178,7 @@ struct md_ctx {
   // evaluated in FP64; strong_w4sq is that threshold in kernel units
   // (squared, for |mu_i|^2 |mu_j|^2 > w4sq r^8; < 0: off).
   double kself[6] = {0, 0, 0, 0, 0, 0};  // k-space self-interaction matrix (IntParams::kself)
-  double strong_theta = 3.0;
+  double strong_theta = kStrongTheta;
   float strong_w4sq = -1.f;
   int2* snbr = nullptr;
   int *snbr_cnt = nullptr, *snbr_off = nullptr;

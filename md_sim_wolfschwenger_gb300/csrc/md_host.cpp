@@ -679,6 +679,12 @@ MeshTables mesh_tables(int kc, int M) {
 
 // Cells of edge >= rc / reach; a stencil of +-reach cells must not wrap onto
 // itself (ncx >= 2 reach + 1), otherwise all pairs are scanned (ncx = 1).
+int64_t list_entries(int64_t n, double rl_box) {
+  // uniform density and a margin (the list is grown on overflow)
+  const double N = (double)n, est = N * N * 4.0 / 3.0 * 3.141592653589793 * rl_box * rl_box * rl_box;
+  return (int64_t)(1.3 * std::min(est, N * (N - 1))) + 64 * n;
+}
+
 md::CellGrid choose_grid(double rc_box, int64_t n, int reach) {
   md::CellGrid g{1, 1, 0};
   if (reach < 1) reach = 2;

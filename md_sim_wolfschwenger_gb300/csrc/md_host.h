@@ -11,6 +11,14 @@
 #include "../../include/md_gb300.h"
 #include "md_types.h"
 
+// Contexts that step in batches only (the request loop's): set before md_set_ewald,
+// they hold no buffers of the engines that batches do not run.
+void ctx_packed_only(md_ctx* c);
+// Device bytes that such a mixed-precision context will hold with the given Ewald
+// parameters and room for `steps` records; < 0 on invalid particles.
+extern "C" double mdi_packed_ctx_bytes(const md_config* cfg, int64_t n, const double* rMag, double alpha, double rc,
+                                       int64_t kc, int64_t steps);
+
 namespace mdh {
 
 // ------------------------------------------------------- configuration
@@ -93,5 +101,7 @@ MeshTables mesh_tables(int kc, int M);
 
 // ----------------------------------------------------------- cell grid
 md::CellGrid choose_grid(double rc_box, int64_t n, int reach);
+// Neighbour-list entries to allocate for a list radius (box units).
+int64_t list_entries(int64_t n, double rl_box);
 
 }  // namespace mdh

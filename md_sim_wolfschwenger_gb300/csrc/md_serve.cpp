@@ -69,7 +69,7 @@ md_config request_config(const md_config& base, const md_request& q) {
 }
 
 // A request's system on the host, with its Ewald parameters from the error
-// model and an upper estimate of the device memory it will hold.
+// model and the device memory it will hold (before tuning).
 struct HostSys {
   int64_t req = -1;
   md_config cfg{};
@@ -77,20 +77,6 @@ struct HostSys {
   double L = 0, alpha = 0, rc = 0, est = 0;
   int64_t kc = 0;
 };
-
-// Device bytes of a mixed-precision context: per-particle state, stage and
-// work arrays (~620 B), phase tables, the neighbour list (uniform-density
-// estimate with the allocator's margin), k-space arrays and records.
-double estimate_bytes(int64_t n, double rc_box, int64_t kc, int64_t steps) {
-  const double pi = 3.141592653589793, N = (double)n;
-  const double rl = rc_box * 1.02;
-  const double nbr = 4.0 * (1.3 * std::min(N * N * 4.0 / 3.0 * pi * rl * rl * rl, N * (N - 1)) + 64.0 * N);
-  const double nk = 2.0 * pi / 3.0 * std::pow((double)kc + 1.0, 3.0) + 64.0;
-  const double nchunk = std::max(1.0, std::ceil(N / 512.0)) + 8.0;
-  const double cells = 8.0 * std::pow(std::max(1.0, std::ceil(2.0 / rc_box)), 3.0);
-  return 1.1 * (620.0 * N + 24.0 * (kc + 1) * N + nbr + nk * (80.0 + 16.0 * nchunk) + cells + 64.0 * (steps + 1024) +
-                (1 << 20));
-}
 
 int prepare_host(const md_config& base, const md_request& q, int64_t qi, HostSys* h) {
   h->req = qi;
@@ -107,8 +93,8 @@ int prepare_host(const md_config& base, const md_request& q, int64_t qi, HostSys
   if ((st = md_ewald_params_host(&h->cfg, q.n, h->rMag.data(), nullptr, 0.0, &h->alpha, &h->rc, &h->kc, nullptr,
                                  nullptr, &L2)))
     return st;
-  h->est = estimate_bytes(q.n, h->rc / h->L, h->kc, q.steps);
-  return MD_OK;
+  h->est = mdi_packed_ctx_bytes(&h->cfg, q.n, h->rMag.data(), h->alpha, h->rc, h->kc, q.steps);
+  return h->est < 0 ? MD_ERR_INVALID : MD_OK;
 }
 
 // Context with state and Ewald parameters (not yet batched).
@@ -120,6 +106,7 @@ int create_device(const HostSys& h, const md_request& q, int autotune, Live* out
     md_ctx_destroy(ctx);
     return s;
   };
+  ctx_packed_only(ctx);
   if ((st = md_set_particles(ctx, h.rMag.data(), nullptr))) return fail(st);
   if ((st = md_state_upload(ctx, h.pos.data(), h.mm.data(), h.ea.data(), 1))) return fail(st);
   if (autotune) {

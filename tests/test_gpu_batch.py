@@ -217,3 +217,33 @@ def test_autotune_single_candidate_is_the_cost_model_choice():
     al, rc, kc, _, _ = a.ewald_params()
     ta, trc, tkc, ms = a.autotune_ewald(1)
     assert (ta, trc, tkc) == (al, rc, kc) and ms > 0
+
+
+@pytest.mark.parametrize("n,phi,lognormal", [(300, 0.05, False), (1001, 0.10, True), (8000, 0.05, True),
+                                             (20011, 0.10, True)])
+def test_served_contexts_hold_what_batches_need(n, phi, lognormal):
+    """A served system holds no buffers of the engines that only md_step has (k rows,
+    mesh): with the tensor cores chosen, a context of its own holds the same.  The
+    admission's estimate is that size, to 1 %."""
+    import ctypes as C
+    L = m._lib.lib()
+    L.mdi_packed_ctx_bytes.restype = C.c_double
+    cfg = m.Configuration.default().set(rMagMean=1e-8, dShell=5e-9, visOverride=1e-3, volFrac=phi,
+                                        SIZE_DIST=1 if lognormal else 0, sigmaLog=0.2 if lognormal else 0.0)
+    steps = 4
+    res, _ = m.serve(cfg, [dict(n=n, steps=steps, dt=1e-12, volFrac=phi, fieldKind=m.MD_FIELD_STEP, fieldAmp=0.02,
+                                fieldFreq=0.0, seed=3, arrival=0.0)], hbm_budget=40e9,
+                     max_systems=1, round_steps=4, realtime=False)
+    assert res[0]["status"] == 0
+    own = cfg.set(numbPartOverride=n)
+    rMag, rHydr, pos, mm, ea, _ = m.init_system(own, n, 3)
+    sim = m.Simulation(own, n, m.MD_PREC_MIXED, rMag=rMag)
+    sim.set_kspace_engine("tc")
+    a, rc, kc = sim.ewald_params()[:3]
+    sim.set_ewald(a, rc, kc)
+    records = 64 * (steps + 1024)
+    assert res[0]["device_bytes"] <= sim.device_bytes() + records
+    r = np.ascontiguousarray(rMag)
+    est = L.mdi_packed_ctx_bytes(C.byref(own.c), C.c_int64(n), r.ctypes.data_as(C.POINTER(C.c_double)), C.c_double(a),
+                                 C.c_double(rc), C.c_int64(kc), C.c_int64(steps))
+    assert res[0]["device_bytes"] <= est < 1.01 * res[0]["device_bytes"] + 1e5
