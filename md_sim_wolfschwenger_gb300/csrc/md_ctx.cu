@@ -1594,10 +1594,11 @@ int prepare_dt(md_ctx* c, double dt) {
   return MD_OK;
 }
 
-// Captures k steps as one graph.
-static int capture_steps(md_ctx* c, int k, double dt, cudaGraph_t* graph, cudaGraphExec_t* exec, int* launches) {
+// Captures k steps as one graph; *launches: its kernels.
+static int capture_steps(md_ctx* c, int k, double dt, cudaGraph_t* graph, cudaGraphExec_t* exec, int64_t* launches) {
+  *launches = 0;
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
-  for (int s = 0; s < k; s++) *launches = issue_step(c, dt, s > 0, s < k - 1);
+  for (int s = 0; s < k; s++) *launches += issue_step(c, dt, s > 0, s < k - 1);
   cudaError_t e = cudaStreamEndCapture(c->stream, graph);
   if (e != cudaSuccess) return set_err(c, MD_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
   CK(c, cudaGraphInstantiate(exec, *graph, 0));
@@ -1627,25 +1628,25 @@ static int enqueue_steps(md_ctx* c, int64_t nsteps, double dt, const double* xi)
     }
     CK(c, cudaGetLastError());
   } else {
-    int lps = 0;
     if (!c->graph_valid) {
-      if ((st = capture_steps(c, 1, dt, &c->graph, &c->gexec, &lps))) return st;
-      c->launches_per_step = lps;
+      if ((st = capture_steps(c, 1, dt, &c->graph, &c->gexec, &c->launches_1))) return st;
       c->graph_valid = true;
     }
+    c->launches = 0;
     int64_t s = 0;
     while (s < nsteps) {
       if (nsteps - s >= kGraphSteps && (c->gexec_n || c->replays >= kGraphAfter) && !c->prof) {
-        if (!c->gexec_n && (st = capture_steps(c, kGraphSteps, dt, &c->graph_n, &c->gexec_n, &lps))) return st;
+        if (!c->gexec_n && (st = capture_steps(c, kGraphSteps, dt, &c->graph_n, &c->gexec_n, &c->launches_n))) return st;
         CK(c, cudaGraphLaunch(c->gexec_n, c->stream));
+        c->launches += c->launches_n;
         s += kGraphSteps;
       } else {
         CK(c, cudaGraphLaunch(c->gexec, c->stream));
+        c->launches += c->launches_1;
         c->replays++;
         s++;
       }
     }
-    c->launches = c->launches_per_step * nsteps;
   }
   c->have_geometry = true;
   return MD_OK;

@@ -80,7 +80,7 @@ struct md_ctx {
   cudaGraph_t graph_n = nullptr;
   cudaGraphExec_t gexec_n = nullptr;
   int64_t replays = 0;
-  int64_t launches = 0, launches_per_step = 0;
+  int64_t launches = 0, launches_1 = 0, launches_n = 0;  // of the last call, of each graph
 
   // device: master state & particle constants
   double *pos = nullptr, *mm = nullptr, *ea = nullptr, *truePos = nullptr, *posRef = nullptr;

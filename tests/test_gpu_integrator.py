@@ -60,3 +60,31 @@ def test_steps_in_one_graph_equal_single_steps(prec):
             b.step(1, dt)
         for x, y in zip(a.get_state(), b.get_state()):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [150, 6001])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_records_and_launches_of_steps_in_one_graph(prec, n):
+    """The records of a step are taken beside the next one in a graph of eight: the
+    same rows, as many as steps, and a kernel more per step but the last.  N = 6001:
+    k space through the mesh (mixed)."""
+    if n < 6000:
+        ini, g = random_system(n, seed=8, rc_frac=0.35, noise=True)
+    else:
+        from test_gpu_parity import random_system_fast
+        ini, g = random_system_fast(n, seed=8, phi=0.10, B0=0.02)
+        g["rc"], g["kc"] = 0.2 * g["lBox"], 16 if prec else 5
+        g["alpha"] = 3.5 / g["rc"]
+    a, b = (gpu_system(ini, g, prec, noise=2, seed=4) for _ in range(2))
+    k, dt = 150, g["dt"]
+    a.step(k, dt)
+    per = []
+    for _ in range(k):
+        b.step(1, dt)
+        per.append(b.launches())
+    ra, rb = a.records(), b.records()
+    assert ra.shape == (k, 8)
+    np.testing.assert_array_equal(ra, rb)
+    for x, y in zip(a.get_state(), b.get_state()):
+        np.testing.assert_array_equal(x, y)
+    assert a.launches() == sum(per) + 7 * ((k - 128) // 8)
