@@ -58,15 +58,6 @@ def tc_mma_flops(n, kc):
     return sf, 3 * 2.0 * nb * (nt_full * 128) * kp, 3 * 2.0 * nb * (nt_field * 128) * kp
 
 
-def kspace_mesh(sim, n, kc):
-    """Whether the default engine takes k space through the mesh for these
-    parameters (mesh_wanted in md_ctx.cu)."""
-    ring, waves, _ = sim.kspace_tiling()
-    m = 8 * ((kc + 1) // 2)
-    return (bool(sim.kspace_tensor_cores()) and ring < 0 and waves == 1 and n >= 6000
-            and (kc >= 15 or (kc >= 13 and n >= 32768)) and m ** 3 <= 100 * n)
-
-
 BYTES_CELLS = 60.0        # per particle (+8 per cell)
 FLOPS_MESH = 729 * 2.0    # per particle and summed component: the window's mesh points
 BYTES_HEUN1 = 252.0       # per particle
@@ -371,7 +362,7 @@ def fp64_plain(n, sysd, ewald, seed, steps=4, warm=1):
             "mixed_error_vs_fp64": err}
 
 
-def segment_rooflines(seg_mean, n, kc, pairs, nk_real, tensor_cores, mesh, peak_fp32, hbm_peak):
+def segment_rooflines(seg_mean, n, kc, pairs, nk_real, engine, peak_fp32, hbm_peak):
     """Per-segment achieved rates of a profiled pass (ms per kernel segment):
     algorithmic FLOPs or bytes per unit (the constants above) over the
     segment's time, against the FP32 FMA-chain peak, the HBM copy peak or the
@@ -382,10 +373,10 @@ def segment_rooflines(seg_mean, n, kc, pairs, nk_real, tensor_cores, mesh, peak_
             "kscat_field": ("fp32", nk_real * n * FLOPS_KSCAT_FIELD),
             "cells": ("hbm", n * BYTES_CELLS), "heun1": ("hbm", n * BYTES_HEUN1), "heun2": ("hbm", n * BYTES_HEUN2)}
     peak_tf32 = peak_f16 = None
-    if mesh:  # spread (3 components), interpolation (3, with derivatives 6); the transforms are kred_*
+    if engine == "mesh":  # spread (3 components), interpolation (3, with derivatives 6); the transforms are kred_*
         work.update(ksf_full=("fp32", n * 3 * FLOPS_MESH), ksf_field=("fp32", n * 3 * FLOPS_MESH),
                     kscat_full=("fp32", n * 6 * FLOPS_MESH), kscat_field=("fp32", n * 3 * FLOPS_MESH))
-    elif tensor_cores:
+    elif engine == "tc":
         # the tensor-core k space: the structure factor's executed 3-pass FP16
         # MMA work against the measured bf16 rate (the same rate), the
         # scatter's 3-pass TF32 work against half of it (nominal 1:2)
@@ -454,8 +445,7 @@ def stress_sample(steps, peak_fp32, hbm_peak, warm=3, fp64_steps=2, seed=1):
         extra = {}
         if prec == MD_PREC_MIXED:
             extra = {"pairs": sim.pairs(), "strong_pair_entries_fp64": sim.strong_pairs(),
-                     "kspace_tensor_cores": sim.kspace_tensor_cores() and not kspace_mesh(sim, n, kc),
-                     "kspace_mesh": kspace_mesh(sim, n, kc)}
+                     "kspace_engine": sim.kspace_engine()}
             # per-kernel segments: a profiled pass (kernels one after another)
             sim.profile(True)
             sim.step(1, 1e-12)
@@ -467,7 +457,7 @@ def stress_sample(steps, peak_fp32, hbm_peak, warm=3, fp64_steps=2, seed=1):
             sim.profile(False)
             seg_mean = {a: b / 3 for a, b in acc.items()}
             segs, _ = segment_rooflines(seg_mean, n, kc, extra["pairs"], len(sim.debug_structure_factor()),
-                                        sim.kspace_tensor_cores(), kspace_mesh(sim, n, kc), peak_fp32, hbm_peak)
+                                        sim.kspace_engine(), peak_fp32, hbm_peak)
             kspace = [q for q in seg_mean if q.startswith("k")]
             extra_segs = {"segments": segs,
                           "kspace_share_of_serialised_step": sum(seg_mean[q] for q in kspace) / sum(seg_mean.values()),
@@ -697,8 +687,7 @@ def run_ours(args):
     pairs = sim.pairs()
     strong = sim.strong_pairs()
     ring, waves, chunk = sim.kspace_tiling()
-    mesh = kspace_mesh(sim, n, kc)
-    kspace = {"tensor_cores": bool(sim.kspace_tensor_cores()) and not mesh, "mesh": mesh, "sf_ring_option": ring, "sf_chunk_waves": waves,
+    kspace = {"engine": sim.kspace_engine(), "sf_ring_option": ring, "sf_chunk_waves": waves,
               "sf_chunk_particles": chunk, "chosen_by": "autotuner" if args.autotune > 0 else "defaults"}
     nk_real = len(sim.debug_structure_factor())
     clk = clocks.stop()  # sampled over both timed runs
@@ -731,8 +720,7 @@ def run_ours(args):
         hbm_peak = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"]
     except Exception:
         pass
-    segs, work = segment_rooflines(seg_mean, n, kc, pairs, nk_real, sim.kspace_tensor_cores(), kspace_mesh(sim, n, kc),
-                                   peak_fp32, hbm_peak)
+    segs, work = segment_rooflines(seg_mean, n, kc, pairs, nk_real, sim.kspace_engine(), peak_fp32, hbm_peak)
     dom = max((k for k in segs if k in work), key=lambda k: segs[k]["ms"])
     traffic = None  # from the ncu capture of this workload, when there is one
     try:
@@ -773,7 +761,7 @@ def run_ours(args):
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
                 "dtype": "f64" if prec == MD_PREC_FP64 else "f32",
                 "precision": ("fp64 (plain)" if prec == MD_PREC_FP64 else
-                              "mixed: FP32 pair maths, k space (through a mesh at this size) and integrator; "
+                              "mixed: FP32 pair maths, k space and integrator; "
                               "real-space pairs above 3 contact forces (strong pairs) in FP64; FP64 self/surface "
                               "terms, positions, reductions"),
                 "data": "synthetic (seeded log-normal radii, random sequential addition, moments and easy axes "

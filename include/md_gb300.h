@@ -58,9 +58,12 @@ enum {
 
 /* Reciprocal-space engine of the mixed path (md_set_kspace_engine). */
 enum {
-  MD_KSPACE_AUTO = 0, /* by size: see md_kspace_engine_active                  */
+  MD_KSPACE_AUTO = 0, /* by size: see md_kspace_engine_used                    */
   MD_KSPACE_SIMT = 1, /* FP32 CUDA-core kernels (row segments, phase recurrences) */
-  MD_KSPACE_TC = 2    /* tensor cores (3-pass TF32 matrix products over k rows) */
+  MD_KSPACE_TC = 2,   /* tensor cores (3-pass TF32 matrix products over k rows) */
+  /* chosen by MD_KSPACE_AUTO only */
+  MD_KSPACE_ROWS = 3, /* CUDA cores by pairs +-nx of k rows (also the FP64 path) */
+  MD_KSPACE_MESH = 4  /* non-uniform Fourier transforms through a mesh          */
 };
 
 /* External field program (DefExtField, src/simulation.cpp:546-556). */
@@ -198,12 +201,17 @@ int md_set_ewald(md_ctx* ctx, double alpha, double rc, int64_t kc);
  * tensor-core kernels' shared memory (kc <= 25).  Applies to the current
  * and later Ewald parameters. */
 int md_set_kspace_engine(md_ctx* ctx, int engine);
-/* *tensor_cores = 1 when the current Ewald parameters are those of the tensor
- * cores.  With MD_KSPACE_AUTO and the default tiling, systems too small to
- * fill them (about 3e6 k vectors x particles) evaluate the same k rows on the
- * CUDA cores under that setting, and systems of 6000 particles and more with
- * kc >= 15 (32768: kc >= 13) take the same sums through a mesh; MD_KSPACE_TC always takes the tensor cores. */
+/* *tensor_cores = 1 when the tensor cores are set up for the current Ewald
+ * parameters: packed batches evaluate with them, and so do a context's own
+ * calls unless MD_KSPACE_AUTO has something better for its size
+ * (md_kspace_engine_used). */
 int md_kspace_engine_active(const md_ctx* ctx, int* tensor_cores);
+/* *engine = the MD_KSPACE_* engine of the context's own calls (md_step,
+ * md_compute_interactions, ..) with the current Ewald parameters; 0 before they
+ * are set.  With MD_KSPACE_AUTO and the default tiling, mixed systems too small to
+ * fill the tensor cores (about 3e6 k vectors x particles) take MD_KSPACE_ROWS and
+ * large ones, by particles and kc, MD_KSPACE_MESH. */
+int md_kspace_engine_used(const md_ctx* ctx, int* engine);
 /* Tiling of the tensor-core structure factor (no counterpart in the
  * reference; the autotuner's knobs): ring = the operand-ring option (0..5,
  * deeper rings first; -1: the deepest that fits shared memory), waves = the

@@ -1466,6 +1466,17 @@ int md_kspace_engine_active(const md_ctx* c, int* tensor_cores) {
   return MD_OK;
 }
 
+int md_kspace_engine_used(const md_ctx* c, int* engine) {
+  if (!c || !engine) return MD_ERR_INVALID;
+  // in the order of launch_kspace
+  *engine = !c->have_ewald ? 0
+            : c->rw_T > 0  ? MD_KSPACE_ROWS
+            : c->gm_M > 0  ? MD_KSPACE_MESH
+            : c->tc_rows > 0 ? MD_KSPACE_TC
+                             : MD_KSPACE_SIMT;
+  return MD_OK;
+}
+
 int md_set_kspace_tiling(md_ctx* c, int ring, int waves) {
   if (!c || ring < -1 || ring > 5 || waves < 1 || waves > 4) return set_err(c, MD_ERR_INVALID, "bad k-space tiling");
   invalidate_graph(c);

@@ -208,8 +208,16 @@ class Simulation:
         self._ck(self.L.md_get_kspace_tiling(self.h, C.byref(r), C.byref(w), C.byref(ch)))
         return r.value, w.value, ch.value
 
+    def kspace_engine(self):
+        """Engine that evaluates this context's k space (md_kspace_engine_used):
+        "rows", "mesh", "tc", "simt", or None before the Ewald parameters are set."""
+        v = C.c_int()
+        self._ck(self.L.md_kspace_engine_used(self.h, C.byref(v)))
+        return (None, "simt", "tc", "rows", "mesh")[v.value]
+
     def kspace_tensor_cores(self):
-        """True when the current Ewald parameters run the k space on the tensor cores."""
+        """True when the tensor cores are set up for the current Ewald parameters
+        (see kspace_engine for the engine of this context's own calls)."""
         v = C.c_int()
         self._ck(self.L.md_kspace_engine_active(self.h, C.byref(v)))
         return bool(v.value)

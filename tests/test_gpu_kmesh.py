@@ -120,3 +120,22 @@ def test_field_after_the_skin_was_changed(skin):
     assert rms(sim.CompDemagField(mm), a) < TOL
     sim.CompInteractions()
     assert rms(sim.CompDemagField(mm), a) < TOL
+
+
+def test_engine_of_the_current_parameters():
+    """kspace_engine names what runs: by size, as chosen, and on the FP64 path."""
+    ini, g = random_system(300, seed=1, rc_frac=0.4)
+    small = gpu_system(ini, g, 1)
+    assert small.kspace_engine() == "rows" and gpu_system(ini, g, 0).kspace_engine() == "rows"
+    small.set_kspace_engine("simt")
+    assert small.kspace_engine() == "simt"
+    ini, g = random_system_fast(20011, seed=2, phi=0.10, B0=0.02)
+    g["kc"] = 15
+    large = gpu_system(ini, g, 1)
+    assert large.kspace_engine() == "mesh" and large.kspace_tensor_cores()
+    large.set_kspace_tiling(0, 1)
+    assert large.kspace_engine() == "tc"
+    large.set_kspace_tiling(-1, 1)
+    assert large.kspace_engine() == "mesh"
+    large.set_kspace_engine("tc")
+    assert large.kspace_engine() == "tc"
