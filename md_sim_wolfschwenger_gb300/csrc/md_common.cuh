@@ -397,7 +397,6 @@ struct RKStage {
   double e[7];              // error weights (last stage)
   int s;                    // stage index (0-based); accept: last weight index
   int last;                 // stage: no next stage, form the error; accept: take (cm, ce)
-  double nf;                // factor on the thermal field and torque (rescaled on rejections)
   unsigned long long* errmax;  // max over particles of the error norm (double bits)
 };
 

@@ -1590,15 +1590,18 @@ int ensure_records(md_ctx* c, int64_t extra) {
 // DefThermFluct prefactors (src/simulation.cpp:563-603) and the other
 // per-particle constants of the integrator, computed on the device for this
 // dt (queued on the stream; the adaptive solvers change dt every step).
-int prepare_dt(md_ctx* c, double dt) {
-  if (dt == c->cur_dt) return MD_OK;
+static int int_consts(md_ctx* c, double dt, double nf) {
   const md_config& g = c->cfg;
   const double kt = 2.0 * g.kB * g.temp / dt;
   const double kb = 2.0 * g.kB * g.temp * g.magDamp / (g.gyroMr * g.satMag * dt);
+  return launch_int_consts(c->stream, (int)c->n, g.ENABLE_THERM_TORQUE ? kt : 0.0, g.ENABLE_THERM_FIELD ? kb : 0.0,
+                           g.ENABLE_THERM_FORCE ? kt : 0.0, nf, c->zetaR, c->zetaT, c->invVol, c->invZt, c->velEa1,
+                           c->velEa2, c->magMom_u, c->rMag_u, c->cA, c->cB, fp64(c));
+}
+int prepare_dt(md_ctx* c, double dt) {
+  if (dt == c->cur_dt) return MD_OK;
   cudaGetLastError();  // an earlier call's error was reported there
-  launch_int_consts(c->stream, (int)c->n, g.ENABLE_THERM_TORQUE ? kt : 0.0, g.ENABLE_THERM_FIELD ? kb : 0.0,
-                    g.ENABLE_THERM_FORCE ? kt : 0.0, c->zetaR, c->zetaT, c->invVol, c->invZt, c->velEa1, c->velEa2,
-                    c->magMom_u, c->rMag_u, c->cA, c->cB, fp64(c));
+  int_consts(c, dt, 1.0);
   CK(c, cudaGetLastError());
   c->cur_dt = dt;
   invalidate_graph(c);
@@ -1779,7 +1782,6 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
     double nf = 1.0, used = dt0;
     while (cond) {
       const double dt = *dt_io;
-      q.nf = nf;
       for (int s = 0; s < tb.stages; s++) {
         const bool start_field = s == 0 && first;  // later: the field last evaluated
         q.p = int_params(c, dt, start_field ? c->Br : c->Br2, start_field ? c->Bk : c->Bk2);
@@ -1819,6 +1821,13 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
       } else {
         tnew = noFailed ? dt * std::min(std::max(0.9 * std::pow(absTol / error, tb.power), 0.2), 5.0) : dt;
         cond = false;
+      }
+      if (cond) {
+        // torque and field rescaled in FP64 and drawn again; the force keeps the scale of
+        // the first trial
+        c->launches += int_consts(c, dt0, nf);
+        c->launches += launch_noise(c->stream, int_params(c, dt0, nullptr, nullptr), fp64(c));
+        c->cur_dt = -1.0;  // the next step's constants are made anew
       }
       *dt_io = std::min(tnew, dtMax);
       *dt_io = std::max(tnew, dtMin);

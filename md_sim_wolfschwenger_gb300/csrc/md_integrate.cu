@@ -179,9 +179,10 @@ __global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
 }
 
 // Per-particle constants of the integrator in T for the step dt: ct, cb, cf
-// are the DefThermFluct prefactors under the square roots (0: switched off).
+// are the DefThermFluct prefactors under the square roots (0: switched off), nf the
+// factor of torque and field after rejected steps of the adaptive solvers.
 template <typename T>
-__global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf,
+__global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf, double nf,
                                                             const double* __restrict__ zr, const double* __restrict__ zt,
                                                             const double* __restrict__ ivol,
                                                             const double* __restrict__ izt,
@@ -192,8 +193,8 @@ __global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, do
   const int i = blockIdx.x * kIntThreads + threadIdx.x;
   if (i >= n) return;
   T4 a, b;
-  a.x = (T)sqrt(ct * zr[i]);
-  a.y = (T)sqrt(cb * ivol[i]);
+  a.x = (T)(sqrt(ct * zr[i]) * nf);
+  a.y = (T)(sqrt(cb * ivol[i]) * nf);
   a.z = (T)sqrt(cf * zt[i]);
   a.w = (T)izt[i];
   b.x = (T)v1[i];
@@ -605,11 +606,10 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
       e[a] = q.s == 0 ? (T)p.ea[a * n + i] : ((const T*)q.ce)[a * n + i];
     }
     demag_si<T>(p, r, bd);
-    const T nf = (T)q.nf;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      tau[a] = nf * ((const T*)p.th)[a * n + i];
-      bth[a] = nf * ((const T*)p.th)[(3 + a) * n + i];
+      tau[a] = ((const T*)p.th)[a * n + i];
+      bth[a] = ((const T*)p.th)[(3 + a) * n + i];
     }
     const T bz = (T)ext_field_z(p, *p.time);
     T km[3], ke[3];
@@ -732,14 +732,14 @@ int launch_noise(cudaStream_t st, const IntParams& p, bool fp64) {
   return 1;
 }
 
-int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, const double* zr, const double* zt,
+int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, double nf, const double* zr, const double* zt,
                       const double* ivol, const double* izt, const double* v1, const double* v2, const double* mu,
                       const double* rm, void* cA, void* cB, bool fp64) {
   const int g = int_blocks(n);
   if (fp64)
-    k_int_consts<double><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+    k_int_consts<double><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, nf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
   else
-    k_int_consts<float><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+    k_int_consts<float><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, nf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
   return 1;
 }
 

@@ -64,3 +64,27 @@ def test_adaptive_philox_vs_oracle_and_stop_time(solver):
     # the loop runs while t <= t_end: one more step, then it stops
     dt2, done2 = sim.step_adaptive(100, dt_gpu, t_end=sim.get_time()[0])
     assert done2 == 1
+
+
+@pytest.mark.parametrize("solver", [0, 1, 2])
+def test_adaptive_philox_after_rejections(solver):
+    """First trials far too long, so that the drawn noise is rescaled, twice in a call
+    with steps in between: the oracle's steps, and torque, field and force each at its
+    own scale (the force keeps the first trial's)."""
+    ini, g = random_system(125, seed=70 + solver, rc_frac=0.4, noise=True, B0=0.02)
+    ini["adaptive_timestepping_solver"]["SOLVER"] = solver
+    ini["solver_settings"]["absTol"] = 1e-4
+    d = O.derive(ini)
+    sim = gpu_system(ini, g, 0, noise=2, seed=35)
+    orc = oracle_system(ini, g)
+    attempts = 0
+    for dt in (3e-10, 1e-10):
+        dt_gpu, done = sim.step_adaptive(3, dt)
+        assert done == 3
+        for _ in range(3):
+            dt, used, att, obs = orc.step_adaptive(solver, dt, d["absTol"], d["deltaTmin"], d["deltaTmax"], 2, None, 35)
+            attempts += att
+        assert abs(dt_gpu - dt) <= 1e-9 * dt
+    assert attempts > 6  # rejections
+    for x, y, tol in zip(sim.get_state(), orc.get_state()[:3], (1e-12 * g["lBox"], 1e-10, 1e-10)):
+        assert np.abs(x - y).max() < tol
