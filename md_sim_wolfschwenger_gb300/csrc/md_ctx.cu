@@ -407,10 +407,10 @@ static int fork_join(md_ctx* c, int q, int seg_real, int seg_k, RP&& real_prep, 
 }
 
 // Field + force evaluation on the current master state (no integrator).
-// dt >= 0: the step's noise is drawn beside it.  after_records: the step before left
+// dt >= 0: the step's noise is drawn beside it (unit: unscaled).  after_records: the step before left
 // its records to the side stream (issue_step); they come before the noise, and with
 // it the integrator.
-static int issue_interactions(md_ctx* c, double dt = -1.0, bool after_records = false) {
+static int issue_interactions(md_ctx* c, double dt = -1.0, bool unit = false, bool after_records = false) {
   int l = 0;
   mark(c, MD_SEG_CELLS);
   if (!c->list_valid) c->cell_skin = c->skin_frac;  // this evaluation sorts anew
@@ -424,7 +424,7 @@ static int issue_interactions(md_ctx* c, double dt = -1.0, bool after_records = 
       [&](cudaStream_t st) {
         int l = launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), &c->sc->flags, fp64(c));
         if (after_records) cudaStreamWaitEvent(st, c->join_ev[2], 0);
-        if (dt >= 0) l += launch_noise(st, int_params(c, dt, nullptr, nullptr), fp64(c));
+        if (dt >= 0) l += launch_noise(st, int_params(c, dt, nullptr, nullptr), unit, fp64(c));
         return l;
       },
       [&](cudaStream_t st) { return launch_real(st, real_params(c, c->Br, c->Fr, c->ov), true, fp64(c)); },
@@ -455,7 +455,7 @@ static int issue_field(md_ctx* c) {
 // one are taken beside the start of that one (the kernel that ends with them in its
 // last block costs the chain of steps ~2 us more: N = 512 49.0 -> 46.8 us per step).
 static int issue_step(md_ctx* c, double dt, bool after_records = false, bool leave_records = false) {
-  int l = issue_interactions(c, dt, after_records);
+  int l = issue_interactions(c, dt, false, after_records);
   mark(c, MD_SEG_HEUN1);
   l += launch_heun1(c->stream, int_params(c, dt, c->Br, c->Bk), fp64(c));
   l += issue_field(c);
@@ -1032,7 +1032,9 @@ int md_ctx_create(const md_config* cfg, int64_t n, int precision, md_ctx** out) 
     if ((st = dalloc(c, &c->xi4, 16 * N))) return fail(st);
   }
   if ((st = dalloc(c, &c->mu, 4 * T * N))) return fail(st);
-  if ((st = dalloc(c, &c->cA, 4 * T * N)) || (st = dalloc(c, &c->cB, 4 * T * N))) return fail(st);
+  if ((st = dalloc(c, &c->cA, 4 * T * N)) || (st = dalloc(c, &c->cB, 4 * T * N)) ||
+      (st = dalloc(c, &c->sTB, 16 * N)))
+    return fail(st);
   void** t3[] = {&c->Br, &c->Fr, &c->ov, &c->Bk, &c->Fk, &c->Br2, &c->Bk2, &c->k1m, &c->k1e, &c->m2, &c->e2};
   for (auto p : t3)
     if ((st = dalloc(c, p, 3 * T * N))) return fail(st);
@@ -1423,7 +1425,7 @@ double mdi_packed_ctx_bytes(const md_config* cfg, int64_t n, const double* rMag,
   const size_t ks = std::max(std::max((size_t)k.nk, k.seg.size()), std::max((size_t)k.nk_scat, k.rseg.size())) + 2;
   int chunk = 0, nchunk = 0;
   segment_chunks(k, n, (int)kc, nsm, &chunk, &nchunk);
-  double b = 661.0 * N + 4096;                                        // state, stages and work arrays
+  double b = 677.0 * N + 4096;                                        // state, stages and work arrays
   b += 8.0 * (cell_grid(rc / L, n, false).ncell + 1);                 // cells
   b += 4.0 * (double)mdh::list_entries(n, rl / L);                    // neighbour list
   if (!cfg->ENABLE_COATING_POT)                                       // strong list and its sums
@@ -1590,18 +1592,15 @@ int ensure_records(md_ctx* c, int64_t extra) {
 // DefThermFluct prefactors (src/simulation.cpp:563-603) and the other
 // per-particle constants of the integrator, computed on the device for this
 // dt (queued on the stream; the adaptive solvers change dt every step).
-static int int_consts(md_ctx* c, double dt, double nf) {
+int prepare_dt(md_ctx* c, double dt) {
+  if (dt == c->cur_dt) return MD_OK;
   const md_config& g = c->cfg;
   const double kt = 2.0 * g.kB * g.temp / dt;
   const double kb = 2.0 * g.kB * g.temp * g.magDamp / (g.gyroMr * g.satMag * dt);
-  return launch_int_consts(c->stream, (int)c->n, g.ENABLE_THERM_TORQUE ? kt : 0.0, g.ENABLE_THERM_FIELD ? kb : 0.0,
-                           g.ENABLE_THERM_FORCE ? kt : 0.0, nf, c->zetaR, c->zetaT, c->invVol, c->invZt, c->velEa1,
-                           c->velEa2, c->magMom_u, c->rMag_u, c->cA, c->cB, fp64(c));
-}
-int prepare_dt(md_ctx* c, double dt) {
-  if (dt == c->cur_dt) return MD_OK;
   cudaGetLastError();  // an earlier call's error was reported there
-  int_consts(c, dt, 1.0);
+  launch_int_consts(c->stream, (int)c->n, g.ENABLE_THERM_TORQUE ? kt : 0.0, g.ENABLE_THERM_FIELD ? kb : 0.0,
+                    g.ENABLE_THERM_FORCE ? kt : 0.0, c->zetaR, c->zetaT, c->invVol, c->invZt, c->velEa1, c->velEa2,
+                    c->magMom_u, c->rMag_u, c->sTB, c->cA, c->cB, fp64(c));
   CK(c, cudaGetLastError());
   c->cur_dt = dt;
   invalidate_graph(c);
@@ -1769,6 +1768,7 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
   q.cm = c->rk_cm;
   q.ce = c->rk_ce;
   q.errmax = &c->sc->errmax;
+  q.sTB = c->sTB;
   int64_t done = 0;
   c->launches = 0;
   while (done < max_steps && t <= t_end) {
@@ -1777,11 +1777,12 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
     if (c->noise == MD_NOISE_UPLOADED)
       CK(c, cudaMemcpyAsync(c->xi, xi + (size_t)done * 9 * c->n, 72 * (size_t)c->n, cudaMemcpyHostToDevice,
                             c->stream));
-    c->launches += issue_interactions(c, dt0);
+    c->launches += issue_interactions(c, dt0, true);
     bool cond = true, noFailed = true, first = true;
     double nf = 1.0, used = dt0;
     while (cond) {
       const double dt = *dt_io;
+      q.nf = nf;
       for (int s = 0; s < tb.stages; s++) {
         const bool start_field = s == 0 && first;  // later: the field last evaluated
         q.p = int_params(c, dt, start_field ? c->Br : c->Br2, start_field ? c->Bk : c->Bk2);
@@ -1821,13 +1822,6 @@ int md_step_adaptive(md_ctx* c, int64_t max_steps, double t_end, double* dt_io, 
       } else {
         tnew = noFailed ? dt * std::min(std::max(0.9 * std::pow(absTol / error, tb.power), 0.2), 5.0) : dt;
         cond = false;
-      }
-      if (cond) {
-        // torque and field rescaled in FP64 and drawn again; the force keeps the scale of
-        // the first trial
-        c->launches += int_consts(c, dt0, nf);
-        c->launches += launch_noise(c->stream, int_params(c, dt0, nullptr, nullptr), fp64(c));
-        c->cur_dt = -1.0;  // the next step's constants are made anew
       }
       *dt_io = std::min(tnew, dtMax);
       *dt_io = std::max(tnew, dtMin);

@@ -88,6 +88,7 @@ struct md_ctx {
   double *magMom_u = nullptr, *rMag_u = nullptr, *invZt = nullptr, *velEa1 = nullptr, *velEa2 = nullptr;
   double *zetaR = nullptr, *zetaT = nullptr, *invVol = nullptr;
   void *cA = nullptr, *cB = nullptr;  // the integrator's constants in T (k_int_consts)
+  double2* sTB = nullptr;             // and the scales of thermal torque and field unrounded
   // cells and sorted views
   int *cellOf = nullptr, *tmp = nullptr, *perm = nullptr, *rank = nullptr, *scell = nullptr;
   int *count = nullptr, *cell_start = nullptr;

@@ -152,9 +152,10 @@ __device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], cons
 
 // Thermal torque, field and force of the step: unit normals (drawn, uploaded
 // or zero) times the particle's scales, into th.  Independent of the fields,
-// so the launch runs beside their evaluation.
+// so the launch runs beside their evaluation.  UNIT: the normals alone (adaptive
+// solvers, which rescale torque and field after a rejected step).
 // Thread = one Box-Muller pair (j of five) of one particle.
-template <typename T>
+template <typename T, bool UNIT>
 __global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
   const int i = blockIdx.x * kIntOne + threadIdx.x, j = blockIdx.y, n = p.n;
   if (i >= n) return;
@@ -169,32 +170,35 @@ __global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
     }
   }
   using T4 = typename V4<T>::t;
-  const T4 c = ((const T4*)p.cA)[i];
+  T4 c;
+  if constexpr (!UNIT) c = ((const T4*)p.cA)[i];
   T* th = (T*)p.th;
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const int q = 2 * j + h;
-    if (q < 9) th[q * n + i] = (q < 3 ? c.x : (q < 6 ? c.y : c.z)) * z[h];
+    if (q < 9) th[q * n + i] = UNIT ? z[h] : (q < 3 ? c.x : (q < 6 ? c.y : c.z)) * z[h];
   }
 }
 
 // Per-particle constants of the integrator in T for the step dt: ct, cb, cf
-// are the DefThermFluct prefactors under the square roots (0: switched off), nf the
-// factor of torque and field after rejected steps of the adaptive solvers.
+// are the DefThermFluct prefactors under the square roots (0: switched off).  sTB: the
+// scales of torque and field unrounded (for the adaptive solvers).
 template <typename T>
-__global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf, double nf,
+__global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf,
                                                             const double* __restrict__ zr, const double* __restrict__ zt,
                                                             const double* __restrict__ ivol,
                                                             const double* __restrict__ izt,
                                                             const double* __restrict__ v1, const double* __restrict__ v2,
                                                             const double* __restrict__ mu, const double* __restrict__ rm,
-                                                            void* cA, void* cB) {
+                                                            double2* __restrict__ sTB, void* cA, void* cB) {
   using T4 = typename V4<T>::t;
   const int i = blockIdx.x * kIntThreads + threadIdx.x;
   if (i >= n) return;
   T4 a, b;
-  a.x = (T)(sqrt(ct * zr[i]) * nf);
-  a.y = (T)(sqrt(cb * ivol[i]) * nf);
+  const double2 s = make_double2(sqrt(ct * zr[i]), sqrt(cb * ivol[i]));
+  sTB[i] = s;
+  a.x = (T)s.x;
+  a.y = (T)s.y;
   a.z = (T)sqrt(cf * zt[i]);
   a.w = (T)izt[i];
   b.x = (T)v1[i];
@@ -606,10 +610,20 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
       e[a] = q.s == 0 ? (T)p.ea[a * n + i] : ((const T*)q.ce)[a * n + i];
     }
     demag_si<T>(p, r, bd);
+    T sT, sB;
+    if (q.nf == 1.0) {
+      const T4 ca = ((const T4*)p.cA)[i];
+      sT = ca.x;
+      sB = ca.y;
+    } else {
+      const double2 s = q.sTB[i];
+      sT = (T)(s.x * q.nf);
+      sB = (T)(s.y * q.nf);
+    }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      tau[a] = ((const T*)p.th)[a * n + i];
-      bth[a] = ((const T*)p.th)[(3 + a) * n + i];
+      tau[a] = sT * ((const T*)p.th)[a * n + i];
+      bth[a] = sB * ((const T*)p.th)[(3 + a) * n + i];
     }
     const T bz = (T)ext_field_z(p, *p.time);
     T km[3], ke[3];
@@ -695,9 +709,10 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_accept(RKStage q) {
     }
     // the thermal force at the scale of the step's first trial (the
     // reference rescales it on rejections only after it entered the force)
+    const typename V4<T>::t ca = ((const typename V4<T>::t*)p.cA)[i];
 #pragma unroll
-    for (int a = 0; a < 3; a++) fth[a] = ((const T*)p.th)[(6 + a) * n + i];
-    finish_particle<T>(p, i, r, mn, en, fth, ((const typename V4<T>::t*)p.cA)[i].w, acc, disp2);
+    for (int a = 0; a < 3; a++) fth[a] = ca.z * ((const T*)p.th)[(6 + a) * n + i];
+    finish_particle<T>(p, i, r, mn, en, fth, ca.w, acc, disp2);
   }
   step_block_sums(p, blockIdx.x, acc, disp2);
 }
@@ -723,23 +738,24 @@ int launch_rk_accept(cudaStream_t st, const RKStage& q, bool fp64) {
 int int_blocks(int n) { return (n + kIntThreads - 1) / kIntThreads; }
 int int_blocks_one(int n) { return (n + kIntOne - 1) / kIntOne; }
 
-int launch_noise(cudaStream_t st, const IntParams& p, bool fp64) {
+int launch_noise(cudaStream_t st, const IntParams& p, bool unit, bool fp64) {
   const dim3 g(int_blocks_one(p.n), 5);
+  auto go = [&](auto kern) { kern<<<g, kIntOne, 0, st>>>(p); };
   if (fp64)
-    k_noise<double><<<g, kIntOne, 0, st>>>(p);
+    unit ? go(k_noise<double, true>) : go(k_noise<double, false>);
   else
-    k_noise<float><<<g, kIntOne, 0, st>>>(p);
+    unit ? go(k_noise<float, true>) : go(k_noise<float, false>);
   return 1;
 }
 
-int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, double nf, const double* zr, const double* zt,
+int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, const double* zr, const double* zt,
                       const double* ivol, const double* izt, const double* v1, const double* v2, const double* mu,
-                      const double* rm, void* cA, void* cB, bool fp64) {
+                      const double* rm, double2* sTB, void* cA, void* cB, bool fp64) {
   const int g = int_blocks(n);
   if (fp64)
-    k_int_consts<double><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, nf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+    k_int_consts<double><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, sTB, cA, cB);
   else
-    k_int_consts<float><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, nf, zr, zt, ivol, izt, v1, v2, mu, rm, cA, cB);
+    k_int_consts<float><<<g, kIntThreads, 0, st>>>(n, ct, cb, cf, zr, zt, ivol, izt, v1, v2, mu, rm, sTB, cA, cB);
   return 1;
 }
 

@@ -157,10 +157,10 @@ size_t ksf_smem(int kc);
 int scatter_particles(int kc);
 
 // Integrator.
-int launch_noise(cudaStream_t st, const IntParams& p, bool fp64);
-int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, double nf, const double* zr,
-                      const double* zt, const double* ivol, const double* izt, const double* v1, const double* v2,
-                      const double* mu, const double* rm, void* cA, void* cB, bool fp64);
+int launch_noise(cudaStream_t st, const IntParams& p, bool unit, bool fp64);
+int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, const double* zr, const double* zt,
+                      const double* ivol, const double* izt, const double* v1, const double* v2, const double* mu,
+                      const double* rm, double2* sTB, void* cA, void* cB, bool fp64);
 int launch_heun1(cudaStream_t st, const IntParams& p, bool fp64);
 int launch_obs(cudaStream_t st, const ObsParams& p);
 // Stage 2 with the step records (k_obs) fused: done = a zeroed block counter.
