@@ -17,14 +17,14 @@
 // the pairs at 500 bins), so the counts are those of the FP64 expression; FP64
 // for every pair in range would cost ~40 instructions of 64 cycles each.
 // Bound: the candidates' loads from L1, ~95 per particle at N = 32768 and a
-// range of 0.047 L: 546 us per call over all pairs -> 86 us (27 of them this walk).
-// Longer ranges: all pairs from the FP64 master positions; block (x, y) takes
-// the particles i of tile x against the 256 particles j of tile y >= x, staged in
-// shared memory; an FP32 pre-test in box units (with a margin) rejects the
-// pairs far outside the range, the rest get their FP64 distance; pairs
-// inside the range go to a per-block shared-memory histogram (integer
-// atomics) added to the global counts at the end (deterministic integer
-// sums).
+// range of 0.047 L: 546 us per call over all pairs -> 71 us (27 of them this walk).
+// Longer ranges, and frames whose particles gather in few cells: all pairs from the
+// FP64 master positions; a block takes the particles i of tile x against the 256
+// particles j of tile y >= x, staged in shared memory, tile pair after tile pair; an
+// FP32 pre-test in box units (with a margin) rejects the pairs far outside the
+// range, the rest get their FP64 distance; pairs inside the range go to a per-block
+// shared-memory histogram (integer atomics) added to the global counts after each
+// tile pair (deterministic integer sums).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -80,14 +80,22 @@ __global__ void __launch_bounds__(kRdfThreads) k_rdf_cells(int n, const double* 
   cs[i] = make_int2(c, atomicAdd(&count[c], 1));
 }
 
-// Exclusive sums of the cell counts (one block of 1024 threads); count is
-// left zero for the next call.
-__global__ void __launch_bounds__(1024) k_rdf_scan(int ncell, int* __restrict__ count, int* __restrict__ start) {
+// Exclusive sums of the cell counts (one block of 1024 threads).  *crowded: the
+// particles' cells hold more than `most` particles on average (count squared, summed).
+__global__ void __launch_bounds__(1024) k_rdf_scan(int ncell, const int* __restrict__ count, int* __restrict__ start,
+                                                   double most, unsigned long long* __restrict__ crowded) {
   __shared__ int wsum[32];
+  __shared__ unsigned long long sq[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int per = (ncell + 1023) / 1024, b = min(t * per, ncell), e = min(ncell, b + per);
   int local = 0;
-  for (int c = b; c < e; c++) local += count[c];
+  unsigned long long s2 = 0;
+#pragma unroll 8
+  for (int c = b; c < e; c++) {
+    const int v = count[c];
+    local += v;
+    s2 += (unsigned long long)v * (unsigned)v;
+  }
   int incl = local;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -95,8 +103,12 @@ __global__ void __launch_bounds__(1024) k_rdf_scan(int ncell, int* __restrict__ 
     if (lane >= o) incl += v;
   }
   if (lane == 31) wsum[w] = incl;
+  s2 = warp_sum(s2);
+  if (lane == 0) sq[w] = s2;
   __syncthreads();
   if (w == 0) {
+    s2 = warp_sum(sq[lane]);
+    if (lane == 0) *crowded = (double)s2 > most;
     const int v = wsum[lane];
     int inc = v;
 #pragma unroll
@@ -108,10 +120,10 @@ __global__ void __launch_bounds__(1024) k_rdf_scan(int ncell, int* __restrict__ 
   }
   __syncthreads();
   int run = wsum[w] + incl - local;
+#pragma unroll 8
   for (int c = b; c < e; c++) {
     start[c] = run;
     run += count[c];
-    count[c] = 0;
   }
   if (t == 1023) start[ncell] = run;
 }
@@ -136,7 +148,9 @@ __global__ void __launch_bounds__(kRdfThreads) k_rdf_near(int n, const int4* __r
                                                           const int* __restrict__ start, int ncx,
                                                           const double* __restrict__ pos, RdfBins rb, float inv_f,
                                                           float tol, int bin_cont, int jmax,
+                                                          const unsigned long long* __restrict__ crowded,
                                                           unsigned long long* __restrict__ counts) {
+  if (*crowded) return;  // left to k_rdf
   extern __shared__ unsigned int hist[];  // [bins]
   for (int b = threadIdx.x; b < rb.bins; b += kRdfThreads) hist[b] = 0;
   __syncthreads();
@@ -180,46 +194,54 @@ __global__ void __launch_bounds__(kRdfThreads) k_rdf_near(int n, const int4* __r
     if (hist[b]) atomicAdd(&counts[b], (unsigned long long)hist[b]);
 }
 
-// Block (x, y): particles i of tile x against the particles j of tile y >= x.
+// All pairs, tile pair after tile pair: particles i of tile x against the particles j
+// of tile y >= x.
 __global__ void __launch_bounds__(kRdfThreads) k_rdf(int n, const double* __restrict__ pos, RdfBins rb,
-                                                     float range2_test, int jmax,
+                                                     float range2_test, int jmax, int ntile,
                                                      unsigned long long* __restrict__ counts) {
-  if (blockIdx.y < blockIdx.x) return;
   extern __shared__ unsigned char smem_raw[];
   double* tile = (double*)smem_raw;                          // [3][kRdfThreads]
   float* tilef = (float*)(tile + 3 * kRdfThreads);           // [3][kRdfThreads] box units
   unsigned int* hist = (unsigned int*)(tilef + 3 * kRdfThreads);  // [bins]
-  for (int b = threadIdx.x; b < rb.bins; b += blockDim.x) hist[b] = 0;
   const float invL = (float)(1.0 / rb.L);
-  const int i = blockIdx.x * kRdfThreads + threadIdx.x;
-  const int j0 = blockIdx.y * kRdfThreads, jl = j0 + threadIdx.x;
-  if (jl < jmax) {
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      tile[a * kRdfThreads + threadIdx.x] = pos[a * n + jl];
-      tilef[a * kRdfThreads + threadIdx.x] = (float)pos[a * n + jl] * invL;
+  const unsigned pairs = (unsigned)ntile * (unsigned)(ntile + 1) / 2;
+  for (unsigned q = blockIdx.x; q < pairs; q += gridDim.x) {
+    // q = y (y + 1) / 2 + x, x <= y
+    unsigned y = min((unsigned)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f), (unsigned)ntile - 1u);
+    while (y * (y + 1) / 2 > q) y--;
+    while ((y + 1) * (y + 2) / 2 <= q) y++;
+    const int i0 = (int)(q - y * (y + 1) / 2) * kRdfThreads, j0 = (int)y * kRdfThreads;
+    __syncthreads();
+    for (int b = threadIdx.x; b < rb.bins; b += kRdfThreads) hist[b] = 0;
+    const int i = i0 + threadIdx.x, jl = j0 + threadIdx.x;
+    if (jl < jmax) {
+      for (int a = 0; a < 3; a++) {
+        const double v = pos[a * n + jl];
+        tile[a * kRdfThreads + threadIdx.x] = v;
+        tilef[a * kRdfThreads + threadIdx.x] = (float)v * invL;
+      }
     }
-  }
-  __syncthreads();
-  if (i < n) {
-    const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
-    const float xf = (float)xi * invL, yf = (float)yi * invL, zf = (float)zi * invL;
-    const int tn = min(kRdfThreads, jmax - j0);
-    for (int t = 0; t < tn; t++) {
-      if (j0 + t <= i) continue;
-      // FP32 pre-test in box units with a margin, FP64 distance for the rest
-      float fx = xf - tilef[t], fy = yf - tilef[kRdfThreads + t], fz = zf - tilef[2 * kRdfThreads + t];
-      fx -= rintf(fx);
-      fy -= rintf(fy);
-      fz -= rintf(fz);
-      if (fx * fx + fy * fy + fz * fz > range2_test) continue;
-      const int b = rb.bin(xi - tile[t], yi - tile[kRdfThreads + t], zi - tile[2 * kRdfThreads + t]);
-      if (b >= 0) atomicAdd(&hist[b], 1u);
+    __syncthreads();
+    if (i < n) {
+      const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
+      const float xf = (float)xi * invL, yf = (float)yi * invL, zf = (float)zi * invL;
+      const int tn = min(kRdfThreads, jmax - j0);
+      for (int t = 0; t < tn; t++) {
+        if (j0 + t <= i) continue;
+        float fx = xf - tilef[t], fy = yf - tilef[kRdfThreads + t], fz = zf - tilef[2 * kRdfThreads + t];
+        // minimum image in box units (|f| may exceed 1/2 just past the faces)
+        fx -= rintf(fx);
+        fy -= rintf(fy);
+        fz -= rintf(fz);
+        if (fx * fx + fy * fy + fz * fz > range2_test) continue;
+        const int b = rb.bin(xi - tile[t], yi - tile[kRdfThreads + t], zi - tile[2 * kRdfThreads + t]);
+        if (b >= 0) atomicAdd(&hist[b], 1u);
+      }
     }
+    __syncthreads();
+    for (int b = threadIdx.x; b < rb.bins; b += kRdfThreads)
+      if (hist[b]) atomicAdd(&counts[b], (unsigned long long)hist[b]);
   }
-  __syncthreads();
-  for (int b = threadIdx.x; b < rb.bins; b += blockDim.x)
-    if (hist[b]) atomicAdd(&counts[b], (unsigned long long)hist[b]);
 }
 
 }  // namespace md
@@ -244,9 +266,10 @@ extern "C" int md_rdf(md_ctx* c, int64_t bins, double range, double r_mag0, int 
   const int ncx = (int)std::min({1.0 / rbox, std::cbrt(0.5 * n), 128.0});
   const bool cells = ncx >= 5;
   const int ncell = cells ? ncx * ncx * ncx : 0;
-  // workspace, kept by the context: counts | sorted x | x | cell, place | cell | cell counts | starts
-  const size_t cb = sizeof(unsigned long long) * (size_t)md::kRdfMaxBins;
-  const size_t need = cb + (cells ? 44 * (size_t)n + 8 * (size_t)(ncell + 1) : 0);
+  // workspace, kept by the context: sorted x | x | cell, place | counts | crowded | cell
+  // counts | starts | cell
+  const size_t cb = sizeof(unsigned long long) * (size_t)(md::kRdfMaxBins + 1);
+  const size_t need = cb + 8 * (size_t)(ncell + 1) + (cells ? 44 * (size_t)n : 0);
   if (need > c->rdf_cap) {
     dfree(c, c->rdf_ws);
     c->rdf_ws = nullptr;
@@ -254,35 +277,50 @@ extern "C" int md_rdf(md_ctx* c, int64_t bins, double range, double r_mag0, int 
     if ((st = dalloc(c, &c->rdf_ws, need))) return st;
     c->rdf_cap = need;
   }
-  char* ws = (char*)c->rdf_ws;
-  unsigned long long* d_counts = (unsigned long long*)ws;
-  if (cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * (size_t)bins, c->stream) != cudaSuccess)
+  const size_t nc = cells ? (size_t)n : 0;
+  int4 *sorted = (int4*)c->rdf_ws, *x = sorted + nc;
+  int2* cs = (int2*)(x + nc);
+  unsigned long long *d_counts = (unsigned long long*)(cs + nc), *crowded = d_counts + bins;
+  int *count = (int*)(crowded + 1), *start = count + ncell, *cellof = start + ncell + 1;
+  const size_t hb = sizeof(unsigned long long) * (size_t)(bins + 1);
+  if (cudaMemsetAsync(d_counts, 0, hb + sizeof(int) * (size_t)ncell, c->stream) != cudaSuccess)
     return set_err(c, MD_ERR_CUDA, "md_rdf: memset failed");
   const int nt = (n + md::kRdfThreads - 1) / md::kRdfThreads;
+  auto all_pairs = [&] {
+    const size_t smem = (sizeof(double) + sizeof(float)) * 3 * md::kRdfThreads + sizeof(unsigned int) * (size_t)bins;
+    md::allow_smem((const void*)md::k_rdf);
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+    // 64 blocks per SM, dealt out as they finish (8, all resident: 689 us against 581
+    // at N = 32768)
+    const int g = (int)std::min<int64_t>((int64_t)nt * (nt + 1) / 2, 64 * nsm);
+    md::k_rdf<<<g, md::kRdfThreads, smem, c->stream>>>(n, c->pos, rb, (float)(rbox * rbox), jmax, nt, d_counts);
+  };
+  std::vector<unsigned long long> h((size_t)bins + 1);
+  auto read = [&] {
+    return cudaGetLastError() == cudaSuccess &&
+           cudaMemcpyAsync(h.data(), d_counts, hb, cudaMemcpyDeviceToHost, c->stream) == cudaSuccess &&
+           cudaStreamSynchronize(c->stream) == cudaSuccess;
+  };
   if (cells) {
-    int4 *sorted = (int4*)(ws + cb), *x = sorted + n;
-    int2* cs = (int2*)(x + n);
-    int *cellof = (int*)(cs + n), *count = cellof + n, *start = count + ncell + 1;
-    if (cudaMemsetAsync(count, 0, sizeof(int) * (size_t)ncell, c->stream) != cudaSuccess)
-      return set_err(c, MD_ERR_CUDA, "md_rdf: memset failed");
+    // A walk takes ~2.3 us for each particle in a cell (its threads walk one after
+    // another); all pairs take 150 us at N = 2048, 201 at 8192, 530 at 32768, 1660 at
+    // 65536, 6240 at 131072: equal at ~45, 60, 180, 500, 1750 particles in a
+    // particle's cell.  Below ~1500 particles the walk is never much longer.
+    const double most = n < 1500 ? 1e300 : (double)n * (45.0 + 1.0e-7 * (double)n * (double)n);
     md::k_rdf_cells<<<nt, md::kRdfThreads, 0, c->stream>>>(n, c->pos, 1.0 / L, ncx, count, x, cs);
-    md::k_rdf_scan<<<1, 1024, 0, c->stream>>>(ncell, count, start);
+    md::k_rdf_scan<<<1, 1024, 0, c->stream>>>(ncell, count, start, most, crowded);
     md::k_rdf_place<<<nt, md::kRdfThreads, 0, c->stream>>>(n, x, cs, start, sorted, cellof);
     const double per_fix = L / 4294967296.0 / bw;  // bins per 2^-32 box lengths
     md::k_rdf_near<<<dim3(nt, 3), md::kRdfThreads, sizeof(unsigned int) * (size_t)bins, c->stream>>>(
         n, sorted, cellof, start, ncx, c->pos, rb, (float)per_fix, (float)(4.0 * per_fix + 1e-9),
-        (int)std::floor(rb.rcont * rb.inv_bw), jmax, d_counts);
-  } else {
-    const size_t smem = (sizeof(double) + sizeof(float)) * 3 * md::kRdfThreads + sizeof(unsigned int) * (size_t)bins;
-    md::allow_smem((const void*)md::k_rdf);
-    md::k_rdf<<<dim3(nt, nt), md::kRdfThreads, smem, c->stream>>>(n, c->pos, rb, (float)(rbox * rbox), jmax, d_counts);
+        (int)std::floor(rb.rcont * rb.inv_bw), jmax, crowded, d_counts);
+    if (!read()) return set_err(c, MD_ERR_CUDA, "md_rdf: kernel or copy failed");
   }
-  std::vector<unsigned long long> h((size_t)bins);
-  if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(h.data(), d_counts, sizeof(unsigned long long) * (size_t)bins, cudaMemcpyDeviceToHost,
-                      c->stream) != cudaSuccess ||
-      cudaStreamSynchronize(c->stream) != cudaSuccess)
-    return set_err(c, MD_ERR_CUDA, "md_rdf: kernel or copy failed");
+  if (!cells || h[(size_t)bins]) {
+    all_pairs();
+    if (!read()) return set_err(c, MD_ERR_CUDA, "md_rdf: kernel or copy failed");
+  }
   // normalisation of the script: L^3 / (2 pi dr^3 N^2) / (k - 1/2)^2
   const double norm = L * L * L / (2.0 * c->cfg.my_pi * bw * bw * bw * (double)n * (double)n);
   for (int64_t k = 0; k < bins; k++) {

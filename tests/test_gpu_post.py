@@ -50,3 +50,26 @@ def test_rdf_routes(n, phi, bins, range_mag, shift):
     ref = np.rint(gr * (np.arange(bins) + 0.5) ** 2 * (2 * np.pi * bw ** 3 * n * n) / g["lBox"] ** 3).astype(np.int64)
     assert (np.abs(cnt.astype(np.int64) - ref) > 0).sum() <= 2
     assert np.abs(cnt.astype(np.int64).sum() - ref.sum()) <= 1 and ref.sum() > 0
+
+
+@pytest.mark.parametrize("n", [1499, 1500, 2049, 6000])
+@pytest.mark.parametrize("include_last", [False, True])
+def test_rdf_of_a_gathered_frame(n, include_last):
+    """All particles in 1/125 of the box, a few hundred in each cell: the cells are
+    left for the tile pairs (from 1500 particles on), with the same counts."""
+    ini, g = random_system(n, seed=n, rc_frac=0.3, phi=0.05)
+    sim = gpu_system(ini, g, 1)
+    L = 5.0 * g["lBox"]
+    sim.set_box(L)
+    sim.set_ewald(0.2 * g["alpha"], 5.0 * g["rc"], g["kc"])
+    r0, bins = float(g["rMag"][0]), 300
+    bw = 20.0 * r0 / bins
+    for pos in (g["pos"], 5.0 * g["pos"], g["pos"]):  # gathered, spread over the box, gathered
+        pos = np.ascontiguousarray(pos)
+        sim.set_state(pos, g["mm"], g["ea"])
+        _, gr = analysis.radial_distribution(pos, L, r0, bins=bins, range_mag=20.0, include_last=include_last)
+        ref = np.rint(gr * (np.arange(bins) + 0.5) ** 2 * (2 * np.pi * bw ** 3 * n * n) / L ** 3).astype(np.int64)
+        _, _, cnt = sim.rdf(bins=bins, range_mag=20.0, r_mag0=r0, include_last=include_last)
+        assert (np.abs(cnt.astype(np.int64) - ref) > 0).sum() <= 2
+        assert np.abs(cnt.astype(np.int64).sum() - ref.sum()) <= 1
+        assert ref.sum() > 0
