@@ -26,6 +26,7 @@
 
 #include "md_common.cuh"
 #include "md_kernels.h"
+#include "md_mesh.cuh"
 
 namespace md {
 
@@ -198,14 +199,29 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(1024) k
   if (blockIdx.x == 0) scan_cells(p);
   cluster_sync();
   for (int i = g; i < p.n; i += G) scatter_one(p, i);
+  for (int b = g >> 5; b < p.mesh.nbrick; b += G >> 5) mesh_plan_count(p.mesh, p.s.cell_start, b, threadIdx.x & 31);
   cluster_sync();
   for (int c = g >> 5; c < p.grid.ncell; c += G >> 5) sort_cell(p, c, threadIdx.x & 31);
+  if (blockIdx.x == kClusterBlocks - 1 && p.mesh.nbrick > 0) mesh_plan_items(p.mesh);
 }
 template <bool FIXED>
 __global__ void __launch_bounds__(kCellThreads) k_cell_assign(CellParams p) { cell_assign<FIXED>(p, blockIdx.x); }
 __global__ void __launch_bounds__(1024) k_cell_scan(CellParams p) { cell_scan(p); }
-__global__ void __launch_bounds__(kCellThreads) k_cell_scatter(CellParams p) { cell_scatter(p, blockIdx.x); }
-__global__ void __launch_bounds__(kCellThreads) k_cell_sort(CellParams p) { cell_sort(p, blockIdx.x); }
+// With the mesh's plan in blocks past the first nb (md_mesh.cuh).
+__global__ void __launch_bounds__(kCellThreads) k_cell_scatter(CellParams p, int nb) {
+  if ((int)blockIdx.x < nb) {
+    cell_scatter(p, blockIdx.x);
+  } else if (!skip(p.flags)) {
+    const int b = ((int)blockIdx.x - nb) * (kCellThreads / 32) + (threadIdx.x >> 5);
+    if (b < p.mesh.nbrick) mesh_plan_count(p.mesh, p.s.cell_start, b, threadIdx.x & 31);
+  }
+}
+__global__ void __launch_bounds__(kCellThreads) k_cell_sort(CellParams p, int nb) {
+  if ((int)blockIdx.x < nb)
+    cell_sort(p, blockIdx.x);
+  else if (!skip(p.flags))
+    mesh_plan_items(p.mesh);
+}
 template <typename T>
 __global__ void __launch_bounds__(kCellThreads) k_sorted_fill(CellParams p) {
   sorted_fill<T>(p, blockIdx.x);
@@ -417,8 +433,9 @@ int launch_cells(cudaStream_t st, const CellParams& p, bool fp64, bool fill) {
     launches++;
     if (p.grid.ncx > 1) {
       k_cell_scan<<<1, 1024, 0, st>>>(p);
-      k_cell_scatter<<<nb, kCellThreads, 0, st>>>(p);
-      k_cell_sort<<<cell_sort_blocks(p.grid), kCellThreads, 0, st>>>(p);
+      const int mb = (p.mesh.nbrick + kCellThreads / 32 - 1) / (kCellThreads / 32), sb = cell_sort_blocks(p.grid);
+      k_cell_scatter<<<nb + mb, kCellThreads, 0, st>>>(p, nb);
+      k_cell_sort<<<sb + (mb > 0), kCellThreads, 0, st>>>(p, sb);
       launches += 3;
     }
   }

@@ -56,6 +56,13 @@ struct StepFlags {
 };
 
 // Cell-list build of one system (positions in particle order, FP64).
+// The mesh's bricks as the cell order sees them (md_mesh.cuh; M = 0: none).
+struct MeshGrid {
+  int M, ncx, nbrick, nitem;
+  float reach;  // distance a particle may be from the cell it is filed in, box units
+  int* plan;
+};
+
 struct CellParams {
   int n;
   double invL;
@@ -71,6 +78,7 @@ struct CellParams {
   SortedView s;
   double* xbuild;           // positions at the last build (may be null)
   StepFlags* flags;
+  MeshGrid mesh;
 };
 
 // A packed launch runs one kernel over the blocks of several independent
@@ -322,6 +330,7 @@ struct KParams {
   void* rw_ad;              // [T][4] T4 (A, D)
   // k space through a mesh (md_kmesh.cu; gm_M = 0: off)
   int gm_M, gm_nbrick;     // mesh points per axis, bricks of the spread
+  int gm_nitem;            // work items that there is room for (>= bricks)
   int gm_ncx;              // cells per axis of the sorted view
   float gm_reach;          // distance a particle may be from the cell it is filed in, box units
   const float* gm_coef;    // [kMeshW][kMeshDeg + 1] window polynomials, lowest order first
@@ -331,6 +340,7 @@ struct KParams {
   float2* gm_z;            // [3][kc + 1][M][M] after the z axis
   float4 *gm_y, *gm_t;     // [kc + 1][2 kc + 1][M] rows before and after the x axis
   float4* gm_b;            // [M][M][M] field mesh
+  int* gm_plan;            // work items of the spread and the interpolation
   long long tc_wait;     // SM clock cycles after which an mbarrier wait gives up
   int* err;              // device error word (kErrTcWait on a wait that gave up)
 };

@@ -191,6 +191,19 @@ RealParams real_params(md_ctx* c, void* B, void* F, void* ov) {
   return p;
 }
 
+static MeshGrid mesh_grid(const md_ctx* c) {
+  MeshGrid m{};
+  if (c->gm_M == 0) return m;
+  m.M = c->gm_M;
+  m.ncx = c->grid.ncx;
+  m.nbrick = md::mesh_bricks(c->gm_M);
+  m.nitem = md::mesh_items(c->gm_M);
+  // half the skin since the build, and rounding
+  m.reach = (float)(0.5 * c->cell_skin * c->rc / c->L * (1.0 + 1e-5) + 2e-6);
+  m.plan = c->gm_plan;
+  return m;
+}
+
 CellParams cell_params(md_ctx* c) {
   CellParams p{};
   p.n = (int)c->n;
@@ -207,6 +220,7 @@ CellParams cell_params(md_ctx* c) {
   p.s = sorted_view(c);
   p.xbuild = c->xbuild;
   p.flags = &c->sc->flags;
+  p.mesh = mesh_grid(c);
   return p;
 }
 
@@ -287,10 +301,11 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.rw_rowt = c->rw_rowt;
   p.rw_ad = c->rw_ad;
   p.gm_M = c->gm_M;
-  if (c->gm_M > 0) p.gm_nbrick = md::mesh_bricks(c->gm_M);
-  p.gm_ncx = c->grid.ncx;
-  // half the skin since the build, and rounding
-  p.gm_reach = (float)(0.5 * c->cell_skin * c->rc / c->L * (1.0 + 1e-5) + 2e-6);
+  const MeshGrid m = mesh_grid(c);
+  p.gm_nbrick = m.nbrick;
+  p.gm_nitem = m.nitem;
+  p.gm_ncx = m.ncx;
+  p.gm_reach = m.reach;
   p.gm_coef = c->gm_coef;
   p.gm_fac = c->gm_fac;
   p.gm_tw = c->gm_tw;
@@ -299,6 +314,7 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.gm_y = c->gm_y;
   p.gm_t = c->gm_t;
   p.gm_b = c->gm_b;
+  p.gm_plan = m.plan;
   p.tc_wait = c->tc_wait;
   p.err = &c->sc->err;
   return p;
@@ -856,7 +872,7 @@ static bool mesh_wanted(const md_ctx* c) {
 static int setup_mesh(md_ctx* c) {
   c->gm_M = 0;
   if (!mesh_wanted(c)) return MD_OK;
-  const int kc = (int)c->kc, M = md::mesh_points(kc), nb = md::mesh_bricks(M);
+  const int kc = (int)c->kc, M = md::mesh_points(kc), items = md::mesh_items(M);
   const size_t kc1 = (size_t)kc + 1, rows = kc1 * (2 * (size_t)kc + 1), M2 = (size_t)M * M;
   const mdh::MeshTables t = mdh::mesh_tables(kc, M);
   // factors in the layout of tc_kmap: row, nx
@@ -878,7 +894,7 @@ static int setup_mesh(md_ctx* c) {
     const double a = 2.0 * std::acos(-1.0) * j / M;
     tw[j] = make_float2((float)std::cos(a), (float)std::sin(a));
   }
-  void* old[] = {c->gm_coef, c->gm_fac, c->gm_tw, c->gm_part, c->gm_z, c->gm_y, c->gm_t, c->gm_b};
+  void* old[] = {c->gm_coef, c->gm_fac, c->gm_tw, c->gm_part, c->gm_z, c->gm_y, c->gm_t, c->gm_b, c->gm_plan};
   for (void* q : old) dfree(c, q);
   c->gm_coef = nullptr;
   c->gm_fac = nullptr;
@@ -886,6 +902,9 @@ static int setup_mesh(md_ctx* c) {
   c->gm_part = nullptr;
   c->gm_z = nullptr;
   c->gm_y = c->gm_t = c->gm_b = nullptr;
+  c->gm_plan = nullptr;
+  std::vector<int> plan;
+  md::mesh_plan_init(M, plan);
   int st;
   if ((st = dalloc(c, &c->gm_coef, sizeof(float) * t.coef.size()))) return st;
   if ((st = dalloc(c, &c->gm_fac, sizeof(float2) * fac.size()))) return st;
@@ -895,16 +914,18 @@ static int setup_mesh(md_ctx* c) {
   if ((st = dalloc(c, &c->gm_y, sizeof(float4) * rows * M))) return st;
   if ((st = dalloc(c, &c->gm_t, sizeof(float4) * rows * M))) return st;
   if ((st = dalloc(c, &c->gm_b, sizeof(float4) * M2 * M))) return st;
-  if (nb > c->musum_cap) {
+  if ((st = dalloc(c, &c->gm_plan, sizeof(int) * plan.size()))) return st;
+  if (items > c->musum_cap) {
     dfree(c, c->musum_part);
     c->musum_part = nullptr;
     c->musum_cap = 0;
-    if ((st = dalloc(c, &c->musum_part, 24 * (size_t)nb))) return st;
-    c->musum_cap = nb;
+    if ((st = dalloc(c, &c->musum_part, 24 * (size_t)items))) return st;
+    c->musum_cap = items;
   }
   CK(c, cudaMemcpy(c->gm_coef, t.coef.data(), sizeof(float) * t.coef.size(), cudaMemcpyHostToDevice));
   CK(c, cudaMemcpy(c->gm_fac, fac.data(), sizeof(float2) * fac.size(), cudaMemcpyHostToDevice));
   CK(c, cudaMemcpy(c->gm_tw, tw.data(), sizeof(float2) * (size_t)M, cudaMemcpyHostToDevice));
+  CK(c, cudaMemcpy(c->gm_plan, plan.data(), sizeof(int) * plan.size(), cudaMemcpyHostToDevice));
   c->gm_M = M;
   return MD_OK;
 }

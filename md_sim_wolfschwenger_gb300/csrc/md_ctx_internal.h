@@ -146,6 +146,7 @@ struct md_ctx {
   float* gm_part = nullptr;
   float2* gm_z = nullptr;
   float4 *gm_y = nullptr, *gm_t = nullptr, *gm_b = nullptr;
+  int* gm_plan = nullptr;
   // tensor-core k space (mixed path; md_ktc.cu): engine choice, k rows and
   // their buffers (tc_rows = 0 while the engine is off)
   int kengine = MD_KSPACE_AUTO;

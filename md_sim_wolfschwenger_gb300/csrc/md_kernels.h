@@ -7,6 +7,8 @@
 // host from the per-system block counts below).  Packed launches exist for
 // the mixed-precision path.
 #pragma once
+#include <vector>
+
 #include "md_common.cuh"
 
 namespace md {
@@ -138,12 +140,16 @@ struct RowShape {
   int nblk, threads, chunk, nchunk;
 };
 RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
-// k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks and
-// partial-mesh floats of the spread.
+// k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks, work
+// items (bricks and parts of crowded ones), partial-mesh floats of the spread, and the
+// plan that says which item is what (its size and its initial content).
 // (kc >= 5: M >= 24, so that a window and its neighbour bricks do not wrap onto themselves)
 inline int mesh_points(int kc) { return 8 * ((kc + 1) / 2); }
 int mesh_bricks(int M);
+int mesh_items(int M);
 size_t mesh_part_floats(int M);
+size_t mesh_plan_ints(int M);
+void mesh_plan_init(int M, std::vector<int>& out);
 int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev);
 int launch_krows(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaEvent_t* ev);
 // Per-particle phase tables (once per step; positions are frozen across the

@@ -27,25 +27,27 @@
 // Measured at N = 32768 (M = 64) / 131072 (M = 80), us: spread 29 / 79, the four
 // transforms 30 / 50, interpolation 36 / 104 with the force, 29 / 80 without;
 // the tensor cores' 135 / 850 and 120 / 700 for the same.
+#include <vector>
+
 #include "md_common.cuh"
 #include "md_kernels.h"
+#include "md_mesh.cuh"
 
 namespace md {
 
-constexpr int kMW = kMeshW;                    // window points per axis (odd: nearest mesh point +- 4)
-constexpr int kMH = kMW / 2;
-constexpr int kMC = kMeshDeg + 1;              // coefficients per interval
-constexpr int kBX = 16, kBY = 8, kBZ = 8;      // brick: mesh points whose particles one block spreads
-constexpr int kPX = kBX + kMW - 1, kPY = kBY + kMW - 1, kPZ = kBZ + kMW - 1;  // with the window's reach
-static_assert(kPZ == 16 && kPY == 16 && kPX == 24, "padded brick");
-constexpr int kPad = kPX * kPY * kPZ;          // points of a padded brick
-constexpr int kBrThreads = kPY * kPZ;          // brick kernels: a thread per (y, z) of the padded brick
-constexpr int kBrWarps = kBrThreads / 32;      // two rows y of 16 z each
-static_assert(kPZ == 16 && kBrThreads == 256, "lanes of a warp: two rows of 16");
-
 static int mesh_nbx(int M) { return (M + kBX - 1) / kBX; }
 int mesh_bricks(int M) { return mesh_nbx(M) * (M / kBY) * (M / kBZ); }
-size_t mesh_part_floats(int M) { return (size_t)mesh_bricks(M) * 3 * kPad; }
+int mesh_items(int M) { return mesh_bricks(M) + mesh_bricks(M) / 8; }
+size_t mesh_part_floats(int M) { return (size_t)mesh_items(M) * 3 * kPad; }
+size_t mesh_plan_ints(int M) { return 2 + 2 * (size_t)mesh_bricks(M) + 2 * (size_t)mesh_items(M); }
+
+// Brick of the block's item, -1 without one.  A brick's own block does not wait for
+// the plan to know where it works.
+__device__ __forceinline__ int mesh_brick(const KParams& p) {
+  if ((int)blockIdx.x < p.gm_nbrick) return blockIdx.x;
+  const int2 item = MeshPlan(p.gm_plan, p.gm_nbrick).item[blockIdx.x];
+  return item.y ? item.x : -1;
+}
 
 // Nearest mesh point of a fixed-point coordinate (2^32 per box) and s = -2 times
 // the distance to it, in [-1, 1]: the argument of the window's polynomials.
@@ -68,12 +70,13 @@ struct BrickScan {
   int wsum[NT / 32];
   int place[NT];      // [class][warp]: particles, then the first one's place
   int start[33];      // first particle of each class, and their number
+  int first, step;    // of the candidates, for the block's item
 };
 
 // Finds the particles of the brick at (x0, y0, z0): the cells that reach into it,
 // grown by the distance a particle may have moved since they were filled, are
-// searched NT candidates at a time.  put(k, j, start, s) stores a particle found
-// (sorted index, window start x | y << 8 | z << 16, arguments of the window's
+// searched NT candidates at a time, the part of the block's item every parts-th
+// time.  put(k, j, start, s) stores a particle found (sorted index, window start x | y << 8 | z << 16, arguments of the window's
 // polynomials); k runs over the classes 4 (x / 2) + y / 2 of the start, and in cell
 // order within a class.  chunk(hits) is then called by the whole block, between
 // barriers.
@@ -82,22 +85,12 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan<NT>&
                                                 C&& chunk) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int M = p.gm_M, wx = min(kBX, M - x0), ncx = p.gm_ncx;
-  // a window starts kMH points below the nearest mesh point
-  auto cells = [&](int b0, int w, int& lo, int& cnt) {
-    const float im = 1.0f / (float)M, f = (float)ncx, h = p.gm_reach;
-    lo = (int)floorf((((float)(b0 + kMH) - 0.5f) * im + 0.5f - h) * f);
-    cnt = (int)floorf((((float)(b0 + w + kMH) - 0.5f) * im + 0.5f + h) * f) - lo + 1;
-    if (cnt >= ncx) {
-      lo = 0;
-      cnt = ncx;
-    }
-    lo %= ncx;
-    if (lo < 0) lo += ncx;
-  };
   int cx, nx, cy, ny, cz, nz;
-  cells(x0, wx, cx, nx);
-  cells(y0, kBY, cy, ny);
-  cells(z0, kBZ, cz, nz);
+  brick_cells(M, ncx, p.gm_reach, x0, wx, cx, nx);
+  brick_cells(M, ncx, p.gm_reach, y0, kBY, cy, ny);
+  brick_cells(M, ncx, p.gm_reach, z0, kBZ, cz, nz);
+  int part = 0;  // waited for after the rows of cells
+  if (tid == 0) part = MeshPlan(p.gm_plan, p.gm_nbrick).item[blockIdx.x].y;
   for (int r0 = 0; r0 < ny * nz; r0 += NT) {
     __syncthreads();
     {  // one row of cells per thread, split where it wraps
@@ -129,11 +122,15 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan<NT>&
       __syncthreads();
       for (int q = 0; q < wid; q++) incl += b.wsum[q];
       b.pre[tid + 1] = incl;
-      if (tid == 0) b.pre[0] = 0;
+      if (tid == 0) {
+        b.pre[0] = 0;
+        b.first = (part & 0xffff) * NT;
+        b.step = (part >> 16) * NT;
+      }
     }
     __syncthreads();
     const int total = b.pre[NT], nrow = min(NT, ny * nz - r0);
-    for (int t0 = 0; t0 < total; t0 += NT) {
+    for (int t0 = b.first; t0 < total; t0 += b.step) {
       const int t = t0 + tid;
       bool in = false;
       int at = 0, j = 0;
@@ -223,7 +220,11 @@ __global__ void __launch_bounds__(kBrThreads, 2) k_mesh_spread(KParams p) {
   SpreadSmem& sm = *(SpreadSmem*)smem;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int M = p.gm_M, nbx = (M + kBX - 1) / kBX, nby = M / kBY;
-  const int bx = blockIdx.x % nbx, by = blockIdx.x / nbx % nby, bz = blockIdx.x / (nbx * nby);
+  const int brick = mesh_brick(p), bx = brick % nbx, by = brick / nbx % nby, bz = brick / (nbx * nby);
+  if (brick < 0) {
+    if (tid < 3) p.musum_part[3 * blockIdx.x + tid] = 0.0;
+    return;
+  }
   for (int e = tid; e < kSub * kWS; e += kBrThreads) sm.w[e] = 0.f;
   for (int e = tid; e < kMW * kMC; e += kBrThreads) sm.coef[e] = p.gm_coef[e];
   const int y = tid >> 4, z = tid & 15;
@@ -351,6 +352,8 @@ __global__ void __launch_bounds__(256) k_mesh_z(KParams p) {
   const int b0 = blockIdx.y, b1 = b0 > 0 ? b0 - 1 : nby - 1;
   const int wid = threadIdx.x >> 5;  // a warp takes one line of each component
   const size_t bs = (size_t)3 * kPad * nbx;
+  const MeshPlan plan(p.gm_plan, p.gm_nbrick);
+  const bool split = *plan.total > 0;
   for (int z = threadIdx.x & 31; z < M; z += 32) {
     const int bz0 = z >> 3, bz1 = bz0 > 0 ? bz0 - 1 : nby - 1, lz = z & 7;
     float v[3][2] = {};
@@ -366,6 +369,21 @@ __global__ void __launch_bounds__(256) k_mesh_z(KParams p) {
         }
 #pragma unroll
     for (int c = 0; c < 3; c++) line[(c * kMZLines + wid) * LS + z] = v[c][0] + v[c][1];
+  }
+  if (split) {  // the extra items of split bricks
+    for (int z = threadIdx.x & 31; z < M; z += 32) {
+      const int bz0 = z >> 3, bz1 = bz0 > 0 ? bz0 - 1 : nby - 1, lz = z & 7;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int i = q >> 2, by = q & 2 ? b1 : b0, bz = q & 1 ? bz1 : bz0;
+        if (i >= ox.n) break;
+        const int b = (bz * nby + by) * nbx + ox.b[i];
+        const float* a = p.gm_part + (size_t)(p.gm_nbrick + plan.first[b]) * 3 * kPad +
+                         (ox.l[i] * kPY + wid + (q & 2 ? 8 : 0)) * kPZ + lz + (q & 1 ? 8 : 0);
+        for (int e = plan.extra[b]; e > 0; e--, a += 3 * kPad)
+          for (int c = 0; c < 3; c++) line[(c * kMZLines + wid) * LS + z] += a[c * kPad];
+      }
+    }
   }
   __syncthreads();
   // even and odd parts: line[z] + line[M - z], line[z] - line[M - z]
@@ -446,7 +464,7 @@ __global__ void __launch_bounds__(512) k_mesh_y(KParams p) {
   if (nz == kc && x0 == 0 && threadIdx.x < 96) {  // total moment, in the block with the fewest rows: fixed order
     const int c = threadIdx.x >> 5;
     double m = 0.0;
-    for (int b = threadIdx.x & 31; b < p.gm_nbrick; b += 32) m += p.musum_part[3 * b + c];
+    for (int b = threadIdx.x & 31; b < p.gm_nitem; b += 32) m += p.musum_part[3 * b + c];
     m = warp_sum(m);
     if ((threadIdx.x & 31) == 0) p.musum[c] = m;
   }
@@ -655,7 +673,9 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
   InterpSmem& sm = *(InterpSmem*)smem;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int M = p.gm_M, n = p.n, nbx = (M + kBX - 1) / kBX, nby = M / kBY;
-  const int x0 = blockIdx.x % nbx * kBX, y0 = blockIdx.x / nbx % nby * kBY, z0 = blockIdx.x / (nbx * nby) * kBZ;
+  const int brick = mesh_brick(p);
+  if (brick < 0) return;
+  const int x0 = brick % nbx * kBX, y0 = brick / nbx % nby * kBY, z0 = brick / (nbx * nby) * kBZ;
   auto fold = [&](int i) { return i >= M ? i - M : i; };
 #pragma unroll 8
   for (int e = tid; e < kPX * kPY * kPZ; e += kInThreads) {
@@ -672,7 +692,8 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
   const float fB = (float)-p.cflux, fF = (float)(p.cforce * (double)M / p.two_pi);
   float *B = (float*)p.B, *F = (float*)p.F;
   brick_particles(
-      p, sm.scan, x0, y0, z0, [&](int k, int j, int, const float (&)[3]) { sm.j[k] = j; },
+      p, sm.scan, x0, y0, z0,
+      [&](int k, int j, int, const float (&)[3]) { sm.j[k] = j; },
       [&](int hits) {
         int kn = 0;
         int4 xn = make_int4(0, 0, 0, 0);
@@ -772,10 +793,19 @@ __global__ void __launch_bounds__(kInThreads, 2) k_mesh_interp(KParams p) {
 
 // ------------------------------------------------------------- launches
 
+// One item per brick, as long as no plan was made.
+void mesh_plan_init(int M, std::vector<int>& out) {
+  const int nb = mesh_bricks(M);
+  out.assign(mesh_plan_ints(M), 0);
+  const MeshPlan plan(out.data(), nb);
+  for (int b = 0; b < nb; b++) plan.item[b] = make_int2(b, 1 << 16);
+}
+
 int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) {
   const int M = p.gm_M, kc1 = p.kc + 1, Q = 2 * p.kc + 1;
   allow_smem((const void*)k_mesh_spread);
-  k_mesh_spread<<<p.gm_nbrick, kBrThreads, sizeof(SpreadSmem), st>>>(p);
+  const int items = p.gm_nitem;
+  k_mesh_spread<<<items, kBrThreads, sizeof(SpreadSmem), st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_mesh_z<<<dim3(M, M / kMZLines), 256, sizeof(float) * (2 * M + 3 * kMZLines * (M + 1)), st>>>(p);
   k_mesh_y<<<dim3(kc1, M / kMYLines), (16 * kc1 + 31) / 32 * 32, sizeof(float2) * (M + 3 * kMYLines * (M + 2)), st>>>(p);
@@ -788,9 +818,9 @@ int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) 
   const size_t smf = sizeof(InterpSmem);
   allow_smem(kern);
   if (full)
-    k_mesh_interp<true><<<p.gm_nbrick, kInThreads, smf, st>>>(p);
+    k_mesh_interp<true><<<items, kInThreads, smf, st>>>(p);
   else
-    k_mesh_interp<false><<<p.gm_nbrick, kInThreads, smf, st>>>(p);
+    k_mesh_interp<false><<<items, kInThreads, smf, st>>>(p);
   return 6;
 }
 

@@ -139,3 +139,25 @@ def test_engine_of_the_current_parameters():
     assert large.kspace_engine() == "mesh"
     large.set_kspace_engine("tc")
     assert large.kspace_engine() == "tc"
+
+
+@pytest.mark.parametrize("n,kc,grow", [(8501, 16, 3.0), (8501, 20, 8.0), (20011, 15, 30.0), (20011, 21, 5.0)])
+def test_gathered_bricks_are_split(n, kc, grow):
+    """All particles in the middle of the box (an edge of 1 / grow): the few bricks
+    that hold them are split into parts, whose sums and particles come together
+    again; spread over the box afterwards, and gathered once more."""
+    ini, g = random_system_fast(n, seed=n + 5, phi=0.05, B0=0.02)
+    L, rc = grow * g["lBox"], 0.12 * grow * g["lBox"]
+    ref, sim = gpu_system(ini, g, 0), gpu_system(ini, g, 1)
+    for s in (ref, sim):
+        s.set_box(L)
+        s.set_ewald(3.5 / rc, rc, kc)
+    sim.set_strong_pairs(0.0)
+    assert sim.kspace_engine() == "mesh"
+    mm = np.roll(g["mm"], 1, axis=1)
+    for pos in (g["pos"] + 0.3 * L, grow * g["pos"], g["pos"] + 0.5 * L):  # across faces at the end
+        for s in (ref, sim):
+            s.set_state(pos, g["mm"], g["ea"])
+        got, want = k_part(sim, mm), k_part(ref, mm)
+        for q in range(4):
+            assert rms(got[q], want[q]) < TOL
