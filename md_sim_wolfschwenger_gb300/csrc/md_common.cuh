@@ -323,6 +323,7 @@ struct KParams {
   int rw_T, rw_R;          // tasks, rows
   int rw_nblk, rw_threads; // structure factor: task blocks, threads per block
   int rw_chunk, rw_nchunk; // particles per chunk, chunks
+  int rw_np;               // particles per scatter block
   const int4* rw_task;      // [T] row, ny, nz, first |nx|
   const int* rw_kidx;       // [T][4][+, -] sorted k index, or -1
   const double2* rw_row;    // [R] (ny, nz)

@@ -295,6 +295,7 @@ KParams k_params(md_ctx* c, void* B, void* F) {
   p.rw_threads = c->rws.threads;
   p.rw_chunk = c->rws.chunk;
   p.rw_nchunk = c->rws.nchunk;
+  p.rw_np = c->rws.np;
   p.rw_task = c->rw_task;
   p.rw_kidx = c->rw_kidx;
   p.rw_row = c->rw_row;
@@ -850,18 +851,21 @@ static int setup_rows(md_ctx* c) {
 }
 
 // Whether the mixed path's default engine goes through a mesh (md_kmesh.cu)
-// instead of the tensor cores.  The mesh's work per particle is that of ~6000 k
-// vectors (half space) on the tensor cores, ~4000 once its kernels fill the GPU;
-// its transforms, ~M^3, must not outweigh the particles.  Measured step times,
-// mesh / tensor cores, us: N = 6000, kc = 20 212 / 237, kc = 25 (M = 104) 377 / 322;
-// N = 8192, kc = 13 174 / 165, kc = 16 179 / 199, kc = 20 241 / 273, kc = 25 397 / 356;
-// N = 12000, kc = 14 236 / 227, kc = 16 237 / 265; N = 16384, kc = 13 286 / 267, kc = 15
-// 285 / 284..297; N = 20011, kc = 15 344 / 388; N = 32768, kc = 12 609 / 595, kc = 13
-// 621 / 626, kc = 15 599 / 664; N = 131072, kc = 13 3135 / 3286, kc = 20 3097 / 4186
-// (the interpolation has become 5 to 25 us faster since).
-// Errors of the k-space part against FP64 (rms, N = 32768): field 1.5e-7 / 1.2e-6,
-// force 2.8e-7 / 1.3e-6.  An engine or a tensor-core tiling that the caller chose is
-// kept.
+// instead of the tensor cores.  The mesh's work is in its particles and, ~M^3, in its
+// transforms, the tensor cores' in particles x k vectors, in steps (at kc = 20 and 24
+// they pad most).  Step times, mesh against tensor cores, both splits from the error
+// model:
+//   N = 20011 and more   10 to 37 % shorter (kc = 15 .. 25)
+//   N = 14000 .. 16384   up to 17 % shorter, 5 % longer at worst (kc = 17); kc = 25
+//                        (M^3 = 80 N) 3 % longer at 14000, 4 % shorter at 15000
+//   N = 8192 .. 13000    kc = 20 5 to 10 %, kc = 24 2 to 9 % shorter, kc = 16 equal to 6 %
+//                        shorter; the others 2 to 16 % longer
+//   N = 6000             2 to 18 % longer
+//   N = 32768, kc = 13   621 / 626 us, kc = 12 609 / 595
+// Where it takes longer it stays for its error, an eighth of the tensor cores' in the
+// field (k-space part against FP64, rms, N = 32768: field 1.5e-7 / 1.2e-6, force 2.8e-7
+// / 1.3e-6); from M^3 = 100 N on and below 6000 particles the time decides.  An engine
+// or a tensor-core tiling that the caller chose is kept.
 static bool mesh_wanted(const md_ctx* c) {
   if (fp64(c) || c->kengine != MD_KSPACE_AUTO || c->packed_only || c->tc_ring >= 0 || c->tc_waves != 1 || c->tc_rows == 0) return false;
   const double M = md::mesh_points((int)c->kc);
@@ -1641,8 +1645,8 @@ static int capture_steps(md_ctx* c, int k, double dt, cudaGraph_t* graph, cudaGr
 
 // Between two graphs lie ~3.4 us, between a graph's own steps ~0.7: a run that has
 // shown to be long (its capture, ~1 ms, then pays) goes on in graphs of several
-// steps.  N = 512 53.3 -> 50.2, N = 1000 67.3 -> 64.4, N = 4096 105.9 -> 104.5, N =
-// 8192 150.6 -> 146.0 us per step (N = 3001 94.3 -> 95.3).
+// steps.  N = 512 51.2 -> 47.4, N = 1000 59.5 -> 55.6, N = 3001 91.6 -> 87.7, N = 8192
+// 153.6 -> 148.9, N = 32768 585.6 -> 579.9 us per step.
 constexpr int kGraphSteps = 8, kGraphAfter = 128;
 
 // md_step's work queued on the stream (no synchronisation).

@@ -138,6 +138,7 @@ int launch_tc_wait_probe(cudaStream_t st, int* err, int arrive, long long limit)
 // the given number of tasks.
 struct RowShape {
   int nblk, threads, chunk, nchunk;
+  int np;  // particles per scatter block
 };
 RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64);
 // k space through a mesh (md_kmesh.cu): mesh points per axis for kc, bricks, work

@@ -424,6 +424,9 @@ RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64) {
   if (!fp64) nch = std::max(nch, (n + 511) / 512);
   s.chunk = ((n + nch - 1) / nch + 3) / 4 * 4;
   s.nchunk = (n + s.chunk - 1) / s.chunk;
+  // few particles per scatter block while that leaves SMs without a block (32 only
+  // where their phases fit)
+  s.np = n <= 16 * nsm ? 8 : (n <= 32 * nsm || kc > 64 ? 16 : 32);
   return s;
 }
 
@@ -456,10 +459,9 @@ static int krows_t(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_red_rows<T><<<dim3((p.rw_T + 31) / 32, 4), 256, 0, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal);
-  // few particles per block while that leaves SMs without a block
-  if (p.n <= 2432)
+  if (p.rw_np == 8)
     scat_rows<T, 8>(st, p, full);
-  else if (p.n <= 4864 || p.kc > 64)
+  else if (p.rw_np == 16)
     scat_rows<T, 16>(st, p, full);
   else
     scat_rows<T, 32>(st, p, full);
