@@ -247,3 +247,24 @@ def test_served_contexts_hold_what_batches_need(n, phi, lognormal):
     est = L.mdi_packed_ctx_bytes(C.byref(own.c), C.c_int64(n), r.ctypes.data_as(C.POINTER(C.c_double)), C.c_double(a),
                                  C.c_double(rc), C.c_int64(kc), C.c_int64(steps))
     assert res[0]["device_bytes"] <= est < 1.01 * res[0]["device_bytes"] + 1e5
+
+
+def test_groups_joined_in_a_large_batch_change_nothing():
+    """With enough groups of particles in a batch a real-space task takes several of
+    them: a system's results stay those of a batch of its own, bit for bit, for sizes
+    that leave tails of groups and of particles."""
+    dt, steps = 1e-12, 6
+    specs = [(n, 40 + i, 0.05, 0.02, m.MD_FIELD_STEP, 0.0, i % 2 == 1, None)
+             for i, n in enumerate((8191, 8192, 257, 5003, 3001, 4097, 1026))]
+    assert sum(s[0] for s in specs) // 4 > 2 * 2500  # more than twice the tasks that are kept
+    alone = [_run_alone(s, steps, dt) for s in specs]
+    sims = [_system(*s) for s in specs]
+    b = m.Batch(len(sims))
+    for sm in sims:
+        b.add(sm, steps, dt)
+    while b.run(4):
+        pass
+    for sm, (st, rec) in zip(sims, alone):
+        for x, y in zip(sm.get_state(), st):
+            np.testing.assert_array_equal(x, y)
+        np.testing.assert_array_equal(sm.records(), rec)

@@ -161,3 +161,87 @@ def test_gathered_bricks_are_split(n, kc, grow):
         got, want = k_part(sim, mm), k_part(ref, mm)
         for q in range(4):
             assert rms(got[q], want[q]) < TOL
+
+
+def test_particles_out_of_their_cells_between_builds():
+    """Particles that moved up to two cells since the last build, across the faces
+    too, without a new one: spread and interpolation find them where they are."""
+    n = 20011
+    ini, g = random_system_fast(n, seed=6, phi=0.10, B0=0.02)
+    g["rc"], g["kc"] = 0.2 * g["lBox"], 15
+    g["alpha"] = 3.5 / g["rc"]
+    sim = gpu_system(ini, g, 1)
+    sim.set_neighbor_skin(1.0)
+    sim.CompInteractions()
+    ncx, _, perm = sim.debug_cells()
+    shift = 0.055 * g["lBox"]  # along each axis: 0.095 L of the 0.1 L before a build
+    assert sim.kspace_engine() == "mesh" and shift * ncx > 0.7 * g["lBox"]
+    g["pos"], g["mm"] = g["pos"] + shift, np.roll(g["mm"], 1, axis=1)
+    sim.set_state(g["pos"], g["mm"], g["ea"])
+    fresh = gpu_system(ini, g, 1)
+    sim.step(1, 1e-13)
+    fresh.step(1, 1e-13)
+    np.testing.assert_array_equal(sim.debug_cells()[2], perm)  # not sorted anew
+    for x, y, s in zip(sim.get_state(), fresh.get_state(), (g["lBox"], 1.0, 1.0)):
+        assert np.abs(x - y).max() < 2e-6 * s
+    mm = np.roll(g["mm"], 1, axis=1)
+    assert rms(sim.CompDemagField(mm), fresh.CompDemagField(mm)) < TOL
+
+
+def test_mesh_beside_an_overflowed_list():
+    """The pairs scan the cells directly while the list grows; k space is the mesh's."""
+    ini, g = random_system_fast(8501, seed=9, phi=0.10, B0=0.02)
+    g["rc"], g["kc"] = 0.25 * g["lBox"], 18
+    g["alpha"] = 3.5 / g["rc"]
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref = k_part(gpu_system(ini, g, 0), mm)
+    sim = gpu_system(ini, g, 1)
+    sim.set_strong_pairs(0.0)
+    sim.CompInteractions()
+    used = sim.neighbor_capacity()
+    sim.neighbor_capacity(cap=used // 10)
+    sim.set_state(g["pos"], g["mm"], g["ea"])
+    for _ in range(2):  # with the list too short, and grown
+        got = k_part(sim, mm)
+        for q in range(4):
+            assert rms(got[q], ref[q]) < TOL
+    assert sim.neighbor_capacity() == used
+
+
+def test_engines_changed_on_a_live_context():
+    """Every engine after every other, with steps in between and after the context
+    was in a batch: each evaluation is that of its own engine."""
+    from md_sim_wolfschwenger_gb300 import Batch
+    n, dt = 8501, 1e-16
+    ini, g = random_system_fast(n, seed=10, phi=0.10, B0=0.02)
+    g["rc"], g["kc"] = 0.25 * g["lBox"], 18
+    g["alpha"] = 3.5 / g["rc"]
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref = k_part(gpu_system(ini, g, 0), mm)
+    sim = gpu_system(ini, g, 1)
+    sim.set_strong_pairs(0.0)
+
+    def check(tol):
+        sim.set_state(g["pos"], g["mm"], g["ea"])  # the steps moved it
+        got = k_part(sim, mm)
+        for q in range(4):
+            assert rms(got[q], ref[q]) < tol
+
+    for engine in ("auto", "tc", "auto", "simt", "tc", "simt", "auto"):
+        sim.set_kspace_engine(engine)
+        assert sim.kspace_engine() == ("mesh" if engine == "auto" else engine)
+        sim.step(2, dt)
+        # tensor cores and row segments: ~1.3e-6
+        check(TOL if engine == "auto" else 5e-6)
+    for ring in (0, -1):
+        sim.set_kspace_tiling(ring, 1)
+        sim.step(2, dt)
+        check(5e-6 if ring == 0 else TOL)
+    a = sim.CompDemagField(mm)  # of other moments: the positions move by 1e-12 of a box
+    b = Batch(1)
+    b.add(sim, 3, dt)
+    assert b.run(3) == 3
+    # the batch's geometry, on the mesh
+    assert rms(sim.CompDemagField(mm), a) < TOL
+    sim.step(2, dt)
+    check(TOL)
