@@ -559,6 +559,10 @@ int alloc_strong(md_ctx* c, long long cap) {
   if (st) return st;
   c->scap = cap;
   invalidate_graph(c);
+  // not in use before the next build has filled it (a field at the last geometry
+  // takes every pair in FP32)
+  static const int one = 1;
+  CK(c, cudaMemcpyAsync(&c->sc->flags.soverflow, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   return MD_OK;
 }
 

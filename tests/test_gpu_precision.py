@@ -125,3 +125,23 @@ def test_strong_pairs_count_once_at_any_splitting(n, alpha):
     ref = gpu_system(ini, g, 0)
     ref.CompInteractions()
     assert O.rms_rel(sim.CompDemagField(mm), ref.CompDemagField(mm), bAl) < TOL_MIXED
+
+
+def test_field_after_the_strong_threshold_was_lowered():
+    """A lower threshold asks for a longer strong list, filled by the next build: a
+    field at the last geometry does without it."""
+    from helpers import gpu_system, random_system, scales
+    ini, g = random_system(2500, seed=5, rc_frac=0.3, lognormal=True)
+    _, bAl, _ = scales(ini, g)
+    mm = np.roll(g["mm"], 1, axis=1)
+    ref, sim = gpu_system(ini, g, 0), gpu_system(ini, g, 1)
+    ref.CompInteractions()
+    sim.CompInteractions()
+    assert sim.strong_pairs() > 0
+    held = sim.device_bytes()
+    sim.set_strong_pairs(0.05)
+    assert sim.device_bytes() > held
+    want = ref.CompDemagField(mm)
+    assert O.rms_rel(sim.CompDemagField(mm), want, bAl) < TOL_MIXED
+    sim.CompInteractions()
+    assert O.rms_rel(sim.CompDemagField(mm), want, bAl) < TOL_MIXED
