@@ -89,8 +89,11 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan<NT>&
   brick_cells(M, ncx, p.gm_reach, x0, wx, cx, nx);
   brick_cells(M, ncx, p.gm_reach, y0, kBY, cy, ny);
   brick_cells(M, ncx, p.gm_reach, z0, kBZ, cz, nz);
-  int part = 0;  // waited for after the rows of cells
-  if (tid == 0) part = MeshPlan(p.gm_plan, p.gm_nbrick).item[blockIdx.x].y;
+  if (tid == NT - 1) {  // in a warp that has no row of cells to load below
+    const int part = MeshPlan(p.gm_plan, p.gm_nbrick).item[blockIdx.x].y;
+    b.first = (part & 0xffff) * NT;
+    b.step = (part >> 16) * NT;
+  }
   for (int r0 = 0; r0 < ny * nz; r0 += NT) {
     __syncthreads();
     {  // one row of cells per thread, split where it wraps
@@ -122,11 +125,7 @@ __device__ __forceinline__ void brick_particles(const KParams& p, BrickScan<NT>&
       __syncthreads();
       for (int q = 0; q < wid; q++) incl += b.wsum[q];
       b.pre[tid + 1] = incl;
-      if (tid == 0) {
-        b.pre[0] = 0;
-        b.first = (part & 0xffff) * NT;
-        b.step = (part >> 16) * NT;
-      }
+      if (tid == 0) b.pre[0] = 0;
     }
     __syncthreads();
     const int total = b.pre[NT], nrow = min(NT, ny * nz - r0);
@@ -464,7 +463,16 @@ __global__ void __launch_bounds__(512) k_mesh_y(KParams p) {
   if (nz == kc && x0 == 0 && threadIdx.x < 96) {  // total moment, in the block with the fewest rows: fixed order
     const int c = threadIdx.x >> 5;
     double m = 0.0;
-    for (int b = threadIdx.x & 31; b < p.gm_nitem; b += 32) m += p.musum_part[3 * b + c];
+    for (int b0 = threadIdx.x & 31; b0 < p.gm_nitem; b0 += 512) {
+      double v[16];  // loaded together: a trip's latency is most of this block's time
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int b = b0 + 32 * i;
+        v[i] = b < p.gm_nitem ? p.musum_part[3 * b + c] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; i++) m += v[i];
+    }
     m = warp_sum(m);
     if ((threadIdx.x & 31) == 0) p.musum[c] = m;
   }

@@ -46,7 +46,7 @@ __device__ __forceinline__ void brick_cells(int M, int ncx, float h, int b0, int
 // up to eight times the mean, or 1024: at uniform density every brick is one item, and
 // the extra items are at most an eighth of the bricks (their idle blocks cost 3 us per
 // step at N = 32768 with a quarter, 1 with an eighth).  N = 32768 all in 0.15^3 of the
-// box, kc = 20: step 4233 -> 1389 us (tensor cores 1413); uniform 575.6 -> 578.  Made in
+// box, kc = 20: step 4233 -> 1389 us (tensor cores 1413); uniform 574.7 -> 576.4.  Made in
 // the launches of the cell order: a launch of its own before the spread let the
 // real-space blocks take the SMs first, 7 us per step at N = 32768.
 
