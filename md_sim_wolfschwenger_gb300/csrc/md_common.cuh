@@ -83,9 +83,9 @@ struct CellParams {
 
 // A packed launch runs one kernel over the blocks of several independent
 // systems: block b of the grid executes block tasks[b].blk of system
-// tasks[b].rep, with that system's parameters.  The kernel bodies are the
-// same as for a single system, so every system gets the same results alone
-// and packed.
+// tasks[b].rep, with that system's parameters.  A system's results in a batch do
+// not depend on what else is in it; a context's own calls may take another engine
+// (small and large systems, md_kspace_engine_used) and agree within rounding.
 struct Task {
   int rep, blk;
 };
@@ -183,7 +183,7 @@ struct RealParams {
   const double2* etab;  //   and [kEEntries]
   CellGrid grid;
   double alpha, rc;      // box units
-  double rc2, rc2_test;  // exact and (slightly larger) candidate cutoff
+  double rc2;
   double c2a;            // 2 alpha / sqrt(pi)
   double al2, al4;       // alpha^2, alpha^4
   double cont_eps;       // 1e-10 m / L (contact offset, interaction.cpp:120)

@@ -145,8 +145,6 @@ RealParams real_params(md_ctx* c, void* B, void* F, void* ov) {
   p.alpha = a;
   p.rc = rcb;
   p.rc2 = rcb * rcb;
-  const double rt = rcb * (1.0 + 1e-6) + 2e-7;
-  p.rc2_test = rt * rt;
   p.pk = make_pair_consts(a, 2.0 * a * g.irPi, 1e-10 / L, p.rc2);
   p.c2a = 2.0 * a * g.irPi;
   p.al2 = a * a;
@@ -439,7 +437,7 @@ static int issue_interactions(md_ctx* c, double dt = -1.0, bool unit = false, bo
   l += fork_join(
       c, 0, MD_SEG_REAL_FULL, MD_SEG_KSF_FULL,
       [&](cudaStream_t st) {
-        int l = launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), &c->sc->flags, fp64(c));
+        int l = launch_nbr(st, real_params(c, nullptr, nullptr, nullptr), fp64(c));
         if (after_records) cudaStreamWaitEvent(st, c->join_ev[2], 0);
         if (dt >= 0) l += launch_noise(st, int_params(c, dt, nullptr, nullptr), unit, fp64(c));
         return l;

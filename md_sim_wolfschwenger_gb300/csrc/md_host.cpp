@@ -437,16 +437,16 @@ void predicted_errors(const md_config& c, const EwaldModel& m, double alpha, dou
   if (errT) *errT = std::sqrt(eKT * eKT + eRT * eRT) / m.tAl;
 }
 
-// Instruction-count model of one step (two field evaluations): per neighbour
-// ~75 for the candidate tests and ~155 for the pair maths; per (k, particle)
-// ~44 (structure factor twice, full and field-only scatter).
 // Relative cost of one step for cutoff rc (box units) and kc: per particle,
 // the ordered pairs within rc (field + force and field-only passes over the
 // Verlet list, which is rebuilt only every many steps) and the k vectors of
 // the half space (structure factor twice, scatter twice).  The weights are
-// the measured per-unit times on GB300 at N = 32768: 9.5 ps per ordered
-// pair; per (k, particle) 2.5 ps on the FP32 CUDA-core k-space kernels and
-// 1.7 ps on the tensor-core ones (used for kc <= kc_tc).
+// per-unit times on GB300 at N = 32768 with the pair passes and the tensor cores of the
+// time: 9.5 ps per ordered pair; per (k, particle) 2.5 ps on the FP32 CUDA-core k-space
+// kernels and 1.7 ps on the tensor-core ones (used for kc <= kc_tc).  The two pair
+// passes take 5.8 ps now and the mesh does not cost particles x k vectors, so the split
+// is no longer the fastest one; the weights stay, and with them every split that a
+// program gets, until splits at equal predicted errors have been timed per engine.
 double model_cost(double rc_box, int64_t kc, int64_t n, int kc_tc) {
   const double pi = 3.141592653589793;
   const double nr = (double)n * 4.0 / 3.0 * pi * rc_box * rc_box * rc_box;

@@ -72,7 +72,7 @@ int launch_fill_tc_prep(cudaStream_t st, const CellParams& c, const KParams& p);
 int launch_cells_packed(cudaStream_t st, const CellParams* ps, int R, const Packed& n256, const Packed& sort,
                         const unsigned* anyrb);
 // Neighbour list within rc + skin (count, scan, fill; skipped unless rebuilding).
-int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64);
+int launch_nbr(cudaStream_t st, const RealParams& p, bool fp64);
 int launch_nbr_packed(cudaStream_t st, const RealParams* ps, int R, const Packed& real, const unsigned* anyrb);
 int launch_set_mu(cudaStream_t st, int n, const double* mm, const double* magMom_u, const double* rMag_u,
                   const SortedView& s, bool fp64);

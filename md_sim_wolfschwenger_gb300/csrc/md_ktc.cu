@@ -642,7 +642,8 @@ __device__ __forceinline__ void sf_reduce_body(const KParams& p, int bx) {
   if (grp != 0) return;
   // the groups' pairs the same way: 2^-48 of the sum, far below its terms' own
   // errors (FP64 additions here were a chain of 64 cycles each: N = 3001 87.4 -> 82.8
-  // us per step, S unchanged to the digits shown, 3.3157e-7 of it off FP64)
+  // us per step).  S off FP64, N = 2000 .. 65536, two systems each: 3.5e-7 .. 1.0e-6
+  // either way, their ratio 0.97 .. 1.03, 1.001 on average.
 #pragma unroll
   for (int g = 1; g < G; g++)
 #pragma unroll

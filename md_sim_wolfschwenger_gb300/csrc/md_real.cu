@@ -55,9 +55,8 @@
 
 namespace md {
 
-constexpr int kRealWarps = 8;  // warps (particles) per block: list build, full pass, packed launches
-// warps per block of the single-system field pass (its packed pair maths
-// needs fewer registers; smaller blocks give finer occupancy steps)
+constexpr int kRealWarps = 8;  // warps per block: list build, field + force with coating
+// of the other passes (smaller blocks give finer occupancy steps)
 constexpr int kFieldWarps = 4;
 
 template <typename T>
@@ -95,7 +94,7 @@ __device__ __forceinline__ double coat_force(const RealParams& p, double rd, int
 }
 
 // Ewald pair terms for the pair vector (dx, dy, dz) from i to j (r2 < rc2),
-// mixed path: with coating potentials and in the direct cell scan.
+// mixed path, in the direct cell scan.
 template <bool FULL, bool COAT>
 __device__ __forceinline__ void pair_terms(const RealParams& p, float dx, float dy, float dz, float r2, const float4& mi,
                                            const float4& mj, int oi, int oj, Acc<float>& a) {
@@ -298,7 +297,6 @@ __device__ __forceinline__ void pair64(const RealParams& p, const double4_32a& d
 // neighbours of the warp's particle.  Special functions stay scalar.
 __device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 pk1(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
@@ -1145,8 +1143,8 @@ constexpr int kNearCap = 128;  // coating pairs a warp queues
 // Mixed path: one warp per particle, lanes take two list entries at a time in
 // the halves of packed FP32 operations.
 //
-// Bound: FP32 issue and the FMA pipe (see pair_terms2); 250 / 188 us for field +
-// force / field at N = 32768, 7.5e7 ordered pairs (273 / 193 with the arithmetic
+// Bound: FP32 issue and the FMA pipe (see pair_terms2); 250 / 185 us for field +
+// force / field at N = 32768 and 7.5e7 ordered pairs (273 / 193 with the arithmetic
 // before).  The list comes from DRAM, ~1 us away, longer than an iteration of a
 // warp, so its entries are loaded two iterations (128) ahead.
 //
@@ -1449,7 +1447,7 @@ int real_blocks(int n) { return (n + kRealWarps - 1) / kRealWarps; }
 int real_pass_blocks(int n, int run) { return (n + kFieldWarps * run - 1) / (kFieldWarps * run); }
 int nbr_blocks(int n, bool fp64) { return real_blocks(fp64 ? n : (n + 1) / 2); }
 
-int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64) {
+int launch_nbr(cudaStream_t st, const RealParams& p, bool fp64) {
   const int nsm = num_sms();
   const int nblk = nbr_blocks(p.n, fp64);
   dim3 grid(std::min(nblk, 8 * nsm)), block(kRealWarps * 32);
@@ -1457,7 +1455,6 @@ int launch_nbr(cudaStream_t st, const RealParams& p, StepFlags* flags, bool fp64
     k_nbr_build<double, false><<<grid, block, 0, st>>>(p, nblk);
   else
     k_nbr_build<float, false><<<grid, block, 0, st>>>(p, nblk);
-  (void)flags;
   k_nbr_scan<<<2, 1024, 0, st>>>(p);
   if (fp64)
     k_nbr_build<double, true><<<grid, block, 0, st>>>(p, nblk);
