@@ -373,7 +373,7 @@ struct IntParams {
     float dt, L, iL, B_unit, F_unit, cself, csurf, anisConst, velMmConst, magDamp;
   } f;
   // work arrays (orig order, T)
-  void *k1m, *k1e, *m2, *e2, *th;   // th: [9][n] scaled noise (adaptive solvers: unit normals)
+  void *k1m, *k1e, *m2, *e2, *th;   // th: [9][n] scaled noise (mixed adaptive solvers: unit normals)
   // stage outputs (sorted order, T)
   const void *Br, *Bk, *Fr, *Fk, *ov;
   // FP64 strong-pair terms: sv.B belongs to the evaluation that gave Br,
@@ -407,7 +407,7 @@ struct RKStage {
   double a[7];              // weights of k_0..k_s: next stage (stage kernel) / solution (accept)
   double e[7];              // error weights (last stage)
   double nf;                // factor on the thermal field and torque (rescaled on rejections)
-  const double2* sTB;       // scales of torque and field, unrounded; p.th holds unit normals
+  const double2* sTB;       // mixed: scales of torque and field, unrounded, of p.th's unit normals
   int s;                    // stage index (0-based); accept: last weight index
   int last;                 // stage: no next stage, form the error; accept: take (cm, ce)
   unsigned long long* errmax;  // max over particles of the error norm (double bits)

@@ -422,7 +422,7 @@ static int fork_join(md_ctx* c, int q, int seg_real, int seg_k, RP&& real_prep, 
 }
 
 // Field + force evaluation on the current master state (no integrator).
-// dt >= 0: the step's noise is drawn beside it (unit: unscaled).  after_records: the step before left
+// dt >= 0: the step's noise is drawn beside it (unit: see launch_noise).  after_records: the step before left
 // its records to the side stream (issue_step); they come before the noise, and with
 // it the integrator.
 static int issue_interactions(md_ctx* c, double dt = -1.0, bool unit = false, bool after_records = false) {

@@ -152,8 +152,9 @@ __device__ __forceinline__ void demag_si(const IntParams& p, int r, R b[3], cons
 
 // Thermal torque, field and force of the step: unit normals (drawn, uploaded
 // or zero) times the particle's scales, into th.  Independent of the fields,
-// so the launch runs beside their evaluation.  UNIT: the normals alone (adaptive
-// solvers, which rescale torque and field after a rejected step).
+// so the launch runs beside their evaluation.  UNIT: the normals alone (the mixed
+// path's adaptive solvers, which rescale torque and field after a rejected step and
+// round their product once).
 // Thread = one Box-Muller pair (j of five) of one particle.
 template <typename T, bool UNIT>
 __global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(kIntOne) k_noise(IntParams p) {
 
 // Per-particle constants of the integrator in T for the step dt: ct, cb, cf
 // are the DefThermFluct prefactors under the square roots (0: switched off).  sTB: the
-// scales of torque and field unrounded (for the adaptive solvers).
+// scales of torque and field unrounded (for the mixed path's adaptive solvers).
 template <typename T>
 __global__ void __launch_bounds__(kIntThreads) k_int_consts(int n, double ct, double cb, double cf,
                                                             const double* __restrict__ zr, const double* __restrict__ zt,
@@ -603,6 +604,16 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
   if (i < n) {
     const int r = p.s.rank[i];
     const T4 cb = ((const T4*)p.cB)[i];
+    // factors of p.th: FP64 holds the scaled noise, FP32 unit normals (one rounding of
+    // the rescaled scale)
+    T sT, sB;
+    if constexpr (std::is_same<T, float>::value) {
+      const double2 sTB = q.sTB[i];
+      sT = (float)(sTB.x * q.nf);
+      sB = (float)(sTB.y * q.nf);
+    } else {
+      sT = sB = q.nf;
+    }
     T m[3], e[3], bd[3], tau[3], bth[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -610,16 +621,6 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_stage(RKStage q) {
       e[a] = q.s == 0 ? (T)p.ea[a * n + i] : ((const T*)q.ce)[a * n + i];
     }
     demag_si<T>(p, r, bd);
-    T sT, sB;
-    if (q.nf == 1.0) {
-      const T4 ca = ((const T4*)p.cA)[i];
-      sT = ca.x;
-      sB = ca.y;
-    } else {
-      const double2 s = q.sTB[i];
-      sT = (T)(s.x * q.nf);
-      sB = (T)(s.y * q.nf);
-    }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       tau[a] = sT * ((const T*)p.th)[a * n + i];
@@ -711,7 +712,10 @@ __global__ void __launch_bounds__(kIntThreads) k_rk_accept(RKStage q) {
     // reference rescales it on rejections only after it entered the force)
     const typename V4<T>::t ca = ((const typename V4<T>::t*)p.cA)[i];
 #pragma unroll
-    for (int a = 0; a < 3; a++) fth[a] = ca.z * ((const T*)p.th)[(6 + a) * n + i];
+    for (int a = 0; a < 3; a++) {
+      const T t = ((const T*)p.th)[(6 + a) * n + i];
+      fth[a] = std::is_same<T, float>::value ? ca.z * t : t;
+    }
     finish_particle<T>(p, i, r, mn, en, fth, ca.w, acc, disp2);
   }
   step_block_sums(p, blockIdx.x, acc, disp2);
@@ -740,11 +744,12 @@ int int_blocks_one(int n) { return (n + kIntOne - 1) / kIntOne; }
 
 int launch_noise(cudaStream_t st, const IntParams& p, bool unit, bool fp64) {
   const dim3 g(int_blocks_one(p.n), 5);
-  auto go = [&](auto kern) { kern<<<g, kIntOne, 0, st>>>(p); };
   if (fp64)
-    unit ? go(k_noise<double, true>) : go(k_noise<double, false>);
+    k_noise<double, false><<<g, kIntOne, 0, st>>>(p);
+  else if (unit)
+    k_noise<float, true><<<g, kIntOne, 0, st>>>(p);
   else
-    unit ? go(k_noise<float, true>) : go(k_noise<float, false>);
+    k_noise<float, false><<<g, kIntOne, 0, st>>>(p);
   return 1;
 }
 
