@@ -22,7 +22,6 @@
 // arrays 8 B) plus 8 B per cell.
 #include <map>
 #include <mutex>
-#include <set>
 
 #include "md_common.cuh"
 #include "md_kernels.h"
@@ -279,20 +278,14 @@ __global__ void __launch_bounds__(kCellThreads) k_sorted_fill_packed(const CellP
   });
 }
 
-void allow_smem(const void* fn) {
-  static std::mutex mu;
-  static std::set<std::pair<int, const void*>> done;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count({dev, fn})) return;
-  int top = 0;
+bool raise_smem(const void* fn) {
+  int dev = 0, top = 0;
   cudaFuncAttributes a;
-  // a failure is reported by the launch that needs more than the default
-  if (cudaDeviceGetAttribute(&top, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
-      cudaFuncGetAttributes(&a, fn) == cudaSuccess &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, top - (int)a.sharedSizeBytes) == cudaSuccess)
-    done.insert({dev, fn});
+  return cudaGetDevice(&dev) == cudaSuccess &&
+         cudaDeviceGetAttribute(&top, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+         cudaFuncGetAttributes(&a, fn) == cudaSuccess &&
+         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, top - (int)a.sharedSizeBytes) ==
+             cudaSuccess;
 }
 
 int persistent_grid(const void* fn, int threads, size_t smem, int ntask) {

@@ -7,6 +7,7 @@
 // host from the per-system block counts below).  Packed launches exist for
 // the mixed-precision path.
 #pragma once
+#include <atomic>
 #include <vector>
 
 #include "md_common.cuh"
@@ -27,7 +28,16 @@ int persistent_grid(const void* fn, int threads, size_t smem, int ntask);
 
 // Raises a kernel's dynamic shared memory limit to what the device allows, once per
 // device: a launch's own size must not depend on what another host thread set last.
-void allow_smem(const void* fn);
+bool raise_smem(const void* fn);  // false: not raised
+template <auto K>
+inline void allow_smem() {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  // without it, a launch that needs more than the default reports the failure
+  if (!(done.load(std::memory_order_relaxed) & bit) && raise_smem((const void*)K)) done.fetch_or(bit);
+}
 
 // Blocks of one system per kernel shape (task-table construction).
 int cell_blocks(int n);                 // cell assign/scatter/fill, integrator
@@ -163,7 +173,7 @@ size_t kscatter_smem(int kc);
 size_t ksf_smem(int kc);
 int scatter_particles(int kc);
 
-// Integrator.
+// Integrator.  unit: unscaled noise on the mixed path.
 int launch_noise(cudaStream_t st, const IntParams& p, bool unit, bool fp64);
 int launch_int_consts(cudaStream_t st, int n, double ct, double cb, double cf, const double* zr, const double* zt,
                       const double* ivol, const double* izt, const double* v1, const double* v2, const double* mu,

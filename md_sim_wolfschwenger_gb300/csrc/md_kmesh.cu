@@ -811,7 +811,7 @@ void mesh_plan_init(int M, std::vector<int>& out) {
 
 int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) {
   const int M = p.gm_M, kc1 = p.kc + 1, Q = 2 * p.kc + 1;
-  allow_smem((const void*)k_mesh_spread);
+  allow_smem<k_mesh_spread>();
   const int items = p.gm_nitem;
   k_mesh_spread<<<items, kBrThreads, sizeof(SpreadSmem), st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
@@ -819,16 +819,17 @@ int launch_kmesh(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) 
   k_mesh_y<<<dim3(kc1, M / kMYLines), (16 * kc1 + 31) / 32 * 32, sizeof(float2) * (M + 3 * kMYLines * (M + 2)), st>>>(p);
   k_mesh_x<<<p.tc_rows, kMXThreads, sizeof(float) * (6 * M + 4 * kc1 + 8 * kMXThreads), st>>>(p);
   const size_t smi = sizeof(float4) * kc1 * Q * kMIx + sizeof(float2) * (M + kMIx * kMIy * kc1 * 3);
-  allow_smem((const void*)k_mesh_yz);
+  allow_smem<k_mesh_yz>();
   k_mesh_yz<<<dim3(M / kMIx, M / kMIy), 256, smi, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[1], st, cudaEventRecordExternal);
-  const void* kern = full ? (const void*)k_mesh_interp<true> : (const void*)k_mesh_interp<false>;
   const size_t smf = sizeof(InterpSmem);
-  allow_smem(kern);
-  if (full)
+  if (full) {
+    allow_smem<k_mesh_interp<true>>();
     k_mesh_interp<true><<<items, kInThreads, smf, st>>>(p);
-  else
+  } else {
+    allow_smem<k_mesh_interp<false>>();
     k_mesh_interp<false><<<items, kInThreads, smf, st>>>(p);
+  }
   return 6;
 }
 

@@ -416,7 +416,7 @@ RowShape krows_shape(int kc, int n, int tasks, int nsm, bool fp64) {
   s.nblk = (tasks + 127) / 128;
   s.threads = ((tasks + s.nblk - 1) / s.nblk + 31) / 32 * 32;
   const size_t sm = sf_rows_smem(kc, s.threads, fp64);
-  allow_smem(sf_rows_fn(fp64));
+  fp64 ? allow_smem<k_sf_rows<double>>() : allow_smem<k_sf_rows<float>>();
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sf_rows_fn(fp64), s.threads, sm) != cudaSuccess || nb < 1)
     nb = 1;
@@ -443,18 +443,21 @@ int launch_fill_phase_rows(cudaStream_t st, const CellParams& c, const KParams& 
 template <typename T, int NP>
 static void scat_rows(cudaStream_t st, const KParams& p, bool full) {
   const size_t sm = scat_rows_smem(p.kc, NP, std::is_same<T, double>::value);
-  auto go = [&](auto kern) {
-    allow_smem((const void*)kern);
-    kern<<<(p.n + NP - 1) / NP, kRowScat, sm, st>>>(p);
-  };
-  full ? go(k_scat_rows<T, NP, true>) : go(k_scat_rows<T, NP, false>);
+  const int g = (p.n + NP - 1) / NP;
+  if (full) {
+    allow_smem<k_scat_rows<T, NP, true>>();
+    k_scat_rows<T, NP, true><<<g, kRowScat, sm, st>>>(p);
+  } else {
+    allow_smem<k_scat_rows<T, NP, false>>();
+    k_scat_rows<T, NP, false><<<g, kRowScat, sm, st>>>(p);
+  }
 }
 
 template <typename T>
 static int krows_t(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) {
   constexpr bool fp64 = std::is_same<T, double>::value;
   const size_t sm = sf_rows_smem(p.kc, p.rw_threads, fp64);
-  allow_smem((const void*)k_sf_rows<T>);
+  allow_smem<k_sf_rows<T>>();
   k_sf_rows<T><<<dim3(p.rw_nblk + 1, p.rw_nchunk), p.rw_threads, sm, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   k_red_rows<T><<<dim3((p.rw_T + 31) / 32, 4), 256, 0, st>>>(p);

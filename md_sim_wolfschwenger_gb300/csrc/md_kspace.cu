@@ -397,7 +397,7 @@ int sk_threads() { return kSkThreads; }
 int sk_resident_blocks(int kc) {
   int nb = 0;
   const size_t sm = ksf_smem(kc);
-  allow_smem((const void*)k_sk);
+  allow_smem<k_sk>();
   const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_sk, kSkThreads, sm);
   return (e == cudaSuccess && nb > 0) ? nb : 1;
 }
@@ -429,10 +429,10 @@ template <int NP>
 static void scatter_launch(cudaStream_t st, const KParams& p, bool full, size_t smem) {
   dim3 grid((p.n + NP - 1) / NP);
   if (full) {
-    allow_smem((const void*)k_kscatter<NP, true>);
+    allow_smem<k_kscatter<NP, true>>();
     k_kscatter<NP, true><<<grid, NP * kScatterParts, smem, st>>>(p);
   } else {
-    allow_smem((const void*)k_kscatter<NP, false>);
+    allow_smem<k_kscatter<NP, false>>();
     k_kscatter<NP, false><<<grid, NP * kScatterParts, smem, st>>>(p);
   }
 }
@@ -442,7 +442,7 @@ int launch_kspace(cudaStream_t st, const KParams& p, bool full, bool fp64, cudaE
   if (p.gm_M > 0) return launch_kmesh(st, p, full, ev);
   if (p.tc_rows > 0) return launch_kspace_tc(st, p, full, ev);
   const size_t sm1 = ksf_smem(p.kc);
-  allow_smem((const void*)k_sk);
+  allow_smem<k_sk>();
   dim3 g1((p.nseg + kSkThreads - 1) / kSkThreads, p.nchunk);
   k_sk<<<g1, kSkThreads, sm1, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
@@ -487,11 +487,11 @@ template <int NP>
 static void scatter_packed(cudaStream_t st, const KParams* ps, const Packed& sc, bool full, int kcmax, size_t smem) {
   const int th = NP * kScatterParts;
   if (full) {
-    allow_smem((const void*)k_kscatter_packed<NP, true>);
+    allow_smem<k_kscatter_packed<NP, true>>();
     const int g = persistent_grid((const void*)k_kscatter_packed<NP, true>, th, smem, sc.n);
     k_kscatter_packed<NP, true><<<g, th, smem, st>>>(ps, sc.tasks, kcmax, sc.n, sc.wq);
   } else {
-    allow_smem((const void*)k_kscatter_packed<NP, false>);
+    allow_smem<k_kscatter_packed<NP, false>>();
     const int g = persistent_grid((const void*)k_kscatter_packed<NP, false>, th, smem, sc.n);
     k_kscatter_packed<NP, false><<<g, th, smem, st>>>(ps, sc.tasks, kcmax, sc.n, sc.wq);
   }
@@ -502,7 +502,7 @@ int launch_kspace_packed(cudaStream_t st, const KParams* ps, const Packed& sk, c
   int l = 0;
   if (sk.n) {
     const size_t sm1 = ksf_smem(kcmax);
-    allow_smem((const void*)k_sk_packed);
+    allow_smem<k_sk_packed>();
     k_sk_packed<<<persistent_grid((const void*)k_sk_packed, kSkThreads, sm1, sk.n), kSkThreads, sm1, st>>>(
         ps, sk.tasks, sk.n, sk.wq);
     l++;

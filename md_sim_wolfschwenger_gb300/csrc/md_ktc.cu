@@ -1073,15 +1073,15 @@ int launch_kspace_tc_prep_packed(cudaStream_t st, const KParams* ps, const Packe
 int launch_kspace_tc_packed(cudaStream_t st, const KParams* ps, const Packed& sf, const Packed& red,
                             const Packed& sc, bool full, size_t sf_smem, size_t sc_smem) {
   if (!sf.n) return 0;
-  allow_smem((const void*)k_sf_tc_packed);
+  allow_smem<k_sf_tc_packed>();
   k_sf_tc_packed<<<sf.n, kSfThreads, sf_smem, st>>>(ps, sf.tasks);
   if (full) {
     k_sf_tc_reduce_packed<true><<<red.n, 64 * kRedGroupsPacked, 0, st>>>(ps, red.tasks);
-    allow_smem((const void*)k_kscat_tc_packed<true>);
+    allow_smem<k_kscat_tc_packed<true>>();
     k_kscat_tc_packed<true><<<sc.n, kScThreads, sc_smem, st>>>(ps, sc.tasks);
   } else {
     k_sf_tc_reduce_packed<false><<<red.n, 64 * kRedGroupsPacked, 0, st>>>(ps, red.tasks);
-    allow_smem((const void*)k_kscat_tc_packed<false>);
+    allow_smem<k_kscat_tc_packed<false>>();
     k_kscat_tc_packed<false><<<sc.n, kScThreads, sc_smem, st>>>(ps, sc.tasks);
   }
   return 3;
@@ -1089,7 +1089,7 @@ int launch_kspace_tc_packed(cudaStream_t st, const KParams* ps, const Packed& sf
 
 int launch_kspace_tc(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* ev) {
   const size_t sm1 = (size_t)SfLayout(p.tc_ns, p.kc + 1, p.tc_sfa, p.tc_sfb).bytes;
-  allow_smem((const void*)k_sf_tc);
+  allow_smem<k_sf_tc>();
   k_sf_tc<<<dim3(p.tc_mt, p.tc_nchunk), kSfThreads, sm1, st>>>(p);
   if (ev) cudaEventRecordWithFlags(ev[0], st, cudaEventRecordExternal);
   const int nred = p.tc_mt * (2 * p.kc + 1);
@@ -1101,10 +1101,10 @@ int launch_kspace_tc(cudaStream_t st, const KParams& p, bool full, cudaEvent_t* 
   const size_t sm2 = (size_t)p.tc_scat_smem;
   const int nb = (p.n + kScParticles - 1) / kScParticles;
   if (full) {
-    allow_smem((const void*)k_kscat_tc<true>);
+    allow_smem<k_kscat_tc<true>>();
     k_kscat_tc<true><<<nb, kScThreads, sm2, st>>>(p);
   } else {
-    allow_smem((const void*)k_kscat_tc<false>);
+    allow_smem<k_kscat_tc<false>>();
     k_kscat_tc<false><<<nb, kScThreads, sm2, st>>>(p);
   }
   return 3;

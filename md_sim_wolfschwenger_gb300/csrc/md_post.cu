@@ -288,7 +288,7 @@ extern "C" int md_rdf(md_ctx* c, int64_t bins, double range, double r_mag0, int 
   const int nt = (n + md::kRdfThreads - 1) / md::kRdfThreads;
   auto all_pairs = [&] {
     const size_t smem = (sizeof(double) + sizeof(float)) * 3 * md::kRdfThreads + sizeof(unsigned int) * (size_t)bins;
-    md::allow_smem((const void*)md::k_rdf);
+    md::allow_smem<md::k_rdf>();
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     // 64 blocks per SM, dealt out as they finish (8, all resident: 689 us against 581

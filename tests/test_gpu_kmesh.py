@@ -141,7 +141,7 @@ def test_engine_of_the_current_parameters():
     assert large.kspace_engine() == "tc"
 
 
-@pytest.mark.parametrize("n,kc,grow", [(8501, 16, 3.0), (8501, 20, 8.0), (20011, 15, 30.0), (20011, 21, 5.0)])
+@pytest.mark.parametrize("n,kc,grow", [(7001, 16, 6.0), (8501, 16, 3.0), (8501, 20, 8.0), (20011, 15, 30.0), (20011, 21, 5.0)])
 def test_gathered_bricks_are_split(n, kc, grow):
     """All particles in the middle of the box (an edge of 1 / grow): the few bricks
     that hold them are split into parts, whose sums and particles come together
