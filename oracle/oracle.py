@@ -25,7 +25,7 @@ _lib = None
 
 
 def build(force=False) -> str:
-    """Compiles md_oracle.c with gcc (portable flags only: x86 here, Arm on the GPU machine)."""
+    """Compiles md_oracle.c with gcc (portable flags only: x86 and Arm)."""
     src = os.path.join(HERE, "md_oracle.c")
     with _lock:
         if force or not os.path.exists(LIB) or os.path.getmtime(LIB) < max(
